@@ -36,22 +36,6 @@ inline int row_blocks(int nk, int kpw) {
   return b < 1 ? 1 : b;
 }
 
-// acc + a*b, acc + conj(a)*b, acc + a*conj(b)
-__device__ __forceinline__ double2 cfma(double2 a, double2 b, double2 acc) {
-  acc.x = fma(a.x, b.x, fma(-a.y, b.y, acc.x));
-  acc.y = fma(a.x, b.y, fma(a.y, b.x, acc.y));
-  return acc;
-}
-__device__ __forceinline__ double2 cfma_cj(double2 a, double2 b, double2 acc) {
-  acc.x = fma(a.x, b.x, fma(a.y, b.y, acc.x));
-  acc.y = fma(a.x, b.y, fma(-a.y, b.x, acc.y));
-  return acc;
-}
-__device__ __forceinline__ double2 cfma_c(double2 a, double2 b, double2 acc) {
-  acc.x = fma(a.x, b.x, fma(a.y, b.y, acc.x));
-  acc.y = fma(a.y, b.x, fma(-a.x, b.y, acc.y));
-  return acc;
-}
 __device__ __forceinline__ double2 crecip(double2 z) {
   const double s = 1.0 / fma(z.x, z.x, z.y * z.y);
   return make_double2(z.x * s, -z.y * s);
@@ -747,11 +731,9 @@ __device__ __forceinline__ void jacobi_reg_cols(double2 (&a)[NB], double2 (&v)[N
 // when Qin already diagonalises a nearby matrix, so the sweeps converge at once) and
 // Qout = Qin V.  Qin may equal Qout: a k-point's rows are read before they are written.
 constexpr int kEigWarps = 2;
-// mode 1 (no starting basis): the eigensolve of herm(i A), the Cayley spectral setup of
-// solver.py:161-166
 template <int NB>
 __device__ __forceinline__ void eig_cols(int nk, const double2* __restrict__ A, const double2* Qin, double2* Qout,
-                                         double* eps, double tol, int mode = 0) {
+                                         double* eps, double tol) {
   const bool rotate = Qin != nullptr;
   using RG = RowGroup<NB>;
   constexpr int G = RG::G, KPW = RG::KPW, LP = RG::LP, MAT = RG::MAT, NP = JacobiPairs<NB>::M / 2;
@@ -769,10 +751,7 @@ __device__ __forceinline__ void eig_cols(int nk, const double2* __restrict__ A, 
     const size_t base = (size_t)k * NB * NB + c;
     if (on) {
 #pragma unroll
-      for (int r = 0; r < NB; ++r) {
-        const double2 x = A[base + (size_t)r * NB];
-        SA[r * LP + c] = mode ? make_double2(-x.y, x.x) : x;
-      }
+      for (int r = 0; r < NB; ++r) SA[r * LP + c] = A[base + (size_t)r * NB];
     }
     if (rotate) {  // SA <- Q^H F Q, column c
       // q_c goes through SQ and t = A q_c through this lane's column of SV (free until V
@@ -872,17 +851,12 @@ __device__ __forceinline__ void eig_cols(int nk, const double2* __restrict__ A, 
   }
 }
 
-template <int NB>
-__global__ void __launch_bounds__(32 * kEigWarps, 8) k_cgr_eig(CgArgs a, const double2* __restrict__ A, int rotate,
-                                                            double tol) {
-  eig_cols<NB>(a.nk, A, rotate ? q_cur(a) : nullptr, a.Q, a.eps, tol);
-}
 // Standalone eigensolve: eps, Qout <- eigh(A) (Qin == nullptr) or with the starting basis Qin.
 template <int NB>
 __global__ void __launch_bounds__(32 * kEigWarps, 8) k_eig_cols(int nk, const double2* __restrict__ A,
                                                              const double2* Qin, double2* Qout, double* eps,
-                                                             double tol, int mode) {
-  eig_cols<NB>(nk, A, Qin, Qout, eps, tol, mode);
+                                                             double tol) {
+  eig_cols<NB>(nk, A, Qin, Qout, eps, tol);
 }
 
 }  // namespace hf

@@ -27,9 +27,9 @@ int jdot_multi(void* stream, size_t nk, int nb, int n, const void* const* aX, co
                double* out, void* ws);
 int gram_row_slot(void* stream, int n, const int* slot, size_t stride, int nk, int nb, const void* R,
                   const double* w, double* b_out, void* ws);
-// eigh of herm(A) (mode 0) or herm(i A) (mode 1), complex128, nb <= 8, ascending, the
-// lane-per-column Jacobi (solver_cg.cu)
-int eigh_cols(void* stream, int nk, int nb, const void* A, double* w, void* V, int mode);
+// eigh of herm(A) (mode 0) or herm(i A) (mode 1), 2 <= nb <= 16, ascending, by
+// tridiagonalisation and QR (eigh.cu); eps and V in A's precision
+int eigh_tri(void* stream, int dtype, int nk, int nb, const void* A, void* eps, void* V, int mode);
 // P = herm(Q diag(p) Q^H), complex128, nb <= 8, lane-per-column kernel (solver_cg.cu)
 int rows_density(void* stream, int nk, int nb, const void* Q, const double* p, void* P);
 int symbol_address(const void* symbol, void** out);
@@ -92,6 +92,23 @@ __host__ __device__ __forceinline__ double2 mul_mi(double2 a) { return make_doub
 __host__ __device__ __forceinline__ float2 mul_mi(float2 a) { return make_float2(a.y, -a.x); }
 __host__ __device__ __forceinline__ double2 mul_pi(double2 a) { return make_double2(-a.y, a.x); }
 __host__ __device__ __forceinline__ float2 mul_pi(float2 a) { return make_float2(-a.y, a.x); }
+
+// acc + a*b, acc + conj(a)*b, acc + a*conj(b)
+__device__ __forceinline__ double2 cfma(double2 a, double2 b, double2 acc) {
+  acc.x = fma(a.x, b.x, fma(-a.y, b.y, acc.x));
+  acc.y = fma(a.x, b.y, fma(a.y, b.x, acc.y));
+  return acc;
+}
+__device__ __forceinline__ double2 cfma_cj(double2 a, double2 b, double2 acc) {
+  acc.x = fma(a.x, b.x, fma(a.y, b.y, acc.x));
+  acc.y = fma(a.x, b.y, fma(-a.y, b.x, acc.y));
+  return acc;
+}
+__device__ __forceinline__ double2 cfma_c(double2 a, double2 b, double2 acc) {
+  acc.x = fma(a.x, b.x, fma(a.y, b.y, acc.x));
+  acc.y = fma(a.y, b.x, fma(-a.x, b.y, acc.y));
+  return acc;
+}
 
 template <typename To, typename From> __device__ __forceinline__ To cvt(From a) {
   To r; r.x = a.x; r.y = a.y; return r;

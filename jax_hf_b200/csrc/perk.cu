@@ -1,7 +1,7 @@
 // Per-k small nb x nb kernels: one warp per matrix, matrices staged in shared
 // memory (double precision internally, storage precision at the boundary).
 //
-// Eigendecomposition: cyclic Jacobi with complex Hermitian rotations in the
+// Eigendecomposition for 2 <= nb <= 16: eigh.cu.  Otherwise cyclic Jacobi with complex Hermitian rotations in the
 // round-robin parallel ordering (Jacobi 1846; Golub & Van Loan, Matrix
 // Computations, sec. 8.5): each round applies nb/2 disjoint rotations at once
 // (lanes over rows/columns), sweeps repeat until no off-diagonal entry exceeds
@@ -283,8 +283,7 @@ static int eigh_common(void* stream, int dtype, int batch, int nb, int mode, con
   if (st) return st;
   if (batch == 0) return HF_OK;
   if (!A || !w || !V) return fail(HF_ERR_INVALID, "NULL argument");
-  // complex128 with nb <= 8: a group of lanes per matrix, one column per lane
-  if (dtype == HF_C128 && nb <= 8) return hf::eigh_cols(stream, batch, nb, A, static_cast<double*>(w), V, mode);
+  if (nb >= 2 && nb <= 16) return hf::eigh_tri(stream, dtype, batch, nb, A, w, V, mode);
   Launch L = warp_launch(batch, jacobi_smem_elems(nb));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (dtype == HF_C128) {

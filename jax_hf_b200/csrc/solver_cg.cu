@@ -844,25 +844,13 @@ static int cg_density(CgRun& r, cudaStream_t s, int force) {
   return HF_OK;
 }
 
-template <int NB>
-static int cg_eig_rows(CgRun& r, cudaStream_t s, const double2* A, int rotate) {
-  const int per_block = kEigWarps * RowGroup<NB>::KPW;
-  int b = (r.a.nk + per_block - 1) / per_block;
-  if (b > 148 * 32) b = 148 * 32;
-  k_cgr_eig<NB><<<b < 1 ? 1 : b, 32 * kEigWarps, 0, s>>>(r.a, A, rotate, kEigTol);
-  HF_LAUNCH_CHECK("k_cgr_eig");
-  return HF_OK;
-}
-
-// eps, Q <- eigh(A) (init) or eigh(Q^H F Q) with Q <- Q V (finalize)
+// eps, Q <- eigh(A): of F0 at init, of the final F at finalize.  The reference decomposes
+// Q^H F Q there and rotates Q (solver.py:622-626), the same eigenvectors up to a phase each;
+// for nb <= 16 decomposing F itself is cheaper than forming Q^H F Q and Q V (144 x 144,
+// nb = 8: 75 us against 195 us for a warm-started Jacobi).
 static int cg_eig(CgRun& r, cudaStream_t s, const double2* A, int rotate) {
-  switch (r.a.nb) {
-#define HF_NB_CASE(N) case N: return cg_eig_rows<N>(r, s, A, rotate);
-    HF_NB_CASE(1) HF_NB_CASE(2) HF_NB_CASE(3) HF_NB_CASE(4) HF_NB_CASE(5) HF_NB_CASE(6) HF_NB_CASE(7) HF_NB_CASE(8)
-#undef HF_NB_CASE
-    default: break;
-  }
   const int nb = r.a.nb;
+  if (nb <= 16) return hf_eigh(s, HF_C128, r.a.nk, nb, A, r.a.eps, r.a.Q);
   k_cg_eig<<<r.nblk, 32 * kSolverWarps, smem_eig(nb), s>>>(r.a, A, rotate);
   HF_LAUNCH_CHECK("k_cg_eig");
   return HF_OK;
@@ -890,28 +878,13 @@ int rows_density(void* stream, int nk, int nb, const void* Q, const double* p, v
 
 template <int NB>
 static int eig_cols_launch(cudaStream_t s, int nk, const double2* A, const double2* Qin, double2* Qout,
-                           double* eps, int mode = 0) {
+                           double* eps) {
   const int per_block = kEigWarps * RowGroup<NB>::KPW;
   int b = (nk + per_block - 1) / per_block;
   if (b > 148 * 32) b = 148 * 32;
-  k_eig_cols<NB><<<b < 1 ? 1 : b, 32 * kEigWarps, 0, s>>>(nk, A, Qin, Qout, eps, kEigTol, mode);
+  k_eig_cols<NB><<<b < 1 ? 1 : b, 32 * kEigWarps, 0, s>>>(nk, A, Qin, Qout, eps, kEigTol);
   HF_LAUNCH_CHECK("k_eig_cols");
   return HF_OK;
-}
-
-// hf_eigh / hf_cayley_spectral for complex128 with nb <= 8 (perk.cu): the lane-per-column
-// Jacobi from the identity; mode 1 decomposes herm(i A)
-int eigh_cols(void* stream, int nk, int nb, const void* A, double* w, void* V, int mode) {
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  auto a = static_cast<const double2*>(A);
-  auto v = static_cast<double2*>(V);
-  switch (nb) {
-#define HF_NB_CASE(N) case N: return eig_cols_launch<N>(s, nk, a, nullptr, v, w, mode);
-    HF_NB_CASE(1) HF_NB_CASE(2) HF_NB_CASE(3) HF_NB_CASE(4) HF_NB_CASE(5) HF_NB_CASE(6) HF_NB_CASE(7) HF_NB_CASE(8)
-#undef HF_NB_CASE
-    default: break;
-  }
-  return fail(HF_ERR_UNSUPPORTED, "eigh_cols: nb > 8");
 }
 
 static int cg_iteration_warp(CgRun& r, cudaStream_t s, const hf_cg_config& cf, bool fp32);

@@ -35,6 +35,17 @@ def eigh(A):
     return w, V
 
 
+def eigh_jacobi(A):
+    """The same decomposition by the cyclic Jacobi of the SCF loop (complex128, nb <= 8)."""
+    A = _as_dev(A)
+    batch, nb = _batch(A)
+    w = torch.empty(A.shape[:-1], dtype=_real(A.dtype), device=A.device)
+    V = torch.empty_like(A)
+    _lib.check(_lib.lib().hf_eigh_warm(_lib.stream_ptr(A.device), batch, nb, A.data_ptr(), None, V.data_ptr(),
+                                       w.data_ptr()))
+    return w, V
+
+
 def density_from_Qp(Q, p):
     """P = herm(Q diag(p) Q^H)."""
     Q = _as_dev(Q)

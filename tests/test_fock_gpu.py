@@ -457,3 +457,43 @@ def test_build_fock_batch_matches_single_calls(cuda, streams):
         assert torch.equal(s1, s2) and torch.equal(f1, f2)
     with pytest.raises(ValueError, match="outs has"):
         G.build_fock_batch(Ps, outs=outs[:2], **kw)
+
+
+@pytest.mark.parametrize("nb", [2, 3, 4, 5, 8, 9, 13, 16, 17])
+@pytest.mark.parametrize("nk,dt", [(1, np.complex128), (33, np.complex128), (300, np.complex64)])
+def test_eigh_shapes_scales_and_clusters(cuda, nb, nk, dt):
+    """hf_eigh over the lane groups and the CTA remainders: random, diagonal, block-split, clustered,
+    zero, huge and tiny matrices.  Backward error and orthogonality within 30 nb ulp (n sweeps of
+    n rotations and n reflections, each a few ulp), eigenvalues within the same of ||A||."""
+    from jax_hf_b200 import linalg as L
+    rng = np.random.default_rng(nb * nk)
+    A = _herm_batch(rng, (nk, nb, nb))
+    special = [np.zeros((nb, nb)), np.diag(np.arange(nb)[::-1] - 1.0), 2.0 * np.eye(nb) + 1e-13 * A[0],
+               np.kron(np.eye(nb // 2 + 1), np.array([[0, 1], [1, 0]]))[:nb, :nb], 1e30 * A[0], 1e-30 * A[0],
+               np.ones((nb, nb))]
+    for i, M in enumerate(special[:nk - 1]):
+        A[1 + i] = M
+    A = A.astype(dt)
+    w, V = L.eigh(torch.as_tensor(A, device="cuda"))
+    w, V = w.cpu().numpy().astype(np.float64), V.cpu().numpy().astype(np.complex128)
+    A = A.astype(np.complex128)
+    tol = 30 * nb * (2.2e-16 if dt == np.complex128 else 1.2e-7)
+    nrm = np.maximum(np.linalg.norm(A, 2, axis=(-2, -1)), 1e-300)
+    assert (np.diff(w, axis=-1) >= 0).all()
+    assert (np.abs(w - np.linalg.eigvalsh(A)).max(-1) <= tol * nrm).all()
+    rec = np.einsum("kin,kn,kjn->kij", V, w, np.conj(V))
+    assert (np.abs(rec - A).max((-2, -1)) <= tol * nrm).all()
+    assert np.abs(np.conj(np.swapaxes(V, -1, -2)) @ V - np.eye(nb)).max() <= tol
+
+
+def test_eigh_non_finite_entries_stay_in_their_matrix(cuda):
+    from jax_hf_b200 import linalg as L
+    A = _herm_batch(np.random.default_rng(3), (9, 6, 6))
+    A[2, 1, 4] = np.nan
+    A[5, 0, 0] = np.inf
+    w, V = L.eigh(torch.as_tensor(A, device="cuda"))
+    bad = torch.tensor([2, 5], device="cuda")
+    assert torch.isnan(w[bad]).all() and torch.isnan(V[bad].real).all()
+    good = [i for i in range(9) if i not in (2, 5)]
+    wo = np.linalg.eigvalsh(A[good])
+    assert np.abs(w.cpu().numpy()[good] - wo).max() < 1e-13 * np.abs(wo).max()
