@@ -63,6 +63,10 @@ extern "C" {
  * hermitised F in separate passes.  A schedule choice (the result is the same
  * to rounding); the autotuner times it as a candidate. */
 #define HF_FOCK_PIPE (1u << 10)
+/* Leaves out the two-factor passes (mesh sides with two factors of at most 16 and no
+ * compile-time line shape): such sides take the Stockham stages.  The SCF drivers set it,
+ * whose DIIS extrapolation amplifies a change of the transform's rounding. */
+#define HF_FOCK_NO_TWO_FACTOR (1u << 11)
 const char* hf_last_error(void);
 const char* hf_status_string(int status);
 int hf_version(void);

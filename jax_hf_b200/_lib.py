@@ -32,6 +32,7 @@ FOCK_GENERIC_FFT = 1 << 7
 FOCK_SYM_V = 1 << 8
 FOCK_TILE_PLAN = 1 << 9
 FOCK_PIPE = 1 << 10
+FOCK_NO_TWO_FACTOR = 1 << 11
 
 vp, i32, u32, f64, sz = C.c_void_p, C.c_int, C.c_uint, C.c_double, C.c_size_t
 pf64 = C.POINTER(C.c_double)

@@ -5,7 +5,7 @@
 // unrolling).  Composite N = A*B is split Cooley-Tukey style: A-point DFTs over
 // x[n2 + B n1], the twiddle W_N^{n2 k1}, B-point DFTs, output X[k1 + A k2].
 // Radices 2/3/4/5/8 are the butterflies of fft_engine.cuh; other primes use a
-// direct DFT.  Inner twiddles are compile-time constants (CtTwiddle).
+// direct DFT with the products of conjugate terms shared.  Inner twiddles are compile-time constants (CtTwiddle).
 //
 // Line FFT of length N = N1*N2 over TPL threads per line (TPL | N1, TPL | N2):
 //   pattern A: thread t holds x[n2 + N2 n1] for n2 = t + TPL i (i < N2/TPL), all n1
@@ -19,6 +19,7 @@
 // a shared-memory table (build_line_twiddles), indexed by compile-time offsets.
 #pragma once
 
+#include <type_traits>
 #include <utility>
 
 #include "fft_engine.cuh"
@@ -93,19 +94,50 @@ __device__ __forceinline__ C ct_twmul(C v) {
 template <int N, int TWN, bool INV, typename C>
 __device__ __forceinline__ void rdft(C* x, const C* __restrict__ tw);
 
-template <int N, bool INV, int K, typename C, int... Ns>
-__device__ __forceinline__ C prime_row(const C* x, std::integer_sequence<int, Ns...>) {
-  C acc = x[0];
-  ((acc = cadd(acc, ct_twmul<(Ns + 1) * K, N, INV>(x[Ns + 1]))), ...);
-  return acc;
+// Prime N: the terms j and N - j of every output share their products, so with
+// p_j = x_j + x_{N-j} and m_j = x_j - x_{N-j} the outputs k and N - k are
+// (x_0 + sum p_j cos) -+ i (sum m_j sin): (N - 1)^2 / 2 real-by-complex products.
+template <int N, int K, typename C, int... Js>
+__device__ __forceinline__ void prime_pair(const C& x0, const C* p, const C* m, C& r, C& q,
+                                           std::integer_sequence<int, Js...>) {
+  using T = decltype(x0.x);
+  r = x0;
+  q = make_c<C>((std::remove_cv_t<std::remove_reference_t<T>>)0, (std::remove_cv_t<std::remove_reference_t<T>>)0);
+  (
+      [&] {
+        using U = std::remove_cv_t<std::remove_reference_t<T>>;
+        constexpr double cw = CtTwiddle<(Js + 1) * K % N, N>::re, sw = -CtTwiddle<(Js + 1) * K % N, N>::im;
+        r = make_c<C>(r.x + (U)cw * p[Js].x, r.y + (U)cw * p[Js].y);
+        q = make_c<C>(q.x + (U)sw * m[Js].x, q.y + (U)sw * m[Js].y);
+      }(),
+      ...);
 }
 template <int N, bool INV, typename C, int... Ks>
-__device__ __forceinline__ void prime_all(const C* x, C* y, std::integer_sequence<int, Ks...>) {
-  ((y[Ks] = prime_row<N, INV, Ks>(x, std::make_integer_sequence<int, N - 1>{})), ...);
+__device__ __forceinline__ void prime_all(C* x, std::integer_sequence<int, Ks...>) {
+  constexpr int H = (N - 1) / 2;
+  C p[H], m[H], s = x[0];
+  const C x0 = x[0];
+#pragma unroll
+  for (int j = 0; j < H; ++j) {
+    p[j] = cadd(x[1 + j], x[N - 1 - j]);
+    m[j] = csub(x[1 + j], x[N - 1 - j]);
+    s = cadd(s, p[j]);
+  }
+  x[0] = s;
+  (
+      [&] {
+        constexpr int k = Ks + 1;
+        C r, q;
+        prime_pair<N, k>(x0, p, m, r, q, std::make_integer_sequence<int, H>{});
+        q = INV ? mul_pi(q) : mul_mi(q);
+        x[k] = cadd(r, q);
+        x[N - k] = csub(r, q);
+      }(),
+      ...);
 }
 template <int N, bool INV, typename C>
-__device__ __forceinline__ void rdft_prime(const C* x, C* y) {
-  prime_all<N, INV>(x, y, std::make_integer_sequence<int, N>{});
+__device__ __forceinline__ void rdft_prime(C* x) {
+  prime_all<N, INV>(x, std::make_integer_sequence<int, (N - 1) / 2>{});
 }
 
 // step 1 of the split for one n2: A-point DFT over x[n2 + B n1], twiddle W_N^{n2 k1}
@@ -155,10 +187,7 @@ __device__ __forceinline__ void rdft(C* x, const C* __restrict__ tw) {
   } else if constexpr (N == 8) {
     bfly8<INV>(x);
   } else if constexpr (ct_is_prime(N)) {
-    C y[N];
-    rdft_prime<N, INV>(x, y);
-#pragma unroll
-    for (int k = 0; k < N; ++k) x[k] = y[k];
+    rdft_prime<N, INV>(x);
   } else {
     constexpr int A = ct_first_factor(N);
     constexpr int B = N / A;

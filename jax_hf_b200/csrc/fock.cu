@@ -508,7 +508,12 @@ static int get_plan(int dtype, unsigned flags, int nk1, int nk2, int nb, SlotPla
     plan_rows(nb, sp);
     return HF_OK;
   }
-  const int max_ls = (fast_length(nk1) && fast_length(nk2)) ? 16 : 32;
+  // 16 slots for the register and two-factor passes, up to 32 for the Stockham stages
+  const bool fast = fast_length(nk1) && fast_length(nk2);
+  if (!fast && !(flags & (HF_FOCK_GENERIC_FFT | HF_FOCK_NO_TWO_FACTOR)) && two_factors(nk1) && two_factors(nk2) &&
+      plan_slots(nb, packing, 1, fft_elem(dtype, flags), 16, sp, inb) == HF_OK)
+    return HF_OK;  // their shared memory (17 lines) fits for every side, so the plan only looks at the padding
+  const int max_ls = fast ? 16 : 32;
   int st = plan_slots(nb, packing, std::max(nk1, nk2), fft_elem(dtype, flags), max_ls, sp, inb);
   if (st != HF_OK) return fail(st, "mesh too large for the shared-memory FFT (nk1, nk2 <= 768 in complex128)");
   return HF_OK;
@@ -625,6 +630,10 @@ static int launch_fock(FockParams& p, cudaStream_t stream, bool need_consts, con
     if (st != HF_OK || handled) return st;
     st = fast_fock<ST, FT>(p, stream, &handled);
     if (st != HF_OK || handled) return st;
+    if (!(p.flags & HF_FOCK_NO_TWO_FACTOR)) {
+      st = two_fock<ST, FT>(p, stream, &handled);
+      if (st != HF_OK || handled) return st;
+    }
   }
   if (exch) {
     k_fock_row_fwd<ST, FT><<<grow, kThreads, sm_row, stream>>>(p);
@@ -662,7 +671,7 @@ static std::map<TuneKey, unsigned> g_tune;
 static TuneKey tune_key(int dtype, unsigned flags, int nk1, int nk2, int nb) {
   int dev = 0;
   cudaGetDevice(&dev);
-  return TuneKey(dev, dtype, flags & ~kEngineFlags, nk1, nk2, nb);
+  return TuneKey(dev, dtype, flags & ~(kEngineFlags | HF_FOCK_NO_TWO_FACTOR), nk1, nk2, nb);
 }
 
 // flags with the stored engine choice applied (unless the caller set an engine flag)

@@ -35,6 +35,7 @@ struct FockParams {
   double* hdiag;      // [nb] Hartree diagonal
   const int* active;  // optional device flag: kernels return at once when *active == 0
   int rows_plan;      // slot groups are whole matrix rows; partner = (group << 8) | slot
+  int two_row, two_col;  // factors N1 | N2 << 5 of nk2 and nk1 (two-factor passes)
   int pipe_ns;        // stages of the pipelined passes (set per launch)
   int* fault;         // device word: a bounded wait of a pipelined pass that ran out records a code here
   CUtensorMap tmap_row;  // pipelined row pass: P as [nk1 nk2][nb^2] 4-byte words, box = SL channels x nk2 k-points
@@ -69,9 +70,20 @@ inline bool fast_length(int n) {
   }
 }
 
+// Factors N1 <= N2 <= 16 of a mesh side as N1 | N2 << 5, the pair nearest to square; 0 when
+// there is none.  Sides the two-factor passes (fock_two.cuh) transform.
+inline int two_factors(int n) {
+  for (int a = 16; a >= 1; --a)
+    if (a * a <= n && n % a == 0) return n / a <= 16 ? a | (n / a) << 5 : 0;
+  return 0;
+}
+
 // Launches the fast passes when both mesh lengths have a fast shape.
 template <typename ST, typename FT>
 int fast_fock(FockParams& p, cudaStream_t stream, bool* handled);
+// Launches the two-factor passes where both sides have two factors of at most 16.
+template <typename ST, typename FT>
+int two_fock(FockParams& p, cudaStream_t stream, bool* handled);
 // Launches the bulk-copy pipelined passes (fock_pipe.cuh) where they apply.
 template <typename ST, typename FT>
 int pipe_fock(FockParams& p, cudaStream_t stream, bool* handled);

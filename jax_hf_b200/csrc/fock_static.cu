@@ -43,6 +43,11 @@ extern "C" int hf_fock_build_static_scratch(void* stream, int dtype, unsigned fl
   size_t need = 0;
   int st = hf_fock_workspace_size(dtype, flags, nk1, nk2, nb, &need);
   if (st != HF_OK) return st;
+  if (need > (size_t)HF_FOCK_STATIC_SCRATCH_BYTES && !(flags & HF_FOCK_NO_TWO_FACTOR)) {
+    // the two-factor passes pad their slot groups differently: without them it may fit
+    flags |= HF_FOCK_NO_TWO_FACTOR;
+    if ((st = hf_fock_workspace_size(dtype, flags, nk1, nk2, nb, &need)) != HF_OK) return st;
+  }
   if (need > (size_t)HF_FOCK_STATIC_SCRATCH_BYTES)
     return hf::fail(HF_ERR_WORKSPACE,
                     "hf_fock_build_static_scratch: this mesh needs " + std::to_string(need) +

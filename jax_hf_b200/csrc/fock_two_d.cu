@@ -1,0 +1,6 @@
+#include "fock_two.cuh"
+
+namespace hf {
+// complex128 storage, FP64 transform
+template int two_fock<double, double>(FockParams&, cudaStream_t, bool*);
+}  // namespace hf

@@ -142,7 +142,7 @@ struct Scf {
       if (cf->fock_cb(cf->cb_user, s, P, Sg, H, F) != 0)
         return fail(HF_ERR_ABORTED, "hf_scf_solve: Fock callback failed");
     } else {
-      const unsigned flags = pb->fock_flags | (fp32 ? HF_FOCK_FFT_FP32 : 0u);
+      const unsigned flags = pb->fock_flags | HF_FOCK_NO_TWO_FACTOR | (fp32 ? HF_FOCK_FFT_FP32 : 0u);
       if ((st = hf_fock_build(s, HF_C128, flags, pb->nk1, pb->nk2, nb, P, pb->h, pb->VR, pb->refP, pb->HH,
                               pb->w2d, pb->n_contact, pb->contact_g, pb->contact_Oi, pb->contact_Oj, Sg, H, F,
                               at<void>(kFOCKWS), fock_ws)))

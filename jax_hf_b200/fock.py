@@ -16,7 +16,9 @@ Differences in form, not in value:
   Stockham engine instead of the register FFT of the specialised mesh lengths;
   ``engine="tile"`` forces the 2x2-tile slot groups in the register engine;
   ``engine="pipe"`` runs the bulk-copy pipelined passes (nb in {4, 8} on
-  register lengths; the default schedule elsewhere).
+  register lengths; the default schedule elsewhere);
+  ``engine="stockham"`` leaves out the two-factor passes (sides without a register
+  shape then take the Stockham stages), as the SCF drivers do;
 * ``autotune=True`` (extension) times the schedules that apply to this shape
   (``hf_fock_autotune``), keeps the fastest for every later build of the same
   shape and flags (solver drivers included) and records the timings in
@@ -137,6 +139,8 @@ def build_fock(P, *, h, VR, refP, HH, w2d, include_exchange: bool, include_hartr
         flags |= _lib.FOCK_TILE_PLAN
     elif engine is not None and str(engine).lower() == "pipe":
         flags |= _lib.FOCK_PIPE
+    elif engine is not None and str(engine).lower() == "stockham":
+        flags |= _lib.FOCK_NO_TWO_FACTOR
     if fft_precision is not None and str(fft_precision).lower() in ("fp32", "float32", "single"):
         if cdt == torch.complex128:
             flags |= _lib.FOCK_FFT_FP32

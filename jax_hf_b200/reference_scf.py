@@ -19,6 +19,7 @@ from __future__ import annotations
 
 import ctypes as C
 from dataclasses import dataclass, field
+from functools import partial
 from typing import Any, Callable
 
 import numpy as np
@@ -167,7 +168,8 @@ def _solve_scf_impl(kernel, P0, n_electrons, cfg, fock_build_fn):
         fock_kw["contact_g"] = kernel.contact_g
         fock_kw["contact_Oi"] = kernel.contact_Oi
         fock_kw["contact_Oj"] = kernel.contact_Oj
-    fn = fock_build_fn or build_fock
+    # the library driver's transforms and eigensolver: the two loops take the same steps
+    fn = fock_build_fn or partial(build_fock, engine="stockham")
 
     def proj_herm(X):
         if project is None:

@@ -497,3 +497,50 @@ def test_eigh_non_finite_entries_stay_in_their_matrix(cuda):
     good = [i for i in range(9) if i not in (2, 5)]
     wo = np.linalg.eigvalsh(A[good])
     assert np.abs(w.cpu().numpy()[good] - wo).max() < 1e-13 * np.abs(wo).max()
+
+
+TWO_FACTOR = [  # sides: prime radices, one-factor sides, unequal factors, the largest, mixed with a register side
+    (13, 13, 3, "layer", "c128"), (1, 30, 2, "scalar", "c128"), (14, 22, 8, "layer", "c128"),
+    (25, 49, 16, "scalar", "c128"), (75, 90, 6, "layer", "c128"), (48, 45, 5, "layer", "c128"),
+    (120, 20, 8, "layer", "c64"), (26, 169, 4, "scalar", "c64"), (256, 10, 1, "layer", "c128"),
+    (60, 27, 8, "layer", "fp32fft"), (208, 15, 9, "scalar", "c128"), (121, 21, 7, "layer", "c128"),
+]
+
+
+@pytest.mark.parametrize("n1,n2,nb,V,mode", TWO_FACTOR)
+@pytest.mark.parametrize("terms", [False, True])
+def test_two_factor_passes_match_stockham(cuda, n1, n2, nb, V, mode, terms):
+    """Sides with two factors of at most 16 against the Stockham engine on the same inputs (FP64: both
+    within 1e-12 of the oracle, so within 2e-12 of each other; FP32 transforms: 2 x 2e-5), with and
+    without the reference density, Hartree and contact terms, for a density that is not Hermitian
+    when every channel is transformed."""
+    import jax_hf_b200 as G
+    rng = np.random.default_rng(n1 + 3 * n2 + nb)
+    q = lambda *s: rng.normal(size=s) + 1j * rng.normal(size=s)
+    h = q(n1, n2, nb, nb)
+    h = h + np.conj(np.swapaxes(h, -1, -2))
+    P = q(n1, n2, nb, nb)
+    if V == "scalar":
+        P = 0.5 * (P + np.conj(np.swapaxes(P, -1, -2)))
+    Vq = rng.uniform(0.1, 1.0, size=(n1, n2) + ((1, 1) if V == "scalar" else (nb, nb)))
+    kw = {}
+    if terms:
+        HH = rng.normal(size=(nb, nb))
+        ref = q(n1, n2, nb, nb)
+        kw = dict(include_hartree=True, hartree_matrix=HH + HH.T, contact_terms=[(0.3, q(nb, nb), q(nb, nb))] * 2,
+                  reference_density=0.25 * (ref + np.conj(np.swapaxes(ref, -1, -2))))
+    dt = np.complex64 if mode == "c64" else np.complex128
+    w = rng.uniform(0.5, 1.5, size=(n1, n2)) / (n1 * n2)
+    K = G.HartreeFockKernel(w, h.astype(dt), Vq, 0.1, **kw)
+    a = K.as_args()
+    run = lambda **e: G.build_fock(
+        torch.as_tensor(P.astype(dt), device="cuda"), h=a["h"], VR=a["VR"], refP=a["refP"], HH=a["HH"], w2d=K.w2d,
+        include_exchange=True, include_hartree=a["include_hartree"],
+        exchange_hermitian_channel_packing=a["exchange_hermitian_channel_packing"], contact_g=a["contact_g"],
+        contact_Oi=a["contact_Oi"], contact_Oj=a["contact_Oj"],
+        fft_precision="fp32" if mode == "fp32fft" else None, **e)
+    tol = 2 * (TOL64 if mode == "c128" else TOL32)
+    for x, y in zip(run(), run(engine="generic")):
+        assert rel(x, y.cpu().numpy()) < tol if y.abs().max() > 0 else torch.equal(x, y)
+    for x, y in zip(run(engine="stockham"), run(engine="generic")):
+        assert torch.equal(x, y)
