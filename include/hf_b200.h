@@ -566,6 +566,13 @@ int hf_energy_vjp(void* stream, int nk1, int nk2, int nb, const void* P, const v
  * inside the entropy clip range [1e-14, 1-1e-14], 0 outside; E_bar = Omega_bar. */
 int hf_free_energy_vjp(void* stream, int nk1, int nk2, int nb, const double* p, const double* w_norm, double T,
                        double Omega_bar, double* p_bar);
+/* The same with the cotangent read from device memory, so a caller whose cotangent is a device
+ * scalar (torch autograd) needs no host read. */
+int hf_energy_vjp_dev(void* stream, int nk1, int nk2, int nb, const void* P, const void* h, const void* Sigma,
+                      const void* H, int H_mode, const double* w2d, const double* E_bar, void* P_bar, void* h_bar,
+                      void* Sigma_bar);
+int hf_free_energy_vjp_dev(void* stream, int nk1, int nk2, int nb, const double* p, const double* w_norm, double T,
+                           const double* Omega_bar, double* p_bar);
 /* hf_fourier_coeffs: out[r] = sum_k w_k exp(-i k.R_r) P_k for nR lattice vectors R (int pairs), k on
  * the centred grid k_m = 2 pi (m - n/2) / n: the gradient of sum_k w_k Re tr(h_k P_k) with respect to
  * an independent Fourier coefficient h_R of h_k = sum_R h_R exp(i k.R) (P Hermitian).  No counterpart

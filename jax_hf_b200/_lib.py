@@ -109,6 +109,8 @@ _SIGS = {
     "hf_fock_build_vjp": ([vp, i32, u32, i32, i32, i32, vp, vp, vp, vp, vp, vp, sz], i32),
     "hf_energy_vjp": ([vp, i32, i32, i32, vp, vp, vp, vp, i32, vp, f64, vp, vp, vp], i32),
     "hf_free_energy_vjp": ([vp, i32, i32, i32, vp, vp, f64, f64, vp], i32),
+    "hf_energy_vjp_dev": ([vp, i32, i32, i32, vp, vp, vp, vp, i32, vp, vp, vp, vp, vp], i32),
+    "hf_free_energy_vjp_dev": ([vp, i32, i32, i32, vp, vp, f64, vp, vp], i32),
     "hf_fourier_coeffs": ([vp, i32, i32, i32, vp, vp, i32, vp, vp], i32),
     "hf_cg_solve_batch": ([vp, vp, i32, vp, i32, vp, sz, vp], i32),
     "hf_cg_solve_batch_graph": ([vp, vp, i32, vp, vp, sz, vp], i32),

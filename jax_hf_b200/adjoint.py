@@ -71,61 +71,97 @@ def _consts(rho, kernel):
     return H, sc
 
 
+def _fock_vjp(kernel, P, gS, gF, gH, want_h):
+    """(P_bar, h_bar) of the Fock build for cotangents of Sigma, F and H (each may be None)."""
+    nk1, nk2, nb = kernel.shape
+    dev = P.device
+    hb = torch.empty_like(P) if want_h and gF is not None else None
+    if gS is None and gF is None:
+        Pb = torch.zeros_like(P)
+    else:
+        VR = kernel._VR_shifted
+        VR_adj = VR.conj().resolve_conj().contiguous() if VR.is_complex() else VR
+        flags = _flags(kernel, VR)
+        gS = None if gS is None else gS.to(torch.complex128).contiguous()
+        gF = None if gF is None else gF.to(torch.complex128).contiguous()
+        Pb = torch.empty_like(P)
+        need = C.c_size_t(0)
+        _lib.check(_lib.lib().hf_fock_vjp_workspace_size(_lib.HF_C128, flags, nk1, nk2, nb, C.byref(need)))
+        ws = _lib.workspace(need.value, dev, "fock_vjp")
+        _lib.check(_lib.lib().hf_fock_build_vjp(_lib.stream_ptr(dev), _lib.HF_C128, flags, nk1, nk2, nb,
+                                                _lib.ptr(gS), _lib.ptr(gF), _lib.ptr(VR_adj), Pb.data_ptr(),
+                                                _lib.ptr(hb), ws.data_ptr(), ws.numel()))
+    if kernel.include_hartree or kernel.has_contact:
+        # the k-independent terms: H enters F at every k; the contact term enters Sigma and F
+        w2d = kernel.w2d.to(torch.float64).contiguous()
+        ones = torch.ones_like(w2d)
+        Fh = None if gF is None else 0.5 * (gF + gF.transpose(-1, -2).conj())
+        terms, cots = [], []
+        refP = kernel.refP
+        dP = P if is_marked_zero(refP) else P - refP.to(torch.complex128)
+        rho = _k_sum(dP, w2d).detach().requires_grad_(True)
+        with torch.enable_grad():
+            Hm, sc = _consts(rho, kernel)
+            if kernel.include_hartree and (Fh is not None or gH is not None):
+                cH = torch.zeros_like(rho) if Fh is None else _k_sum(Fh, ones)
+                if gH is not None:
+                    cH = cH + gH.reshape(nb, nb).to(torch.complex128)
+                terms.append(Hm)
+                cots.append(cH)
+            if kernel.has_contact and (Fh is not None or gS is not None):
+                terms.append(sc)
+                cots.append(_k_sum(gS if Fh is None else Fh if gS is None else Fh + gS, ones))
+            grho = torch.autograd.grad(terms, [rho], cots, allow_unused=True)[0] if terms else None
+        if grho is not None:
+            Pb = Pb + w2d[..., None, None].to(torch.complex128) * grho
+    return Pb, hb
+
+
+def _build(P, h, kernel):
+    from .fock import build_fock
+    a = kernel.as_args()
+    return build_fock(P, h=h, VR=a["VR"], refP=a["refP"], HH=a["HH"], w2d=kernel.w2d,
+                      include_exchange=kernel.include_exchange, include_hartree=kernel.include_hartree,
+                      exchange_hermitian_channel_packing=a["exchange_hermitian_channel_packing"],
+                      contact_g=a["contact_g"], contact_Oi=a["contact_Oi"], contact_Oj=a["contact_Oj"])
+
+
+def _energy_vjp(gE, P, h, Sigma, H, w2d, want_P, want_h, want_S):
+    """Cotangents of hf_energy's P, h and Sigma (None where not wanted); gE stays on the device."""
+    nk1, nk2, nb = P.shape[0], P.shape[1], P.shape[-1]
+    Ht = H.reshape(nb, nb).to(torch.complex128).contiguous()
+    out = [torch.empty_like(P) if w else None for w in (want_P, want_h, want_S)]
+    _lib.check(_lib.lib().hf_energy_vjp_dev(_lib.stream_ptr(P.device), nk1, nk2, nb, P.data_ptr(), h.data_ptr(),
+                                            Sigma.data_ptr(), Ht.data_ptr(), 1, w2d.data_ptr(), gE.data_ptr(),
+                                            *[_lib.ptr(t) for t in out]))
+    return out
+
+
+def _energy_vjp_H(gE, P, w2d):
+    """Cotangent of hf_energy's k-independent H: E_bar / 2 sum_k w_k P_k^H."""
+    return (0.5 * gE) * _k_sum(P, w2d).transpose(-1, -2).conj()
+
+
+def _dev_scalar(g, dev):
+    """A cotangent as a contiguous float64 device scalar (no host read)."""
+    return g.to(dev, torch.float64).contiguous()
+
+
 class _FockBuildFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, P, h, kernel):
-        from .fock import build_fock
-        a = kernel.as_args()
-        Sg, H, F = build_fock(P, h=h, VR=a["VR"], refP=a["refP"], HH=a["HH"], w2d=kernel.w2d,
-                              include_exchange=kernel.include_exchange, include_hartree=kernel.include_hartree,
-                              exchange_hermitian_channel_packing=a["exchange_hermitian_channel_packing"],
-                              contact_g=a["contact_g"], contact_Oi=a["contact_Oi"], contact_Oj=a["contact_Oj"])
+        Sg, H, F = _build(P, h, kernel)
+        ctx.set_materialize_grads(False)
         ctx.kernel = kernel
         ctx.save_for_backward(P)
         return Sg, H, F
 
     @staticmethod
     def backward(ctx, gS, gH, gF):
-        kernel = ctx.kernel
         (P,) = ctx.saved_tensors
-        nk1, nk2, nb = kernel.shape
-        dev = P.device
-        VR = kernel._VR_shifted
-        VR_adj = VR.conj().resolve_conj().contiguous() if VR.is_complex() else VR
-        flags = _flags(kernel, VR)
-        gS = torch.zeros_like(P) if gS is None else gS.to(torch.complex128).contiguous()
-        gF = torch.zeros_like(P) if gF is None else gF.to(torch.complex128).contiguous()
-        Pb = torch.empty_like(P)
-        hb = torch.empty_like(P)
-        need = C.c_size_t(0)
-        _lib.check(_lib.lib().hf_fock_vjp_workspace_size(_lib.HF_C128, flags, nk1, nk2, nb, C.byref(need)))
-        ws = _lib.workspace(need.value, dev, "fock_vjp")
-        _lib.check(_lib.lib().hf_fock_build_vjp(_lib.stream_ptr(dev), _lib.HF_C128, flags, nk1, nk2, nb,
-                                                gS.data_ptr(), gF.data_ptr(), _lib.ptr(VR_adj), Pb.data_ptr(),
-                                                hb.data_ptr(), ws.data_ptr(), ws.numel()))
-        if kernel.include_hartree or kernel.has_contact:
-            # the k-independent terms: H enters F at every k; the contact term enters Sigma and F
-            w2d = kernel.w2d.to(torch.float64).contiguous()
-            ones = torch.ones_like(w2d)
-            Fh = 0.5 * (gF + gF.transpose(-1, -2).conj())
-            terms, cots = [], []
-            refP = kernel.refP
-            dP = P if is_marked_zero(refP) else P - refP.to(torch.complex128)
-            rho = _k_sum(dP, w2d).detach().requires_grad_(True)
-            with torch.enable_grad():
-                Hm, sc = _consts(rho, kernel)
-                if kernel.include_hartree:
-                    cH = _k_sum(Fh, ones)
-                    if gH is not None:
-                        cH = cH + gH.reshape(nb, nb).to(torch.complex128)
-                    terms.append(Hm)
-                    cots.append(cH)
-                if kernel.has_contact:
-                    terms.append(sc)
-                    cots.append(_k_sum(Fh + gS, ones))
-                (grho,) = torch.autograd.grad(terms, [rho], cots, allow_unused=True)
-            if grho is not None:
-                Pb = Pb + w2d[..., None, None].to(torch.complex128) * grho
+        Pb, hb = _fock_vjp(ctx.kernel, P, gS, gF, gH, ctx.needs_input_grad[1])
+        if hb is None and ctx.needs_input_grad[1]:
+            hb = torch.zeros_like(P)
         return Pb, hb, None
 
 
@@ -147,14 +183,10 @@ class _EnergyFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gE):
         P, h, Sigma, H, w2d = ctx.saved_tensors
-        nk1, nk2, nb = P.shape[0], P.shape[1], P.shape[-1]
-        Ht = H.reshape(nb, nb).to(torch.complex128).contiguous()
-        Pb, hb, Sb = torch.empty_like(P), torch.empty_like(P), torch.empty_like(P)
-        Eb = float(gE)
-        _lib.check(_lib.lib().hf_energy_vjp(_lib.stream_ptr(P.device), nk1, nk2, nb, P.data_ptr(), h.data_ptr(),
-                                            Sigma.data_ptr(), Ht.data_ptr(), 1, w2d.data_ptr(), Eb, Pb.data_ptr(),
-                                            hb.data_ptr(), Sb.data_ptr()))
-        Hb = (0.5 * Eb) * _k_sum(P.transpose(-1, -2).conj(), w2d).reshape(H.shape)
+        gE = _dev_scalar(gE, P.device)
+        need = ctx.needs_input_grad
+        Pb, hb, Sb = _energy_vjp(gE, P, h, Sigma, H, w2d, *need[:3])
+        Hb = _energy_vjp_H(gE, P, w2d).reshape(H.shape) if need[3] else None
         return Pb, hb, Sb, Hb, None
 
 
@@ -162,6 +194,14 @@ def hf_energy(P, h, Sigma, H, w2d):
     """Differentiable E = sum_k w_k Re tr((h + (Sigma + H)/2) P) (fock.py:100-111); H is (1, 1, nb, nb)."""
     return _EnergyFn.apply(P.contiguous(), h.contiguous(), Sigma.contiguous(), H.contiguous(),
                            w2d.to(torch.float64).contiguous())
+
+
+def _free_energy_vjp(gO, p, w_norm, T):
+    nb = p.shape[-1]
+    pb = torch.empty_like(p)
+    _lib.check(_lib.lib().hf_free_energy_vjp_dev(_lib.stream_ptr(p.device), p.numel() // nb, 1, nb, p.data_ptr(),
+                                                 w_norm.data_ptr(), T, gO.data_ptr(), pb.data_ptr()))
+    return pb
 
 
 class _FreeEnergyFn(torch.autograd.Function):
@@ -175,11 +215,7 @@ class _FreeEnergyFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gO):
         p, w_norm = ctx.saved_tensors
-        nb = p.shape[-1]
-        nk = p.numel() // nb
-        pb = torch.empty_like(p)
-        _lib.check(_lib.lib().hf_free_energy_vjp(_lib.stream_ptr(p.device), nk, 1, nb, p.data_ptr(),
-                                                 w_norm.data_ptr(), ctx.T, float(gO), pb.data_ptr()))
+        pb = _free_energy_vjp(_dev_scalar(gO, p.device), p, w_norm, ctx.T) if ctx.needs_input_grad[1] else None
         return gO, pb, None, None
 
 
@@ -188,13 +224,47 @@ def free_energy(E, p, w_norm, T):
     return _FreeEnergyFn.apply(E, p.to(torch.float64).contiguous(), w_norm.to(torch.float64).contiguous(), T)
 
 
+class _ObjectiveFn(torch.autograd.Function):
+    """Omega(P, p, h) as one node: the three calls forward, the three adjoints backward, with no
+    cotangent of Sigma, H or E passing through the autograd graph and nothing read on the host.
+    At 96 x 96, nb = 4 the calls are latency-bound: as three nodes (two of which read their cotangent
+    on the host, and materialised zero cotangents of F and H) value and gradients took 559 us."""
+
+    @staticmethod
+    def forward(ctx, P, p, h, kernel):
+        from .fock import free_energy, hf_energy
+        Sg, H, _ = _build(P, h, kernel)
+        w2d = kernel.w2d.to(torch.float64)
+        E = hf_energy(P, h=h, Sigma=Sg, H=H, weights_b=w2d[..., None, None])
+        wn = w2d / max(float(kernel.weight_sum), 1e-30)
+        ctx.kernel = kernel
+        ctx.save_for_backward(P, p, h, Sg, H, wn)
+        return free_energy(E, p, wn, kernel.T)
+
+    @staticmethod
+    def backward(ctx, gO):
+        kernel = ctx.kernel
+        P, p, h, Sg, H, wn = ctx.saved_tensors
+        want_P, want_p, want_h = ctx.needs_input_grad[:3]
+        gO = _dev_scalar(gO, P.device)
+        w2d = kernel.w2d.to(torch.float64).contiguous()
+        Pb = pb = hb = None
+        if want_P or want_h:
+            Pb, hb, Sb = _energy_vjp(gO, P, h, Sg, H, w2d, want_P, want_h, want_P)
+        if want_P:
+            gH = _energy_vjp_H(gO, P, w2d) if kernel.include_hartree else None
+            Pb += _fock_vjp(kernel, P, Sb, None, gH, False)[0]
+        if want_p:
+            pb = _free_energy_vjp(gO, p, wn, float(kernel.T))
+        return Pb, pb, hb, None
+
+
 def objective(P, p, kernel, h=None):
     """Omega(P, p) = hf_energy(P, h, Sigma[P], H[P]) - T S(p), differentiable in P, p and h."""
     h = kernel.h.to(torch.complex128) if h is None else h
-    Sg, H, _ = fock_build(P, h, kernel)
-    E = hf_energy(P, h, Sg, H.reshape(1, 1, *H.shape[-2:]), kernel.w2d)
-    wn = kernel.w2d.to(torch.float64) / max(float(kernel.weight_sum), 1e-30)
-    return free_energy(E, p, wn, kernel.T)
+    if kernel.dtype != torch.complex128:
+        raise ValueError("the hand-written adjoint runs in complex128; build the kernel in complex128")
+    return _ObjectiveFn.apply(P.contiguous(), p.to(torch.float64).contiguous(), h.contiguous(), kernel)
 
 
 def shifted_vr(dV, weights):

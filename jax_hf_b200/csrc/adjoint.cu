@@ -61,9 +61,10 @@ __global__ void k_vjp_xbar(size_t nk, int nb, const double2* __restrict__ Sb, co
 // Sigma_bar = Eb w P^H / 2 (the shared H's cotangent is a k-sum formed by the caller).
 __global__ void k_energy_vjp(size_t nk, int nb, const double2* __restrict__ P, const double2* __restrict__ h,
                              const double2* __restrict__ S, const double2* __restrict__ H, int H_mode,
-                             const double* __restrict__ w, double Eb, double2* __restrict__ Pb,
-                             double2* __restrict__ hb, double2* __restrict__ Sb) {
+                             const double* __restrict__ w, double Eb, const double* __restrict__ Eb_dev,
+                             double2* __restrict__ Pb, double2* __restrict__ hb, double2* __restrict__ Sb) {
   const size_t nb2 = (size_t)nb * nb, n = nk * nb2;
+  if (Eb_dev) Eb = Eb_dev[0];
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
     const size_t k = e / nb2;
     const int r = (int)(e - k * nb2), i = r / nb, j = r - i * nb;
@@ -91,8 +92,10 @@ __global__ void k_energy_vjp(size_t nk, int nb, const double2* __restrict__ P, c
 // Omega = E - max(T, 1e-14) S(p), S = -sum_k wn_k sum_i s(clip(p)), s(p) = p log p + (1-p) log1p(-p):
 // p_bar = Ob T wn (log p - log1p(-p)) inside the clip range, 0 outside (fock.py:114-129).
 __global__ void k_free_energy_vjp(size_t n, int nb, const double* __restrict__ p, const double* __restrict__ wn,
-                                  double T, double Ob, double* __restrict__ pb) {
+                                  double T, double Ob, const double* __restrict__ Ob_dev,
+                                  double* __restrict__ pb) {
   const double Tm = fmax(T, 1e-14);
+  if (Ob_dev) Ob = Ob_dev[0];
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
     const double pv = p[e];
     double g = 0.0;
@@ -164,12 +167,17 @@ extern "C" int hf_fock_build_vjp(void* stream, int dtype, unsigned flags, int nk
   size_t fws = 0;
   if (flags & HF_FOCK_EXCHANGE) hf_fock_workspace_size(dtype, vjp_flags(flags), nk1, nk2, nb, &fws);
   char* ws = static_cast<char*>(workspace);
-  double2* X = reinterpret_cast<double2*>(ws + align_up(fws, 256));
-  double2* Fs = X + align_up(nq * sizeof(double2), 256) / sizeof(double2);
-  k_vjp_xbar<<<adj_blocks(nq), kAdjThreads, 0, s>>>(nk, nb, static_cast<const double2*>(Sigma_bar),
-                                                   static_cast<const double2*>(F_bar), X,
-                                                   static_cast<double2*>(h_bar));
-  HF_LAUNCH_CHECK("k_vjp_xbar");
+  double2* xw = reinterpret_cast<double2*>(ws + align_up(fws, 256));
+  double2* Fs = xw + align_up(nq * sizeof(double2), 256) / sizeof(double2);
+  const void* X = xw;
+  if (F_bar || h_bar || P_bar == Sigma_bar) {
+    k_vjp_xbar<<<adj_blocks(nq), kAdjThreads, 0, s>>>(nk, nb, static_cast<const double2*>(Sigma_bar),
+                                                     static_cast<const double2*>(F_bar), xw,
+                                                     static_cast<double2*>(h_bar));
+    HF_LAUNCH_CHECK("k_vjp_xbar");
+  } else {
+    X = Sigma_bar;  // nothing to add: the cotangent itself is transformed
+  }
   if (!(flags & HF_FOCK_EXCHANGE)) {
     HF_CUDA(cudaMemsetAsync(P_bar, 0, nq * sizeof(double2), s));
     return HF_OK;
@@ -179,9 +187,10 @@ extern "C" int hf_fock_build_vjp(void* stream, int dtype, unsigned flags, int nk
                              nullptr, 0, nullptr, nullptr, nullptr, P_bar, nullptr, Fs, ws, fws, nullptr);
 }
 
-extern "C" int hf_energy_vjp(void* stream, int nk1, int nk2, int nb, const void* P, const void* h,
-                             const void* Sigma, const void* H, int H_mode, const double* w2d, double E_bar,
-                             void* P_bar, void* h_bar, void* Sigma_bar) {
+namespace hf {
+static int energy_vjp(void* stream, int nk1, int nk2, int nb, const void* P, const void* h, const void* Sigma,
+                      const void* H, int H_mode, const double* w2d, double E_bar, const double* E_bar_dev,
+                      void* P_bar, void* h_bar, void* Sigma_bar) {
   if (nk1 < 1 || nk2 < 1 || nb < 1) return fail(HF_ERR_INVALID, "bad shape");
   if (!P || !w2d) return fail(HF_ERR_INVALID, "P and w2d must be non-NULL");
   if (H_mode < 0 || H_mode > 2) return fail(HF_ERR_INVALID, "H_mode must be 0, 1 or 2");
@@ -189,21 +198,46 @@ extern "C" int hf_energy_vjp(void* stream, int nk1, int nk2, int nb, const void*
   const size_t nq = (size_t)nk1 * nk2 * nb * nb;
   k_energy_vjp<<<adj_blocks(nq), kAdjThreads, 0, static_cast<cudaStream_t>(stream)>>>(
       (size_t)nk1 * nk2, nb, static_cast<const double2*>(P), static_cast<const double2*>(h),
-      static_cast<const double2*>(Sigma), static_cast<const double2*>(H), H_mode, w2d, E_bar,
+      static_cast<const double2*>(Sigma), static_cast<const double2*>(H), H_mode, w2d, E_bar, E_bar_dev,
       static_cast<double2*>(P_bar), static_cast<double2*>(h_bar), static_cast<double2*>(Sigma_bar));
   HF_LAUNCH_CHECK("k_energy_vjp");
   return HF_OK;
 }
 
-extern "C" int hf_free_energy_vjp(void* stream, int nk1, int nk2, int nb, const double* p, const double* w_norm,
-                                  double T, double Omega_bar, double* p_bar) {
+static int free_energy_vjp(void* stream, int nk1, int nk2, int nb, const double* p, const double* w_norm, double T,
+                           double Omega_bar, const double* Omega_bar_dev, double* p_bar) {
   if (nk1 < 1 || nk2 < 1 || nb < 1) return fail(HF_ERR_INVALID, "bad shape");
   if (!p || !w_norm || !p_bar) return fail(HF_ERR_INVALID, "NULL argument");
   const size_t n = (size_t)nk1 * nk2 * nb;
-  k_free_energy_vjp<<<adj_blocks(n), kAdjThreads, 0, static_cast<cudaStream_t>(stream)>>>(n, nb, p, w_norm, T,
-                                                                                          Omega_bar, p_bar);
+  k_free_energy_vjp<<<adj_blocks(n), kAdjThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+      n, nb, p, w_norm, T, Omega_bar, Omega_bar_dev, p_bar);
   HF_LAUNCH_CHECK("k_free_energy_vjp");
   return HF_OK;
+}
+}  // namespace hf
+
+extern "C" int hf_energy_vjp(void* stream, int nk1, int nk2, int nb, const void* P, const void* h,
+                             const void* Sigma, const void* H, int H_mode, const double* w2d, double E_bar,
+                             void* P_bar, void* h_bar, void* Sigma_bar) {
+  return hf::energy_vjp(stream, nk1, nk2, nb, P, h, Sigma, H, H_mode, w2d, E_bar, nullptr, P_bar, h_bar, Sigma_bar);
+}
+
+extern "C" int hf_energy_vjp_dev(void* stream, int nk1, int nk2, int nb, const void* P, const void* h,
+                                 const void* Sigma, const void* H, int H_mode, const double* w2d,
+                                 const double* E_bar, void* P_bar, void* h_bar, void* Sigma_bar) {
+  if (!E_bar) return fail(HF_ERR_INVALID, "E_bar is NULL");
+  return hf::energy_vjp(stream, nk1, nk2, nb, P, h, Sigma, H, H_mode, w2d, 0.0, E_bar, P_bar, h_bar, Sigma_bar);
+}
+
+extern "C" int hf_free_energy_vjp(void* stream, int nk1, int nk2, int nb, const double* p, const double* w_norm,
+                                  double T, double Omega_bar, double* p_bar) {
+  return hf::free_energy_vjp(stream, nk1, nk2, nb, p, w_norm, T, Omega_bar, nullptr, p_bar);
+}
+
+extern "C" int hf_free_energy_vjp_dev(void* stream, int nk1, int nk2, int nb, const double* p,
+                                      const double* w_norm, double T, const double* Omega_bar, double* p_bar) {
+  if (!Omega_bar) return fail(HF_ERR_INVALID, "Omega_bar is NULL");
+  return hf::free_energy_vjp(stream, nk1, nk2, nb, p, w_norm, T, 0.0, Omega_bar, p_bar);
 }
 
 extern "C" int hf_fourier_coeffs(void* stream, int nk1, int nk2, int nb, const void* P, const double* w2d,

@@ -208,3 +208,38 @@ def test_torch_library_ops(cuda):
     A.hf_energy(P2, h2, Sg2, H2, K.w2d).backward()
     torch.testing.assert_close(P1.grad, P2.grad, rtol=0, atol=1e-13)
     torch.testing.assert_close(h1.grad, h2.grad, rtol=0, atol=1e-13)
+
+
+@pytest.mark.parametrize("hartree", [False, True])
+@pytest.mark.parametrize("want", ["P", "p", "h", "Pph"])
+def test_objective_node_matches_the_separate_nodes(cuda, hartree, want):
+    """The one-node objective against fock_build -> hf_energy -> free_energy on the same inputs: the same
+    kernels in the same order, one sum of two P cotangents apart (4 ulp of the largest entry)."""
+    import jax_hf_b200 as G
+    from jax_hf_b200 import adjoint as A
+    rng = np.random.default_rng(11)
+    n, nb = 6, 3
+    q = lambda *s: rng.normal(size=s) + 1j * rng.normal(size=s)
+    h = q(n, n, nb, nb)
+    kw = {}
+    if hartree:
+        HH = rng.normal(size=(nb, nb))
+        kw = dict(include_hartree=True, hartree_matrix=HH + HH.T, reference_density=q(n, n, nb, nb),
+                  contact_terms=[(0.4, q(nb, nb), q(nb, nb))])
+    K = G.HartreeFockKernel(np.full((n, n), 1.0 / n ** 2), h + np.conj(np.swapaxes(h, -1, -2)),
+                            rng.uniform(0.1, 1.0, size=(n, n, nb, nb)), 0.1, **kw)
+    P0 = torch.as_tensor(q(n, n, nb, nb), device="cuda")
+    p0 = torch.as_tensor(rng.uniform(0.05, 0.95, size=(n, n, nb)), device="cuda")
+
+    def leaves():
+        return [t.clone().requires_grad_(c in want) for t, c in ((P0, "P"), (p0, "p"), (K.h, "h"))]
+
+    a, b = leaves(), leaves()
+    (2.5 * A.objective(a[0], a[1], K, a[2])).backward()
+    Sg, H, _ = A.fock_build(b[0], b[2], K)
+    E = A.hf_energy(b[0], b[2], Sg, H.reshape(1, 1, nb, nb), K.w2d)
+    (2.5 * A.free_energy(E, b[1], K.w2d / K.weight_sum, K.T)).backward()
+    for x, y in zip(a, b):
+        assert (x.grad is None) == (y.grad is None)
+        if x.grad is not None:
+            assert float((x.grad - y.grad).abs().max()) <= 4 * 2.2e-16 * float(y.grad.abs().max())
