@@ -165,8 +165,15 @@ def require_cuda(t: torch.Tensor) -> None:
         raise RuntimeError("jax_hf_b200 runs on CUDA tensors only (no CPU fallback)")
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def stream_ptr(device=None) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    """The current stream's handle (without building a Stream object where torch offers that)."""
+    if _raw_stream is None:
+        return torch.cuda.current_stream(device).cuda_stream
+    index = None if device is None else torch.device(device).index
+    return _raw_stream(torch.cuda.current_device() if index is None else index)
 
 
 def ptr(t) -> int | None:
@@ -186,13 +193,13 @@ def dtype_code(t: torch.Tensor) -> int:
 _ws_cache: dict = {}
 
 
-def workspace(nbytes: int, device, tag: str = "ws") -> torch.Tensor:
+def workspace(nbytes: int, device, tag: str = "ws", stream: int | None = None) -> torch.Tensor:
     """Caller-owned scratch from torch's caching allocator (256-byte aligned).
 
     One buffer per (tag, device, current stream): calls on different streams may
     run at the same time and never share scratch; calls on one stream are ordered.
     """
-    key = (tag, str(device), torch.cuda.current_stream(device).cuda_stream)
+    key = (tag, torch.device(device), stream_ptr(device) if stream is None else stream)
     buf = _ws_cache.get(key)
     if buf is None or buf.numel() < nbytes:
         buf = torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=device)

@@ -5,6 +5,7 @@
 #include <mutex>
 #include <set>
 #include <string>
+#include <tuple>
 
 #include "common.cuh"
 
@@ -77,6 +78,48 @@ int allow_max_dynamic_smem(const void* fn) {
   HF_CUDA(cudaFuncGetAttributes(&fa, fn));
   HF_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes));
   done.insert({fn, ctx});
+  return HF_OK;
+}
+
+// CTAs of a launch shape resident on the whole device, and clusters of csize CTAs when
+// csize > 0, asked once per (kernel, context, shape): the queries cost more host time
+// than the launches they size.
+int resident_ctas(const void* fn, int threads, size_t smem, int csize, int* out) {
+  static std::mutex mu;
+  static std::map<std::tuple<const void*, unsigned long long, int, size_t, int>, int> cache;
+  unsigned long long ctx = 0;
+  int st = context_id(&ctx);
+  if (st) return st;
+  const auto key = std::make_tuple(fn, ctx, threads, smem, csize);
+  std::lock_guard<std::mutex> lock(mu);
+  auto it = cache.find(key);
+  if (it == cache.end()) {
+    int n = 1;
+    if (csize > 0) {
+      cudaLaunchConfig_t cfg = {};
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = (unsigned)csize;
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cfg.gridDim = dim3((unsigned)csize);
+      cfg.blockDim = dim3((unsigned)threads);
+      cfg.dynamicSmemBytes = smem;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) != cudaSuccess || n < 1) n = 1;
+    } else {
+      int dev = 0, sms = 148, per_sm = 1;
+      cudaGetDevice(&dev);
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem) != cudaSuccess || per_sm < 1)
+        per_sm = 1;
+      n = sms * per_sm;
+    }
+    cudaGetLastError();  // a refused query leaves the fallback of one
+    it = cache.emplace(key, n).first;
+  }
+  *out = it->second;
   return HF_OK;
 }
 

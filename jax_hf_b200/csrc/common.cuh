@@ -16,6 +16,7 @@ int fail(int status, const std::string& msg);
 int cuda_check(cudaError_t e, const char* what);
 int allow_max_dynamic_smem(const void* fn);
 int context_id(unsigned long long* id);
+int resident_ctas(const void* fn, int threads, size_t smem, int csize, int* out);
 // Slot-indexed DIIS steps for the device-resident SCF loop (ops.cu): the history slot is
 // a device int, so one captured iteration serves every slot
 int scf_residuals_slot(void* stream, int nk, int nb, const void* F, const void* P, const void* Pn, const double* w,

@@ -207,6 +207,7 @@ __global__ void __launch_bounds__(kThreads) k_fock_row_fwd(const __grid_constant
   if (p.active && !*p.active) return;
   using SC = cpx_t<ST>;
   using FC = cpx_t<FT>;
+  zero_h<SC>(p);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int N = p.nk2, LS = p.LS;
   FC* tw = reinterpret_cast<FC*>(smem_raw);
@@ -519,8 +520,7 @@ static void plan_rows(int nb, SlotPlan& out) {
   }
 }
 
-static int get_plan(int dtype, unsigned flags, int nk1, int nk2, int nb, SlotPlan& sp,
-                    const unsigned char* inb = nullptr) {
+static int make_plan(int dtype, unsigned flags, int nk1, int nk2, int nb, SlotPlan& sp, const unsigned char* inb) {
   const bool packing = (flags & HF_FOCK_PACKING) != 0;
   if (!inb && !packing && nb <= 8 && !(flags & (HF_FOCK_GENERIC_FFT | HF_FOCK_TILE_PLAN)) && fast_length(nk1) &&
       fast_length(nk2)) {
@@ -535,6 +535,32 @@ static int get_plan(int dtype, unsigned flags, int nk1, int nk2, int nb, SlotPla
   const int max_ls = fast ? 16 : 32;
   int st = plan_slots(nb, packing, std::max(nk1, nk2), fft_elem(dtype, flags), max_ls, sp, inb);
   if (st != HF_OK) return fail(st, "mesh too large for the shared-memory FFT (nk1, nk2 <= 768 in complex128)");
+  return HF_OK;
+}
+
+// The plan of a shape, kept for later builds of it (packing the slot groups of 16 bands
+// takes ~40 us of host time; a build of 49 x 49 x 16 spent 180 us in it).  Masked builds
+// make theirs each time.
+static int get_plan(int dtype, unsigned flags, int nk1, int nk2, int nb, SlotPlan& sp,
+                    const unsigned char* inb = nullptr) {
+  if (inb) return make_plan(dtype, flags, nk1, nk2, nb, sp, inb);
+  constexpr unsigned kPlanFlags = HF_FOCK_PACKING | HF_FOCK_GENERIC_FFT | HF_FOCK_TILE_PLAN | HF_FOCK_NO_TWO_FACTOR;
+  static std::mutex mu;
+  static std::map<std::tuple<unsigned, size_t, int, int, int>, SlotPlan> plans;
+  const auto key = std::make_tuple(flags & kPlanFlags, fft_elem(dtype, flags), nk1, nk2, nb);
+  {
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = plans.find(key);
+    if (it != plans.end()) {
+      sp = it->second;
+      return HF_OK;
+    }
+  }
+  const int st = make_plan(dtype, flags, nk1, nk2, nb, sp, nullptr);
+  if (st != HF_OK) return st;
+  std::lock_guard<std::mutex> lk(mu);
+  if (plans.size() >= 1024) plans.clear();
+  plans.emplace(key, sp);
   return HF_OK;
 }
 
@@ -804,7 +830,11 @@ static int fock_build_exact(void* stream, int dtype, unsigned flags, int nk1, in
   std::copy(sp.chan.begin(), sp.chan.end(), p.chan);
   std::copy(sp.partner.begin(), sp.partner.end(), p.partner);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (H && !need_consts && !active) {
+  // without constant terms H is zero: the forward row pass writes it, except where the
+  // pipelined passes or a mask without in-block channels leave that pass out
+  const bool zero = H && !need_consts && !active;
+  p.zero_h = zero && !inb && !(flags & HF_FOCK_PIPE);
+  if (zero && !p.zero_h) {
     const size_t hb = (size_t)nb * nb * (dtype == HF_C128 ? sizeof(double2) : sizeof(float2));
     HF_CUDA(cudaMemsetAsync(H, 0, hb, s));
   }

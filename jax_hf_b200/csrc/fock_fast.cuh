@@ -113,6 +113,7 @@ __global__ void __launch_bounds__(16 * S::TPL) k_fast_row_fwd(const __grid_const
   pdl_launch_dependents();
   using SC = cpx_t<ST>;
   using FC = cpx_t<FT>;
+  zero_h<SC>(p);
   constexpr bool kStage = sizeof(SC) == sizeof(FC);  // mixed precision converts in registers
   extern __shared__ __align__(16) unsigned char smem_raw[];
   FC* twf = reinterpret_cast<FC*>(smem_raw);
@@ -503,16 +504,15 @@ constexpr size_t fast_smem_rows() {
   return (size_t)(2 * S::TPL * S::TS) * sizeof(cpx_t<FT>) + 16 * (size_t)S::N * e + 16 * (size_t)S::N * sizeof(cpx_t<FT>);
 }
 
-// Persistent grid: CTAs resident on the device (2 per SM for the large shapes).
+// Grid of a persistent pass: the CTAs resident on the device (at least 2 per SM for the
+// large shapes), or one per item when there are fewer.  Also lifts the kernel's cap.
 template <typename K>
-inline int persistent_grid(K kernel, int threads, size_t smem, int items) {
-  int dev = 0, sms = 148, per_sm = 1;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess || per_sm < 1)
-    per_sm = 1;
-  const int g = sms * per_sm;
-  return items < g ? items : g;
+inline int persistent_grid(K kernel, int threads, size_t smem, int items, int* grid) {
+  const void* fn = (const void*)kernel;
+  int st = allow_max_dynamic_smem(fn), g = 1;
+  if (!st) st = resident_ctas(fn, threads, smem, 0, &g);
+  *grid = items < g ? items : g;
+  return st;
 }
 
 // Launches the three passes when both mesh lengths have a fast shape; returns
@@ -526,57 +526,44 @@ int fast_fock(FockParams& p, cudaStream_t stream, bool* handled) {
   auto row = [&](auto shape) {
     using S = decltype(shape);
     constexpr size_t sm = fast_smem<S, FT>();
-    if (exch) {
-      cudaFuncSetAttribute(k_fast_row_fwd<ST, FT, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-      const int grid = persistent_grid(k_fast_row_fwd<ST, FT, S>, 16 * S::TPL, sm, p.ngroups * p.nk1);
-      k_fast_row_fwd<ST, FT, S><<<grid, 16 * S::TPL, sm, stream>>>(p);
-    }
+    if (!exch) return;
+    int grid = 0;
+    st = persistent_grid(k_fast_row_fwd<ST, FT, S>, 16 * S::TPL, sm, p.ngroups * p.nk1, &grid);
+    if (!st) k_fast_row_fwd<ST, FT, S><<<grid, 16 * S::TPL, sm, stream>>>(p);
+  };
+  auto pass = [&](auto kern, int threads, size_t sm, int items, const char* what) {
+    int grid = 0;
+    st = persistent_grid(kern, threads, sm, items, &grid);
+    if (st) return;
+    const cudaError_t e = launch_pass(kern, grid, threads, sm, stream, p);
+    if (e != cudaSuccess) st = cuda_check(e, what);
   };
   auto col = [&](auto shape) {
     using S = decltype(shape);
-    constexpr size_t sm = fast_smem<S, FT>();
     auto kern = (p.flags & HF_FOCK_VR_REAL) ? k_fast_col<ST, FT, S, true> : k_fast_col<ST, FT, S, false>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    const int grid = persistent_grid(kern, 16 * S::TPL, sm, p.ngroups * p.nk2);
-    const cudaError_t e = launch_pass(kern, grid, 16 * S::TPL, sm, stream, p);
-    if (e != cudaSuccess) st = cuda_check(e, "k_fast_col");
+    pass(kern, 16 * S::TPL, fast_smem<S, FT>(), p.ngroups * p.nk2, "k_fast_col");
   };
   auto inv = [&](auto shape) {
     using S = decltype(shape);
     if (p.rows_plan) {
       constexpr size_t sm = fast_smem_rows<S, ST, FT>();
       auto kern = k_fast_row_inv_rows<ST, FT, S>;
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-      cudaLaunchConfig_t cfg = {};
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = (unsigned)p.ngroups;
-      attr[0].val.clusterDim.y = 1;
-      attr[0].val.clusterDim.z = 1;
-      cfg.gridDim = dim3((unsigned)p.ngroups);
-      cfg.blockDim = dim3(16 * S::TPL);
-      cfg.dynamicSmemBytes = sm;
-      cfg.stream = stream;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      int ncl = 0;
-      if (cudaOccupancyMaxActiveClusters(&ncl, kern, &cfg) != cudaSuccess || ncl < 1) ncl = 1;
+      int ncl = 1;
+      if ((st = allow_max_dynamic_smem((const void*)kern))) return;
+      if ((st = resident_ctas((const void*)kern, 16 * S::TPL, sm, p.ngroups, &ncl))) return;
       if (ncl > p.nk1) ncl = p.nk1;
       const cudaError_t e = launch_pass(kern, ncl * p.ngroups, 16 * S::TPL, sm, stream, p, p.ngroups);
       if (e != cudaSuccess) st = cuda_check(e, "k_fast_row_inv_rows");
       return;
     }
-    constexpr size_t sm = fast_smem<S, FT>();
-    cudaFuncSetAttribute(k_fast_row_inv<ST, FT, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    const int grid = persistent_grid(k_fast_row_inv<ST, FT, S>, 16 * S::TPL, sm, p.ngroups * p.nk1);
-    const cudaError_t e = launch_pass(k_fast_row_inv<ST, FT, S>, grid, 16 * S::TPL, sm, stream, p);
-    if (e != cudaSuccess) st = cuda_check(e, "k_fast_row_inv");
+    pass(k_fast_row_inv<ST, FT, S>, 16 * S::TPL, fast_smem<S, FT>(), p.ngroups * p.nk1, "k_fast_row_inv");
   };
   switch (p.nk2) {
 #define HF_CASE(N, A, B, T) case N: row(LineShape<N, A, B, T>{}); break;
     HF_FAST_SHAPES(HF_CASE)
 #undef HF_CASE
   }
+  if (st) return st;
   HF_LAUNCH_CHECK("k_fast_row_fwd");
   if (exch) {
     switch (p.nk1) {
@@ -584,14 +571,13 @@ int fast_fock(FockParams& p, cudaStream_t stream, bool* handled) {
       HF_FAST_SHAPES(HF_CASE)
 #undef HF_CASE
     }
-    HF_LAUNCH_CHECK("k_fast_col");
+    if (st) return st;
   }
   switch (p.nk2) {
 #define HF_CASE(N, A, B, T) case N: inv(LineShape<N, A, B, T>{}); break;
     HF_FAST_SHAPES(HF_CASE)
 #undef HF_CASE
   }
-  HF_LAUNCH_CHECK("k_fast_row_inv");
   *handled = true;
   return st;
 }

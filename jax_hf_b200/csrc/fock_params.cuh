@@ -33,6 +33,7 @@ struct FockParams {
   double2* rho_part;  // [nk1][ngroups*LS]
   double2* sigc;      // [nb*nb] contact sigma
   double* hdiag;      // [nb] Hartree diagonal
+  int zero_h;         // the forward row pass zeroes Hout (a build without constant terms)
   const int* active;  // optional device flag: kernels return at once when *active == 0
   int rows_plan;      // slot groups are whole matrix rows; partner = (group << 8) | slot
   int two_row, two_col;  // factors N1 | N2 << 5 of nk2 and nk1 (two-factor passes)
@@ -43,6 +44,13 @@ struct FockParams {
   int16_t chan[kMaxSlotTable];
   int16_t partner[kMaxSlotTable];
 };
+
+// The first CTA of the forward row pass: H = 0 when nothing forms it (in place of a memset).
+template <typename SC>
+__device__ __forceinline__ void zero_h(const FockParams& p) {
+  if (!p.zero_h || blockIdx.x != 0 || blockIdx.y != 0) return;
+  for (int c = threadIdx.x; c < p.nb2; c += blockDim.x) static_cast<SC*>(p.Hout)[c] = mk<SC>(0.0, 0.0);
+}
 
 // Mesh lengths with a specialised register-FFT pass: N = N1 * N2 split over TPL
 // threads per line (see fft_reg.cuh).

@@ -73,6 +73,7 @@ __global__ void __launch_bounds__(16 * kTwoRadix, 2) k_two_row_fwd(const __grid_
   pdl_launch_dependents();
   using SC = cpx_t<ST>;
   using FC = cpx_t<FT>;
+  zero_h<SC>(p);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   FC* tw = reinterpret_cast<FC*>(smem_raw);
   const int N = p.nk2, LS = p.LS;
@@ -299,8 +300,8 @@ int two_fock(FockParams& p, cudaStream_t stream, bool* handled) {
   auto threads = [](int f) { return 16 * ((f & 31) > (f >> 5) ? (f & 31) : (f >> 5)); };
   auto smem = [](int n) { return (size_t)17 * n * sizeof(cpx_t<FT>); };  // twiddles and 16 lines
   auto pass = [&](auto kern, int f, int n, int items, const char* what) -> int {
-    HF_SMEM_CAP(kern);
-    const int grid = persistent_grid(kern, threads(f), smem(n), items);
+    int grid = 0;
+    if (int e = persistent_grid(kern, threads(f), smem(n), items, &grid)) return e;
     const cudaError_t e = launch_pass(kern, grid, threads(f), smem(n), stream, p);
     return e == cudaSuccess ? HF_OK : cuda_check(e, what);
   };
@@ -308,8 +309,8 @@ int two_fock(FockParams& p, cudaStream_t stream, bool* handled) {
   if (exch) {
     // a plain launch: with programmatic serialisation this pass could overwrite the scratch
     // while an earlier build on the stream still reads it
-    HF_SMEM_CAP(k_two_row_fwd<ST, FT>);
-    const int grid = persistent_grid(k_two_row_fwd<ST, FT>, threads(fr), smem(p.nk2), p.ngroups * p.nk1);
+    int grid = 0;
+    if ((st = persistent_grid(k_two_row_fwd<ST, FT>, threads(fr), smem(p.nk2), p.ngroups * p.nk1, &grid))) return st;
     k_two_row_fwd<ST, FT><<<grid, threads(fr), smem(p.nk2), stream>>>(p);
     HF_LAUNCH_CHECK("k_two_row_fwd");
     if (p.flags & HF_FOCK_VR_REAL) st = pass(k_two_col<ST, FT, true>, fc, p.nk1, p.ngroups * p.nk2, "k_two_col");

@@ -37,6 +37,8 @@ from .problem import is_marked_zero
 def _as_dev(x, device=None, dtype=None):
     if isinstance(x, torch.Tensor):
         t = x
+        if (t.dtype is dtype or dtype is None) and (device is None or t.device == device):
+            return t if t.is_contiguous() else t.contiguous()
         if device is not None and t.device != device:
             t = t.to(device)
     else:
@@ -64,6 +66,7 @@ def _real_of(dt: torch.dtype) -> torch.dtype:
 
 
 _block_ws: dict = {}  # workspace sizes of block-spec builds, per (dtype, flags, shape, masks)
+_plain_ws: dict = {}  # workspace sizes of plain builds, per (dtype, flags, nk1, nk2, nb)
 
 
 def build_fock(P, *, h, VR, refP, HH, w2d, include_exchange: bool, include_hartree: bool,
@@ -113,18 +116,18 @@ def build_fock(P, *, h, VR, refP, HH, w2d, include_exchange: bool, include_hartr
     VRt = None
     if include_exchange:
         VRt = VR if isinstance(VR, torch.Tensor) else torch.as_tensor(np.asarray(VR))
-        VRt = VRt.to(dev)
         if VRt.is_complex():
-            VRt = VRt.to(cdt).contiguous()
+            VRt = _as_dev(VRt, dev, cdt)
         else:
-            VRt = VRt.to(rdt).contiguous()
+            VRt = _as_dev(VRt, dev, rdt)
             flags |= _lib.FOCK_VR_REAL
-        if tuple(VRt.shape[-2:]) == (1, 1):
+        vshape = tuple(VRt.shape[-2:])
+        if vshape == (1, 1):
             flags |= _lib.FOCK_VR_SCALAR
-        elif tuple(VRt.shape[-2:]) != (nb, nb):
+        elif vshape != (nb, nb):
             raise ValueError(f"VR must have shape (nk1, nk2, 1, 1) or (nk1, nk2, nb, nb), got {tuple(VRt.shape)}")
     if exchange_hermitian_channel_packing:
-        if VRt is not None and tuple(VRt.shape[-2:]) != (1, 1):
+        if VRt is not None and vshape != (1, 1):
             raise ValueError("hermitian_channel_packing requires a scalar interaction kernel with shape (..., 1, 1).")
         flags |= _lib.FOCK_PACKING
     elif hermitian_density and include_exchange and sym_v and exchange_block_specs is None:
@@ -161,7 +164,8 @@ def build_fock(P, *, h, VR, refP, HH, w2d, include_exchange: bool, include_hartr
         F = torch.empty_like(P)
         H = torch.empty((1, 1, nb, nb), dtype=cdt, device=dev)
     dt = _lib.dtype_code(P)
-    need = _lib.C.c_size_t(0)
+    if _inblock is not None:
+        need = _lib.C.c_size_t(0)
     if _inblock is not None and _spec_check is not None:
         masks = np.ascontiguousarray(np.asarray(_inblock, dtype=np.uint8).reshape(-1, nb, nb))
         mptr = masks.ctypes.data_as(_lib.C.c_void_p)
@@ -195,9 +199,17 @@ def build_fock(P, *, h, VR, refP, HH, w2d, include_exchange: bool, include_hartr
         if project_fn is not None:
             F = _herm(torch.as_tensor(project_fn(F)).to(cdt))
         return Sigma, H, F
-    _lib.check(_lib.lib().hf_fock_workspace_size(dt, flags, nk1, nk2, nb, _lib.C.byref(need)))
-    ws = _lib.workspace(need.value, dev, "fock")
-    args = (_lib.stream_ptr(dev), dt, flags, nk1, nk2, nb, P.data_ptr(), h.data_ptr(), _lib.ptr(VRt),
+    key = (dt, flags, nk1, nk2, nb)
+    nbytes = _plain_ws.get(key)
+    if nbytes is None:
+        need = _lib.C.c_size_t(0)
+        _lib.check(_lib.lib().hf_fock_workspace_size(dt, flags, nk1, nk2, nb, _lib.C.byref(need)))
+        if len(_plain_ws) >= 4096:
+            _plain_ws.clear()
+        nbytes = _plain_ws[key] = int(need.value)
+    stream = _lib.stream_ptr(dev)
+    ws = _lib.workspace(nbytes, dev, "fock", stream)
+    args = (stream, dt, flags, nk1, nk2, nb, P.data_ptr(), h.data_ptr(), _lib.ptr(VRt),
             _lib.ptr(refPt), _lib.ptr(HHt), _lib.ptr(w2dt), n_contact, _lib.ptr(cg), _lib.ptr(cOi),
             _lib.ptr(cOj), Sigma.data_ptr(), H.data_ptr(), F.data_ptr(), ws.data_ptr(), ws.numel())
     if autotune:
@@ -268,10 +280,16 @@ def build_fock_batch(Ps, *, h, VR, refP, HH, w2d, include_exchange: bool, includ
     return results
 
 
-def _reduce_ws(dev):
-    need = _lib.C.c_size_t(0)
-    _lib.check(_lib.lib().hf_reduce_workspace_size(1, 1, 1, _lib.C.byref(need)))
-    return _lib.workspace(need.value, dev, "reduce")
+_reduce_bytes = None  # workspace of the objective reductions (the same for every shape)
+
+
+def _reduce_ws(dev, stream):
+    global _reduce_bytes
+    if _reduce_bytes is None:
+        need = _lib.C.c_size_t(0)
+        _lib.check(_lib.lib().hf_reduce_workspace_size(1, 1, 1, _lib.C.byref(need)))
+        _reduce_bytes = int(need.value)
+    return _lib.workspace(_reduce_bytes, dev, "reduce", stream)
 
 
 def hf_energy(P, *, h, Sigma, H, weights_b, out=None):
@@ -294,8 +312,9 @@ def hf_energy(P, *, h, Sigma, H, weights_b, out=None):
             H_mode = 2
     w = _as_dev(weights_b, dev, _real_of(cdt)).reshape(nk1, nk2).contiguous()
     E = out if out is not None else torch.empty((), dtype=torch.float64, device=dev)
-    ws = _reduce_ws(dev)
-    _lib.check(_lib.lib().hf_energy(_lib.stream_ptr(dev), _lib.dtype_code(P), nk1, nk2, nb, P.data_ptr(),
+    stream = _lib.stream_ptr(dev)
+    ws = _reduce_ws(dev, stream)
+    _lib.check(_lib.lib().hf_energy(stream, _lib.dtype_code(P), nk1, nk2, nb, P.data_ptr(),
                                     h.data_ptr(), Sigma.data_ptr(), _lib.ptr(Ht), H_mode, w.data_ptr(),
                                     E.data_ptr(), ws.data_ptr(), ws.numel()))
     return E
@@ -309,8 +328,9 @@ def occupation_entropy(p, w_norm, out=None):
     nb = int(p.shape[-1])
     nk = p.numel() // nb
     S = out if out is not None else torch.empty((), dtype=torch.float64, device=dev)
-    ws = _reduce_ws(dev)
-    _lib.check(_lib.lib().hf_occupation_entropy(_lib.stream_ptr(dev), _lib.dtype_code(p), nk, 1, nb,
+    stream = _lib.stream_ptr(dev)
+    ws = _reduce_ws(dev, stream)
+    _lib.check(_lib.lib().hf_occupation_entropy(stream, _lib.dtype_code(p), nk, 1, nb,
                                                 p.data_ptr(), w.data_ptr(), S.data_ptr(), ws.data_ptr(),
                                                 ws.numel()))
     return S
@@ -326,8 +346,9 @@ def free_energy(E, p, w_norm, T, out=None):
     Et = E if isinstance(E, torch.Tensor) else torch.tensor(float(E), dtype=torch.float64, device=dev)
     Et = Et.to(dev, torch.float64).reshape(()).contiguous()
     Om = out if out is not None else torch.empty((), dtype=torch.float64, device=dev)
-    ws = _reduce_ws(dev)
-    _lib.check(_lib.lib().hf_free_energy(_lib.stream_ptr(dev), _lib.dtype_code(p), nk, 1, nb, Et.data_ptr(),
+    stream = _lib.stream_ptr(dev)
+    ws = _reduce_ws(dev, stream)
+    _lib.check(_lib.lib().hf_free_energy(stream, _lib.dtype_code(p), nk, 1, nb, Et.data_ptr(),
                                          p.data_ptr(), w.data_ptr(), float(T), Om.data_ptr(), ws.data_ptr(),
                                          ws.numel()))
     return Om
