@@ -529,9 +529,9 @@ static int make_plan(int dtype, unsigned flags, int nk1, int nk2, int nb, SlotPl
   }
   // 16 slots for the register and two-factor passes, up to 32 for the Stockham stages
   const bool fast = fast_length(nk1) && fast_length(nk2);
-  if (!fast && !(flags & (HF_FOCK_GENERIC_FFT | HF_FOCK_NO_TWO_FACTOR)) && two_factors(nk1) && two_factors(nk2) &&
+  if (!fast && !(flags & (HF_FOCK_GENERIC_FFT | HF_FOCK_NO_TWO_FACTOR)) && line_factors(nk1) && line_factors(nk2) &&
       plan_slots(nb, packing, 1, fft_elem(dtype, flags), 16, sp, inb) == HF_OK)
-    return HF_OK;  // their shared memory (17 lines) fits for every side, so the plan only looks at the padding
+    return HF_OK;  // their shared memory fits for every side, so the plan only looks at the padding
   const int max_ls = fast ? 16 : 32;
   int st = plan_slots(nb, packing, std::max(nk1, nk2), fft_elem(dtype, flags), max_ls, sp, inb);
   if (st != HF_OK) return fail(st, "mesh too large for the shared-memory FFT (nk1, nk2 <= 768 in complex128)");

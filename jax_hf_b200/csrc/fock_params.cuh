@@ -37,6 +37,7 @@ struct FockParams {
   const int* active;  // optional device flag: kernels return at once when *active == 0
   int rows_plan;      // slot groups are whole matrix rows; partner = (group << 8) | slot
   int two_row, two_col;  // factors N1 | N2 << 5 of nk2 and nk1 (two-factor passes)
+  int dense_row, dense_col;  // output pairs per walk where N2 is a direct sum
   int pipe_ns;        // stages of the pipelined passes (set per launch)
   int* fault;         // device word: a bounded wait of a pipelined pass that ran out records a code here
   CUtensorMap tmap_row;  // pipelined row pass: P as [nk1 nk2][nb^2] 4-byte words, box = SL channels x nk2 k-points
@@ -78,11 +79,23 @@ inline bool fast_length(int n) {
   }
 }
 
-// Factors N1 <= N2 <= 16 of a mesh side as N1 | N2 << 5, the pair nearest to square; 0 when
-// there is none.  Sides the two-factor passes (fock_two.cuh) transform.
-inline int two_factors(int n) {
+// Factors of a mesh side as N1 | N2 << 5 for the two-factor passes, 0 when they leave the side
+// to the Stockham stages: N1 <= N2 <= 16, the pair nearest to square (fock_two.cuh); else, for
+// a side with a prime factor of 17 or more, the largest N1 <= 16 that keeps it in N2 <= 224
+// (fock_dense.cuh; the Stockham stages would take that prime by a direct sum as well).
+inline int line_factors(int n) {
   for (int a = 16; a >= 1; --a)
-    if (a * a <= n && n % a == 0) return n / a <= 16 ? a | (n / a) << 5 : 0;
+    if (a * a <= n && n % a == 0) {
+      if (n / a <= 16) return a | (n / a) << 5;
+      break;
+    }
+  int prime = 1, m = n;
+  for (int d = 2; d * d <= m; ++d)
+    while (m % d == 0) { prime = d; m /= d; }
+  if (m > 1) prime = m;
+  if (prime < 17) return 0;
+  for (int a = 16; a >= 1; --a)
+    if (n % a == 0 && (n / a) % prime == 0) return n / a <= 224 && n <= 430 ? a | (n / a) << 5 : 0;
   return 0;
 }
 

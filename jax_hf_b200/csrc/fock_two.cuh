@@ -200,26 +200,83 @@ __global__ void __launch_bounds__(16 * kTwoRadix, 2) k_two_col(const __grid_cons
   }
 }
 
+// Column t of an inverse row (N1 points at t, t + N2, ... in buf): the last register IDFT and
+// the outputs of its k-points (contact sigma, Hartree diagonal, herm with the transposed
+// channel, + h).  The 16 slot lanes of a line part call it together.
+template <typename ST, typename FT>
+__device__ __forceinline__ void two_epilogue(const FockParams& p, const cpx_t<FT>* buf, bool exch, int g, int k1,
+                                             int t, int s, int N1, int N2) {
+  using SC = cpx_t<ST>;
+  using FC = cpx_t<FT>;
+  const int LS = p.LS, nb = p.nb;
+  const unsigned half = 0xffffu << (threadIdx.x & 16);  // these 16 lanes
+  const bool packing = (p.flags & HF_FOCK_PACKING) != 0;
+  const int c = s < LS ? p.chan[g * LS + s] : -1, pl = s < LS ? p.partner[g * LS + s] : s;
+  const int a = c >= 0 ? c / nb : 0, b = c >= 0 ? c - a * nb : 0, cab = a * nb + b, cba = b * nb + a;
+  const size_t at = ((size_t)k1 * N1 * N2 + t) * p.nb2, st = (size_t)N2 * p.nb2;
+  const SC* h = static_cast<const SC*>(p.h) + at;
+  SC* Sg = static_cast<SC*>(p.Sigma) + at;
+  SC* F = static_cast<SC*>(p.F) + at;
+  SC zab = mk<SC>(0.0, 0.0), zba = mk<SC>(0.0, 0.0);
+  double hd = 0.0;
+  if (p.sigc != nullptr && c >= 0) {
+    zab = cvt<SC>(p.sigc[cab]);
+    zba = cvt<SC>(p.sigc[cba]);
+    if (a == b) hd = p.hdiag[a];
+  }
+  two_switch(N1, [&](auto rc) {
+    constexpr int R = decltype(rc)::value;
+    SC hv[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) hv[i] = c >= 0 ? ld_stream(h + i * st + cab) : mk<SC>(0.0, 0.0);
+    FC x[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) x[i] = exch ? buf[((size_t)i * N2 + t) * 16 + s] : mk<FC>(0.0, 0.0);
+    if (exch) two_dft<R, true>(x);
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      SC sab = cvt<SC>(x[i]), sba, hba;
+      if (packing) {
+        sba = a == b ? sab : conj(sab);
+        hba = c >= 0 ? ld_stream(h + i * st + cba) : mk<SC>(0.0, 0.0);
+      } else {  // the transposed channel is another slot lane of the same k-point
+        sba.x = __shfl_sync(half, sab.x, pl, 16);
+        sba.y = __shfl_sync(half, sab.y, pl, 16);
+        hba.x = __shfl_sync(half, hv[i].x, pl, 16);
+        hba.y = __shfl_sync(half, hv[i].y, pl, 16);
+      }
+      if (c < 0) continue;
+      sab = cadd(sab, zab);
+      sba = cadd(sba, zba);
+      SC f = mk<SC>(0.5 * ((double)hv[i].x + (double)hba.x) + 0.5 * ((double)sab.x + (double)sba.x),
+                    0.5 * ((double)hv[i].y - (double)hba.y) + 0.5 * ((double)sab.y - (double)sba.y));
+      f.x += (ST)hd;
+      st_stream(Sg + i * st + cab, sab);
+      st_stream(F + i * st + cab, f);
+      if (packing && a != b) {
+        st_stream(Sg + i * st + cba, sba);
+        st_stream(F + i * st + cba, conj(f));
+      }
+    }
+  });
+}
+
 template <typename ST, typename FT>
 __global__ void __launch_bounds__(16 * kTwoRadix, 2) k_two_row_inv(const __grid_constant__ FockParams p) {
-  using SC = cpx_t<ST>;
   using FC = cpx_t<FT>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   FC* tw = reinterpret_cast<FC*>(smem_raw);
-  const int N = p.nk2, LS = p.LS, nb = p.nb;
+  const int N = p.nk2, LS = p.LS;
   FC* buf = tw + N;
   const int s = threadIdx.x & 15;
   const bool exch = (p.flags & HF_FOCK_EXCHANGE) != 0;
-  const bool packing = (p.flags & HF_FOCK_PACKING) != 0;
   if (exch) build_twiddles<FT>(tw, N);
   pdl_wait();  // the column pass has finished writing the scratch
   if (p.active && !*p.active) return;
   __syncthreads();
-  const unsigned half = 0xffffu << (threadIdx.x & 16);  // the 16 slot lanes of this line part
   for (int item = blockIdx.x; item < p.ngroups * p.nk1; item += gridDim.x) {
     const int t = in_loop(threadIdx.x >> 4), N1 = in_loop(p.two_row & 31), N2 = in_loop(p.two_row >> 5);
     const int g = item % p.ngroups, k1 = item / p.ngroups;
-    const int c = s < LS ? p.chan[g * LS + s] : -1;
     if (exch) {
       if (t < N1) {
         const FC* row = static_cast<const FC*>(p.scratch) + (((size_t)g * p.nk1 + k1) * N + t) * LS + (s < LS ? s : 0);
@@ -234,92 +291,9 @@ __global__ void __launch_bounds__(16 * kTwoRadix, 2) k_two_row_inv(const __grid_
       }
       __syncthreads();
     }
-    if (t < N2) {
-      const int pl = s < LS ? p.partner[g * LS + s] : s;
-      const int a = c >= 0 ? c / nb : 0, b = c >= 0 ? c - a * nb : 0, cab = a * nb + b, cba = b * nb + a;
-      const size_t at = ((size_t)k1 * N + t) * p.nb2, st = (size_t)N2 * p.nb2;
-      const SC* h = static_cast<const SC*>(p.h) + at;
-      SC* Sg = static_cast<SC*>(p.Sigma) + at;
-      SC* F = static_cast<SC*>(p.F) + at;
-      SC zab = mk<SC>(0.0, 0.0), zba = mk<SC>(0.0, 0.0);
-      double hd = 0.0;
-      if (p.sigc != nullptr && c >= 0) {
-        zab = cvt<SC>(p.sigc[cab]);
-        zba = cvt<SC>(p.sigc[cba]);
-        if (a == b) hd = p.hdiag[a];
-      }
-      two_switch(N1, [&](auto rc) {
-        constexpr int R = decltype(rc)::value;
-        SC hv[R];
-#pragma unroll
-        for (int i = 0; i < R; ++i) hv[i] = c >= 0 ? ld_stream(h + i * st + cab) : mk<SC>(0.0, 0.0);
-        FC x[R];
-#pragma unroll
-        for (int i = 0; i < R; ++i) x[i] = exch ? buf[(i * N2 + t) * 16 + s] : mk<FC>(0.0, 0.0);
-        if (exch) two_dft<R, true>(x);
-#pragma unroll
-        for (int i = 0; i < R; ++i) {
-          SC sab = cvt<SC>(x[i]), sba, hba;
-          if (packing) {
-            sba = a == b ? sab : conj(sab);
-            hba = c >= 0 ? ld_stream(h + i * st + cba) : mk<SC>(0.0, 0.0);
-          } else {  // the transposed channel is another slot lane of the same k-point
-            sba.x = __shfl_sync(half, sab.x, pl, 16);
-            sba.y = __shfl_sync(half, sab.y, pl, 16);
-            hba.x = __shfl_sync(half, hv[i].x, pl, 16);
-            hba.y = __shfl_sync(half, hv[i].y, pl, 16);
-          }
-          if (c < 0) continue;
-          sab = cadd(sab, zab);
-          sba = cadd(sba, zba);
-          SC f = mk<SC>(0.5 * ((double)hv[i].x + (double)hba.x) + 0.5 * ((double)sab.x + (double)sba.x),
-                        0.5 * ((double)hv[i].y - (double)hba.y) + 0.5 * ((double)sab.y - (double)sba.y));
-          f.x += (ST)hd;
-          st_stream(Sg + i * st + cab, sab);
-          st_stream(F + i * st + cab, f);
-          if (packing && a != b) {
-            st_stream(Sg + i * st + cba, sba);
-            st_stream(F + i * st + cba, conj(f));
-          }
-        }
-      });
-    }
+    if (t < N2) two_epilogue<ST, FT>(p, buf, exch, g, k1, t, s, N1, N2);
     __syncthreads();  // buf is rewritten by the next item
   }
-}
-
-// Launches the three passes when both sides have two factors of at most 16; sets *handled.
-template <typename ST, typename FT>
-int two_fock(FockParams& p, cudaStream_t stream, bool* handled) {
-  *handled = false;
-  const int fr = two_factors(p.nk2), fc = two_factors(p.nk1);
-  if (p.LS > 16 || p.rows_plan || !fr || !fc) return HF_OK;
-  p.two_row = fr;
-  p.two_col = fc;
-  const bool exch = (p.flags & HF_FOCK_EXCHANGE) != 0;
-  auto threads = [](int f) { return 16 * ((f & 31) > (f >> 5) ? (f & 31) : (f >> 5)); };
-  auto smem = [](int n) { return (size_t)17 * n * sizeof(cpx_t<FT>); };  // twiddles and 16 lines
-  auto pass = [&](auto kern, int f, int n, int items, const char* what) -> int {
-    int grid = 0;
-    if (int e = persistent_grid(kern, threads(f), smem(n), items, &grid)) return e;
-    const cudaError_t e = launch_pass(kern, grid, threads(f), smem(n), stream, p);
-    return e == cudaSuccess ? HF_OK : cuda_check(e, what);
-  };
-  int st;
-  if (exch) {
-    // a plain launch: with programmatic serialisation this pass could overwrite the scratch
-    // while an earlier build on the stream still reads it
-    int grid = 0;
-    if ((st = persistent_grid(k_two_row_fwd<ST, FT>, threads(fr), smem(p.nk2), p.ngroups * p.nk1, &grid))) return st;
-    k_two_row_fwd<ST, FT><<<grid, threads(fr), smem(p.nk2), stream>>>(p);
-    HF_LAUNCH_CHECK("k_two_row_fwd");
-    if (p.flags & HF_FOCK_VR_REAL) st = pass(k_two_col<ST, FT, true>, fc, p.nk1, p.ngroups * p.nk2, "k_two_col");
-    else st = pass(k_two_col<ST, FT, false>, fc, p.nk1, p.ngroups * p.nk2, "k_two_col");
-    if (st) return st;
-  }
-  if ((st = pass(k_two_row_inv<ST, FT>, fr, p.nk2, p.ngroups * p.nk1, "k_two_row_inv"))) return st;
-  *handled = true;
-  return HF_OK;
 }
 
 }  // namespace hf

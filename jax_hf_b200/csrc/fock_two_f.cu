@@ -1,4 +1,4 @@
-#include "fock_two.cuh"
+#include "fock_two_launch.cuh"
 
 namespace hf {
 // complex64 storage, FP32 transform

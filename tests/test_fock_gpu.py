@@ -544,3 +544,16 @@ def test_two_factor_passes_match_stockham(cuda, n1, n2, nb, V, mode, terms):
         assert rel(x, y.cpu().numpy()) < tol if y.abs().max() > 0 else torch.equal(x, y)
     for x, y in zip(run(engine="stockham"), run(engine="generic")):
         assert torch.equal(x, y)
+
+
+DENSE = [  # sides with a prime factor of 17 or more: one row, several rows, an even N2, both sides, the largest
+    (17, 17, 3, "layer", "c128"), (34, 37, 8, "layer", "c128"), (61, 24, 4, "scalar", "c64"),
+    (191, 3, 2, "layer", "c128"), (74, 19, 6, "layer", "fp32fft"), (12, 97, 8, "layer", "c128"),
+    (306, 4, 1, "layer", "c128"), (5, 430, 2, "scalar", "c128"), (23, 29, 16, "scalar", "c128"),
+]
+
+
+@pytest.mark.parametrize("n1,n2,nb,V,mode", DENSE)
+@pytest.mark.parametrize("terms", [False, True])
+def test_dense_line_sums_match_stockham(cuda, n1, n2, nb, V, mode, terms):
+    test_two_factor_passes_match_stockham(cuda, n1, n2, nb, V, mode, terms)
