@@ -271,6 +271,14 @@ int hf_free_energy(void* stream, int dtype, int nk1, int nk2, int nb, const doub
 int hf_find_mu(void* stream, int dtype, int method, int nk1, int nk2, int nb, const void* eps,
                const void* weights, double n_electrons, double T, int maxiter, const double* mu0,
                double* mu_out);
+/* The same with a workspace (hf_mu_workspace_size bytes, 256-byte aligned): from some ten
+ * thousand eigenvalues on, the bisection without a hint and the warm-started Newton rule run
+ * their evaluations over the whole device instead of one cluster.  The bisection's result is
+ * bit-identical to hf_find_mu's. */
+int hf_mu_workspace_size(size_t* bytes);
+int hf_find_mu_ws(void* stream, int dtype, int method, int nk1, int nk2, int nb, const void* eps,
+                  const void* weights, double n_electrons, double T, int maxiter, const double* mu0,
+                  double* mu_out, void* workspace, size_t workspace_bytes);
 
 /* ---- Per-k small matrices (one warp per k-point) ------------------------------
  * batch = number of nb x nb matrices (nk1*nk2 for mesh arrays).

@@ -69,6 +69,8 @@ _SIGS = {
     "hf_occupation_entropy": ([vp, i32, i32, i32, i32, vp, vp, vp, vp, sz], i32),
     "hf_free_energy": ([vp, i32, i32, i32, i32, vp, vp, vp, f64, vp, vp, sz], i32),
     "hf_find_mu": ([vp, i32, i32, i32, i32, i32, vp, vp, f64, f64, i32, vp, vp], i32),
+    "hf_mu_workspace_size": ([psz], i32),
+    "hf_find_mu_ws": ([vp, i32, i32, i32, i32, i32, vp, vp, f64, f64, i32, vp, vp, vp, sz], i32),
     "hf_density_from_Qp": ([vp, i32, i32, i32, vp, vp, vp], i32),
     "hf_fock_orbital": ([vp, i32, i32, i32, vp, vp, vp], i32),
     "hf_eigh": ([vp, i32, i32, i32, vp, vp, vp], i32),

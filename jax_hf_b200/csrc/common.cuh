@@ -111,6 +111,22 @@ __device__ __forceinline__ double2 cfma_c(double2 a, double2 b, double2 acc) {
   return acc;
 }
 
+// 1 / sqrt(x) and 1 / x for serial chains, for arguments well inside the range of normal
+// numbers: the hardware's approximate seed and one step of third order
+// (Householder's iteration), four and three dependent FP64 operations, errors of about
+// one ulp.
+__device__ __forceinline__ double rsqrt_seeded(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x * y, y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
+__device__ __forceinline__ double recip_seeded(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
 template <typename To, typename From> __device__ __forceinline__ To cvt(From a) {
   To r; r.x = a.x; r.y = a.y; return r;
 }

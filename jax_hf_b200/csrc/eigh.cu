@@ -31,22 +31,6 @@ namespace {
 
 constexpr double kHalfUlp = 0x1p-53;
 
-// 1 / sqrt(x) and 1 / x for the serial chains, for arguments well inside the range (here
-// at least 1e-36): the hardware's approximate seed and one step of third order
-// (Householder's iteration), four and three dependent FP64 operations, errors of about
-// one ulp.
-__device__ __forceinline__ double rsqrt_seeded(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x * y, y, 1.0);
-  return fma(y * e, fma(0.375, e, 0.5), y);
-}
-__device__ __forceinline__ double recip_seeded(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x, y, 1.0);
-  return fma(y, fma(e, e, e), y);
-}
 constexpr double kTiny2 = 1e-36;  // squares below this are zero next to entries of order one
 
 template <int NB>

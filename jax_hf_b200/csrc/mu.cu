@@ -49,6 +49,17 @@ struct MuArgs {
   double* out;
   const int* active;  // optional device flag: return at once when *active == 0
   int cache;          // elements per thread kept in shared memory as (eps, w); 0: read from L2
+  int kpt;                    // eigenvalues per thread of the cluster kernel
+  const struct MuState* pre;  // what the grid-wide passes found, or nullptr
+};
+
+// Root-find state of the grid-wide passes (device memory, in the caller's workspace).
+struct MuState {
+  unsigned counter;  // CTAs of the running pass that have published; zero between passes
+  int done, it;
+  double lo, hi, mu;        // method 2: bracket and iterate
+  double mn, mx, W;         // extreme eigenvalues, total weight
+  double A, B, m, d;        // bisection: certified bracket, next iterate and probe offset
 };
 // loads in flight per thread when the elements are read from L2
 constexpr int kMuCacheU = 4;
@@ -224,6 +235,282 @@ __device__ __forceinline__ double div_by(double x, double b, double rb) {
   return fma(r, rb, q);
 }
 
+// Twice the error bound of two evaluations of N with ka and kb terms summed per thread (the
+// sum below twice the evaluation's rounding error, see the certified bracket below), with
+// 25% to spare: evaluations by different kernels may be compared with each other.
+__device__ __forceinline__ double cert_margin(int ka, int kb, double W) {
+  return 1.25 * ((double)ka + (double)kb + 60.0) * 1.1102230246251565e-16 * W;
+}
+
+// One step of the Newton-bracket rule (solver.py:62-101) from g = N(mu) - target and
+// Z = N'(mu); true once the accepted Newton step is below 4 ulp of mu.
+__device__ __forceinline__ bool newton_step(double g, double Z, double& lo, double& hi, double& mu) {
+  if (g < 0) lo = mu;
+  if (g > 0) hi = mu;
+  double mn2 = mu - g / fmax(Z, 1e-18);
+  const double mb = 0.5 * (lo + hi);
+  bool newton = true;
+  if (mn2 <= lo || mn2 >= hi) { mn2 = mb; newton = false; }
+  mn2 = fmin(fmax(mn2, lo), hi);
+  if (!isfinite(mn2)) { mn2 = mb; newton = false; }
+  const double step = fabs(mn2 - mu);
+  mu = mn2;
+  return newton && step <= 4.0 * 2.220446049250313e-16 * fmax(1.0, fabs(mu));
+}
+
+// ------------------------------------------------------------ grid-wide passes ---
+// The cluster kernel below has 16 SMs: from a few ten thousand eigenvalues on it is bound
+// by their FP64 pipes (one exp and one division per eigenvalue and evaluation).  These
+// passes run one evaluation each over the whole grid; the last CTA to publish its sums
+// (atomic ticket, no spin) takes the step, and the cluster kernel finishes from MuState.
+// Every pass returns at once when the state says done.  The bisection's passes certify a
+// bracket (see the hinted bisection below); only the levels inside it are left to evaluate.
+// 144 x 144, nb = 8 (166k eigenvalues): the bisection of the cluster kernel alone takes 353 us.
+constexpr int kPassThreads = 256;
+constexpr int kPassBlocks = 296;   // two CTAs per SM
+constexpr int kPassSums = 8;
+constexpr int kGridMin = 16384;    // eigenvalues from which the passes are used
+constexpr int kNewtonPasses = 5;   // method 2: Newton steps queued ahead of the cluster kernel
+constexpr int kCertPasses = 7;     // bisection: certifying passes, the first one a scan of 8 points
+constexpr size_t kMuWsBytes = 256 + sizeof(double) * kPassBlocks * kPassSums;  // also 4 per warp of k_mu_newton
+static_assert(kPassBlocks * kPassSums >= 4 * 32 * kMuMaxCluster, "workspace of k_mu_newton");
+
+enum MuStage { kStageRange, kStageScan, kStageCertify };
+
+template <typename RT, int STAGE>
+__global__ void __launch_bounds__(kPassThreads) k_mu_pass(const MuArgs a, MuState* st, double* part) {
+  if (a.active && !*a.active) return;
+  if (STAGE != kStageRange && st->done) return;
+  constexpr int K = STAGE == kStageRange ? 3 : STAGE == kStageScan ? 8 : 5;
+  __shared__ double red[(kPassThreads / 32) * K];
+  __shared__ bool last;
+  const int gt = blockIdx.x * blockDim.x + threadIdx.x, gs = gridDim.x * blockDim.x;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const double Td = a.T + 1e-12;
+  double v[K];
+#pragma unroll
+  for (int j = 0; j < K; ++j) v[j] = 0.0;
+  auto fermi = [](double x) { return recip_seeded(1.0 + exp(fmin(x, 600.0))); };
+  if constexpr (STAGE == kStageRange) {  // extremes and total weight
+    v[0] = INFINITY;
+    v[1] = -INFINITY;
+    for_each_eps<RT, kMuCacheU>(a, gt, gs, [&](double e, double w) {
+      v[0] = fmin(v[0], e);
+      v[1] = fmax(v[1], e);
+      v[2] += w;
+    });
+  } else if constexpr (STAGE == kStageScan) {  // N at 8 points inside [mn, mx]
+    const double r = 1.0 / Td, m0 = st->mn, h = (st->mx - st->mn) * (1.0 / 9.0);
+    for_each_eps<RT, kMuCacheU>(a, gt, gs, [&](double e, double w) {
+#pragma unroll
+      for (int j = 0; j < K; ++j) v[j] += w * fermi((e - fma(j + 1.0, h, m0)) * r);
+    });
+  } else {
+    const double r = 1.0 / Td, m = st->m, pl = m - st->d, ph = m + st->d;
+    for_each_eps<RT, kMuCacheU>(a, gt, gs, [&](double e, double w) {
+      const double f = fermi((e - m) * r);
+      v[0] += w * f;
+      v[1] += w * (f * (1.0 - f));
+      v[2] += w * fermi((e - pl) * r);
+      v[3] += w * fermi((e - ph) * r);
+      v[4] += w;
+    });
+  }
+  // block, then grid: fixed trees, so the sums do not depend on the order of arrival
+  auto combine = [](int j, double x, double y) {
+    return STAGE == kStageRange && j == 0 ? fmin(x, y) : STAGE == kStageRange && j == 1 ? fmax(x, y) : x + y;
+  };
+  auto block_all = [&]() {  // v: the block's values in thread 0
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      for (int off = 16; off > 0; off >>= 1) v[j] = combine(j, v[j], __shfl_xor_sync(0xffffffffu, v[j], off));
+      if (lane == 0) red[wid * K + j] = v[j];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+      for (int j = 0; j < K; ++j) {
+        double t = red[j];
+#pragma unroll
+        for (int q = 1; q < kPassThreads / 32; ++q) t = combine(j, t, red[q * K + j]);
+        v[j] = t;
+      }
+    }
+  };
+  block_all();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int j = 0; j < K; ++j) part[blockIdx.x * K + j] = v[j];
+    __threadfence();
+    last = atomicAdd(&st->counter, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+#pragma unroll
+  for (int j = 0; j < K; ++j) v[j] = STAGE == kStageRange && j < 2 ? (j ? -INFINITY : INFINITY) : 0.0;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += kPassThreads)
+#pragma unroll
+    for (int j = 0; j < K; ++j) v[j] = combine(j, v[j], __ldcg(part + b * K + j));
+  block_all();
+  if (threadIdx.x != 0) return;
+  st->counter = 0u;
+  if constexpr (STAGE == kStageRange) {
+    const double mn = v[0], mx = v[1];
+    st->mn = mn;
+    st->mx = mx;
+    st->W = v[2];
+    st->done = 0;
+    st->A = INFINITY;
+    st->B = -INFINITY;
+    st->m = 0.5 * (mn + mx);
+    st->d = 0.0;
+  } else {
+    const int gk = (a.n + gs - 1) / gs;
+    const double margin = cert_margin(gk, a.kpt, st->W);
+    double A = st->A, B = st->B;
+    auto note = [&](double x, double n) {
+      if (n > a.target + margin) A = fmin(A, x);
+      if (n < a.target - margin) B = fmax(B, x);
+    };
+    double r = 0.0, d = 0.0;
+    if constexpr (STAGE == kStageScan) {
+      const double m0 = st->mn, h = (st->mx - st->mn) * (1.0 / 9.0);
+      double xl = m0, nl = 0.0, xh = st->mx, nh = st->W;  // the points next to the target
+#pragma unroll
+      for (int j = 0; j < K; ++j) {
+        const double x = fma(j + 1.0, h, m0);
+        note(x, v[j]);
+        if (v[j] < a.target) { xl = x; nl = v[j]; }
+        else if (x < xh) { xh = x; nh = v[j]; }
+      }
+      r = nh > nl ? xl + (xh - xl) * fmin(fmax((a.target - nl) / (nh - nl), 0.0), 1.0) : 0.5 * (xl + xh);
+    } else {
+      const double m = st->m;
+      note(m, v[0]);
+      note(m - st->d, v[2]);
+      note(m + st->d, v[3]);
+      const double span = st->mx - st->mn + 10.0 * fmax(a.T, 1e-6);
+      const double bl = fmax(B, st->mn - span), bh = fmin(A, st->mx + span), Z = v[1] / Td;
+      r = m - (v[0] - a.target) / Z;
+      if (!(Z > 0.0) || !isfinite(r) || r <= bl || r >= bh) r = 0.5 * (bl + bh);
+      const double fw = Z > 0.0 ? margin / Z : INFINITY;
+      st->done = A - B <= 4.0 * fw;  // as narrow as the margin allows
+      d = fmax(2.0 * fabs(r - m), 1.5 * fw);
+    }
+    st->A = A;
+    st->B = B;
+    st->m = r;
+    st->d = d;
+  }
+}
+
+// One evaluation of the Newton-bracket rule over the whole grid, in the summation order of
+// the cluster kernel: its csize CTAs of 32 warps are spread over csize * 8 CTAs of four,
+// every warp visits the elements of "its" threads in the same order, and the last CTA
+// combines the warp sums by the same trees.  The iterates are the cluster kernel's bit for
+// bit, which the conjugate-gradient solver needs: a last-digit change of mu moves its
+// plateau stop on some problems.  FIRST: the extremes and the evaluation at mu0.
+template <typename RT, bool FIRST>
+__global__ void __launch_bounds__(128) k_mu_newton(const MuArgs a, int csize, MuState* st, double* part) {
+  if (a.active && !*a.active) return;
+  if (!FIRST && st->done) return;
+  __shared__ double sb[kMuMaxCluster][4];
+  __shared__ bool last;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, vw = blockIdx.x * 4 + wid;
+  const int gt = vw * 32 + lane, gs = csize * kMuThreads;
+  const double Tj = fmax(a.T, 1e-12), rTj = recip_of(Tj);
+  const double mu0 = FIRST ? a.mu0[0] : 0.0, mu = FIRST ? mu0 : st->mu;
+  double mn = INFINITY, mx = -INFINITY, N = 0.0, Z = 0.0;
+  for_each_eps<RT, kMuCacheU>(a, gt, gs, [&](double ev, double w) {
+    if (FIRST) {
+      mn = fmin(mn, ev);
+      mx = fmax(mx, ev);
+    }
+    const double p = expit(div_by(mu - ev, Tj, rTj));
+    N += w * p;
+    Z += div_by(w * (p * (1.0 - p)), Tj, rTj);
+  });
+  auto reduce = [&] {
+    N = warp_sum(N);
+    Z = warp_sum(Z);
+    if (FIRST)
+      for (int off = 16; off > 0; off >>= 1) {
+        mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, off));
+        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+      }
+  };
+  reduce();
+  if (lane == 0) {
+    double* q = part + 4 * vw;
+    q[0] = N;
+    q[1] = Z;
+    if (FIRST) {
+      q[2] = mn;
+      q[3] = mx;
+    }
+    __threadfence();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&st->counter, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int b = wid; b < csize; b += 4) {
+    const double* q = part + 4 * (b * 32 + lane);
+    N = __ldcg(q);
+    Z = __ldcg(q + 1);
+    if (FIRST) {
+      mn = __ldcg(q + 2);
+      mx = __ldcg(q + 3);
+    }
+    reduce();
+    if (lane == 0) {
+      sb[b][0] = N;
+      sb[b][1] = Z;
+      sb[b][2] = mn;
+      sb[b][3] = mx;
+    }
+  }
+  __syncthreads();
+  if (wid != 0) return;
+  const bool in = lane < csize;
+  N = in ? sb[lane][0] : 0.0;
+  Z = in ? sb[lane][1] : 0.0;
+  mn = in ? sb[lane][2] : INFINITY;
+  mx = in ? sb[lane][3] : -INFINITY;
+  reduce();
+  if (lane != 0) return;
+  st->counter = 0u;
+  double lo, hi, m;
+  int it;
+  bool have = true;
+  if (FIRST) {
+    st->mn = mn;
+    st->mx = mx;
+    lo = mn - 50.0 * Tj;
+    hi = mx + 50.0 * Tj;
+    m = fmin(fmax(mu0, lo), hi);
+    it = 0;
+    have = m == mu0;  // the first Newton evaluation is in hand
+  } else {
+    lo = st->lo;
+    hi = st->hi;
+    m = mu;
+    it = st->it;
+  }
+  int done = 0;
+  if (have) {
+    done = newton_step(N - a.target, Z, lo, hi, m);
+    done = ++it >= a.maxiter || done;
+  }
+  st->done = done;
+  st->it = it;
+  st->lo = lo;
+  st->hi = hi;
+  st->mu = m;
+}
+
 // BT threads per CTA; the bisection evaluates L levels per pass (L = 2 for the
 // 256-thread variant, 1 for the 1024-thread variant, whose register budget is 64).
 // NEWTON: methods 1 and 2 only (1024 threads); otherwise the bisection only, so that
@@ -232,6 +519,10 @@ template <typename RT, int BT, bool NEWTON>
 __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
   constexpr int L = BT <= 256 ? kBisLevels : 1, NODES = (1 << L) - 1;
   if (a.active && !*a.active) return;  // uniform across the cluster: no barrier is skipped by a subset
+  if (NEWTON && a.pre && a.pre->done) {  // the grid-wide passes converged (uniform as well)
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.out[0] = a.pre->mu;
+    return;
+  }
   cg::cluster_group cl = cg::this_cluster();
   __shared__ double slots[3][2];
   __shared__ double wsm[66];
@@ -265,10 +556,10 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
 
   // method 0 with a hint (the caller's previous mu): read before any CTA can write a.out
   const double hint = (!NEWTON && a.mu0 != nullptr) ? a.mu0[0] : 0.0;
-  const bool has_hint = !NEWTON && a.mu0 != nullptr && isfinite(hint);
+  const bool has_hint = !NEWTON && a.mu0 != nullptr && isfinite(hint) && a.pre == nullptr;
   // Method 2 with a warm start: the min/max pass also forms N and Z at mu0, which
   // are the first Newton evaluation whenever mu0 lies inside the bracket.
-  const bool fuse_first = NEWTON && a.method == 2 && a.mu0 != nullptr;
+  const bool fuse_first = NEWTON && a.method == 2 && a.mu0 != nullptr && a.pre == nullptr;
   const double mu0v = fuse_first ? a.mu0[0] : 0.0;
   const double Tf = fmax(a.T, 1e-12), rTf = recip_of(Tf);
   double mn = INFINITY, mx = -INFINITY, N0 = 0.0, Z0 = 0.0;
@@ -280,13 +571,18 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
       N0 += w * p;
       Z0 += div_by(w * (p * (1.0 - p)), Tf, rTf);
     });
-  } else {
+  } else if (!a.pre) {
     visit([&](double v, double) {
       mn = fmin(mn, v);
       mx = fmax(mx, v);
     });
   }
-  cluster_minmax(cl, mn, mx, slots, wsm);
+  if (a.pre) {
+    mn = a.pre->mn;
+    mx = a.pre->mx;
+  } else {
+    cluster_minmax(cl, mn, mx, slots, wsm);
+  }
   int parity = 0;
   if (fuse_first) {
     cluster_sum2(cl, N0, Z0, slots, wsm, parity);
@@ -306,12 +602,13 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
     const double Td = T + 1e-12, iTd = 1.0 / Td;
     int it = 0;
     bool fixed = false;
+    double A = INFINITY, B = -INFINITY;
     if (has_hint) {
       // Certified bracket from the hint.  N(x) = sum w / (1 + exp((e - x) / Td)) is
       // increasing in x; an evaluation N~(x) differs from it by at most E = (kpt + 24) u W
       // (kpt terms summed per thread, a reduction tree of depth <= 14, about 6 u per term
       // and u W for the rounding of the exponent's argument; W = sum w).  So once
-      // N~(A) > target + margin with margin = 8 (kpt + 24) u W >= 2E, every x >= A has
+      // N~(A) > target + margin with margin = cert_margin(...) >= 2E, every x >= A has
       // N~(x) > target: the bisection's decision at a midpoint m >= A is "above" without
       // an evaluation, and likewise "below" for m <= B once N~(B) < target - margin.
       // Newton passes from the hint put A and B within a few margin / N' of the root,
@@ -320,7 +617,6 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
       // only the last few levels are evaluated.  The decisions, and so the result, are
       // those of evaluating every level.
       const int kpt = (a.n + gs - 1) / gs;
-      double A = INFINITY, B = -INFINITY;
       double m = fmin(fmax(hint, lo), hi), d = 0.0;
       for (int t = 0; t < kMuCertPasses; ++t) {
         const double pl = m - d, ph = m + d;
@@ -335,7 +631,7 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
         });
         cluster_sum_n<5>(cl, v, cslots, csm, parity);
         parity ^= 1;
-        const double margin = 8.0 * (kpt + 24) * 1.1102230246251565e-16 * v[4];
+        const double margin = cert_margin(kpt, kpt, v[4]);
         const double xs[3] = {m, pl, ph}, ns[3] = {v[0], v[2], v[3]};
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
@@ -346,22 +642,25 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
         const double bl = fmax(B, lo), bh = fmin(A, hi);
         double r = m - (v[0] - a.target) / Z;
         if (!(Z > 0.0) || !isfinite(r) || r <= bl || r >= bh) r = 0.5 * (bl + bh);
-        const double floor_w = Z > 0.0 ? 2.0 * margin / Z : INFINITY;
+        const double floor_w = Z > 0.0 ? margin / Z : INFINITY;
         if (A - B <= 4.0 * floor_w) break;  // as narrow as the margin allows
-        d = fmax(2.0 * fabs(r - m), floor_w);
+        d = fmax(2.0 * fabs(r - m), 1.5 * floor_w);
         m = r;
       }
-      while (it < a.maxiter) {  // the levels decided by the certified bracket
-        const double mid = 0.5 * (lo + hi);
-        double nl, nh;
-        if (mid >= A) { nl = lo; nh = mid; }
-        else if (mid <= B) { nl = mid; nh = hi; }
-        else break;
-        if (nl == lo && nh == hi) { fixed = true; break; }
-        lo = nl;
-        hi = nh;
-        ++it;
-      }
+    } else if (a.pre) {  // the bracket certified by the grid-wide passes
+      A = a.pre->A;
+      B = a.pre->B;
+    }
+    while (it < a.maxiter) {  // the levels decided by the certified bracket (none without one)
+      const double mid = 0.5 * (lo + hi);
+      double nl, nh;
+      if (mid >= A) { nl = lo; nh = mid; }
+      else if (mid <= B) { nl = mid; nh = hi; }
+      else break;
+      if (nl == lo && nh == hi) { fixed = true; break; }
+      lo = nl;
+      hi = nh;
+      ++it;
     }
     while (it < a.maxiter && !fixed) {
       double nlo[NODES + 1], nhi[NODES + 1], mid[NODES + 1];
@@ -446,8 +745,15 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
       const double m0 = a.mu0 ? a.mu0[0] : 0.0;
       mu = fmin(fmax(m0, lo), hi);
     }
+    int it = 0;
+    if (a.pre) {  // method 2, carried on from the grid-wide passes
+      lo = a.pre->lo;
+      hi = a.pre->hi;
+      mu = a.pre->mu;
+      it = a.pre->it;
+    }
     const bool have_first = fuse_first && mu == mu0v;
-    for (int it = 0; it < a.maxiter; ++it) {
+    for (; it < a.maxiter; ++it) {
       double N = 0.0, Z = 0.0;
       if (it == 0 && have_first) {
         N = N0;
@@ -461,18 +767,7 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
         cluster_sum2(cl, N, Z, slots, wsm, parity);
         parity ^= 1;
       }
-      const double g = N - a.target;
-      if (g < 0) lo = mu;
-      if (g > 0) hi = mu;
-      double mn2 = mu - g / fmax(Z, 1e-18);
-      const double mb = 0.5 * (lo + hi);
-      bool newton = true;
-      if (mn2 <= lo || mn2 >= hi) { mn2 = mb; newton = false; }
-      mn2 = fmin(fmax(mn2, lo), hi);
-      if (!isfinite(mn2)) { mn2 = mb; newton = false; }
-      const double step = fabs(mn2 - mu);
-      mu = mn2;
-      if (newton && step <= 4.0 * 2.220446049250313e-16 * fmax(1.0, fabs(mu))) break;
+      if (newton_step(N - a.target, Z, lo, hi, mu)) break;
     }
     if (a.method == 1) {
       double N = 0.0, dummy = 0.0;
@@ -494,19 +789,55 @@ using namespace hf;
 namespace hf {
 int find_mu_internal(void* stream, int dtype, int method, int nk1, int nk2, int nb, const void* eps,
                      const void* weights, double n_electrons, double T, int maxiter, const double* mu0,
-                     double* mu_out, const int* active);
+                     double* mu_out, const int* active, void* ws, size_t ws_bytes, bool ws_ready);
+
+// Queues the grid-wide passes in front of the cluster kernel (a.kpt set).
+template <typename RT>
+static int launch_passes(cudaStream_t s, const MuArgs& a, int csize, MuState* st, double* part, bool ready) {
+  if (!ready) HF_CUDA(cudaMemsetAsync(st, 0, sizeof(MuState), s));  // the ticket; the passes set the rest
+  if (a.method == 2) {
+    k_mu_newton<RT, true><<<csize * 8, 128, 0, s>>>(a, csize, st, part);
+    for (int i = 0; i < kNewtonPasses; ++i) k_mu_newton<RT, false><<<csize * 8, 128, 0, s>>>(a, csize, st, part);
+    HF_LAUNCH_CHECK("k_mu_newton");
+    return HF_OK;
+  }
+  int blocks = (a.n + kPassThreads - 1) / kPassThreads;
+  if (blocks > kPassBlocks) blocks = kPassBlocks;
+  k_mu_pass<RT, kStageRange><<<blocks, kPassThreads, 0, s>>>(a, st, part);
+  k_mu_pass<RT, kStageScan><<<blocks, kPassThreads, 0, s>>>(a, st, part);
+  for (int i = 1; i < kCertPasses; ++i) k_mu_pass<RT, kStageCertify><<<blocks, kPassThreads, 0, s>>>(a, st, part);
+  HF_LAUNCH_CHECK("k_mu_pass");
+  return HF_OK;
+}
+}
+
+extern "C" int hf_mu_workspace_size(size_t* bytes) {
+  if (!bytes) return fail(HF_ERR_INVALID, "bytes is NULL");
+  *bytes = kMuWsBytes;
+  return HF_OK;
+}
+
+extern "C" int hf_find_mu_ws(void* stream, int dtype, int method, int nk1, int nk2, int nb, const void* eps,
+                             const void* weights, double n_electrons, double T, int maxiter, const double* mu0,
+                             double* mu_out, void* workspace, size_t workspace_bytes) {
+  if (!workspace || workspace_bytes < kMuWsBytes)
+    return fail(HF_ERR_WORKSPACE, "workspace too small: need " + std::to_string(kMuWsBytes) + " bytes");
+  if (reinterpret_cast<uintptr_t>(workspace) % 256 != 0)
+    return fail(HF_ERR_WORKSPACE, "workspace must be 256-byte aligned");
+  return hf::find_mu_internal(stream, dtype, method, nk1, nk2, nb, eps, weights, n_electrons, T, maxiter, mu0,
+                              mu_out, nullptr, workspace, workspace_bytes, false);
 }
 
 extern "C" int hf_find_mu(void* stream, int dtype, int method, int nk1, int nk2, int nb,
                           const void* eps, const void* weights, double n_electrons, double T,
                           int maxiter, const double* mu0, double* mu_out) {
   return hf::find_mu_internal(stream, dtype, method, nk1, nk2, nb, eps, weights, n_electrons, T, maxiter, mu0,
-                              mu_out, nullptr);
+                              mu_out, nullptr, nullptr, 0, false);
 }
 
 int hf::find_mu_internal(void* stream, int dtype, int method, int nk1, int nk2, int nb, const void* eps,
                          const void* weights, double n_electrons, double T, int maxiter, const double* mu0,
-                         double* mu_out, const int* active) {
+                         double* mu_out, const int* active, void* ws, size_t ws_bytes, bool ws_ready) {
   if (dtype != HF_C128 && dtype != HF_C64) return fail(HF_ERR_INVALID, "bad dtype");
   if (method < 0 || method > 2) return fail(HF_ERR_INVALID, "method must be 0, 1 or 2");
   if (nk1 < 1 || nk2 < 1 || nb < 1) return fail(HF_ERR_INVALID, "bad shape");
@@ -519,7 +850,7 @@ int hf::find_mu_internal(void* stream, int dtype, int method, int nk1, int nk2, 
   }
   const size_t n_all = (size_t)nk1 * (size_t)nk2 * (size_t)nb;
   if (n_all > (size_t)INT_MAX) return fail(HF_ERR_UNSUPPORTED, "more than 2^31 - 1 eigenvalues");
-  MuArgs a;
+  MuArgs a = {};
   a.eps = eps; a.w = weights;
   a.n = (int)n_all; a.nb = nb; a.method = method; a.maxiter = maxiter;
   a.target = n_electrons; a.T = T; a.mu0 = mu0; a.out = mu_out; a.active = active;
@@ -575,6 +906,18 @@ int hf::find_mu_internal(void* stream, int dtype, int method, int nk1, int nk2, 
   {
     const long long per = ((long long)a.n + (long long)csize * threads - 1) / ((long long)csize * threads);
     a.cache = per <= kMuCacheMax ? (int)per : 0;
+    a.kpt = (int)per;
+  }
+  // the grid-wide passes, given a workspace: for the bisection without a hint (with one, the
+  // cluster kernel certifies its own bracket) and the warm-started Newton rule
+  if (ws && ws_bytes >= kMuWsBytes && a.n >= kGridMin && (method == 2 ? mu0 != nullptr : method == 0 && !mu0)) {
+    MuState* st = static_cast<MuState*>(ws);
+    double* part = reinterpret_cast<double*>(static_cast<char*>(ws) + 256);
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const int e = single ? launch_passes<float>(s, a, csize, st, part, ws_ready)
+                         : launch_passes<double>(s, a, csize, st, part, ws_ready);
+    if (e) return e;
+    a.pre = st;
   }
   const size_t cache_bytes = (size_t)a.cache * threads * sizeof(double2);
   cudaLaunchConfig_t cfg = {};

@@ -33,7 +33,7 @@ int energy_internal(void* stream, int dtype, int nk1, int nk2, int nb, const voi
                     void* workspace, size_t workspace_bytes, const int* active);
 int find_mu_internal(void* stream, int dtype, int method, int nk1, int nk2, int nb, const void* eps,
                      const void* weights, double n_electrons, double T, int maxiter, const double* mu0,
-                     double* mu_out, const int* active);
+                     double* mu_out, const int* active, void* ws, size_t ws_bytes, bool ws_ready);
 
 struct CgScalars {
   int k, active, accepted, converged, k_base;
@@ -707,6 +707,8 @@ struct CgLayout {
   size_t total;
 };
 
+constexpr size_t kCgMuWs = 32 * 1024;  // at least hf_mu_workspace_size
+
 static size_t cg_layout(const hf_cg_problem& pb, size_t fock_ws, size_t red_ws, CgLayout& L) {
   const size_t nk = (size_t)pb.nk1 * pb.nk2, nb = pb.nb, nq = nk * nb * nb, nv = nk * nb;
   const size_t sizes[] = {
@@ -716,7 +718,7 @@ static size_t cg_layout(const hf_cg_problem& pb, size_t fock_ws, size_t red_ws, 
       nb * nb * 16,                                                    // H
       sizeof(CgScalars), 64,                                           // scalars, counter
       (size_t)148 * 16 * kMaxSums * 2 * 8,                             // partials
-      fock_ws, red_ws};
+      fock_ws, red_ws, kCgMuWs};
   size_t o = 0;
   const int n = sizeof(sizes) / sizeof(sizes[0]);
   for (int i = 0; i < n; ++i) { L.off[i] = o; o += align_up(sizes[i], 256); }
@@ -742,6 +744,7 @@ struct CgRun {
   size_t fock_ws_bytes;
   void* red_ws;
   size_t red_ws_bytes;
+  void* mu_ws;
   double2* Sigma;
   double2* H;
   int nblk;
@@ -777,7 +780,7 @@ static int cg_energy(CgRun& r, cudaStream_t s, double* out, const int* active) {
 static int cg_mu(CgRun& r, cudaStream_t s, int maxiter, const int* active) {
   const hf_cg_problem& pb = *r.pb;
   return find_mu_internal(s, HF_C128, 2, pb.nk1, pb.nk2, pb.nb, r.a.eps, r.a.w_norm, r.a.n_target_norm, r.a.T_r,
-                          maxiter, &r.a.sc->mu, &r.a.sc->mu, active);
+                          maxiter, &r.a.sc->mu, &r.a.sc->mu, active, r.mu_ws, kCgMuWs, true);
 }
 
 // Grid of an elementwise pass: a few elements per thread, at most 8 CTAs of 256 per SM.
@@ -1060,6 +1063,7 @@ int CgSolver::setup(const hf_cg_problem* pb_, const hf_cg_config* cf_, void* Q, 
   r.fock_ws = ws + L.off[18];
   r.fock_ws_bytes = fws > f2 ? fws : f2;
   r.red_ws = ws + L.off[19];
+  r.mu_ws = ws + L.off[20];
   r.red_ws_bytes = rws;
   a.hist_E = hist_E ? hist_E : reinterpret_cast<double*>(ws + L.total);
   a.hist_G = hist_grad ? hist_grad : reinterpret_cast<double*>(ws + L.total) + cf->max_iter;
@@ -1086,6 +1090,7 @@ int CgSolver::init_ops(const void* P0) {
   const int nb = pb->nb, nb2 = nb * nb;
   int st;
   HF_CUDA(cudaMemsetAsync(r.H, 0, sizeof(double2) * nb2, s));  // H stays zero without Hartree
+  HF_CUDA(cudaMemsetAsync(r.mu_ws, 0, 256, s));                // the ticket of the mu passes
   if (cf->max_iter > 0) HF_CUDA(cudaMemsetAsync(a.hist_E, 0, sizeof(double) * cf->max_iter, s));
   if (cf->max_iter > 0) HF_CUDA(cudaMemsetAsync(a.hist_G, 0, sizeof(double) * cf->max_iter, s));
   // ---- init (solver.py:377-394) ----

@@ -1,7 +1,7 @@
 """Occupations, chemical potential and validation (drop-in for jax_hf.utils).
 
 ``find_chemical_potential`` runs the cluster-wide mu root find on the GPU
-(``hf_find_mu``); ``validate_electron_count`` is the reference's host check
+(``hf_find_mu_ws``); ``validate_electron_count`` is the reference's host check
 (utils.py:21-43) with the same ValueError text; ``resample_kgrid`` (utils.py:477-535)
 resamples a centered periodic k-grid array on the GPU (``hf_resample_kgrid``).
 """
@@ -60,10 +60,24 @@ def find_chemical_potential(bands, weights, n_electrons: float, T: float, *, max
     nb = int(bands.shape[-1])
     nk = bands.numel() // nb
     mu = torch.empty((), dtype=torch.float64, device=dev)
-    _lib.check(_lib.lib().hf_find_mu(_lib.stream_ptr(dev), _lib.dtype_code(bands), _METHODS[m], nk, 1, nb,
-                                     bands.data_ptr(), w.data_ptr(), float(n_electrons), float(T),
-                                     int(maxiter or 0), None, mu.data_ptr()))
+    _find_mu(dev, bands, _METHODS[m], nk, nb, w, n_electrons, T, int(maxiter or 0), None, mu)
     return mu
+
+
+_mu_bytes = None  # workspace of the grid-wide passes (the same for every shape)
+
+
+def _find_mu(dev, eps, method, nk, nb, w, n, T, maxiter, mu0, out):
+    global _mu_bytes
+    if _mu_bytes is None:
+        need = _lib.C.c_size_t(0)
+        _lib.check(_lib.lib().hf_mu_workspace_size(_lib.C.byref(need)))
+        _mu_bytes = int(need.value)
+    stream = _lib.stream_ptr(dev)
+    ws = _lib.workspace(_mu_bytes, dev, "mu", stream)
+    _lib.check(_lib.lib().hf_find_mu_ws(stream, _lib.dtype_code(eps), method, nk, 1, nb, eps.data_ptr(),
+                                        w.data_ptr(), float(n), float(T), maxiter, _lib.ptr(mu0), out.data_ptr(),
+                                        ws.data_ptr(), ws.numel()))
 
 
 def solve_mu(eps, w_norm, n_target_norm: float, mu0, T: float, maxiter: int = 25, out=None):
@@ -76,9 +90,7 @@ def solve_mu(eps, w_norm, n_target_norm: float, mu0, T: float, maxiter: int = 25
     m0 = mu0 if isinstance(mu0, torch.Tensor) else torch.tensor(float(mu0), dtype=torch.float64, device=dev)
     m0 = m0.to(dev, torch.float64).reshape(()).contiguous()
     mu = out if out is not None else torch.empty((), dtype=torch.float64, device=dev)
-    _lib.check(_lib.lib().hf_find_mu(_lib.stream_ptr(dev), _lib.dtype_code(eps), 2, nk, 1, nb, eps.data_ptr(),
-                                     w.data_ptr(), float(n_target_norm), float(T), int(maxiter), m0.data_ptr(),
-                                     mu.data_ptr()))
+    _find_mu(dev, eps, 2, nk, nb, w, n_target_norm, T, int(maxiter), m0, mu)
     return mu
 
 

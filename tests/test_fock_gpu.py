@@ -557,3 +557,40 @@ DENSE = [  # sides with a prime factor of 17 or more: one row, several rows, an 
 @pytest.mark.parametrize("terms", [False, True])
 def test_dense_line_sums_match_stockham(cuda, n1, n2, nb, V, mode, terms):
     test_two_factor_passes_match_stockham(cuda, n1, n2, nb, V, mode, terms)
+
+
+@pytest.mark.parametrize("shape,T,kind", [((70, 59, 4), 0.1, "metal"), ((128, 128, 1), 0.02, "metal"),
+                                          ((96, 96, 4), 1e-4, "metal"), ((64, 64, 8), 0.01, "gapped"),
+                                          ((80, 80, 3), 0.0, "metal"), ((144, 144, 8), 0.05, "metal")])
+@pytest.mark.parametrize("fill", [0.01, 0.43, 0.5, 1.0])
+def test_grid_wide_mu_equals_the_cluster_bisection(cuda, shape, T, kind, fill):
+    """hf_find_mu_ws (certifying passes over the grid) against hf_find_mu on the same eigenvalues: the
+    bisection bit for bit; the Newton rule's root within the noise of the count (sum of n terms,
+    (n / threads + 40) ulp of the total weight over N') or, where N' vanishes, the same count."""
+    from jax_hf_b200 import _lib
+    rng = np.random.default_rng(shape[0] + shape[2])
+    eps = rng.normal(size=shape)
+    if kind == "gapped":
+        eps += 3.0 * np.sign(np.arange(shape[2]) - shape[2] / 2 + 0.5)
+    w = rng.uniform(0.5, 1.5, size=shape[:2])
+    w /= w.sum()
+    nb, nk = shape[2], shape[0] * shape[1]
+    e, wt = torch.as_tensor(eps, device="cuda").contiguous(), torch.as_tensor(w, device="cuda")
+    L = _lib.lib()
+    n = _lib.C.c_size_t(0)
+    _lib.check(L.hf_mu_workspace_size(_lib.C.byref(n)))
+    ws = torch.full((n.value,), 255, dtype=torch.uint8, device="cuda")
+    mu0 = torch.tensor(0.1, dtype=torch.float64, device="cuda")
+    out = torch.empty(4, dtype=torch.float64, device="cuda")
+    s = _lib.stream_ptr(e.device)
+    ne = fill * nb
+    for i, (meth, m0) in enumerate(((0, None), (2, mu0.data_ptr()))):
+        _lib.check(L.hf_find_mu(s, _lib.HF_C128, meth, nk, 1, nb, e.data_ptr(), wt.data_ptr(), ne, T, 0, m0,
+                                out[2 * i:].data_ptr()))
+        _lib.check(L.hf_find_mu_ws(s, _lib.HF_C128, meth, nk, 1, nb, e.data_ptr(), wt.data_ptr(), ne, T, 0, m0,
+                                   out[2 * i + 1:].data_ptr(), ws.data_ptr(), ws.numel()))
+    mu = out.cpu().numpy()
+    assert mu[0] == mu[1]
+    count = lambda m: float((w[..., None] / (1.0 + np.exp(np.clip((eps - m) / max(T, 1e-12), -700, 700)))).sum())
+    if abs(mu[2] - mu[3]) > 1e-11 * max(1.0, abs(mu[2])):
+        assert abs(count(mu[2]) - count(mu[3])) <= 60 * 2.2e-16 * nb
