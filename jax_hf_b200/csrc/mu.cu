@@ -56,8 +56,8 @@ struct MuArgs {
 // Root-find state of the grid-wide passes (device memory, in the caller's workspace).
 struct MuState {
   unsigned counter;  // CTAs of the running pass that have published; zero between passes
-  int done, it;
-  double lo, hi, mu;        // method 2: bracket and iterate
+  int done, it, fixed;      // fixed: the bisection's interval no longer changes
+  double lo, hi, mu;        // bracket; method 2: iterate
   double mn, mx, W;         // extreme eigenvalues, total weight
   double A, B, m, d;        // bisection: certified bracket, next iterate and probe offset
 };
@@ -242,6 +242,23 @@ __device__ __forceinline__ double cert_margin(int ka, int kb, double W) {
   return 1.25 * ((double)ka + (double)kb + 60.0) * 1.1102230246251565e-16 * W;
 }
 
+// Bisection levels that need no evaluation: every midpoint >= A is decided "above", every one
+// <= B "below".  True when the interval stops changing.
+__device__ __forceinline__ bool replay_levels(double A, double B, int maxiter, double& lo, double& hi, int& it) {
+  while (it < maxiter) {
+    const double mid = 0.5 * (lo + hi);
+    double nl, nh;
+    if (mid >= A) { nl = lo; nh = mid; }
+    else if (mid <= B) { nl = mid; nh = hi; }
+    else return false;
+    if (nl == lo && nh == hi) return true;
+    lo = nl;
+    hi = nh;
+    ++it;
+  }
+  return false;
+}
+
 // One step of the Newton-bracket rule (solver.py:62-101) from g = N(mu) - target and
 // Z = N'(mu); true once the accepted Newton step is below 4 ulp of mu.
 __device__ __forceinline__ bool newton_step(double g, double Z, double& lo, double& hi, double& mu) {
@@ -264,21 +281,23 @@ __device__ __forceinline__ bool newton_step(double g, double Z, double& lo, doub
 // passes run one evaluation each over the whole grid; the last CTA to publish its sums
 // (atomic ticket, no spin) takes the step, and the cluster kernel finishes from MuState.
 // Every pass returns at once when the state says done.  The bisection's passes certify a
-// bracket (see the hinted bisection below); only the levels inside it are left to evaluate.
+// bracket (see the hinted bisection below), the levels inside it are evaluated two per pass,
+// and the cluster kernel finishes what is left.
 // 144 x 144, nb = 8 (166k eigenvalues): the bisection of the cluster kernel alone takes 353 us.
 constexpr int kPassThreads = 256;
 constexpr int kPassBlocks = 296;   // two CTAs per SM
 constexpr int kPassSums = 8;
 constexpr int kGridMin = 16384;    // eigenvalues from which the passes are used
 constexpr int kNewtonPasses = 5;   // method 2: Newton steps queued ahead of the cluster kernel
+constexpr int kLevelPasses = 5;    // bisection: passes of two levels each behind them
 constexpr int kCertPasses = 7;     // bisection: certifying passes, the first one a scan of 8 points
-constexpr size_t kMuWsBytes = 256 + sizeof(double) * kPassBlocks * kPassSums;  // also 4 per warp of k_mu_newton
-static_assert(kPassBlocks * kPassSums >= 4 * 32 * kMuMaxCluster, "workspace of k_mu_newton");
+constexpr size_t kMuWsBytes = 256 + sizeof(double) * kPassBlocks * kPassSums;  // also 3 per warp of k_mu_levels
+static_assert(kPassBlocks * kPassSums >= 3 * 32 * kMuMaxCluster, "workspace of k_mu_levels");
 
 enum MuStage { kStageRange, kStageScan, kStageCertify };
 
 template <typename RT, int STAGE>
-__global__ void __launch_bounds__(kPassThreads) k_mu_pass(const MuArgs a, MuState* st, double* part) {
+__global__ void __launch_bounds__(kPassThreads) k_mu_pass(const MuArgs a, MuState* st, double* part, bool final_pass) {
   if (a.active && !*a.active) return;
   if (STAGE != kStageRange && st->done) return;
   constexpr int K = STAGE == kStageRange ? 3 : STAGE == kStageScan ? 8 : 5;
@@ -327,13 +346,11 @@ __global__ void __launch_bounds__(kPassThreads) k_mu_pass(const MuArgs a, MuStat
       if (lane == 0) red[wid * K + j] = v[j];
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (wid == 0) {
 #pragma unroll
       for (int j = 0; j < K; ++j) {
-        double t = red[j];
-#pragma unroll
-        for (int q = 1; q < kPassThreads / 32; ++q) t = combine(j, t, red[q * K + j]);
-        v[j] = t;
+        v[j] = red[(lane & (kPassThreads / 32 - 1)) * K + j];
+        for (int off = kPassThreads / 64; off > 0; off >>= 1) v[j] = combine(j, v[j], __shfl_xor_sync(0xffffffffu, v[j], off));
       }
     }
   };
@@ -402,94 +419,117 @@ __global__ void __launch_bounds__(kPassThreads) k_mu_pass(const MuArgs a, MuStat
     st->B = B;
     st->m = r;
     st->d = d;
+    if (STAGE == kStageCertify && (st->done || final_pass)) {
+      // the levels that the bracket decides (none outside [B, A] needs an evaluation)
+      const double span = st->mx - st->mn + 10.0 * fmax(a.T, 1e-6);
+      double lo = st->mn - span, hi = st->mx + span;
+      int it = 0;
+      st->fixed = replay_levels(A, B, a.maxiter, lo, hi, it);
+      st->lo = lo;
+      st->hi = hi;
+      st->it = it;
+    }
   }
 }
 
-// One evaluation of the Newton-bracket rule over the whole grid, in the summation order of
-// the cluster kernel: its csize CTAs of 32 warps are spread over csize * 8 CTAs of four,
-// every warp visits the elements of "its" threads in the same order, and the last CTA
-// combines the warp sums by the same trees.  The iterates are the cluster kernel's bit for
-// bit, which the conjugate-gradient solver needs: a last-digit change of mu moves its
-// plateau stop on some problems.  FIRST: the extremes and the evaluation at mu0.
-template <typename RT, bool FIRST>
-__global__ void __launch_bounds__(128) k_mu_newton(const MuArgs a, int csize, MuState* st, double* part) {
-  if (a.active && !*a.active) return;
-  if (!FIRST && st->done) return;
-  __shared__ double sb[kMuMaxCluster][4];
+// Evaluations over the whole grid in the summation order of the cluster kernel: its csize
+// CTAs of 32 warps are spread over csize * 8 CTAs of four of them.  kOrdParts threads share
+// the elements of one of "its" threads: they form the terms, the first of them adds them in
+// order from shared memory, and the last CTA combines the warp sums by the same trees.  The
+// results are the cluster kernel's bit for bit, which its callers need: a last-digit change
+// of mu moves the plateau stop of the conjugate-gradient solver on some problems.
+constexpr int kOrdWarps = 4, kOrdParts = 4, kOrdThreads = 32 * kOrdWarps * kOrdParts;
+
+// term(e, w, t): the K term values of an element; add(t, w, acc): acc += them.  acc is the
+// thread's own sum (part 0 only).
+template <typename RT, int K, class Term, class Add>
+__device__ __forceinline__ void ordered_terms(const MuArgs& a, int csize, double (*buf)[kOrdParts][32 * kOrdWarps][K + 1],
+                                              Term&& term, Add&& add) {
+  const int vt = threadIdx.x % (32 * kOrdWarps), part = threadIdx.x / (32 * kOrdWarps);
+  const int gt = blockIdx.x * 32 * kOrdWarps + vt, gs = csize * kMuThreads;
+  int side = 0;
+  for (int base = gt - vt; base < a.n; base += kOrdParts * gs, side ^= 1) {  // uniform over the CTA
+    const int e = base + vt + part * gs;
+    double* t = buf[side][part][vt];
+    if (e < a.n) {
+      const double w = load_w<RT>(a, e);
+      term(load_eps<RT>(a, e), w, t);
+      t[K] = w;
+    }
+    __syncthreads();
+    if (part == 0) {
+#pragma unroll
+      for (int q = 0; q < kOrdParts; ++q)
+        if (base + vt + q * gs < a.n) add(buf[side][q][vt]);
+    }
+  }
+}
+
+// v: sums of the virtual threads (part 0); publishes the warp sums and returns true in the
+// last CTA, where warp 0 then holds the totals in every lane.
+template <int K>
+__device__ __forceinline__ bool ordered_totals(double (&v)[K], int csize, MuState* st, double* part) {
+  __shared__ double sb[kMuMaxCluster][K];
   __shared__ bool last;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, vw = blockIdx.x * 4 + wid;
-  const int gt = vw * 32 + lane, gs = csize * kMuThreads;
-  const double Tj = fmax(a.T, 1e-12), rTj = recip_of(Tj);
-  const double mu0 = FIRST ? a.mu0[0] : 0.0, mu = FIRST ? mu0 : st->mu;
-  double mn = INFINITY, mx = -INFINITY, N = 0.0, Z = 0.0;
-  for_each_eps<RT, kMuCacheU>(a, gt, gs, [&](double ev, double w) {
-    if (FIRST) {
-      mn = fmin(mn, ev);
-      mx = fmax(mx, ev);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (wid < kOrdWarps) {
+    const int vw = blockIdx.x * kOrdWarps + wid;
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      v[j] = warp_sum(v[j]);
+      if (lane == 0) part[K * vw + j] = v[j];
     }
-    const double p = expit(div_by(mu - ev, Tj, rTj));
-    N += w * p;
-    Z += div_by(w * (p * (1.0 - p)), Tj, rTj);
-  });
-  auto reduce = [&] {
-    N = warp_sum(N);
-    Z = warp_sum(Z);
-    if (FIRST)
-      for (int off = 16; off > 0; off >>= 1) {
-        mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, off));
-        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-      }
-  };
-  reduce();
-  if (lane == 0) {
-    double* q = part + 4 * vw;
-    q[0] = N;
-    q[1] = Z;
-    if (FIRST) {
-      q[2] = mn;
-      q[3] = mx;
-    }
-    __threadfence();
+    if (lane == 0) __threadfence();
   }
   __syncthreads();
   if (threadIdx.x == 0) last = atomicAdd(&st->counter, 1u) == gridDim.x - 1;
   __syncthreads();
-  if (!last) return;
+  if (!last) return false;
   __threadfence();
-  for (int b = wid; b < csize; b += 4) {
-    const double* q = part + 4 * (b * 32 + lane);
-    N = __ldcg(q);
-    Z = __ldcg(q + 1);
-    if (FIRST) {
-      mn = __ldcg(q + 2);
-      mx = __ldcg(q + 3);
-    }
-    reduce();
-    if (lane == 0) {
-      sb[b][0] = N;
-      sb[b][1] = Z;
-      sb[b][2] = mn;
-      sb[b][3] = mx;
+  if (wid < csize) {  // one warp per CTA of the cluster kernel (csize <= kOrdThreads / 32)
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      const double x = warp_sum(__ldcg(part + K * (wid * 32 + lane) + j));
+      if (lane == 0) sb[wid][j] = x;
     }
   }
   __syncthreads();
-  if (wid != 0) return;
-  const bool in = lane < csize;
-  N = in ? sb[lane][0] : 0.0;
-  Z = in ? sb[lane][1] : 0.0;
-  mn = in ? sb[lane][2] : INFINITY;
-  mx = in ? sb[lane][3] : -INFINITY;
-  reduce();
-  if (lane != 0) return;
+  if (wid == 0) {
+#pragma unroll
+    for (int j = 0; j < K; ++j) v[j] = warp_sum(lane < csize ? sb[lane][j] : 0.0);
+  }
+  return true;
+}
+static_assert(kOrdThreads / 32 >= kMuMaxCluster, "a warp per CTA of the cluster kernel");
+
+// One evaluation of the Newton-bracket rule.  FIRST: at mu0, with the extremes already in st.
+template <typename RT, bool FIRST>
+__global__ void __launch_bounds__(kOrdThreads) k_mu_newton(const MuArgs a, int csize, MuState* st, double* part) {
+  if (a.active && !*a.active) return;
+  if (!FIRST && st->done) return;
+  __shared__ double buf[2][kOrdParts][32 * kOrdWarps][3];
+  const double Tj = fmax(a.T, 1e-12), rTj = recip_of(Tj);
+  const double mu0 = FIRST ? a.mu0[0] : 0.0, mu = FIRST ? mu0 : st->mu;
+  double v[2] = {0.0, 0.0};
+  ordered_terms<RT, 2>(
+      a, csize, buf,
+      [&](double ev, double w, double* t) {
+        const double p = expit(div_by(mu - ev, Tj, rTj));
+        t[0] = p;
+        t[1] = div_by(w * (p * (1.0 - p)), Tj, rTj);
+      },
+      [&](const double* t) {
+        v[0] = fma(t[2], t[0], v[0]);
+        v[1] += t[1];
+      });
+  if (!ordered_totals<2>(v, csize, st, part) || threadIdx.x != 0) return;
   st->counter = 0u;
   double lo, hi, m;
-  int it;
+  int it, done = 0;
   bool have = true;
   if (FIRST) {
-    st->mn = mn;
-    st->mx = mx;
-    lo = mn - 50.0 * Tj;
-    hi = mx + 50.0 * Tj;
+    lo = st->mn - 50.0 * Tj;
+    hi = st->mx + 50.0 * Tj;
     m = fmin(fmax(mu0, lo), hi);
     it = 0;
     have = m == mu0;  // the first Newton evaluation is in hand
@@ -499,9 +539,8 @@ __global__ void __launch_bounds__(128) k_mu_newton(const MuArgs a, int csize, Mu
     m = mu;
     it = st->it;
   }
-  int done = 0;
   if (have) {
-    done = newton_step(N - a.target, Z, lo, hi, m);
+    done = newton_step(v[0] - a.target, v[1], lo, hi, m);
     done = ++it >= a.maxiter || done;
   }
   st->done = done;
@@ -509,6 +548,52 @@ __global__ void __launch_bounds__(128) k_mu_newton(const MuArgs a, int csize, Mu
   st->lo = lo;
   st->hi = hi;
   st->mu = m;
+}
+
+// Two levels of the bisection: the counts at the three midpoints, then the two decisions.
+template <typename RT>
+__global__ void __launch_bounds__(kOrdThreads) k_mu_levels(const MuArgs a, int csize, MuState* st, double* part) {
+  if (a.active && !*a.active) return;
+  if (st->fixed || st->it >= a.maxiter) return;
+  __shared__ double buf[2][kOrdParts][32 * kOrdWarps][4];
+  const double iTd = 1.0 / (a.T + 1e-12);
+  double lo = st->lo, hi = st->hi;
+  const double m1 = 0.5 * (lo + hi), m2 = 0.5 * (lo + m1), m3 = 0.5 * (m1 + hi);
+  double v[3] = {0.0, 0.0, 0.0};
+  ordered_terms<RT, 3>(
+      a, csize, buf,
+      [&](double ev, double w, double* t) {
+        t[0] = w / (1.0 + exp((ev - m1) * iTd));
+        t[1] = w / (1.0 + exp((ev - m2) * iTd));
+        t[2] = w / (1.0 + exp((ev - m3) * iTd));
+      },
+      [&](const double* t) {
+        v[0] += t[0];
+        v[1] += t[1];
+        v[2] += t[2];
+      });
+  if (!ordered_totals<3>(v, csize, st, part) || threadIdx.x != 0) return;
+  st->counter = 0u;
+  int it = st->it;
+  bool fixed = false;
+  double cn = v[0], mid = m1;
+  for (int l = 0; l < 2 && !fixed && it < a.maxiter; ++l) {
+    const bool above = cn > a.target;
+    const double nl = above ? lo : mid, nh = above ? mid : hi;
+    if (nl == lo && nh == hi) {
+      fixed = true;
+    } else {
+      lo = nl;
+      hi = nh;
+      ++it;
+      cn = above ? v[1] : v[2];
+      mid = above ? m2 : m3;
+    }
+  }
+  st->lo = lo;
+  st->hi = hi;
+  st->it = it;
+  st->fixed = fixed;
 }
 
 // BT threads per CTA; the bisection evaluates L levels per pass (L = 2 for the
@@ -519,8 +604,9 @@ template <typename RT, int BT, bool NEWTON>
 __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
   constexpr int L = BT <= 256 ? kBisLevels : 1, NODES = (1 << L) - 1;
   if (a.active && !*a.active) return;  // uniform across the cluster: no barrier is skipped by a subset
-  if (NEWTON && a.pre && a.pre->done) {  // the grid-wide passes converged (uniform as well)
-    if (blockIdx.x == 0 && threadIdx.x == 0) a.out[0] = a.pre->mu;
+  // the grid-wide passes got there (uniform as well)
+  if (a.pre && (NEWTON ? a.pre->done : a.pre->fixed || a.pre->it >= a.maxiter)) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.out[0] = NEWTON ? a.pre->mu : 0.5 * (a.pre->lo + a.pre->hi);
     return;
   }
   cg::cluster_group cl = cg::this_cluster();
@@ -647,21 +733,16 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
         d = fmax(2.0 * fabs(r - m), 1.5 * floor_w);
         m = r;
       }
-    } else if (a.pre) {  // the bracket certified by the grid-wide passes
+    } else if (a.pre) {  // what the grid-wide passes left
       A = a.pre->A;
       B = a.pre->B;
+      lo = a.pre->lo;
+      hi = a.pre->hi;
+      it = a.pre->it;
+      fixed = a.pre->fixed != 0;
     }
-    while (it < a.maxiter) {  // the levels decided by the certified bracket (none without one)
-      const double mid = 0.5 * (lo + hi);
-      double nl, nh;
-      if (mid >= A) { nl = lo; nh = mid; }
-      else if (mid <= B) { nl = mid; nh = hi; }
-      else break;
-      if (nl == lo && nh == hi) { fixed = true; break; }
-      lo = nl;
-      hi = nh;
-      ++it;
-    }
+    // the levels decided by the certified bracket (none without one)
+    if (!fixed) fixed = replay_levels(A, B, a.maxiter, lo, hi, it);
     while (it < a.maxiter && !fixed) {
       double nlo[NODES + 1], nhi[NODES + 1], mid[NODES + 1];
       nlo[1] = lo;
@@ -795,17 +876,20 @@ int find_mu_internal(void* stream, int dtype, int method, int nk1, int nk2, int 
 template <typename RT>
 static int launch_passes(cudaStream_t s, const MuArgs& a, int csize, MuState* st, double* part, bool ready) {
   if (!ready) HF_CUDA(cudaMemsetAsync(st, 0, sizeof(MuState), s));  // the ticket; the passes set the rest
+  int blocks = (a.n + kPassThreads - 1) / kPassThreads;
+  if (blocks > kPassBlocks) blocks = kPassBlocks;
+  const int ord = csize * (kMuThreads / (32 * kOrdWarps));
+  k_mu_pass<RT, kStageRange><<<blocks, kPassThreads, 0, s>>>(a, st, part, false);
   if (a.method == 2) {
-    k_mu_newton<RT, true><<<csize * 8, 128, 0, s>>>(a, csize, st, part);
-    for (int i = 0; i < kNewtonPasses; ++i) k_mu_newton<RT, false><<<csize * 8, 128, 0, s>>>(a, csize, st, part);
+    k_mu_newton<RT, true><<<ord, kOrdThreads, 0, s>>>(a, csize, st, part);
+    for (int i = 0; i < kNewtonPasses; ++i) k_mu_newton<RT, false><<<ord, kOrdThreads, 0, s>>>(a, csize, st, part);
     HF_LAUNCH_CHECK("k_mu_newton");
     return HF_OK;
   }
-  int blocks = (a.n + kPassThreads - 1) / kPassThreads;
-  if (blocks > kPassBlocks) blocks = kPassBlocks;
-  k_mu_pass<RT, kStageRange><<<blocks, kPassThreads, 0, s>>>(a, st, part);
-  k_mu_pass<RT, kStageScan><<<blocks, kPassThreads, 0, s>>>(a, st, part);
-  for (int i = 1; i < kCertPasses; ++i) k_mu_pass<RT, kStageCertify><<<blocks, kPassThreads, 0, s>>>(a, st, part);
+  k_mu_pass<RT, kStageScan><<<blocks, kPassThreads, 0, s>>>(a, st, part, false);
+  for (int i = 1; i < kCertPasses; ++i)
+    k_mu_pass<RT, kStageCertify><<<blocks, kPassThreads, 0, s>>>(a, st, part, i == kCertPasses - 1);
+  for (int i = 0; i < kLevelPasses; ++i) k_mu_levels<RT><<<ord, kOrdThreads, 0, s>>>(a, csize, st, part);
   HF_LAUNCH_CHECK("k_mu_pass");
   return HF_OK;
 }
