@@ -594,3 +594,18 @@ def test_grid_wide_mu_equals_the_cluster_bisection(cuda, shape, T, kind, fill):
     count = lambda m: float((w[..., None] / (1.0 + np.exp(np.clip((eps - m) / max(T, 1e-12), -700, 700)))).sum())
     if abs(mu[2] - mu[3]) > 1e-11 * max(1.0, abs(mu[2])):
         assert abs(count(mu[2]) - count(mu[3])) <= 60 * 2.2e-16 * nb
+
+
+@pytest.mark.parametrize("nb", [2, 7, 8, 9, 13, 16, 17])
+@pytest.mark.parametrize("nk,dt", [(1, np.complex128), (37, np.complex64), (130, np.complex128)])
+def test_density_from_orbitals_shapes(cuda, nb, nk, dt):
+    """P = herm(Q diag(p) Q^H) over the lane groups and CTA remainders: nb products of numbers of
+    modulus <= 1, so 4 nb ulp of the storage precision."""
+    from jax_hf_b200 import linalg as L
+    rng = np.random.default_rng(nb + nk)
+    Q = S.haar_unitaries((nk,), nb, rng).astype(dt)
+    p = rng.uniform(0, 1, size=(nk, nb)).astype(np.zeros(1, dt).real.dtype)
+    P = L.density_from_Qp(torch.as_tensor(Q, device="cuda"), torch.as_tensor(p, device="cuda")).cpu().numpy()
+    ref = np.einsum("kin,kn,kjn->kij", Q.astype(np.complex128), p.astype(float), np.conj(Q.astype(np.complex128)))
+    assert np.abs(P - ref).max() <= 4 * nb * (1.2e-7 if dt == np.complex64 else 2.3e-16)
+    assert np.abs(P - np.conj(np.swapaxes(P, -1, -2))).max() == 0.0
