@@ -9,10 +9,10 @@
 // reading along a row of the copy stays clear of bank conflicts).
 // The retraction solves the Cayley transform directly,
 //   U(tau) = (I + tau d / 2)^{-1} (I - tau d / 2) = 2 (I + tau d / 2)^{-1} - I,
-// the form of _cayley_retract (solver.py:122-138), by Gauss-Jordan elimination
-// with partial pivoting (|re| + |im| pivots, as LAPACK's izamax); it equals the
-// spectral form of the reference loop (solver.py:161-197, eigh(i d)) up to
-// rounding and needs ~5x fewer FP64 operations per trial than a Jacobi eigh.
+// the form of _cayley_retract (solver.py:122-138), by in-place Gauss-Jordan
+// elimination; it equals the spectral form of the reference loop (solver.py:161-197,
+// eigh(i d)) up to rounding and needs ~10x fewer FP64 operations per trial than a
+// Jacobi eigh.
 #pragma once
 
 #include "common.cuh"
@@ -41,82 +41,48 @@ __device__ __forceinline__ double2 crecip(double2 z) {
   return make_double2(z.x * s, -z.y * s);
 }
 
-// element r of a register column (r runtime): a select chain, no local memory
-template <int NB>
-__device__ __forceinline__ double2 pick(const double2 (&v)[NB], int r) {
-  double2 o = v[0];
-#pragma unroll
-  for (int i = 1; i < NB; ++i)
-    if (i == r) o = v[i];
-  return o;
-}
-
 // Column c of U(tau) into u[] from column c of d (skew-Hermitian).  `on`: this lane
-// holds a real column of a live k-point.  SC: NB complex (pivot column), SX: one
-// shared matrix copy.  Warp-uniform control flow.
+// holds a real column of a live k-point.  SC: NB complex (the broadcast column).
+// Warp-uniform control flow.
+//
+// (I + tau d / 2)^{-1} by in-place Gauss-Jordan: step j turns column j into column j of the
+// inverse so far, so a lane updates one column of NB entries per step.  No pivoting: the
+// Hermitian part of I + tau d / 2 is I, and every Schur complement keeps a Hermitian part
+// >= I, so a pivot has modulus >= 1 and the elimination is stable (Golub & Van Loan,
+// Matrix Computations, sec. 4.3, on matrices with a positive definite Hermitian part).
+// Against the pivoted elimination of [M | I] it replaced (pivot search and run-time row
+// selects in every step, two columns per lane): the first line-search trial at 144 x 144,
+// nb = 8 takes 45 us (62 before; cold, launch list).
 template <int NB>
 __device__ __forceinline__ void cayley_cols(const double2 (&d)[NB], double tau, int c, bool on, double2* SC,
-                                            double2* SX, double2 (&u)[NB]) {
-  constexpr int LP = RowGroup<NB>::LP;
-  double2 m[NB], x[NB];
+                                            double2 (&u)[NB]) {
   const double h = 0.5 * tau;
 #pragma unroll
-  for (int r = 0; r < NB; ++r) {
-    m[r] = make_double2((r == c ? 1.0 : 0.0) + h * d[r].x, h * d[r].y);
-    x[r] = make_double2(r == c ? 1.0 : 0.0, 0.0);
-  }
-  unsigned used = 0;
-  int piv[NB];
+  for (int r = 0; r < NB; ++r) u[r] = make_double2((r == c ? 1.0 : 0.0) + h * d[r].x, h * d[r].y);
 #pragma unroll
   for (int j = 0; j < NB; ++j) {
     if (on && c == j) {
 #pragma unroll
-      for (int r = 0; r < NB; ++r) SC[r] = m[r];
+      for (int r = 0; r < NB; ++r) SC[r] = u[r];
     }
     __syncwarp();
-    // every lane finds the same pivot from the shared column (first maximum)
-    int p = 0;
-    double best = -1.0;
-#pragma unroll
-    for (int r = 0; r < NB; ++r) {
-      const double2 v = SC[r];
-      const double key = ((used >> r) & 1u) ? -1.0 : fabs(v.x) + fabs(v.y);
-      if (key > best) { best = key; p = r; }
-    }
-    piv[j] = p;
-    used |= 1u << p;
     if (on) {
-      const double2 ip = crecip(SC[p]);
-      const double2 mp = pick<NB>(m, p), xp = pick<NB>(x, p);
+      const double2 ip = crecip(SC[j]);
+      const double2 pj = c == j ? ip : cmul(u[j], ip);  // row j of the updated column
+      const double2 np = make_double2(-pj.x, -pj.y);
 #pragma unroll
       for (int r = 0; r < NB; ++r) {
-        if (r == p) continue;
-        const double2 l = cmul(SC[r], ip);
-        m[r] = csub(m[r], cmul(l, mp));
-        x[r] = csub(x[r], cmul(l, xp));
+        if (r == j) continue;
+        u[r] = cfma(SC[r], np, c == j ? make_double2(0.0, 0.0) : u[r]);
       }
+      u[j] = pj;
     }
     __syncwarp();
   }
-  // row piv[j] holds column j's only non-zero: (M^-1)[j][c] = x[piv[j]] / m_j, m_j = M'[piv[j]][j]
   if (on) {
 #pragma unroll
-    for (int r = 0; r < NB; ++r) SX[r * LP + c] = x[r];
-    int pc = piv[0];
-#pragma unroll
-    for (int i = 1; i < NB; ++i)
-      if (i == c) pc = piv[i];
-    SC[c] = pick<NB>(m, pc);  // lane c holds column c: its pivot entry M'[piv[c]][c]
+    for (int r = 0; r < NB; ++r) u[r] = make_double2(2.0 * u[r].x - (r == c ? 1.0 : 0.0), 2.0 * u[r].y);
   }
-  __syncwarp();
-  if (on) {
-#pragma unroll
-    for (int j = 0; j < NB; ++j) {
-      const double2 v = cmul(SX[piv[j] * LP + c], crecip(SC[j]));
-      u[j] = make_double2(2.0 * v.x - (j == c ? 1.0 : 0.0), 2.0 * v.y);
-    }
-  }
-  __syncwarp();
 }
 
 // ------------------------------------------------ density: p and P = herm(Q p Q^H)
@@ -403,7 +369,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, NT == 1 ? 3 : 1) k_cgr_trials(
     for (int it = 0; it < NT; ++it) {
       if (it < nt) {  // warp-uniform
         double2 u[NB];
-        cayley_cols<NB>(d, taus[it], c, on, SC, SX, u);  // ends with a warp barrier: SX is free again
+        cayley_cols<NB>(d, taus[it], c, on, SC, u);
         if (on) {
           const double et = diag_uhfu_col<NB>(u, SFt);
           const double pt = clip(pv - taus[it] * dpv, 1e-8, 1.0 - 1e-8);
@@ -426,7 +392,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, NT == 1 ? 3 : 1) k_cgr_trials(
               q_alt(a)[base + (size_t)r * NB] = acc;
             }
           }
-          __syncwarp();  // SX is the Cayley stage of the next k-point group
+          __syncwarp();  // SX takes the Q of the next k-point group
         }
       }
     }
@@ -471,7 +437,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, 3) k_cgr_update(CgArgs a) {
   __shared__ double2 st[kRowWarps][KPW][2 * MAT + NB];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane / G, c = lane % G;
   double2* SFt = st[w][g];
-  double2* SX = SFt + MAT;  // Cayley stage, then the copy of Q
+  double2* SX = SFt + MAT;  // copy of Q
   double2* SC = SX + MAT;
   const double tau = a.sc->tau_final;
   for (int kb = (blockIdx.x * kRowWarps + w) * KPW; kb < a.nk; kb += gridDim.x * kRowWarps * KPW) {
@@ -491,7 +457,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, 3) k_cgr_update(CgArgs a) {
     }
     __syncwarp();
     double2 u[NB];
-    cayley_cols<NB>(d, tau, c, on, SC, SX, u);  // ends with a warp barrier: SX is free again
+    cayley_cols<NB>(d, tau, c, on, SC, u);
     if (on) {
       a.eps[(size_t)k * NB + c] = diag_uhfu_col<NB>(u, SFt);
 #pragma unroll
