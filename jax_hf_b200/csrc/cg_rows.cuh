@@ -197,7 +197,6 @@ __global__ void __launch_bounds__(32 * kRowWarps, 4) k_cgr_grad1(CgArgs a) {
   constexpr int G = RG::G, KPW = RG::KPW, LP = RG::LP, MAT = RG::MAT;
   __shared__ double2 st[kRowWarps][KPW][2 * MAT];
   __shared__ double spv[kRowWarps][KPW][NB];
-  __shared__ double red[64];
   __shared__ double tot[kMaxSums];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane / G, c = lane % G;
   double2* SQ = st[w][g];
@@ -284,8 +283,8 @@ __global__ void __launch_bounds__(32 * kRowWarps, 4) k_cgr_grad1(CgArgs a) {
   acc[1].add(s1);
   acc[2].add(s2);
   acc[3].add(s3);
-  if (publish_partials<4>(acc, a.part, a.counter, red)) {
-    gather_partials<4>(a.part, a.counter, tot, red);
+  if (publish_partials<4>(acc, a.part, a.counter)) {
+    gather_partials<4>(a.part, a.counter, tot);
     if (threadIdx.x == 0) {
       CgScalars* s = a.sc;
       s->grad_norm = sqrt(fmax(0.0, tot[0]));
@@ -326,7 +325,6 @@ __global__ void __launch_bounds__(32 * kRowWarps, NT == 1 ? 3 : 1) k_cgr_trials(
   using RG = RowGroup<NB>;
   constexpr int G = RG::G, KPW = RG::KPW, LP = RG::LP, MAT = RG::MAT;
   __shared__ double2 st[kRowWarps][KPW][2 * MAT + NB];
-  __shared__ double red[64];
   __shared__ double tot[kMaxSums];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane / G, c = lane % G;
   double2* SFt = st[w][g];
@@ -404,8 +402,8 @@ __global__ void __launch_bounds__(32 * kRowWarps, NT == 1 ? 3 : 1) k_cgr_trials(
     acc[2 * i].add(se[i]);
     acc[2 * i + 1].add(sh[i]);
   }
-  if (publish_partials<2 * NT>(acc, a.part, a.counter, red)) {
-    gather_partials<2 * NT>(a.part, a.counter, tot, red);
+  if (publish_partials<2 * NT>(acc, a.part, a.counter)) {
+    gather_partials<2 * NT>(a.part, a.counter, tot);
     if (threadIdx.x == 0) {
       CgScalars* s = a.sc;
       const double Tm = fmax(a.T_r, 1e-14);

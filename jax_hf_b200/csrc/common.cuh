@@ -178,4 +178,45 @@ __device__ __forceinline__ KSum block_reduce(KSum v, double* sm) {
   return r;
 }
 
+// Block-wide compensated sums of NS quantities (block_reduce on each, the same trees), side by side: a compensated merge is a chain of ten dependent additions, so one
+// quantity after the other left the block waiting 2 NS times.  The warps' results go
+// through shared memory once, and warp w finishes quantities w, w + nw, ...  Returns the sums of
+// quantity q in lane 0 of warp q % nw; call with every thread.
+template <int NS, class Sink>
+__device__ __forceinline__ void block_reduce_all(KSum (&acc)[NS], Sink&& sink) {
+  constexpr int MW = 8;  // warps per block at most (256 threads)
+  __shared__ double2 part[NS][MW];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+#pragma unroll
+    for (int q = 0; q < NS; ++q) {
+      KSum o;
+      o.s = __shfl_xor_sync(0xffffffffu, acc[q].s, off);
+      o.c = __shfl_xor_sync(0xffffffffu, acc[q].c, off);
+      acc[q].merge(o);
+    }
+  }
+  __syncthreads();  // the previous use of part
+  if (lane == 0) {
+#pragma unroll
+    for (int q = 0; q < NS; ++q) part[q][wid] = make_double2(acc[q].s, acc[q].c);
+  }
+  __syncthreads();
+  for (int q = wid; q < NS; q += nw) {
+    KSum r;
+    if (lane < nw) {
+      r.s = part[q][lane].x;
+      r.c = part[q][lane].y;
+    }
+    for (int off = MW / 2; off > 0; off >>= 1) {  // the lanes from 8 on hold zeros, which change nothing
+      KSum o;
+      o.s = __shfl_xor_sync(0xffffffffu, r.s, off);
+      o.c = __shfl_xor_sync(0xffffffffu, r.c, off);
+      r.merge(o);
+    }
+    if (lane == 0) sink(q, r);
+  }
+}
+
 }  // namespace hf

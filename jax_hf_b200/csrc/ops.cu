@@ -17,14 +17,12 @@ constexpr int kOpsMaxSums = 32;
 __device__ __forceinline__ double sigm(double x) { return 1.0 / (1.0 + exp(-x)); }
 
 template <int NS>
-__device__ __forceinline__ void write_partials(KSum (&acc)[NS], double* part, double* sm) {
-  for (int q = 0; q < NS; ++q) {
-    KSum r = block_reduce(acc[q], sm);
-    if (threadIdx.x == 0) {
-      part[((size_t)blockIdx.x * NS + q) * 2] = r.s;
-      part[((size_t)blockIdx.x * NS + q) * 2 + 1] = r.c;
-    }
-  }
+__device__ __forceinline__ void write_partials(KSum (&acc)[NS], double* part, int ns = NS) {
+  block_reduce_all<NS>(acc, [&](int q, const KSum& r) {
+    if (q >= ns) return;
+    part[((size_t)blockIdx.x * ns + q) * 2] = r.s;
+    part[((size_t)blockIdx.x * ns + q) * 2 + 1] = r.c;
+  });
 }
 
 // Finish of the device reductions: sum q of ns gets one CTA, whose threads take the
@@ -76,7 +74,6 @@ __global__ void k_scf_residuals(int nk, int nb, const double2* __restrict__ F, c
                                 const int* __restrict__ comm_slot, size_t comm_stride) {
   if (comm && comm_slot) comm += (size_t)(*comm_slot) * comm_stride;
   extern __shared__ double2 smd[];
-  __shared__ double red[64];
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   const int nb2 = nb * nb;
   double2* f = smd + (size_t)wi * 3 * nb2;
@@ -109,7 +106,7 @@ __global__ void k_scf_residuals(int nk, int nb, const double2* __restrict__ F, c
     }
     __syncwarp();
   }
-  write_partials<3>(acc, part, red);
+  write_partials<3>(acc, part);
 }
 
 // ------------------------------------------------------- DIIS Gram matrix --
@@ -119,7 +116,6 @@ __global__ void k_scf_residuals(int nk, int nb, const double2* __restrict__ F, c
 template <int N>
 __global__ void k_gram(size_t stride, size_t len, int nb2, const double2* __restrict__ R,
                        const double* __restrict__ w, double* part) {
-  __shared__ double red[64];
   constexpr int np = N * (N + 1) / 2;
   // a thread sums its few elements in plain FP64; the thread, block and grid partials
   // are then merged with compensated (Neumaier) sums
@@ -137,16 +133,10 @@ __global__ void k_gram(size_t stride, size_t len, int nb2, const double2* __rest
 #pragma unroll
       for (int j = i; j < N; ++j, ++q) acc[q] = fma(wk, fma(r[i].x, r[j].x, r[i].y * r[j].y), acc[q]);
   }
+  KSum t[np];
 #pragma unroll
-  for (int q = 0; q < np; ++q) {
-    KSum t;
-    t.add(acc[q]);
-    KSum rr = block_reduce(t, red);
-    if (threadIdx.x == 0) {
-      part[((size_t)blockIdx.x * np + q) * 2] = rr.s;
-      part[((size_t)blockIdx.x * np + q) * 2 + 1] = rr.c;
-    }
-  }
+  for (int q = 0; q < np; ++q) t[q].add(acc[q]);
+  write_partials<np>(t, part);
 }
 
 // One row of the DIIS Gram matrix: b[j] = sum_k w_k Re tr(R_i^H R_j) for j < N and a
@@ -157,7 +147,6 @@ template <int N>
 __global__ void k_gram_row(size_t stride, size_t len, int nb2, const double2* __restrict__ R, int inew,
                            const double* __restrict__ w, double* part, const int* __restrict__ inew_dev = nullptr) {
   if (inew_dev) inew = *inew_dev;
-  __shared__ double red[64];
   double acc[N];
 #pragma unroll
   for (int q = 0; q < N; ++q) acc[q] = 0.0;
@@ -170,16 +159,10 @@ __global__ void k_gram_row(size_t stride, size_t len, int nb2, const double2* __
       acc[j] = fma(wk, fma(a.x, b.x, a.y * b.y), acc[j]);
     }
   }
+  KSum t[N];
 #pragma unroll
-  for (int q = 0; q < N; ++q) {
-    KSum t;
-    t.add(acc[q]);
-    KSum rr = block_reduce(t, red);
-    if (threadIdx.x == 0) {
-      part[((size_t)blockIdx.x * N + q) * 2] = rr.s;
-      part[((size_t)blockIdx.x * N + q) * 2 + 1] = rr.c;
-    }
-  }
+  for (int q = 0; q < N; ++q) t[q].add(acc[q]);
+  write_partials<N>(t, part);
 }
 
 // out = sum_i c_i X_i (+ optional herm)
@@ -218,7 +201,6 @@ __global__ void k_axpby_real(size_t n, double a, const double* __restrict__ x, d
 __global__ void k_jdot(size_t nk, int nb, const double2* __restrict__ aX, const double2* __restrict__ bX,
                        const double* __restrict__ wX, const double* __restrict__ ap, const double* __restrict__ bp,
                        const double* __restrict__ wp, double* part) {
-  __shared__ double red[64];
   KSum acc[1];
   const int nb2 = nb * nb;
   if (aX) {
@@ -235,7 +217,7 @@ __global__ void k_jdot(size_t nk, int nb, const double2* __restrict__ aX, const 
       acc[0].add(wk * ap[e] * bp[e]);
     }
   }
-  write_partials<1>(acc, part, red);
+  write_partials<1>(acc, part);
 }
 
 // Up to four joint inner products in one pass: product q is accumulated by every thread
@@ -251,7 +233,6 @@ struct JdotMulti {
 };
 
 __global__ void k_jdot_multi(size_t nk, int nb, const __grid_constant__ JdotMulti m, double* part) {
-  __shared__ double red[64];
   KSum acc[4];
   const int nb2 = nb * nb;
 #pragma unroll
@@ -273,15 +254,7 @@ __global__ void k_jdot_multi(size_t nk, int nb, const __grid_constant__ JdotMult
       }
     }
   }
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    if (q >= m.n) break;
-    KSum r = block_reduce(acc[q], red);
-    if (threadIdx.x == 0) {
-      part[((size_t)blockIdx.x * m.n + q) * 2] = r.s;
-      part[((size_t)blockIdx.x * m.n + q) * 2 + 1] = r.c;
-    }
-  }
+  write_partials<4>(acc, part, m.n);
 }
 
 // ---------------------------------------------------------------- Newton --
@@ -310,7 +283,6 @@ __global__ void k_newton_prec(size_t nk, int nb, const double2* __restrict__ rX,
                               const double* __restrict__ eps, const double* __restrict__ p, double lam, double T,
                               double clipv, const double* __restrict__ w2d, double2* __restrict__ zX,
                               double* __restrict__ zp, double* part) {
-  __shared__ double red[64];
   KSum acc[1];
   const int nb2 = nb * nb;
   const size_t n = nk * nb2;
@@ -328,7 +300,7 @@ __global__ void k_newton_prec(size_t nk, int nb, const double2* __restrict__ rX,
     zp[e] = z;
     acc[0].add(w2d[e / nb] * z);
   }
-  write_partials<1>(acc, part, red);
+  write_partials<1>(acc, part);
 }
 
 __global__ void k_sub_scalar(size_t n, double* __restrict__ x, const double* __restrict__ c, double scale) {
@@ -389,7 +361,6 @@ __global__ void k_newton_hvp(int nk, int nb, const double2* __restrict__ Q, cons
                              const double2* __restrict__ dPpen, double2* __restrict__ HX, double* __restrict__ Hp,
                              const double* __restrict__ w2d, double* part) {
   extern __shared__ double2 smd[];
-  __shared__ double red[64];
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   const int nb2 = nb * nb;
   double2* q = smd + (size_t)wi * 5 * nb2;
@@ -440,7 +411,7 @@ __global__ void k_newton_hvp(int nk, int nb, const double2* __restrict__ Q, cons
     }
     __syncwarp();
   }
-  write_partials<1>(acc, part, red);
+  write_partials<1>(acc, part);
 }
 
 // C = A B per k

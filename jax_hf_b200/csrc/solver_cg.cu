@@ -205,7 +205,6 @@ __global__ void k_cg_density(CgArgs a, int force) {
 __global__ void k_cg_grad1(CgArgs a) {
   if (!cg_active(a)) return;
   extern __shared__ double2 sm[];
-  __shared__ double red[64];
   __shared__ double tot[kMaxSums];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   const int nb = a.nb, nb2 = nb * nb;
@@ -252,8 +251,8 @@ __global__ void k_cg_grad1(CgArgs a) {
     }
     __syncwarp();
   }
-  if (publish_partials<4>(acc, a.part, a.counter, red)) {
-    gather_partials<4>(a.part, a.counter, tot, red);
+  if (publish_partials<4>(acc, a.part, a.counter)) {
+    gather_partials<4>(a.part, a.counter, tot);
     if (threadIdx.x == 0) {
       CgScalars* s = a.sc;
       s->grad_norm = sqrt(fmax(0.0, tot[0]));
@@ -276,7 +275,6 @@ __device__ __forceinline__ double2 precond(double2 g, double ei, double ej, doub
 template <int NB>
 __global__ void __launch_bounds__(256) k_cg_grad2_t(CgArgs a) {
   if (!cg_active(a)) return;
-  __shared__ double red[64];
   __shared__ double tot[kMaxSums];
   constexpr unsigned nb2 = NB * NB;
   const int par = a.sc->k & 1;
@@ -308,8 +306,8 @@ __global__ void __launch_bounds__(256) k_cg_grad2_t(CgArgs a) {
   acc[1].add(s1);
   acc[2].add(s2);
   acc[3].add(s3);
-  if (publish_partials<4>(acc, a.part, a.counter, red)) {
-    gather_partials<4>(a.part, a.counter, tot, red);
+  if (publish_partials<4>(acc, a.part, a.counter)) {
+    gather_partials<4>(a.part, a.counter, tot);
     if (threadIdx.x == 0) {
       CgScalars* sc = a.sc;
       const double num = tot[0] - tot[1] + tot[2] - tot[3];
@@ -324,7 +322,6 @@ __global__ void __launch_bounds__(256) k_cg_grad2_t(CgArgs a) {
 template <int NB>
 __global__ void __launch_bounds__(256) k_cg_dir_t(CgArgs a) {
   if (!cg_active(a)) return;
-  __shared__ double red[64];
   __shared__ double tot[kMaxSums];
   constexpr unsigned nb2 = NB * NB;
   const int par = a.sc->k & 1;
@@ -355,8 +352,8 @@ __global__ void __launch_bounds__(256) k_cg_dir_t(CgArgs a) {
   acc[0].add(s0);
   acc[1].add(s1);
   acc[2].add(s2);
-  if (publish_partials<3>(acc, a.part, a.counter, red)) {
-    gather_partials<3>(a.part, a.counter, tot, red);
+  if (publish_partials<3>(acc, a.part, a.counter)) {
+    gather_partials<3>(a.part, a.counter, tot);
     if (threadIdx.x == 0) {
       CgScalars* sc = a.sc;
       const double dn = sqrt(fmax(0.0, tot[0]));
@@ -372,7 +369,6 @@ __global__ void __launch_bounds__(256) k_cg_dir_t(CgArgs a) {
 // --------------------------------------------- grad2: PR+ inner products ---
 __global__ void k_cg_grad2(CgArgs a) {
   if (!cg_active(a)) return;
-  __shared__ double red[64];
   __shared__ double tot[kMaxSums];
   const int par = a.sc->k & 1;
   const double2* G = par ? a.G1 : a.G0;
@@ -400,8 +396,8 @@ __global__ void k_cg_grad2(CgArgs a) {
       acc[3].add(wk * gpp[vi] * hp);
     }
   }
-  if (publish_partials<4>(acc, a.part, a.counter, red)) {
-    gather_partials<4>(a.part, a.counter, tot, red);
+  if (publish_partials<4>(acc, a.part, a.counter)) {
+    gather_partials<4>(a.part, a.counter, tot);
     if (threadIdx.x == 0) {
       CgScalars* s = a.sc;
       const double num = tot[0] - tot[1] + tot[2] - tot[3];
@@ -417,7 +413,6 @@ __global__ void k_cg_grad2(CgArgs a) {
 __global__ void k_cg_dir(CgArgs a) {
   if (!cg_active(a)) return;
   extern __shared__ double2 sm[];
-  __shared__ double red[64];
   __shared__ double tot[kMaxSums];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   const int nb = a.nb, nb2 = nb * nb;
@@ -480,8 +475,8 @@ __global__ void k_cg_dir(CgArgs a) {
     for (int e = lane; e < nb2; e += 32) a.Fe[base + e] = ft[e];
     __syncwarp();
   }
-  if (publish_partials<3>(acc, a.part, a.counter, red)) {
-    gather_partials<3>(a.part, a.counter, tot, red);
+  if (publish_partials<3>(acc, a.part, a.counter)) {
+    gather_partials<3>(a.part, a.counter, tot);
     if (threadIdx.x == 0) {
       CgScalars* s = a.sc;
       const double dn = sqrt(fmax(0.0, tot[0]));
@@ -498,7 +493,6 @@ __global__ void k_cg_dir(CgArgs a) {
 // of the lane-per-row path needs no eigendecomposition of d.
 __global__ void k_cg_dir_lu(CgArgs a) {
   if (!cg_active(a)) return;
-  __shared__ double red[64];
   __shared__ double tot[kMaxSums];
   const int par = a.sc->k & 1;
   const double2* G = par ? a.G1 : a.G0;
@@ -524,8 +518,8 @@ __global__ void k_cg_dir_lu(CgArgs a) {
     acc[1].add(wk * ps * a.epsF[v]);
     acc[2].add(wk * ent_term(ps));
   }
-  if (publish_partials<3>(acc, a.part, a.counter, red)) {
-    gather_partials<3>(a.part, a.counter, tot, red);
+  if (publish_partials<3>(acc, a.part, a.counter)) {
+    gather_partials<3>(a.part, a.counter, tot);
     if (threadIdx.x == 0) {
       CgScalars* s = a.sc;
       const double dn = sqrt(fmax(0.0, tot[0]));
@@ -544,7 +538,6 @@ __global__ void k_cg_trials(CgArgs a, int i0, int i1, int last_chunk) {
   if (!cg_active(a)) return;
   if (a.sc->accepted) return;
   extern __shared__ double2 sm[];
-  __shared__ double red[64];
   __shared__ double tot[kMaxSums];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   const int nb = a.nb, nb2 = nb * nb;
@@ -576,8 +569,8 @@ __global__ void k_cg_trials(CgArgs a, int i0, int i1, int last_chunk) {
     }
     __syncwarp();
   }
-  if (publish_partials<2 * NT>(acc, a.part, a.counter, red)) {
-    gather_partials<2 * NT>(a.part, a.counter, tot, red);
+  if (publish_partials<2 * NT>(acc, a.part, a.counter)) {
+    gather_partials<2 * NT>(a.part, a.counter, tot);
     if (threadIdx.x == 0) {
       CgScalars* s = a.sc;
       const double Tm = fmax(a.T_r, 1e-14);

@@ -14,16 +14,13 @@ constexpr int kMaxSums = 20;     // partial sums per reduction
 // reads all partials (fixed order -> deterministic) through L2.
 template <int NS>
 __device__ __forceinline__ bool publish_partials(KSum (&acc)[NS], double* __restrict__ part,
-                                                 unsigned* __restrict__ counter, double* sm) {
-  for (int q = 0; q < NS; ++q) {
-    KSum r = block_reduce(acc[q], sm);
-    if (threadIdx.x == 0) {
-      part[((size_t)blockIdx.x * NS + q) * 2] = r.s;
-      part[((size_t)blockIdx.x * NS + q) * 2 + 1] = r.c;
-    }
-  }
+                                                 unsigned* __restrict__ counter) {
+  block_reduce_all<NS>(acc, [&](int q, const KSum& r) {
+    part[((size_t)blockIdx.x * NS + q) * 2] = r.s;
+    part[((size_t)blockIdx.x * NS + q) * 2 + 1] = r.c;
+    __threadfence();
+  });
   __shared__ bool s_last;
-  __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
     const unsigned t = atomicAdd(counter, 1u);
@@ -34,11 +31,12 @@ __device__ __forceinline__ bool publish_partials(KSum (&acc)[NS], double* __rest
 }
 
 // In the last CTA: totals[q] = sum over blocks.  Every thread sums a fixed
-// strided subset of the block partials, then one compensated block reduction per
-// quantity (fixed assignment and tree -> deterministic for a launch shape).
+// strided subset of the block partials, then one compensated block reduction
+// (fixed assignment and tree -> deterministic for a launch shape).
 template <int NS>
 __device__ __forceinline__ void gather_partials(const double* __restrict__ part, unsigned* __restrict__ counter,
-                                                double* totals, double* sm) {
+                                                double* totals) {
+  __threadfence();
   KSum t[NS];
   for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
 #pragma unroll
@@ -47,11 +45,7 @@ __device__ __forceinline__ void gather_partials(const double* __restrict__ part,
       t[q].add(__ldcg(part + ((size_t)b * NS + q) * 2 + 1));
     }
   }
-#pragma unroll
-  for (int q = 0; q < NS; ++q) {
-    const KSum r = block_reduce(t[q], sm);
-    if (threadIdx.x == 0) totals[q] = r.value();
-  }
+  block_reduce_all<NS>(t, [&](int q, const KSum& r) { totals[q] = r.value(); });
   __syncthreads();
   if (threadIdx.x == 0) *counter = 0u;
 }
