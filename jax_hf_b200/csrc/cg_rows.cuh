@@ -88,6 +88,7 @@ __device__ __forceinline__ void cayley_cols(const double2 (&d)[NB], double tau, 
 // ------------------------------------------------ density: p and P = herm(Q p Q^H)
 template <int NB>
 __global__ void __launch_bounds__(32 * kRowWarps) k_cgr_density(CgArgs a, int force) {
+  pdl_begin();
   if (!force && !cg_active(a)) return;
   double2* const Qc = q_cur(a);
   using RG = RowGroup<NB>;
@@ -143,6 +144,7 @@ template <int NB>
 __global__ void __launch_bounds__(32 * kRowWarps) k_rows_density(int nk, const double2* __restrict__ Q,
                                                                  const double* __restrict__ p,
                                                                  double2* __restrict__ P) {
+  pdl_begin();
   using RG = RowGroup<NB>;
   constexpr int G = RG::G, KPW = RG::KPW, LP = RG::LP, MAT = RG::MAT;
   __shared__ double2 st[kRowWarps][KPW][2 * MAT];
@@ -191,6 +193,7 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_rows_density(int nk, const d
 // 4 CTAs per SM: 128 registers without spills (16 warps per SM instead of 12)
 template <int NB>
 __global__ void __launch_bounds__(32 * kRowWarps, 4) k_cgr_grad1(CgArgs a) {
+  pdl_begin();
   if (!cg_active(a)) return;
   double2* const Qc = q_cur(a);
   using RG = RowGroup<NB>;
@@ -320,6 +323,7 @@ __device__ __forceinline__ double diag_uhfu_col(const double2 (&u)[NB], const do
 // trials keep the registers they need
 template <int NB, int NT>
 __global__ void __launch_bounds__(32 * kRowWarps, NT == 1 ? 3 : 1) k_cgr_trials(CgArgs a, int i0, int i1, int last_chunk) {
+  pdl_begin();
   if (!cg_active(a)) return;
   if (a.sc->accepted) return;
   using RG = RowGroup<NB>;
@@ -427,6 +431,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, NT == 1 ? 3 : 1) k_cgr_trials(
 // ----------------- retraction: U(tau), Q <- Q U, eps_new = diag(U^H Ft U)
 template <int NB>
 __global__ void __launch_bounds__(32 * kRowWarps, 3) k_cgr_update(CgArgs a) {
+  pdl_begin();
   if (!cg_active(a)) return;
   if (a.sc->first_ok) return;  // tau0 accepted: the first trial formed eps and Q U(tau0) already
   double2* const Qc = q_cur(a);
@@ -820,6 +825,7 @@ template <int NB>
 __global__ void __launch_bounds__(32 * kEigWarps, 8) k_eig_cols(int nk, const double2* __restrict__ A,
                                                              const double2* Qin, double2* Qout, double* eps,
                                                              double tol) {
+  pdl_begin();
   eig_cols<NB>(nk, A, Qin, Qout, eps, tol);
 }
 

@@ -219,4 +219,37 @@ __device__ __forceinline__ void block_reduce_all(KSum (&acc)[NS], Sink&& sink) {
   }
 }
 
+// ------------------------------------------------ programmatic dependent launch ----
+// griddepcontrol.wait: the grids before this one have completed and their writes are
+// visible (without the launch attribute it returns at once); launch_dependents lets the
+// next grid take its place on the SMs once every CTA of this one has got here.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+
+// First statement of every kernel that launch_pdl launches, ahead of any early return: a
+// grid that ended without waiting would let its successor start before its predecessor ended.
+__device__ __forceinline__ void pdl_begin() {
+  pdl_wait();
+  pdl_launch_dependents();
+}
+
+// Launches a kernel that starts with pdl_begin() so that its launch overlaps the end of the
+// one before it: the loops of the solvers are chains of kernels of a few microseconds, and
+// a plain launch in such a chain costs 1 to 1.5 us of idle GPU.  Errors are left for
+// HF_LAUNCH_CHECK.
+template <typename... P, typename... A>
+inline void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 }  // namespace hf

@@ -125,6 +125,7 @@ __device__ __forceinline__ bool qr_sweep(double (&d)[NB], double (&e)[NB], doubl
 template <typename RT, int NB>
 __global__ void __launch_bounds__(TriShape<NB>::MAXM * TriShape<NB>::G, TriShape<NB>::CTAS)
     k_eigh_tri(int nk, int mode, const cpx_t<RT>* __restrict__ A, RT* __restrict__ eps, cpx_t<RT>* V) {
+  pdl_begin();
   using S = TriShape<NB>;
   constexpr int G = S::G, LP = S::LP;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -372,7 +373,7 @@ int launch_tri(cudaStream_t s, int nk, int mode, const void* A, void* eps, void*
   while (mpc > 32 / S::G && (nk + mpc - 1) / mpc < 148) mpc >>= 1;
   const size_t smem = (size_t)mpc * S::BYTES;
   HF_SMEM_CAP(k_eigh_tri<RT, NB>);
-  k_eigh_tri<RT, NB><<<(nk + mpc - 1) / mpc, mpc * S::G, smem, s>>>(nk, mode, static_cast<const cpx_t<RT>*>(A),
+  launch_pdl(k_eigh_tri<RT, NB>, (nk + mpc - 1) / mpc, mpc * S::G, smem, s, nk, mode, static_cast<const cpx_t<RT>*>(A),
                                                                    static_cast<RT*>(eps), static_cast<cpx_t<RT>*>(V));
   HF_LAUNCH_CHECK("k_eigh_tri");
   return HF_OK;

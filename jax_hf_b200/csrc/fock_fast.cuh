@@ -48,15 +48,10 @@ __device__ __forceinline__ void cp_async8(void* dst, const void* src, bool valid
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
-// Programmatic dependent launch: the column and inverse row passes are launched
-// with programmatic stream serialization, so their CTAs may start (twiddle
-// tables, index setup) while the previous pass finishes; pdl_wait()
-// (griddepcontrol.wait: the previous grid has completed and its writes are
-// visible) comes before the first read of anything an earlier kernel wrote.
-// Without the launch attribute griddepcontrol.wait returns at once.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
-__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
-
+// Programmatic dependent launch: the passes are launched with programmatic stream
+// serialization, so their CTAs may start (twiddle tables, index setup) while the
+// previous pass, or whatever kernel comes before the build, finishes; pdl_wait() comes before the
+// first read of anything an earlier kernel wrote.
 // Launches kernel<<<grid, block, smem, stream>>>(p) with programmatic stream
 // serialization (and a cluster shape when csize > 0).
 template <typename K>
@@ -109,11 +104,8 @@ __device__ __forceinline__ void stage_row_fwd(const FockParams& p, cpx_t<FT>* st
 
 template <typename ST, typename FT, class S>
 __global__ void __launch_bounds__(16 * S::TPL) k_fast_row_fwd(const __grid_constant__ FockParams p) {
-  if (p.active && !*p.active) return;
-  pdl_launch_dependents();
   using SC = cpx_t<ST>;
   using FC = cpx_t<FT>;
-  zero_h<SC>(p);
   constexpr bool kStage = sizeof(SC) == sizeof(FC);  // mixed precision converts in registers
   extern __shared__ __align__(16) unsigned char smem_raw[];
   FC* twf = reinterpret_cast<FC*>(smem_raw);
@@ -123,6 +115,9 @@ __global__ void __launch_bounds__(16 * S::TPL) k_fast_row_fwd(const __grid_const
   const int t = threadIdx.x >> 4, s = threadIdx.x & 15, LS = p.LS;
   const int nitems = p.ngroups * p.nk1;
   build_line_twiddles<S, FT>(twf, twi);
+  pdl_begin();  // an earlier build on the stream may still read the scratch
+  if (p.active && !*p.active) return;
+  zero_h<SC>(p);
   const bool has_ref = (p.flags & HF_FOCK_HAS_REFP) != 0;
   int item = blockIdx.x;
   if (kStage && item < nitems) {
@@ -523,20 +518,16 @@ int fast_fock(FockParams& p, cudaStream_t stream, bool* handled) {
   if (p.LS > 16 || !fast_length(p.nk1) || !fast_length(p.nk2)) return HF_OK;
   const bool exch = (p.flags & HF_FOCK_EXCHANGE) != 0;
   int st = HF_OK;
-  auto row = [&](auto shape) {
-    using S = decltype(shape);
-    constexpr size_t sm = fast_smem<S, FT>();
-    if (!exch) return;
-    int grid = 0;
-    st = persistent_grid(k_fast_row_fwd<ST, FT, S>, 16 * S::TPL, sm, p.ngroups * p.nk1, &grid);
-    if (!st) k_fast_row_fwd<ST, FT, S><<<grid, 16 * S::TPL, sm, stream>>>(p);
-  };
   auto pass = [&](auto kern, int threads, size_t sm, int items, const char* what) {
     int grid = 0;
     st = persistent_grid(kern, threads, sm, items, &grid);
     if (st) return;
     const cudaError_t e = launch_pass(kern, grid, threads, sm, stream, p);
     if (e != cudaSuccess) st = cuda_check(e, what);
+  };
+  auto row = [&](auto shape) {
+    using S = decltype(shape);
+    if (exch) pass(k_fast_row_fwd<ST, FT, S>, 16 * S::TPL, fast_smem<S, FT>(), p.ngroups * p.nk1, "k_fast_row_fwd");
   };
   auto col = [&](auto shape) {
     using S = decltype(shape);
@@ -564,7 +555,6 @@ int fast_fock(FockParams& p, cudaStream_t stream, bool* handled) {
 #undef HF_CASE
   }
   if (st) return st;
-  HF_LAUNCH_CHECK("k_fast_row_fwd");
   if (exch) {
     switch (p.nk1) {
 #define HF_CASE(N, A, B, T) case N: col(LineShape<N, A, B, T>{}); break;

@@ -69,17 +69,17 @@ __device__ __forceinline__ void two_first_inv(FC* x, FC* buf, const FC* tw, int 
 
 template <typename ST, typename FT>
 __global__ void __launch_bounds__(16 * kTwoRadix, 2) k_two_row_fwd(const __grid_constant__ FockParams p) {
-  if (p.active && !*p.active) return;
-  pdl_launch_dependents();
   using SC = cpx_t<ST>;
   using FC = cpx_t<FT>;
-  zero_h<SC>(p);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   FC* tw = reinterpret_cast<FC*>(smem_raw);
   const int N = p.nk2, LS = p.LS;
   FC* buf = tw + N;
   const int s = threadIdx.x & 15;
   build_twiddles<FT>(tw, N);
+  pdl_begin();  // an earlier build on the stream may still read the scratch
+  if (p.active && !*p.active) return;
+  zero_h<SC>(p);
   const bool has_ref = (p.flags & HF_FOCK_HAS_REFP) != 0;
   __syncthreads();
   for (int item = blockIdx.x; item < p.ngroups * p.nk1; item += gridDim.x) {

@@ -30,32 +30,25 @@ int two_fock(FockParams& p, cudaStream_t stream, bool* handled) {
   auto dense = [](int f) { return (f >> 5) > kTwoRadix; };
   if (dense(fr)) p.dense_row = dense_pairs_per_walk(fr);
   if (dense(fc)) p.dense_col = dense_pairs_per_walk(fc);
-  auto pass = [&](auto kern, int f, int n, int items, bool pdl, const char* what) -> int {
+  auto pass = [&](auto kern, int f, int n, int items, const char* what) -> int {
     const int threads = dense(f) ? 16 * kDenseWorkers : 16 * ((f & 31) > (f >> 5) ? (f & 31) : (f >> 5));
     // twiddles and one or two buffers of 16 lines
     const size_t smem = (size_t)(dense(f) ? 33 : 17) * n * sizeof(cpx_t<FT>);
     int grid = 0;
     if (int e = persistent_grid(kern, threads, smem, items, &grid)) return e;
-    if (!pdl) {
-      kern<<<grid, threads, smem, stream>>>(p);
-      HF_LAUNCH_CHECK(what);
-      return HF_OK;
-    }
     const cudaError_t e = launch_pass(kern, grid, threads, smem, stream, p);
     return e == cudaSuccess ? HF_OK : cuda_check(e, what);
   };
   int st;
   if (exch) {
-    // a plain launch: with programmatic serialisation this pass could overwrite the scratch
-    // while an earlier build on the stream still reads it
-    st = pass(dense(fr) ? k_dense_row_fwd<ST, FT> : k_two_row_fwd<ST, FT>, fr, p.nk2, p.ngroups * p.nk1, false,
+    st = pass(dense(fr) ? k_dense_row_fwd<ST, FT> : k_two_row_fwd<ST, FT>, fr, p.nk2, p.ngroups * p.nk1,
               "k_two_row_fwd");
     if (st) return st;
     auto col = (p.flags & HF_FOCK_VR_REAL) ? (dense(fc) ? k_dense_col<ST, FT, true> : k_two_col<ST, FT, true>)
                                            : (dense(fc) ? k_dense_col<ST, FT, false> : k_two_col<ST, FT, false>);
-    if ((st = pass(col, fc, p.nk1, p.ngroups * p.nk2, true, "k_two_col"))) return st;
+    if ((st = pass(col, fc, p.nk1, p.ngroups * p.nk2, "k_two_col"))) return st;
   }
-  st = pass(dense(fr) ? k_dense_row_inv<ST, FT> : k_two_row_inv<ST, FT>, fr, p.nk2, p.ngroups * p.nk1, true,
+  st = pass(dense(fr) ? k_dense_row_inv<ST, FT> : k_two_row_inv<ST, FT>, fr, p.nk2, p.ngroups * p.nk1,
             "k_two_row_inv");
   if (st) return st;
   *handled = true;

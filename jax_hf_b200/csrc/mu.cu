@@ -298,6 +298,7 @@ enum MuStage { kStageRange, kStageScan, kStageCertify };
 
 template <typename RT, int STAGE>
 __global__ void __launch_bounds__(kPassThreads) k_mu_pass(const MuArgs a, MuState* st, double* part, bool final_pass) {
+  pdl_begin();
   if (a.active && !*a.active) return;
   if (STAGE != kStageRange && st->done) return;
   constexpr int K = STAGE == kStageRange ? 3 : STAGE == kStageScan ? 8 : 5;
@@ -505,6 +506,7 @@ static_assert(kOrdThreads / 32 >= kMuMaxCluster, "a warp per CTA of the cluster 
 // One evaluation of the Newton-bracket rule.  FIRST: at mu0, with the extremes already in st.
 template <typename RT, bool FIRST>
 __global__ void __launch_bounds__(kOrdThreads) k_mu_newton(const MuArgs a, int csize, MuState* st, double* part) {
+  pdl_begin();
   if (a.active && !*a.active) return;
   if (!FIRST && st->done) return;
   __shared__ double buf[2][kOrdParts][32 * kOrdWarps][3];
@@ -553,6 +555,7 @@ __global__ void __launch_bounds__(kOrdThreads) k_mu_newton(const MuArgs a, int c
 // Two levels of the bisection: the counts at the three midpoints, then the two decisions.
 template <typename RT>
 __global__ void __launch_bounds__(kOrdThreads) k_mu_levels(const MuArgs a, int csize, MuState* st, double* part) {
+  pdl_begin();
   if (a.active && !*a.active) return;
   if (st->fixed || st->it >= a.maxiter) return;
   __shared__ double buf[2][kOrdParts][32 * kOrdWarps][4];
@@ -602,6 +605,7 @@ __global__ void __launch_bounds__(kOrdThreads) k_mu_levels(const MuArgs a, int c
 // neither variant carries the other's registers (1024-thread CTAs have 64 per thread).
 template <typename RT, int BT, bool NEWTON>
 __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
+  pdl_begin();
   constexpr int L = BT <= 256 ? kBisLevels : 1, NODES = (1 << L) - 1;
   if (a.active && !*a.active) return;  // uniform across the cluster: no barrier is skipped by a subset
   // the grid-wide passes got there (uniform as well)
@@ -879,17 +883,17 @@ static int launch_passes(cudaStream_t s, const MuArgs& a, int csize, MuState* st
   int blocks = (a.n + kPassThreads - 1) / kPassThreads;
   if (blocks > kPassBlocks) blocks = kPassBlocks;
   const int ord = csize * (kMuThreads / (32 * kOrdWarps));
-  k_mu_pass<RT, kStageRange><<<blocks, kPassThreads, 0, s>>>(a, st, part, false);
+  launch_pdl(k_mu_pass<RT, kStageRange>, blocks, kPassThreads, 0, s, a, st, part, false);
   if (a.method == 2) {
-    k_mu_newton<RT, true><<<ord, kOrdThreads, 0, s>>>(a, csize, st, part);
-    for (int i = 0; i < kNewtonPasses; ++i) k_mu_newton<RT, false><<<ord, kOrdThreads, 0, s>>>(a, csize, st, part);
+    launch_pdl(k_mu_newton<RT, true>, ord, kOrdThreads, 0, s, a, csize, st, part);
+    for (int i = 0; i < kNewtonPasses; ++i) launch_pdl(k_mu_newton<RT, false>, ord, kOrdThreads, 0, s, a, csize, st, part);
     HF_LAUNCH_CHECK("k_mu_newton");
     return HF_OK;
   }
-  k_mu_pass<RT, kStageScan><<<blocks, kPassThreads, 0, s>>>(a, st, part, false);
+  launch_pdl(k_mu_pass<RT, kStageScan>, blocks, kPassThreads, 0, s, a, st, part, false);
   for (int i = 1; i < kCertPasses; ++i)
-    k_mu_pass<RT, kStageCertify><<<blocks, kPassThreads, 0, s>>>(a, st, part, i == kCertPasses - 1);
-  for (int i = 0; i < kLevelPasses; ++i) k_mu_levels<RT><<<ord, kOrdThreads, 0, s>>>(a, csize, st, part);
+    launch_pdl(k_mu_pass<RT, kStageCertify>, blocks, kPassThreads, 0, s, a, st, part, i == kCertPasses - 1);
+  for (int i = 0; i < kLevelPasses; ++i) launch_pdl(k_mu_levels<RT>, ord, kOrdThreads, 0, s, a, csize, st, part);
   HF_LAUNCH_CHECK("k_mu_pass");
   return HF_OK;
 }
@@ -1002,6 +1006,7 @@ int hf::find_mu_internal(void* stream, int dtype, int method, int nk1, int nk2, 
                          : launch_passes<double>(s, a, csize, st, part, ws_ready);
     if (e) return e;
     a.pre = st;
+    a.cache = 0;  // mostly nothing is left to do: no shared-memory cache to set up (the same order without it)
   }
   const size_t cache_bytes = (size_t)a.cache * threads * sizeof(double2);
   cudaLaunchConfig_t cfg = {};
@@ -1009,13 +1014,15 @@ int hf::find_mu_internal(void* stream, int dtype, int method, int nk1, int nk2, 
   cfg.blockDim = dim3(threads, 1, 1);
   cfg.dynamicSmemBytes = a.cache ? cache_bytes : 0;
   cfg.stream = static_cast<cudaStream_t>(stream);
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = csize;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   if (method != 0) {
     if (single) HF_CUDA(cudaLaunchKernelEx(&cfg, k_find_mu<float, kMuThreads, true>, a));
     else HF_CUDA(cudaLaunchKernelEx(&cfg, k_find_mu<double, kMuThreads, true>, a));

@@ -32,6 +32,7 @@ __device__ __forceinline__ void write_partials(KSum (&acc)[NS], double* part, in
 constexpr int kSumThreads = 128;
 __global__ void __launch_bounds__(kSumThreads) k_sum_partials(const double* __restrict__ part, int nblk, int ns,
                                                               double* __restrict__ out) {
+  pdl_begin();
   __shared__ double sm[2 * 32];
   const int q = blockIdx.x;
   KSum t;
@@ -56,6 +57,7 @@ static int nblocks(size_t n) {
 // mode 2: eps + level_shift (1 - fermidirac(eps - mu, T))           (reference_scf.py:92)
 __global__ void k_fermi(size_t n, const double* __restrict__ eps, const double* __restrict__ mu, double T,
                         int mode, double shift, double* __restrict__ out) {
+  pdl_begin();
   const double m = mu[0];
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
     const double x = eps[e];
@@ -72,6 +74,7 @@ __global__ void k_scf_residuals(int nk, int nb, const double2* __restrict__ F, c
                                 const double2* __restrict__ Pn, const double* __restrict__ w,
                                 double2* __restrict__ comm, double2* __restrict__ delta, double* part,
                                 const int* __restrict__ comm_slot, size_t comm_stride) {
+  pdl_begin();
   if (comm && comm_slot) comm += (size_t)(*comm_slot) * comm_stride;
   extern __shared__ double2 smd[];
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5, wpb = blockDim.x >> 5;
@@ -116,6 +119,7 @@ __global__ void k_scf_residuals(int nk, int nb, const double2* __restrict__ F, c
 template <int N>
 __global__ void k_gram(size_t stride, size_t len, int nb2, const double2* __restrict__ R,
                        const double* __restrict__ w, double* part) {
+  pdl_begin();
   constexpr int np = N * (N + 1) / 2;
   // a thread sums its few elements in plain FP64; the thread, block and grid partials
   // are then merged with compensated (Neumaier) sums
@@ -146,6 +150,7 @@ __global__ void k_gram(size_t stride, size_t len, int nb2, const double2* __rest
 template <int N>
 __global__ void k_gram_row(size_t stride, size_t len, int nb2, const double2* __restrict__ R, int inew,
                            const double* __restrict__ w, double* part, const int* __restrict__ inew_dev = nullptr) {
+  pdl_begin();
   if (inew_dev) inew = *inew_dev;
   double acc[N];
 #pragma unroll
@@ -168,6 +173,7 @@ __global__ void k_gram_row(size_t stride, size_t len, int nb2, const double2* __
 // out = sum_i c_i X_i (+ optional herm)
 __global__ void k_lincomb(int n, size_t stride, size_t len, int nb, const double2* __restrict__ X,
                           const double* __restrict__ c, double2* __restrict__ out) {
+  pdl_begin();
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < len; e += (size_t)gridDim.x * blockDim.x) {
     double2 acc = make_double2(0.0, 0.0);
     for (int i = 0; i < n; ++i) acc = cadd(acc, cscale(X[i * stride + e], c[i]));
@@ -178,6 +184,7 @@ __global__ void k_lincomb(int n, size_t stride, size_t len, int nb, const double
 // out = a x + b y, hermitised when herm != 0 (complex arrays, nb x nb per k)
 __global__ void k_axpby(size_t nk, int nb, double a, const double2* __restrict__ x, double b,
                         const double2* __restrict__ y, int herm, double2* __restrict__ out) {
+  pdl_begin();
   const int nb2 = nb * nb;
   const size_t n = nk * nb2;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
@@ -193,6 +200,7 @@ __global__ void k_axpby(size_t nk, int nb, double a, const double2* __restrict__
 
 __global__ void k_axpby_real(size_t n, double a, const double* __restrict__ x, double b,
                              const double* __restrict__ y, double* __restrict__ out) {
+  pdl_begin();
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x)
     out[e] = a * x[e] + (y ? b * y[e] : 0.0);
 }
@@ -201,6 +209,7 @@ __global__ void k_axpby_real(size_t n, double a, const double* __restrict__ x, d
 __global__ void k_jdot(size_t nk, int nb, const double2* __restrict__ aX, const double2* __restrict__ bX,
                        const double* __restrict__ wX, const double* __restrict__ ap, const double* __restrict__ bp,
                        const double* __restrict__ wp, double* part) {
+  pdl_begin();
   KSum acc[1];
   const int nb2 = nb * nb;
   if (aX) {
@@ -233,6 +242,7 @@ struct JdotMulti {
 };
 
 __global__ void k_jdot_multi(size_t nk, int nb, const __grid_constant__ JdotMulti m, double* part) {
+  pdl_begin();
   KSum acc[4];
   const int nb2 = nb * nb;
 #pragma unroll
@@ -261,6 +271,7 @@ __global__ void k_jdot_multi(size_t nk, int nb, const __grid_constant__ JdotMult
 // G = skew((p_j - p_i) Ft) offdiag, eps = Re diag(Ft)                 (solver.py:898-900)
 __global__ void k_orbital_grad(size_t nk, int nb, const double2* __restrict__ Ft, const double* __restrict__ p,
                                double2* __restrict__ G, double* __restrict__ eps) {
+  pdl_begin();
   const int nb2 = nb * nb;
   const size_t n = nk * nb2;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
@@ -283,6 +294,7 @@ __global__ void k_newton_prec(size_t nk, int nb, const double2* __restrict__ rX,
                               const double* __restrict__ eps, const double* __restrict__ p, double lam, double T,
                               double clipv, const double* __restrict__ w2d, double2* __restrict__ zX,
                               double* __restrict__ zp, double* part) {
+  pdl_begin();
   KSum acc[1];
   const int nb2 = nb * nb;
   const size_t n = nk * nb2;
@@ -304,6 +316,7 @@ __global__ void k_newton_prec(size_t nk, int nb, const double2* __restrict__ rX,
 }
 
 __global__ void k_sub_scalar(size_t n, double* __restrict__ x, const double* __restrict__ c, double scale) {
+  pdl_begin();
   const double v = c[0] * scale;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) x[e] -= v;
 }
@@ -311,6 +324,7 @@ __global__ void k_sub_scalar(size_t n, double* __restrict__ x, const double* __r
 // dP = herm(Q M Q^H), M = X o (p_j - p_i) + diag(dp)                 (solver.py:916-919)
 __global__ void k_newton_dP(int nk, int nb, const double2* __restrict__ Q, const double2* __restrict__ X,
                             const double* __restrict__ dp, const double* __restrict__ p, double2* __restrict__ dP) {
+  pdl_begin();
   extern __shared__ double2 smd[];
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   const int nb2 = nb * nb;
@@ -360,6 +374,7 @@ __global__ void k_newton_hvp(int nk, int nb, const double2* __restrict__ Q, cons
                              const double2* __restrict__ h, double T, double clipv, double pen,
                              const double2* __restrict__ dPpen, double2* __restrict__ HX, double* __restrict__ Hp,
                              const double* __restrict__ w2d, double* part) {
+  pdl_begin();
   extern __shared__ double2 smd[];
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   const int nb2 = nb * nb;
@@ -417,6 +432,7 @@ __global__ void k_newton_hvp(int nk, int nb, const double2* __restrict__ Q, cons
 // C = A B per k
 __global__ void k_matmul(int nk, int nb, const double2* __restrict__ A, const double2* __restrict__ B,
                          double2* __restrict__ Cm) {
+  pdl_begin();
   extern __shared__ double2 smd[];
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   const int nb2 = nb * nb;
@@ -437,6 +453,7 @@ __global__ void k_matmul(int nk, int nb, const double2* __restrict__ A, const do
 }
 
 __global__ void k_real_diag(size_t nk, int nb, const double2* __restrict__ A, double* __restrict__ d) {
+  pdl_begin();
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < nk * nb; e += (size_t)gridDim.x * blockDim.x) {
     const size_t k = e / nb;
     const int i = (int)(e - k * nb);
@@ -452,7 +469,7 @@ static int perk_grid(int nk) {
 
 static int finish(cudaStream_t s, double* part, int nblk, int ns, double* out) {
   HF_LAUNCH_CHECK("reduction kernel");
-  k_sum_partials<<<ns, kSumThreads, 0, s>>>(part, nblk, ns, out);
+  launch_pdl(k_sum_partials, ns, kSumThreads, 0, s, part, nblk, ns, out);
   HF_LAUNCH_CHECK("k_sum_partials");
   return HF_OK;
 }
@@ -473,7 +490,7 @@ extern "C" int hf_fermi(void* stream, size_t n, const double* eps, const double*
                         double shift, double* out) {
   if (!eps || !mu || !out || mode < 0 || mode > 2) return fail(HF_ERR_INVALID, "hf_fermi: bad argument");
   if (n == 0) return HF_OK;
-  k_fermi<<<nblocks(n), kOpsThreads, 0, HF_S>>>(n, eps, mu, T, mode, shift, out);
+  launch_pdl(k_fermi, nblocks(n), kOpsThreads, 0, HF_S, n, eps, mu, T, mode, shift, out);
   HF_LAUNCH_CHECK("k_fermi");
   return HF_OK;
 }
@@ -484,7 +501,7 @@ extern "C" int hf_scf_residuals(void* stream, int nk, int nb, const void* F, con
   const int g = perk_grid(nk);
   const size_t sm = (size_t)3 * nb * nb * sizeof(double2) * 4;
   HF_SMEM_CAP(k_scf_residuals);
-  k_scf_residuals<<<g, 128, sm, HF_S>>>(nk, nb, (const double2*)F, (const double2*)P, (const double2*)Pn, w,
+  launch_pdl(k_scf_residuals, g, 128, sm, HF_S, nk, nb, (const double2*)F, (const double2*)P, (const double2*)Pn, w,
                                         (double2*)comm, (double2*)delta, (double*)ws, nullptr, 0);
   return finish(HF_S, (double*)ws, g, 3, sums3);
 }
@@ -498,20 +515,21 @@ int hf::scf_residuals_slot(void* stream, int nk, int nb, const void* F, const vo
   const int g = perk_grid(nk);
   const size_t sm = (size_t)3 * nb * nb * sizeof(double2) * 4;
   HF_SMEM_CAP(k_scf_residuals);
-  k_scf_residuals<<<g, 128, sm, HF_S>>>(nk, nb, (const double2*)F, (const double2*)P, (const double2*)Pn, w,
+  launch_pdl(k_scf_residuals, g, 128, sm, HF_S, nk, nb, (const double2*)F, (const double2*)P, (const double2*)Pn, w,
                                         (double2*)R, (double2*)delta, (double*)ws, slot, stride);
   return finish(HF_S, (double*)ws, g, 3, sums3);
 }
 
 __global__ void k_copy_to_slot(size_t n, const double2* __restrict__ x, double2* __restrict__ hist,
                                const int* __restrict__ slot) {
+  pdl_begin();
   double2* dst = hist + (size_t)(*slot) * n;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x)
     dst[e] = x[e];
 }
 
 int hf::copy_to_slot(void* stream, size_t n, const void* x, void* hist, const int* slot) {
-  k_copy_to_slot<<<nblocks(n), kOpsThreads, 0, HF_S>>>(n, (const double2*)x, (double2*)hist, slot);
+  launch_pdl(k_copy_to_slot, nblocks(n), kOpsThreads, 0, HF_S, n, (const double2*)x, (double2*)hist, slot);
   HF_LAUNCH_CHECK("k_copy_to_slot");
   return HF_OK;
 }
@@ -524,7 +542,7 @@ int hf::gram_row_slot(void* stream, int n, const int* slot, size_t stride, int n
   switch (n) {
 #define HF_GRAM_ROW(N)                                                                                      \
   case N:                                                                                                   \
-    k_gram_row<N><<<g, kOpsThreads, 0, HF_S>>>(stride, len, nb * nb, (const double2*)R, 0, w, (double*)ws, \
+    launch_pdl(k_gram_row<N>, g, kOpsThreads, 0, HF_S, stride, len, nb * nb, (const double2*)R, 0, w, (double*)ws, \
                                                 slot);                                                      \
     break;
     HF_GRAM_ROW(1) HF_GRAM_ROW(2) HF_GRAM_ROW(3) HF_GRAM_ROW(4) HF_GRAM_ROW(5) HF_GRAM_ROW(6) HF_GRAM_ROW(7)
@@ -542,7 +560,7 @@ extern "C" int hf_gram(void* stream, int n, size_t stride, int nk, int nb, const
   const int g = nblocks(len);
   switch (n) {
 #define HF_GRAM(N) \
-  case N: k_gram<N><<<g, kOpsThreads, 0, HF_S>>>(stride, len, nb * nb, (const double2*)R, w, (double*)ws); break;
+  case N: launch_pdl(k_gram<N>, g, kOpsThreads, 0, HF_S, stride, len, nb * nb, (const double2*)R, w, (double*)ws); break;
     HF_GRAM(1) HF_GRAM(2) HF_GRAM(3) HF_GRAM(4) HF_GRAM(5) HF_GRAM(6)
 #undef HF_GRAM
   }
@@ -558,7 +576,7 @@ extern "C" int hf_gram_row(void* stream, int n, int i, size_t stride, int nk, in
   switch (n) {
 #define HF_GRAM_ROW(N)                                                                                    \
   case N:                                                                                                 \
-    k_gram_row<N><<<g, kOpsThreads, 0, HF_S>>>(stride, len, nb * nb, (const double2*)R, i, w, (double*)ws); \
+    launch_pdl(k_gram_row<N>, g, kOpsThreads, 0, HF_S, stride, len, nb * nb, (const double2*)R, i, w, (double*)ws, nullptr); \
     break;
     HF_GRAM_ROW(1) HF_GRAM_ROW(2) HF_GRAM_ROW(3) HF_GRAM_ROW(4) HF_GRAM_ROW(5) HF_GRAM_ROW(6) HF_GRAM_ROW(7)
     HF_GRAM_ROW(8) HF_GRAM_ROW(9) HF_GRAM_ROW(10) HF_GRAM_ROW(11) HF_GRAM_ROW(12) HF_GRAM_ROW(13)
@@ -570,7 +588,7 @@ extern "C" int hf_gram_row(void* stream, int n, int i, size_t stride, int nk, in
 
 extern "C" int hf_lincomb(void* stream, int n, size_t stride, size_t len, const void* X, const double* c, void* out) {
   if (n < 1 || !X || !c || !out) return fail(HF_ERR_INVALID, "hf_lincomb: bad argument");
-  k_lincomb<<<nblocks(len), kOpsThreads, 0, HF_S>>>(n, stride, len, 0, (const double2*)X, c, (double2*)out);
+  launch_pdl(k_lincomb, nblocks(len), kOpsThreads, 0, HF_S, n, stride, len, 0, (const double2*)X, c, (double2*)out);
   HF_LAUNCH_CHECK("k_lincomb");
   return HF_OK;
 }
@@ -579,7 +597,7 @@ extern "C" int hf_axpby(void* stream, size_t nk, int nb, double a, const void* x
                         int herm, void* out) {
   if (!x || !out) return fail(HF_ERR_INVALID, "hf_axpby: bad argument");
   if (herm && (out == x || out == y)) return fail(HF_ERR_INVALID, "hf_axpby: herm output may not alias inputs");
-  k_axpby<<<nblocks(nk * nb * nb), kOpsThreads, 0, HF_S>>>(nk, nb, a, (const double2*)x, b, (const double2*)y,
+  launch_pdl(k_axpby, nblocks(nk * nb * nb), kOpsThreads, 0, HF_S, nk, nb, a, (const double2*)x, b, (const double2*)y,
                                                          herm, (double2*)out);
   HF_LAUNCH_CHECK("k_axpby");
   return HF_OK;
@@ -588,7 +606,7 @@ extern "C" int hf_axpby(void* stream, size_t nk, int nb, double a, const void* x
 extern "C" int hf_axpby_real(void* stream, size_t n, double a, const double* x, double b, const double* y,
                              double* out) {
   if (!x || !out) return fail(HF_ERR_INVALID, "hf_axpby_real: bad argument");
-  k_axpby_real<<<nblocks(n), kOpsThreads, 0, HF_S>>>(n, a, x, b, y, out);
+  launch_pdl(k_axpby_real, nblocks(n), kOpsThreads, 0, HF_S, n, a, x, b, y, out);
   HF_LAUNCH_CHECK("k_axpby_real");
   return HF_OK;
 }
@@ -597,7 +615,7 @@ extern "C" int hf_jdot(void* stream, size_t nk, int nb, const void* aX, const vo
                        const double* ap, const double* bp, const double* wp, double* out, void* ws) {
   if (!out || !ws) return fail(HF_ERR_INVALID, "hf_jdot: bad argument");
   const int g = nblocks(nk * nb * nb);
-  k_jdot<<<g, kOpsThreads, 0, HF_S>>>(nk, nb, (const double2*)aX, (const double2*)bX, wX, ap, bp, wp, (double*)ws);
+  launch_pdl(k_jdot, g, kOpsThreads, 0, HF_S, nk, nb, (const double2*)aX, (const double2*)bX, wX, ap, bp, wp, (double*)ws);
   return finish(HF_S, (double*)ws, g, 1, out);
 }
 
@@ -618,13 +636,13 @@ int hf::jdot_multi(void* stream, size_t nk, int nb, int n, const void* const* aX
     m.d[q].wp = on ? wp[q] : nullptr;
   }
   const int g = nblocks(nk * nb * nb);
-  k_jdot_multi<<<g, kOpsThreads, 0, HF_S>>>(nk, nb, m, (double*)ws);
+  launch_pdl(k_jdot_multi, g, kOpsThreads, 0, HF_S, nk, nb, m, (double*)ws);
   return finish(HF_S, (double*)ws, g, n, out);
 }
 
 extern "C" int hf_orbital_grad(void* stream, size_t nk, int nb, const void* Ft, const double* p, void* G, double* eps) {
   if (!Ft || !p || !G) return fail(HF_ERR_INVALID, "hf_orbital_grad: bad argument");
-  k_orbital_grad<<<nblocks(nk * nb * nb), kOpsThreads, 0, HF_S>>>(nk, nb, (const double2*)Ft, p, (double2*)G, eps);
+  launch_pdl(k_orbital_grad, nblocks(nk * nb * nb), kOpsThreads, 0, HF_S, nk, nb, (const double2*)Ft, p, (double2*)G, eps);
   HF_LAUNCH_CHECK("k_orbital_grad");
   return HF_OK;
 }
@@ -635,14 +653,14 @@ extern "C" int hf_newton_prec(void* stream, size_t nk, int nb, const void* rX, c
   if (!rX || !rp || !eps || !p || !w2d || !zX || !zp || !wsum_out || !ws)
     return fail(HF_ERR_INVALID, "hf_newton_prec: bad argument");
   const int g = nblocks(nk * nb * nb);
-  k_newton_prec<<<g, kOpsThreads, 0, HF_S>>>(nk, nb, (const double2*)rX, rp, eps, p, lam, T, clipv, w2d,
+  launch_pdl(k_newton_prec, g, kOpsThreads, 0, HF_S, nk, nb, (const double2*)rX, rp, eps, p, lam, T, clipv, w2d,
                                              (double2*)zX, zp, (double*)ws);
   return finish(HF_S, (double*)ws, g, 1, wsum_out);
 }
 
 extern "C" int hf_sub_scalar(void* stream, size_t n, double* x, const double* c, double scale) {
   if (!x || !c) return fail(HF_ERR_INVALID, "hf_sub_scalar: bad argument");
-  k_sub_scalar<<<nblocks(n), kOpsThreads, 0, HF_S>>>(n, x, c, scale);
+  launch_pdl(k_sub_scalar, nblocks(n), kOpsThreads, 0, HF_S, n, x, c, scale);
   HF_LAUNCH_CHECK("k_sub_scalar");
   return HF_OK;
 }
@@ -652,7 +670,7 @@ extern "C" int hf_newton_dP(void* stream, int nk, int nb, const void* Q, const v
   if (!Q || !X || !dp || !p || !dP || nb > 32) return fail(HF_ERR_INVALID, "hf_newton_dP: bad argument");
   const size_t sm = (size_t)3 * nb * nb * sizeof(double2) * 4;
   HF_SMEM_CAP(k_newton_dP);
-  k_newton_dP<<<perk_grid(nk), 128, sm, HF_S>>>(nk, nb, (const double2*)Q, (const double2*)X, dp, p, (double2*)dP);
+  launch_pdl(k_newton_dP, perk_grid(nk), 128, sm, HF_S, nk, nb, (const double2*)Q, (const double2*)X, dp, p, (double2*)dP);
   HF_LAUNCH_CHECK("k_newton_dP");
   return HF_OK;
 }
@@ -666,7 +684,7 @@ extern "C" int hf_newton_hvp(void* stream, int nk, int nb, const void* Q, const 
   const int g = perk_grid(nk);
   const size_t sm = (size_t)5 * nb * nb * sizeof(double2) * 4;
   HF_SMEM_CAP(k_newton_hvp);
-  k_newton_hvp<<<g, 128, sm, HF_S>>>(nk, nb, (const double2*)Q, (const double2*)Ft, (const double2*)X, dp, p,
+  launch_pdl(k_newton_hvp, g, 128, sm, HF_S, nk, nb, (const double2*)Q, (const double2*)Ft, (const double2*)X, dp, p,
                                      (const double2*)Fr, (const double2*)h, T, clipv, pen, (const double2*)dPpen,
                                      (double2*)HX, Hp, w2d, (double*)ws);
   return finish(HF_S, (double*)ws, g, 1, wsum_out);
@@ -676,14 +694,14 @@ extern "C" int hf_matmul(void* stream, int nk, int nb, const void* A, const void
   if (!A || !B || !C || nb > 32) return fail(HF_ERR_INVALID, "hf_matmul: bad argument");
   const size_t sm = (size_t)2 * nb * nb * sizeof(double2) * 4;
   HF_SMEM_CAP(k_matmul);
-  k_matmul<<<perk_grid(nk), 128, sm, HF_S>>>(nk, nb, (const double2*)A, (const double2*)B, (double2*)C);
+  launch_pdl(k_matmul, perk_grid(nk), 128, sm, HF_S, nk, nb, (const double2*)A, (const double2*)B, (double2*)C);
   HF_LAUNCH_CHECK("k_matmul");
   return HF_OK;
 }
 
 extern "C" int hf_real_diag(void* stream, size_t nk, int nb, const void* A, double* d) {
   if (!A || !d) return fail(HF_ERR_INVALID, "hf_real_diag: bad argument");
-  k_real_diag<<<nblocks(nk * nb), kOpsThreads, 0, HF_S>>>(nk, nb, (const double2*)A, d);
+  launch_pdl(k_real_diag, nblocks(nk * nb), kOpsThreads, 0, HF_S, nk, nb, (const double2*)A, d);
   HF_LAUNCH_CHECK("k_real_diag");
   return HF_OK;
 }

@@ -17,11 +17,9 @@ static int red_blocks(size_t n) {
   return (int)b;
 }
 
-// Launched with programmatic stream serialization behind its partial sums: it is in place
-// when they end, and griddepcontrol.wait holds it until their writes are visible.
 __global__ void k_red_final(const double* __restrict__ part, int nparts, int mode, double T,
                             const double* __restrict__ E, double* __restrict__ out, const int* active) {
-  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  pdl_begin();
   if (active && !*active) return;
   __shared__ double sm[64];
   KSum acc;
@@ -43,6 +41,7 @@ __global__ void __launch_bounds__(kRedThreads)
 k_energy_part(int nk, int nb, const cpx_t<RT>* __restrict__ P, const cpx_t<RT>* __restrict__ h,
               const cpx_t<RT>* __restrict__ S, const cpx_t<RT>* __restrict__ H, int H_mode,
               const RT* __restrict__ w, double* __restrict__ part, const int* active) {
+  pdl_begin();
   if (active && !*active) return;
   __shared__ double sm[64];
   const int nb2 = nb * nb;
@@ -71,6 +70,7 @@ template <typename RT>
 __global__ void __launch_bounds__(kRedThreads)
 k_entropy_part(int nk, int nb, const RT* __restrict__ p, const RT* __restrict__ w,
                double* __restrict__ part) {
+  pdl_begin();
   __shared__ double sm[64];
   const size_t n = (size_t)nk * nb;
   KSum acc;
@@ -85,16 +85,8 @@ k_entropy_part(int nk, int nb, const RT* __restrict__ p, const RT* __restrict__ 
 
 static int launch_final(cudaStream_t s, const double* part, int nparts, int mode, double T, const double* E,
                         double* out, const int* active) {
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.gridDim = dim3(1);
-  cfg.blockDim = dim3(256);
-  cfg.stream = s;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  HF_CUDA(cudaLaunchKernelEx(&cfg, k_red_final, part, nparts, mode, T, E, out, active));
+  launch_pdl(k_red_final, 1, 256, 0, s, part, nparts, mode, T, E, out, active);
+  HF_LAUNCH_CHECK("k_red_final");
   return HF_OK;
 }
 
@@ -142,11 +134,11 @@ int hf::energy_internal(void* stream, int dtype, int nk1, int nk2, int nb, const
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   double* part = static_cast<double*>(workspace);
   if (dtype == HF_C128)
-    k_energy_part<double><<<nbk, kRedThreads, 0, s>>>(nk, nb, (const double2*)P, (const double2*)h,
+    launch_pdl(k_energy_part<double>, nbk, kRedThreads, 0, s, nk, nb, (const double2*)P, (const double2*)h,
                                                       (const double2*)Sigma, (const double2*)H, H_mode,
                                                       (const double*)w2d, part, active);
   else
-    k_energy_part<float><<<nbk, kRedThreads, 0, s>>>(nk, nb, (const float2*)P, (const float2*)h,
+    launch_pdl(k_energy_part<float>, nbk, kRedThreads, 0, s, nk, nb, (const float2*)P, (const float2*)h,
                                                      (const float2*)Sigma, (const float2*)H, H_mode,
                                                      (const float*)w2d, part, active);
   HF_LAUNCH_CHECK("k_energy_part");
@@ -168,9 +160,9 @@ static int entropy_common(void* stream, int dtype, int nk1, int nk2, int nb, con
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   double* part = static_cast<double*>(workspace);
   if (dtype == HF_C128)
-    k_entropy_part<double><<<nbk, kRedThreads, 0, s>>>(nk, nb, (const double*)p, (const double*)w_norm, part);
+    launch_pdl(k_entropy_part<double>, nbk, kRedThreads, 0, s, nk, nb, (const double*)p, (const double*)w_norm, part);
   else
-    k_entropy_part<float><<<nbk, kRedThreads, 0, s>>>(nk, nb, (const float*)p, (const float*)w_norm, part);
+    launch_pdl(k_entropy_part<float>, nbk, kRedThreads, 0, s, nk, nb, (const float*)p, (const float*)w_norm, part);
   HF_LAUNCH_CHECK("k_entropy_part");
   return launch_final(s, part, nbk, mode, T, E, out, nullptr);
 }

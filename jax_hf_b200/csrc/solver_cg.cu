@@ -274,6 +274,7 @@ __device__ __forceinline__ double2 precond(double2 g, double ei, double ej, doub
 // double partials and compensated sums across threads and blocks.
 template <int NB>
 __global__ void __launch_bounds__(256) k_cg_grad2_t(CgArgs a) {
+  pdl_begin();
   if (!cg_active(a)) return;
   __shared__ double tot[kMaxSums];
   constexpr unsigned nb2 = NB * NB;
@@ -321,6 +322,7 @@ __global__ void __launch_bounds__(256) k_cg_grad2_t(CgArgs a) {
 
 template <int NB>
 __global__ void __launch_bounds__(256) k_cg_dir_t(CgArgs a) {
+  pdl_begin();
   if (!cg_active(a)) return;
   __shared__ double tot[kMaxSums];
   constexpr unsigned nb2 = NB * NB;
@@ -624,6 +626,7 @@ __global__ void k_cg_update(CgArgs a) {
 // floor phase_rel |E|; k_base restarts the plateau window at the FP64 switch
 // (k_base = 0 reproduces the reference rule exactly).
 __global__ void k_cg_step_end(CgArgs a, double phase_rel) {
+  pdl_begin();
   if (!cg_active(a)) return;
   CgScalars* s = a.sc;
   const int k = s->k;
@@ -789,40 +792,40 @@ static int cg_iteration_rows(CgRun& r, cudaStream_t s, const hf_cg_config& cf, b
   const int* act = &r.a.sc->active;
   const int rb = row_blocks(r.a.nk, RowGroup<NB>::KPW);
   const int eb = perk_blocks(r.a.nk);
-  k_cgr_density<NB><<<rb, 32 * kRowWarps, 0, s>>>(r.a, 0);
+  launch_pdl(k_cgr_density<NB>, rb, 32 * kRowWarps, 0, s, r.a, 0);
   HF_LAUNCH_CHECK("k_cgr_density");
   int st = cg_project(r, s);
   if (st) return st;
   if ((st = cg_fock(r, s, fp32, act))) return st;
   if ((st = cg_energy(r, s, &r.a.sc->E, act))) return st;
-  k_cgr_grad1<NB><<<rb, 32 * kRowWarps, 0, s>>>(r.a);
+  launch_pdl(k_cgr_grad1<NB>, rb, 32 * kRowWarps, 0, s, r.a);
   HF_LAUNCH_CHECK("k_cgr_grad1");
   const int gb = elem_blocks((size_t)r.a.nk * NB * NB);
-  k_cg_grad2_t<NB><<<gb, 256, 0, s>>>(r.a);
+  launch_pdl(k_cg_grad2_t<NB>, gb, 256, 0, s, r.a);
   HF_LAUNCH_CHECK("k_cg_grad2");
-  k_cg_dir_t<NB><<<gb, 256, 0, s>>>(r.a);
+  launch_pdl(k_cg_dir_t<NB>, gb, 256, 0, s, r.a);
   HF_LAUNCH_CHECK("k_cg_dir");
   const int bt = cf.bt_max;
   if (bt >= 1) {
-    k_cgr_trials<NB, 1><<<rb, 32 * kRowWarps, 0, s>>>(r.a, 0, 1, bt == 1);
+    launch_pdl(k_cgr_trials<NB, 1>, rb, 32 * kRowWarps, 0, s, r.a, 0, 1, bt == 1);
     HF_LAUNCH_CHECK("k_cgr_trials");
     for (int i0 = 1; i0 < bt; i0 += 8) {
       const int i1 = i0 + 8 < bt ? i0 + 8 : bt;
-      k_cgr_trials<NB, 8><<<rb, 32 * kRowWarps, 0, s>>>(r.a, i0, i1, i1 == bt);
+      launch_pdl(k_cgr_trials<NB, 8>, rb, 32 * kRowWarps, 0, s, r.a, i0, i1, i1 == bt);
       HF_LAUNCH_CHECK("k_cgr_trials");
     }
   }
-  k_cgr_update<NB><<<rb, 32 * kRowWarps, 0, s>>>(r.a);
+  launch_pdl(k_cgr_update<NB>, rb, 32 * kRowWarps, 0, s, r.a);
   HF_LAUNCH_CHECK("k_cgr_update");
   if ((st = cg_mu(r, s, cf.mu_maxiter, act))) return st;
-  k_cg_step_end<<<1, 1, 0, s>>>(r.a, fp32 ? cf.fp32_switch_rel : 0.0);
+  launch_pdl(k_cg_step_end, 1, 1, 0, s, r.a, fp32 ? cf.fp32_switch_rel : 0.0);
   HF_LAUNCH_CHECK("k_cg_step_end");
   return HF_OK;
 }
 
 template <int NB>
 static int cg_density_rows(CgRun& r, cudaStream_t s, int force) {
-  k_cgr_density<NB><<<row_blocks(r.a.nk, RowGroup<NB>::KPW), 32 * kRowWarps, 0, s>>>(r.a, force);
+  launch_pdl(k_cgr_density<NB>, row_blocks(r.a.nk, RowGroup<NB>::KPW), 32 * kRowWarps, 0, s, r.a, force);
   HF_LAUNCH_CHECK("k_cgr_density");
   return HF_OK;
 }
@@ -854,7 +857,7 @@ static int cg_eig(CgRun& r, cudaStream_t s, const double2* A, int rotate) {
 
 template <int NB>
 static int rows_density_launch(cudaStream_t s, int nk, const double2* Q, const double* p, double2* P) {
-  k_rows_density<NB><<<row_blocks(nk, RowGroup<NB>::KPW), 32 * kRowWarps, 0, s>>>(nk, Q, p, P);
+  launch_pdl(k_rows_density<NB>, row_blocks(nk, RowGroup<NB>::KPW), 32 * kRowWarps, 0, s, nk, Q, p, P);
   HF_LAUNCH_CHECK("k_rows_density");
   return HF_OK;
 }
@@ -878,7 +881,7 @@ static int eig_cols_launch(cudaStream_t s, int nk, const double2* A, const doubl
   const int per_block = kEigWarps * RowGroup<NB>::KPW;
   int b = (nk + per_block - 1) / per_block;
   if (b > 148 * 32) b = 148 * 32;
-  k_eig_cols<NB><<<b < 1 ? 1 : b, 32 * kEigWarps, 0, s>>>(nk, A, Qin, Qout, eps, kEigTol);
+  launch_pdl(k_eig_cols<NB>, b < 1 ? 1 : b, 32 * kEigWarps, 0, s, nk, A, Qin, Qout, eps, kEigTol);
   HF_LAUNCH_CHECK("k_eig_cols");
   return HF_OK;
 }
@@ -932,7 +935,7 @@ static int cg_iteration_warp(CgRun& r, cudaStream_t s, const hf_cg_config& cf, b
   HF_LAUNCH_CHECK("k_cg_update");
   st = cg_mu(r, s, cf.mu_maxiter, act);
   if (st) return st;
-  k_cg_step_end<<<1, 1, 0, s>>>(r.a, phase_rel);
+  launch_pdl(k_cg_step_end, 1, 1, 0, s, r.a, phase_rel);
   HF_LAUNCH_CHECK("k_cg_step_end");
   return HF_OK;
 }
