@@ -673,9 +673,21 @@ static int launch_fock(FockParams& p, cudaStream_t stream, bool need_consts, con
     bool handled = false;
     int st = pipe_fock<ST, FT>(p, stream, &handled);
     if (st != HF_OK || handled) return st;
-    st = fast_fock<ST, FT>(p, stream, &handled);
-    if (st != HF_OK || handled) return st;
-    if (!(p.flags & HF_FOCK_NO_TWO_FACTOR)) {
+    // Sides with a line shape take the register passes, but on the tile plan not those whose shape puts 24
+    // elements on a thread (96 and 192: 64 and 128 threads a CTA, too few in flight behind the gathers of the
+    // slots).  The two-factor passes put 12 threads on a line of 96 and 16 on one of 192: packed c128 builds of
+    // 96 x 96 x 4, x 8, x 16 take 17.0, 22.9, 67.4 us against 20.4, 32.8, 85.3, of 192 x 192 x 4, x 8 30.2, 69.8
+    // against 33.7, 83.6 (c64 x 8: 19.5 against 22.2, 53.4 against 58.4).  The shapes with 8 to 16 elements a
+    // thread keep the register passes, whose DFTs have no run-time switch: 72 and 144 sides lose 3 to 25 %, 16 to
+    // 36 up to 40 %; and so does the row plan (96 x 96 x 4 14.4 us against 16.8).
+    const bool two = !(p.flags & HF_FOCK_NO_TWO_FACTOR);
+    const bool deep = two && !p.rows_plan && !(p.flags & HF_FOCK_TILE_PLAN) && fast_per_thread(p.nk1) >= 24 &&
+                      fast_per_thread(p.nk2) >= 24;
+    if (!deep) {
+      st = fast_fock<ST, FT>(p, stream, &handled);
+      if (st != HF_OK || handled) return st;
+    }
+    if (two) {
       st = two_fock<ST, FT>(p, stream, &handled);
       if (st != HF_OK || handled) return st;
     }

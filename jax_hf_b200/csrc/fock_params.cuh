@@ -79,6 +79,16 @@ inline bool fast_length(int n) {
   }
 }
 
+// Elements of a line that a thread of the side's shape holds (0 without a shape).
+inline int fast_per_thread(int n) {
+  switch (n) {
+#define HF_CASE(N, A, B, T) case N: return N / T;
+    HF_FAST_SHAPES(HF_CASE)
+#undef HF_CASE
+    default: return 0;
+  }
+}
+
 // Factors of a mesh side as N1 | N2 << 5 for the two-factor passes, 0 when they leave the side
 // to the Stockham stages: N1 <= N2 <= 16, the pair nearest to square (fock_two.cuh); else, for
 // a side with a prime factor of 17 or more, the largest N1 <= 16 that keeps it in N2 <= 224

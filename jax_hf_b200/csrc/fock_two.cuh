@@ -1,6 +1,7 @@
 // Fock-build passes for mesh sides that are a product of two factors of at most 16
 // (every composite side up to 256 without a prime factor above 13; 25, 49, 75, 90, 100,
-// 120, ...) and have no compile-time line shape of their own.
+// 120, ...) and have no compile-time line shape of their own, and for 96 and 192 on the tile
+// plan, where they are faster than the register passes (launch_fock has the figures).
 //
 // A line of N = N1 N2 points is transformed in two register DFTs with one exchange through
 // shared memory, as in the register engine (fft_reg.cuh), but N1 and N2 are run-time

@@ -509,7 +509,7 @@ TWO_FACTOR = [  # sides: prime radices, one-factor sides, unequal factors, the l
 
 @pytest.mark.parametrize("n1,n2,nb,V,mode", TWO_FACTOR)
 @pytest.mark.parametrize("terms", [False, True])
-def test_two_factor_passes_match_stockham(cuda, n1, n2, nb, V, mode, terms):
+def test_two_factor_passes_match_stockham(cuda, n1, n2, nb, V, mode, terms, register_side=False):
     """Sides with two factors of at most 16 against the Stockham engine on the same inputs (FP64: both
     within 1e-12 of the oracle, so within 2e-12 of each other; FP32 transforms: 2 x 2e-5), with and
     without the reference density, Hartree and contact terms, for a density that is not Hermitian
@@ -542,8 +542,8 @@ def test_two_factor_passes_match_stockham(cuda, n1, n2, nb, V, mode, terms):
     tol = 2 * (TOL64 if mode == "c128" else TOL32)
     for x, y in zip(run(), run(engine="generic")):
         assert rel(x, y.cpu().numpy()) < tol if y.abs().max() > 0 else torch.equal(x, y)
-    for x, y in zip(run(engine="stockham"), run(engine="generic")):
-        assert torch.equal(x, y)
+    for x, y in zip(run(engine="stockham"), run(engine="generic")):  # the register passes at their sides
+        assert register_side or torch.equal(x, y)
 
 
 DENSE = [  # sides with a prime factor of 17 or more: one row, several rows, an even N2, both sides, the largest
@@ -557,6 +557,18 @@ DENSE = [  # sides with a prime factor of 17 or more: one row, several rows, an 
 @pytest.mark.parametrize("terms", [False, True])
 def test_dense_line_sums_match_stockham(cuda, n1, n2, nb, V, mode, terms):
     test_two_factor_passes_match_stockham(cuda, n1, n2, nb, V, mode, terms)
+
+
+DEEP = [  # register sides that the slot tiles leave to the two-factor passes, and one that keeps the pair on the other
+    (96, 96, 4, "scalar", "c128"), (96, 192, 9, "layer", "c64"), (192, 96, 3, "scalar", "fp32fft"),
+    (192, 128, 4, "scalar", "c128"),
+]
+
+
+@pytest.mark.parametrize("n1,n2,nb,V,mode", DEEP)
+@pytest.mark.parametrize("terms", [False, True])
+def test_slot_tiles_of_deep_line_shapes_match_stockham(cuda, n1, n2, nb, V, mode, terms):
+    test_two_factor_passes_match_stockham(cuda, n1, n2, nb, V, mode, terms, register_side=True)
 
 
 @pytest.mark.parametrize("shape,T,kind", [((70, 59, 4), 0.1, "metal"), ((128, 128, 1), 0.02, "metal"),
