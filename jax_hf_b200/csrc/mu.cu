@@ -136,21 +136,31 @@ __device__ __forceinline__ void cluster_sum2(cg::cluster_group& cl, double& x, d
 
 // Cluster-wide sums of K values (as cluster_sum2); v[] holds this thread's terms
 // on entry and the totals on return.  bsm: 32 * K + K doubles, slots: [2][K].
-template <int K>
+// RANGE: v[0] is a minimum and v[1] a maximum instead.
+template <int K, bool RANGE = false>
 __device__ __forceinline__ void cluster_sum_n(cg::cluster_group& cl, double (&v)[K], double (*slots)[K], double* bsm,
                                               int parity) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  auto reduce = [](int j, double x) {
+    if (!RANGE || j > 1) return warp_sum(x);
+    for (int off = 16; off > 0; off >>= 1) {
+      const double y = __shfl_xor_sync(0xffffffffu, x, off);
+      x = j ? fmax(x, y) : fmin(x, y);
+    }
+    return x;
+  };
+  auto none = [](int j) { return !RANGE || j > 1 ? 0.0 : j ? -INFINITY : INFINITY; };
 #pragma unroll
   for (int j = 0; j < K; ++j) {
-    v[j] = warp_sum(v[j]);
+    v[j] = reduce(j, v[j]);
     if (lane == 0) bsm[wid * K + j] = v[j];
   }
   __syncthreads();
   if (wid == 0) {
 #pragma unroll
     for (int j = 0; j < K; ++j) {
-      double t = lane < nw ? bsm[lane * K + j] : 0.0;
-      t = warp_sum(t);
+      double t = lane < nw ? bsm[lane * K + j] : none(j);
+      t = reduce(j, t);
       if (lane == 0) slots[parity][j] = t;
     }
   }
@@ -159,10 +169,10 @@ __device__ __forceinline__ void cluster_sum_n(cg::cluster_group& cl, double (&v)
     double(*rs)[K] = lane < (int)cl.num_blocks() ? cl.map_shared_rank(slots, lane) : nullptr;
     double t[K];
 #pragma unroll
-    for (int j = 0; j < K; ++j) t[j] = rs ? rs[parity][j] : 0.0;
+    for (int j = 0; j < K; ++j) t[j] = rs ? rs[parity][j] : none(j);
 #pragma unroll
     for (int j = 0; j < K; ++j) {
-      t[j] = warp_sum(t[j]);
+      t[j] = reduce(j, t[j]);
       if (lane == 0) bsm[32 * K + j] = t[j];
     }
   }
@@ -242,6 +252,14 @@ __device__ __forceinline__ double cert_margin(int ka, int kb, double W) {
   return 1.25 * ((double)ka + (double)kb + 60.0) * 1.1102230246251565e-16 * W;
 }
 
+// Offset of the two probes around a Newton iterate of N(x) = target that was moved by `step`.
+// |N''| <= N' / Td for every sum of Fermi functions, so a step of at most Td / 2 leaves the
+// iterate within step^2 / Td of the root; longer steps (and bracket midpoints) take twice the
+// step.  `noise` is the distance that the margin is worth.
+__device__ __forceinline__ double probe_offset(double step, bool newton, double iTd, double noise) {
+  return newton && step * iTd <= 0.5 ? fma(step * step, iTd, 1.5 * noise) : fmax(2.0 * step, 1.5 * noise);
+}
+
 // Bisection levels that need no evaluation: every midpoint >= A is decided "above", every one
 // <= B "below".  True when the interval stops changing.
 __device__ __forceinline__ bool replay_levels(double A, double B, int maxiter, double& lo, double& hi, int& it) {
@@ -310,7 +328,7 @@ __global__ void __launch_bounds__(kPassThreads) k_mu_pass(const MuArgs a, MuStat
   double v[K];
 #pragma unroll
   for (int j = 0; j < K; ++j) v[j] = 0.0;
-  auto fermi = [](double x) { return recip_seeded(1.0 + exp(fmin(x, 600.0))); };
+  auto fermi = [](double x) { return recip_seeded(1.0 + exp(x > 600.0 ? 600.0 : x)); };  // a NaN stays one
   if constexpr (STAGE == kStageRange) {  // extremes and total weight
     v[0] = INFINITY;
     v[1] = -INFINITY;
@@ -411,10 +429,11 @@ __global__ void __launch_bounds__(kPassThreads) k_mu_pass(const MuArgs a, MuStat
       const double span = st->mx - st->mn + 10.0 * fmax(a.T, 1e-6);
       const double bl = fmax(B, st->mn - span), bh = fmin(A, st->mx + span), Z = v[1] / Td;
       r = m - (v[0] - a.target) / Z;
-      if (!(Z > 0.0) || !isfinite(r) || r <= bl || r >= bh) r = 0.5 * (bl + bh);
+      const bool newton = Z > 0.0 && isfinite(r) && r > bl && r < bh;
+      if (!newton) r = 0.5 * (bl + bh);
       const double fw = Z > 0.0 ? margin / Z : INFINITY;
       st->done = A - B <= 4.0 * fw;  // as narrow as the margin allows
-      d = fmax(2.0 * fabs(r - m), 1.5 * fw);
+      d = probe_offset(fabs(r - m), newton, 1.0 / Td, fw);
     }
     st->A = A;
     st->B = B;
@@ -653,6 +672,10 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
   const double mu0v = fuse_first ? a.mu0[0] : 0.0;
   const double Tf = fmax(a.T, 1e-12), rTf = recip_of(Tf);
   double mn = INFINITY, mx = -INFINITY, N0 = 0.0, Z0 = 0.0;
+  double hv[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // has_hint: extremes, N and N' Td at the hint, W
+  // 1 / (1 + x) for x = exp(.), kept inside the range of recip_seeded; a NaN stays one
+  auto cert_fermi = [](double x) { return recip_seeded(1.0 + (x > 0x1p+860 ? 0x1p+860 : x)); };
+  int parity = 0;
   if (fuse_first) {
     visit([&](double v, double w) {
       mn = fmin(mn, v);
@@ -660,6 +683,18 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
       const double p = expit(div_by(mu0v - v, Tf, rTf));
       N0 += w * p;
       Z0 += div_by(w * (p * (1.0 - p)), Tf, rTf);
+    });
+  } else if (has_hint) {  // the first Newton evaluation of the hinted bisection with the extremes
+    hv[0] = mn;
+    hv[1] = mx;
+    const double r = 1.0 / (a.T + 1e-12);
+    visit([&](double v, double w) {
+      hv[0] = fmin(hv[0], v);
+      hv[1] = fmax(hv[1], v);
+      const double f = cert_fermi(exp((v - hint) * r));
+      hv[2] += w * f;
+      hv[3] += w * (f * (1.0 - f));
+      hv[4] += w;
     });
   } else if (!a.pre) {
     visit([&](double v, double) {
@@ -670,10 +705,14 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
   if (a.pre) {
     mn = a.pre->mn;
     mx = a.pre->mx;
+  } else if (has_hint) {
+    if constexpr (!NEWTON) cluster_sum_n<5, true>(cl, hv, cslots, csm, parity);
+    parity ^= 1;
+    mn = hv[0];
+    mx = hv[1];
   } else {
     cluster_minmax(cl, mn, mx, slots, wsm);
   }
-  int parity = 0;
   if (fuse_first) {
     cluster_sum2(cl, N0, Z0, slots, wsm, parity);
     parity ^= 1;
@@ -706,23 +745,15 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
       // levels whose midpoints lie outside (B, A) are replayed without evaluations and
       // only the last few levels are evaluated.  The decisions, and so the result, are
       // those of evaluating every level.
+      // The first evaluation came with the extremes, at the hint itself.  With that and the
+      // probes at step^2 / Td a call on 2304 eigenvalues (T = 0.1) takes 17.8 us for 19.4 with
+      // a hint 1e-7 off the root and 19.9 for 23.8 with one 1e-2 off, on 165888 83 for 106 and 93 for 121.
       const int kpt = (a.n + gs - 1) / gs;
-      double m = fmin(fmax(hint, lo), hi), d = 0.0;
-      for (int t = 0; t < kMuCertPasses; ++t) {
-        const double pl = m - d, ph = m + d;
-        double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // N(m), N'(m) Td, N(pl), N(ph), W
-        visit([&](double ev, double w) {
-          const double f = 1.0 / (1.0 + exp((ev - m) * iTd));
-          v[0] += w * f;
-          v[1] += w * (f * (1.0 - f));
-          v[2] += w / (1.0 + exp((ev - pl) * iTd));
-          v[3] += w / (1.0 + exp((ev - ph) * iTd));
-          v[4] += w;
-        });
-        cluster_sum_n<5>(cl, v, cslots, csm, parity);
-        parity ^= 1;
+      double m = hint, d = 0.0;
+      double v[5] = {hv[2], hv[3], hv[2], hv[2], hv[4]};  // N(m), N'(m) Td, N(m - d), N(m + d), W
+      for (int t = 0;;) {
         const double margin = cert_margin(kpt, kpt, v[4]);
-        const double xs[3] = {m, pl, ph}, ns[3] = {v[0], v[2], v[3]};
+        const double xs[3] = {m, m - d, m + d}, ns[3] = {v[0], v[2], v[3]};
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
           if (ns[q] > a.target + margin) A = fmin(A, xs[q]);
@@ -731,11 +762,28 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
         const double Z = v[1] * iTd;
         const double bl = fmax(B, lo), bh = fmin(A, hi);
         double r = m - (v[0] - a.target) / Z;
-        if (!(Z > 0.0) || !isfinite(r) || r <= bl || r >= bh) r = 0.5 * (bl + bh);
+        const bool newton = Z > 0.0 && isfinite(r) && r > bl && r < bh;
+        if (!newton) r = 0.5 * (bl + bh);
         const double floor_w = Z > 0.0 ? margin / Z : INFINITY;
-        if (A - B <= 4.0 * floor_w) break;  // as narrow as the margin allows
-        d = fmax(2.0 * fabs(r - m), 1.5 * floor_w);
+        if (A - B <= 4.0 * floor_w || ++t == kMuCertPasses) break;  // as narrow as the margin allows
+        d = probe_offset(fabs(r - m), newton, iTd, floor_w);
         m = r;
+        // exp((e - m +- d) / Td) as a product where the factor is far from the range's ends
+        const bool fac = d * iTd < 30.0;
+        const double up = exp(d * iTd), dn = exp(-d * iTd);
+#pragma unroll
+        for (int j = 0; j < 5; ++j) v[j] = 0.0;
+        visit([&](double ev, double w) {
+          const double g = exp((ev - m) * iTd);
+          const double f = cert_fermi(g);
+          v[0] += w * f;
+          v[1] += w * (f * (1.0 - f));
+          v[2] += w * cert_fermi(fac ? g * up : exp((ev - (m - d)) * iTd));
+          v[3] += w * cert_fermi(fac ? g * dn : exp((ev - (m + d)) * iTd));
+          v[4] += w;
+        });
+        cluster_sum_n<5>(cl, v, cslots, csm, parity);
+        parity ^= 1;
       }
     } else if (a.pre) {  // what the grid-wide passes left
       A = a.pre->A;

@@ -608,6 +608,31 @@ def test_grid_wide_mu_equals_the_cluster_bisection(cuda, shape, T, kind, fill):
         assert abs(count(mu[2]) - count(mu[3])) <= 60 * 2.2e-16 * nb
 
 
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), -float("inf")])
+@pytest.mark.parametrize("method", [0, 2])
+def test_grid_wide_mu_with_a_non_finite_eigenvalue(cuda, method, bad):
+    """A non-finite eigenvalue drives hf_find_mu_ws to the bits of hf_find_mu (the certifying passes must not
+    take a NaN for an empty state)."""
+    from jax_hf_b200 import _lib
+    rng = np.random.default_rng(5)
+    nk, nb = 96 * 96, 4
+    eps = rng.normal(size=(nk, nb))
+    eps[1234, 2] = bad
+    e, w = torch.as_tensor(eps, device="cuda"), torch.full((nk,), 1.0 / nk, dtype=torch.float64, device="cuda")
+    L = _lib.lib()
+    n = _lib.C.c_size_t(0)
+    _lib.check(L.hf_mu_workspace_size(_lib.C.byref(n)))
+    ws = torch.full((n.value,), 255, dtype=torch.uint8, device="cuda")
+    mu0 = torch.tensor(0.1, dtype=torch.float64, device="cuda")
+    m0 = mu0.data_ptr() if method else None
+    out = torch.zeros(2, dtype=torch.float64, device="cuda")
+    s = _lib.stream_ptr(e.device)
+    _lib.check(L.hf_find_mu(s, _lib.HF_C128, method, nk, 1, nb, e.data_ptr(), w.data_ptr(), 1.7, 0.1, 0, m0, out.data_ptr()))
+    _lib.check(L.hf_find_mu_ws(s, _lib.HF_C128, method, nk, 1, nb, e.data_ptr(), w.data_ptr(), 1.7, 0.1, 0, m0,
+                               out[1:].data_ptr(), ws.data_ptr(), ws.numel()))
+    assert torch.equal(out[:1], out[1:]) or torch.isnan(out).all()
+
+
 @pytest.mark.parametrize("nb", [2, 7, 8, 9, 13, 16, 17])
 @pytest.mark.parametrize("nk,dt", [(1, np.complex128), (37, np.complex64), (130, np.complex128)])
 def test_density_from_orbitals_shapes(cuda, nb, nk, dt):
