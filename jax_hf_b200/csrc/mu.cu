@@ -9,10 +9,11 @@
 // The bisection evaluates two levels per pass (the 3 midpoints of the next two
 // levels in one reduction, then the two decisions in order).  Each pass costs a
 // chain of block and cluster reductions whose latency grows with the number of
-// sums: on 2304 eigenvalues (9 CTAs) the 54 steps take 52 us at two levels per
-// pass (27 passes), 59 us at three, 65 us at one and 91 us at four; storing the
+// sums: on 2304 eigenvalues (9 CTAs) the 54 steps take 49.7 us at two levels per
+// pass (27 passes) and 51.4 at three; before the trees of a pass ran side by side 52, 59,
+// and 65 us at one, 91 at four levels; storing the
 // warp partials into every CTA's shared memory behind a single cluster barrier
-// instead of the two-stage reduction measured slower (63 us at two levels).
+// instead of the two-stage reduction measured slower (63 us at two levels, before).
 //
 // Methods (reference):
 //   0  _find_mu_bisection  utils.py:353-382 (maxiter 54 f64 / 30 f32)
@@ -134,34 +135,42 @@ __device__ __forceinline__ void cluster_sum2(cg::cluster_group& cl, double& x, d
   y = wsm[65];
 }
 
-// Cluster-wide sums of K values (as cluster_sum2); v[] holds this thread's terms
-// on entry and the totals on return.  bsm: 32 * K + K doubles, slots: [2][K].
-// RANGE: v[0] is a minimum and v[1] a maximum instead.
-template <int K, bool RANGE = false>
+// Cluster-wide sums of K values (as cluster_sum2) over CTAs of NW warps; v[] holds this
+// thread's terms on entry and the totals on return.  bsm: 33 K doubles, slots: [2][K].
+// RANGE: v[0] is a minimum and v[1] a maximum instead.  A pass is a chain of three shuffle
+// trees and a cluster barrier; the trees of the K values advance level by level (one tree
+// after the other, a store between them, made a pass of 3 sums 2.0 us instead of 1.8), and
+// levels that would only add the zeros of absent warps and CTAs are left out.
+template <int K, int NW, bool RANGE = false>
 __device__ __forceinline__ void cluster_sum_n(cg::cluster_group& cl, double (&v)[K], double (*slots)[K], double* bsm,
                                               int parity) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  auto reduce = [](int j, double x) {
-    if (!RANGE || j > 1) return warp_sum(x);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  auto reduce = [](double (&x)[K], int first) {
+#pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
-      const double y = __shfl_xor_sync(0xffffffffu, x, off);
-      x = j ? fmax(x, y) : fmin(x, y);
+      if (off > first) continue;
+      double y[K];
+#pragma unroll
+      for (int j = 0; j < K; ++j) y[j] = __shfl_xor_sync(0xffffffffu, x[j], off);
+#pragma unroll
+      for (int j = 0; j < K; ++j) x[j] = !RANGE || j > 1 ? x[j] + y[j] : j ? fmax(x[j], y[j]) : fmin(x[j], y[j]);
     }
-    return x;
   };
   auto none = [](int j) { return !RANGE || j > 1 ? 0.0 : j ? -INFINITY : INFINITY; };
+  reduce(v, 16);
+  if (lane == 0) {
 #pragma unroll
-  for (int j = 0; j < K; ++j) {
-    v[j] = reduce(j, v[j]);
-    if (lane == 0) bsm[wid * K + j] = v[j];
+    for (int j = 0; j < K; ++j) bsm[wid * K + j] = v[j];
   }
   __syncthreads();
   if (wid == 0) {
+    double t[K];
 #pragma unroll
-    for (int j = 0; j < K; ++j) {
-      double t = lane < nw ? bsm[lane * K + j] : none(j);
-      t = reduce(j, t);
-      if (lane == 0) slots[parity][j] = t;
+    for (int j = 0; j < K; ++j) t[j] = lane < NW ? bsm[lane * K + j] : none(j);
+    reduce(t, NW / 2);
+    if (lane == 0) {
+#pragma unroll
+      for (int j = 0; j < K; ++j) slots[parity][j] = t[j];
     }
   }
   cl.sync();
@@ -170,10 +179,10 @@ __device__ __forceinline__ void cluster_sum_n(cg::cluster_group& cl, double (&v)
     double t[K];
 #pragma unroll
     for (int j = 0; j < K; ++j) t[j] = rs ? rs[parity][j] : none(j);
+    reduce(t, kMuMaxCluster / 2);
+    if (lane == 0) {
 #pragma unroll
-    for (int j = 0; j < K; ++j) {
-      t[j] = reduce(j, t[j]);
-      if (lane == 0) bsm[32 * K + j] = t[j];
+      for (int j = 0; j < K; ++j) bsm[32 * K + j] = t[j];
     }
   }
   __syncthreads();
@@ -706,7 +715,7 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
     mn = a.pre->mn;
     mx = a.pre->mx;
   } else if (has_hint) {
-    if constexpr (!NEWTON) cluster_sum_n<5, true>(cl, hv, cslots, csm, parity);
+    if constexpr (!NEWTON) cluster_sum_n<5, BT / 32, true>(cl, hv, cslots, csm, parity);
     parity ^= 1;
     mn = hv[0];
     mx = hv[1];
@@ -747,7 +756,8 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
       // those of evaluating every level.
       // The first evaluation came with the extremes, at the hint itself.  With that and the
       // probes at step^2 / Td a call on 2304 eigenvalues (T = 0.1) takes 17.8 us for 19.4 with
-      // a hint 1e-7 off the root and 19.9 for 23.8 with one 1e-2 off, on 165888 83 for 106 and 93 for 121.
+      // a hint 1e-7 off the root and 19.9 for 23.8 with one 1e-2 off, on 165888 83 for 106 and 93 for 121 (then
+      // 16.0, 17.8, 82 and 92 with the interleaved trees of cluster_sum_n).
       const int kpt = (a.n + gs - 1) / gs;
       double m = hint, d = 0.0;
       double v[5] = {hv[2], hv[3], hv[2], hv[2], hv[4]};  // N(m), N'(m) Td, N(m - d), N(m + d), W
@@ -782,7 +792,7 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
           v[3] += w * cert_fermi(fac ? g * dn : exp((ev - (m + d)) * iTd));
           v[4] += w;
         });
-        cluster_sum_n<5>(cl, v, cslots, csm, parity);
+        cluster_sum_n<5, BT / 32>(cl, v, cslots, csm, parity);
         parity ^= 1;
       }
     } else if (a.pre) {  // what the grid-wide passes left
@@ -839,7 +849,7 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
           cnt[j - 1] += w / (1.0 + x);
         }
       });
-      cluster_sum_n<NODES>(cl, cnt, bslots, bsm, parity);
+      cluster_sum_n<NODES, BT / 32>(cl, cnt, bslots, bsm, parity);
       parity ^= 1;
       int node = 1;
 #pragma unroll
