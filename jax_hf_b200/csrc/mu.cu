@@ -314,7 +314,12 @@ __device__ __forceinline__ bool newton_step(double g, double Z, double& lo, doub
 constexpr int kPassThreads = 256;
 constexpr int kPassBlocks = 296;   // two CTAs per SM
 constexpr int kPassSums = 8;
-constexpr int kGridMin = 16384;    // eigenvalues from which the passes are used
+// Eigenvalues from which the passes are used.  Bisection: 116 us by the cluster kernel against
+// 58 on 16384, 344 against 78 on 165888.  The warm-started Newton rule has only 4 to 8 evaluations,
+// each a launch here and a cluster barrier there: 20 us (cluster) against 27 on 41472, 25
+// against 29 to 45 against 39 on 131072 (T = 0.2, 0.01), 40 against 36 on 165888, 65 against
+// 45 on 294912.
+constexpr int kGridMin = 16384, kGridMinNewton = 131072;
 constexpr int kNewtonPasses = 5;   // method 2: Newton steps queued ahead of the cluster kernel
 constexpr int kLevelPasses = 5;    // bisection: passes of two levels each behind them
 constexpr int kCertPasses = 7;     // bisection: certifying passes, the first one a scan of 8 points
@@ -1056,7 +1061,8 @@ int hf::find_mu_internal(void* stream, int dtype, int method, int nk1, int nk2, 
   }
   // the grid-wide passes, given a workspace: for the bisection without a hint (with one, the
   // cluster kernel certifies its own bracket) and the warm-started Newton rule
-  if (ws && ws_bytes >= kMuWsBytes && a.n >= kGridMin && (method == 2 ? mu0 != nullptr : method == 0 && !mu0)) {
+  if (ws && ws_bytes >= kMuWsBytes && a.n >= (method == 2 ? kGridMinNewton : kGridMin) &&
+      (method == 2 ? mu0 != nullptr : method == 0 && !mu0)) {
     MuState* st = static_cast<MuState*>(ws);
     double* part = reinterpret_cast<double*>(static_cast<char*>(ws) + 256);
     cudaStream_t s = static_cast<cudaStream_t>(stream);

@@ -615,7 +615,7 @@ def test_grid_wide_mu_with_a_non_finite_eigenvalue(cuda, method, bad):
     take a NaN for an empty state)."""
     from jax_hf_b200 import _lib
     rng = np.random.default_rng(5)
-    nk, nb = 96 * 96, 4
+    nk, nb = 128 * 128, 8
     eps = rng.normal(size=(nk, nb))
     eps[1234, 2] = bad
     e, w = torch.as_tensor(eps, device="cuda"), torch.full((nk,), 1.0 / nk, dtype=torch.float64, device="cuda")
