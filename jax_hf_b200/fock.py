@@ -243,7 +243,7 @@ def build_fock_batch(Ps, *, h, VR, refP, HH, w2d, include_exchange: bool, includ
     SMs that another build's passes leave idle (the last round of a pass, its memory-
     or FP64-bound phases): a density scan or any batch of independent builds runs at a
     higher rate than the same builds one after another (192x192, nb = 8, complex128 on a
-    B200: 81.4 us per build on one stream, 68.0 on two, 65.5 on three, 66.6 on four).
+    B200: 77.6 us per build on one stream, 66.1 on three).
     Each stream has its own workspace.  ``outs``: optional list of (Sigma, H, F) per
     density; build i uses stream i % streams, so an output set shared by builds i and
     i + k * streams is written in order.
