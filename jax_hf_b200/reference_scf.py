@@ -177,7 +177,9 @@ def _solve_scf_impl(kernel, P0, n_electrons, cfg, fock_build_fn):
         return ops.herm(torch.as_tensor(project(X)).to(cd).contiguous())
 
     def fock(P):
-        return fn(P, project_fn=project, **fock_kw)
+        Sg, Hh, F = fn(P, project_fn=project, **fock_kw)
+        # the loop's operations read 16-byte elements; a caller's build may return another type
+        return Sg, Hh, torch.as_tensor(F).to(dev, cd).contiguous()
 
     def density_from_fock(F):
         """reference_scf.py:87-96: eigh, bisection mu, level shift, occupations."""

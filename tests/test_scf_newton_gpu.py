@@ -346,3 +346,25 @@ def test_cg_project_fn_and_block_sizes_hooks(cuda):
     r2 = solve(K, torch.as_tensor(P0, device="cuda"), 16.0, config=SolverConfig(block_sizes=(1, 1), **cfg))
     ro2 = O.solve(Ko, P0, 16.0, config=O.SolverConfig(block_sizes=(1, 1), **cfg))
     assert abs(float(r2.energy) - ro2["energy"]) < 1e-8 * abs(ro2["energy"])
+
+
+@pytest.mark.parametrize("nb", [3, 9])
+def test_python_scf_loop_takes_a_single_precision_fock_matrix(cuda, nb):
+    """A caller's Fock build that returns complex64 (diis_size > 16 runs the Python loop): the loop converts
+    it, so its buffers hold 16-byte elements, and the solve ends where the complex128 build's does (the
+    energy is stationary in the density, so tolerances of 1e-4 and F's rounding leave far less than 1e-6)."""
+    import jax_hf_b200 as G
+    from jax_hf_b200.reference_scf import SCFConfig, solve_scf
+    K = G.HartreeFockKernel(**_multiband(nk=4, nb=nb))
+    P0 = np.zeros(tuple(K.h.shape), complex)
+    cfg = SCFConfig(acceleration="diis", diis_size=17, max_iter=100, density_tol=1e-5, comm_tol=1e-4)
+
+    def single(P, **kw):
+        Sg, H, F = G.build_fock(P, **kw)
+        return Sg, H, F.to(torch.complex64)
+
+    ne = 16 * 0.4 * nb
+    a = solve_scf(K, P0, ne, config=cfg, fock_build_fn=single)
+    b = solve_scf(K, P0, ne, config=cfg, fock_build_fn=G.build_fock)
+    assert a.converged and b.converged and a.fock_matrix.dtype == torch.complex128
+    assert abs(float(a.energy) - float(b.energy)) < 1e-6 * max(1.0, abs(float(b.energy)))
