@@ -264,7 +264,9 @@ def objective(P, p, kernel, h=None):
     h = kernel.h.to(torch.complex128) if h is None else h
     if kernel.dtype != torch.complex128:
         raise ValueError("the hand-written adjoint runs in complex128; build the kernel in complex128")
-    return _ObjectiveFn.apply(P.contiguous(), p.to(torch.float64).contiguous(), h.contiguous(), kernel)
+    # the adjoints read 16-byte elements; autograd carries the conversion back to the caller's type
+    P, h = (t.to(torch.complex128).contiguous() for t in (P, h))
+    return _ObjectiveFn.apply(P, p.to(torch.float64).contiguous(), h, kernel)
 
 
 def shifted_vr(dV, weights):

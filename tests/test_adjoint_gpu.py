@@ -243,3 +243,29 @@ def test_objective_node_matches_the_separate_nodes(cuda, hartree, want):
         assert (x.grad is None) == (y.grad is None)
         if x.grad is not None:
             assert float((x.grad - y.grad).abs().max()) <= 4 * 2.2e-16 * float(y.grad.abs().max())
+
+
+def test_objective_gradients_of_single_precision_inputs(cuda):
+    """complex64 P and h against the same numbers in complex128: value and gradients agree, the gradients
+    rounded to complex64 (6e-8 of the largest entry)."""
+    import jax_hf_b200 as G
+    from jax_hf_b200 import adjoint as A
+    rng = np.random.default_rng(5)
+    n, nb = 5, 3
+    q = lambda *s: rng.normal(size=s) + 1j * rng.normal(size=s)
+    h = q(n, n, nb, nb)
+    K = G.HartreeFockKernel(np.full((n, n), 1.0 / n ** 2), h + np.conj(np.swapaxes(h, -1, -2)),
+                            rng.uniform(0.1, 1.0, size=(n, n, nb, nb)), 0.1)
+    P0 = torch.as_tensor(q(n, n, nb, nb).astype(np.complex64), device="cuda")
+    h0 = K.h.to(torch.complex64)
+    p0 = torch.as_tensor(rng.uniform(0.05, 0.95, size=(n, n, nb)), device="cuda")
+    out = []
+    for dt in (torch.complex64, torch.complex128):
+        P, hh = P0.to(dt).requires_grad_(True), h0.to(dt).requires_grad_(True)
+        Om = A.objective(P, p0, K, hh)
+        Om.backward()
+        assert P.grad.dtype == dt and hh.grad.dtype == dt
+        out.append((float(Om.detach()), P.grad.to(torch.complex128), hh.grad.to(torch.complex128)))
+    assert out[0][0] == out[1][0]
+    for x, y in zip(out[0][1:], out[1][1:]):
+        assert float((x - y).abs().max()) <= 6e-8 * float(y.abs().max())

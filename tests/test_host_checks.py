@@ -30,3 +30,18 @@ def test_eigh_jacobi_refuses_other_element_sizes(no_library, dtype):
 def test_eigh_jacobi_refuses_more_bands_than_the_kernel(no_library):
     with pytest.raises(ValueError, match="nb"):
         linalg.eigh_jacobi(torch.zeros((3, 9, 9), dtype=torch.complex128))
+
+
+@pytest.mark.parametrize("dtype", [torch.complex64, torch.complex128, torch.float64])
+def test_objective_hands_complex128_to_its_node(monkeypatch, dtype):
+    """The node's backward passes P and h to kernels that read 16-byte elements."""
+    from types import SimpleNamespace
+
+    from jax_hf_b200 import adjoint
+    seen = []
+    monkeypatch.setattr(adjoint._ObjectiveFn, "apply", staticmethod(lambda *a: seen.append(a)))
+    P = torch.zeros((2, 3, 4, 4), dtype=dtype).transpose(-1, -2)
+    adjoint.objective(P, torch.zeros(2, 3, 4), SimpleNamespace(dtype=torch.complex128), torch.zeros_like(P))
+    P1, p1, h1, _ = seen[0]
+    assert P1.dtype == h1.dtype == torch.complex128 and p1.dtype == torch.float64
+    assert P1.is_contiguous() and h1.is_contiguous()
