@@ -234,20 +234,19 @@ class _ObjectiveFn(torch.autograd.Function):
     def forward(ctx, P, p, h, kernel):
         from .fock import free_energy, hf_energy
         Sg, H, _ = _build(P, h, kernel)
-        w2d = kernel.w2d.to(torch.float64)
+        w2d = kernel.w2d.to(torch.float64).contiguous()
         E = hf_energy(P, h=h, Sigma=Sg, H=H, weights_b=w2d[..., None, None])
         wn = w2d / max(float(kernel.weight_sum), 1e-30)
-        ctx.kernel = kernel
-        ctx.save_for_backward(P, p, h, Sg, H, wn)
-        return free_energy(E, p, wn, kernel.T)
+        ctx.kernel, ctx.T = kernel, float(kernel.T)
+        ctx.save_for_backward(P, p, h, Sg, H, wn, w2d)
+        return free_energy(E, p, wn, ctx.T)
 
     @staticmethod
     def backward(ctx, gO):
         kernel = ctx.kernel
-        P, p, h, Sg, H, wn = ctx.saved_tensors
+        P, p, h, Sg, H, wn, w2d = ctx.saved_tensors
         want_P, want_p, want_h = ctx.needs_input_grad[:3]
         gO = _dev_scalar(gO, P.device)
-        w2d = kernel.w2d.to(torch.float64).contiguous()
         Pb = pb = hb = None
         if want_P or want_h:
             Pb, hb, Sb = _energy_vjp(gO, P, h, Sg, H, w2d, want_P, want_h, want_P)
@@ -255,7 +254,7 @@ class _ObjectiveFn(torch.autograd.Function):
             gH = _energy_vjp_H(gO, P, w2d) if kernel.include_hartree else None
             Pb += _fock_vjp(kernel, P, Sb, None, gH, False)[0]
         if want_p:
-            pb = _free_energy_vjp(gO, p, wn, float(kernel.T))
+            pb = _free_energy_vjp(gO, p, wn, ctx.T)
         return Pb, pb, hb, None
 
 

@@ -269,3 +269,19 @@ def test_objective_gradients_of_single_precision_inputs(cuda):
     assert out[0][0] == out[1][0]
     for x, y in zip(out[0][1:], out[1][1:]):
         assert float((x - y).abs().max()) <= 6e-8 * float(y.abs().max())
+
+
+def test_objective_backward_uses_the_temperature_of_its_forward(cuda):
+    """A temperature sweep sets kernel.T between the value and its gradients: the gradients are those of the
+    value (entropy term T w log(p / (1 - p)), exact in the order of its two products to 4 ulp)."""
+    import jax_hf_b200 as G
+    from jax_hf_b200 import adjoint as A
+    K = G.HartreeFockKernel(**_kernel_kwargs(4, 2, "scalar", 3))
+    P = torch.as_tensor(S.haar_density(4, 2, 1), device="cuda")
+    p = torch.full((4, 4, 2), 0.25, dtype=torch.float64, device="cuda", requires_grad=True)
+    T = K.T
+    Om = A.objective(P, p, K)
+    K.T = 7.0 * T
+    Om.backward()
+    want = T * float(np.log(0.25 / 0.75)) * (K.w2d / K.weight_sum)[..., None].expand(4, 4, 2)
+    assert float((p.grad - want).abs().max()) <= 1e-15 * float(want.abs().max())
