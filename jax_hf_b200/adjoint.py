@@ -71,6 +71,11 @@ def _consts(rho, kernel):
     return H, sc
 
 
+def _cotangent(g):
+    """A complex cotangent as its numbers in memory: autograd may hand over a lazily conjugated view."""
+    return None if g is None else g.to(torch.complex128).resolve_conj().resolve_neg().contiguous()
+
+
 def _fock_vjp(kernel, P, gS, gF, gH, want_h):
     """(P_bar, h_bar) of the Fock build for cotangents of Sigma, F and H (each may be None)."""
     nk1, nk2, nb = kernel.shape
@@ -82,8 +87,7 @@ def _fock_vjp(kernel, P, gS, gF, gH, want_h):
         VR = kernel._VR_shifted
         VR_adj = VR.conj().resolve_conj().contiguous() if VR.is_complex() else VR
         flags = _flags(kernel, VR)
-        gS = None if gS is None else gS.to(torch.complex128).contiguous()
-        gF = None if gF is None else gF.to(torch.complex128).contiguous()
+        gS, gF = _cotangent(gS), _cotangent(gF)
         Pb = torch.empty_like(P)
         need = C.c_size_t(0)
         _lib.check(_lib.lib().hf_fock_vjp_workspace_size(_lib.HF_C128, flags, nk1, nk2, nb, C.byref(need)))
@@ -144,7 +148,7 @@ def _energy_vjp_H(gE, P, w2d):
 
 def _dev_scalar(g, dev):
     """A cotangent as a contiguous float64 device scalar (no host read)."""
-    return g.to(dev, torch.float64).contiguous()
+    return g.to(dev, torch.float64).resolve_neg().contiguous()
 
 
 class _FockBuildFn(torch.autograd.Function):

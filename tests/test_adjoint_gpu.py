@@ -285,3 +285,20 @@ def test_objective_backward_uses_the_temperature_of_its_forward(cuda):
     Om.backward()
     want = T * float(np.log(0.25 / 0.75)) * (K.w2d / K.weight_sum)[..., None].expand(4, 4, 2)
     assert float((p.grad - want).abs().max()) <= 1e-15 * float(want.abs().max())
+
+
+def test_fock_build_gradient_of_a_conjugated_output(cuda):
+    """Re sum(conj(Sigma) A) and Re sum(Sigma conj(A)) are one number; the first one's backward hands over a
+    conjugated view as the cotangent."""
+    import jax_hf_b200 as G
+    from jax_hf_b200 import adjoint as A
+    K = G.HartreeFockKernel(**_kernel_kwargs(6, 3, "layer", 2))
+    rng = np.random.default_rng(0)
+    q = lambda: torch.as_tensor(rng.normal(size=(6, 6, 3, 3)) + 1j * rng.normal(size=(6, 6, 3, 3)), device="cuda")
+    B, P0 = q(), q()
+    grads = []
+    for f in (lambda S_: (S_.conj() * B).real.sum(), lambda S_: (S_ * B.conj()).real.sum()):
+        P = P0.clone().requires_grad_(True)
+        f(A.fock_build(P, K.h, K)[0]).backward()
+        grads.append(P.grad)
+    torch.testing.assert_close(grads[0], grads[1], rtol=0, atol=1e-13)

@@ -45,3 +45,15 @@ def test_objective_hands_complex128_to_its_node(monkeypatch, dtype):
     P1, p1, h1, _ = seen[0]
     assert P1.dtype == h1.dtype == torch.complex128 and p1.dtype == torch.float64
     assert P1.is_contiguous() and h1.is_contiguous()
+
+
+def test_cotangents_are_materialised():
+    """Autograd passes conj() and negated views without writing their numbers; the kernels read memory."""
+    from jax_hf_b200 import adjoint
+    x = torch.randn(2, 3, 3, dtype=torch.complex128)
+    g = adjoint._cotangent(x.conj())
+    assert not g.is_conj() and torch.equal(torch.view_as_real(g), torch.view_as_real(x.conj().resolve_conj()))
+    y = torch.randn((), dtype=torch.complex128).conj().imag
+    assert y.is_neg()
+    z = adjoint._dev_scalar(y, y.device)
+    assert not z.is_neg() and float(z) == float(y)
