@@ -261,7 +261,7 @@ def test_objective_gradients_of_single_precision_inputs(cuda):
     p0 = torch.as_tensor(rng.uniform(0.05, 0.95, size=(n, n, nb)), device="cuda")
     out = []
     for dt in (torch.complex64, torch.complex128):
-        P, hh = P0.to(dt).requires_grad_(True), h0.to(dt).requires_grad_(True)
+        P, hh = (t.to(dt).clone().requires_grad_(True) for t in (P0, h0))
         Om = A.objective(P, p0, K, hh)
         Om.backward()
         assert P.grad.dtype == dt and hh.grad.dtype == dt
