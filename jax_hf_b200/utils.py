@@ -73,9 +73,10 @@ def _find_mu(dev, eps, method, nk, nb, w, n, T, maxiter, mu0, out):
         need = _lib.C.c_size_t(0)
         _lib.check(_lib.lib().hf_mu_workspace_size(_lib.C.byref(need)))
         _mu_bytes = int(need.value)
-    stream = _lib.stream_ptr(dev)
-    ws = _lib.workspace(_mu_bytes, dev, "mu", stream)
-    _lib.check(_lib.lib().hf_find_mu_ws(stream, _lib.dtype_code(eps), method, nk, 1, nb, eps.data_ptr(),
+    # a call is a chain of launches that pass their state on in the workspace, so it is this call's own: two
+    # threads may queue their chains on one stream at the same time
+    ws = torch.empty(_mu_bytes, dtype=torch.uint8, device=dev)
+    _lib.check(_lib.lib().hf_find_mu_ws(_lib.stream_ptr(dev), _lib.dtype_code(eps), method, nk, 1, nb, eps.data_ptr(),
                                         w.data_ptr(), float(n), float(T), maxiter, _lib.ptr(mu0), out.data_ptr(),
                                         ws.data_ptr(), ws.numel()))
 

@@ -646,3 +646,26 @@ def test_density_from_orbitals_shapes(cuda, nb, nk, dt):
     ref = np.einsum("kin,kn,kjn->kij", Q.astype(np.complex128), p.astype(float), np.conj(Q.astype(np.complex128)))
     assert np.abs(P - ref).max() <= 4 * nb * (1.2e-7 if dt == np.complex64 else 2.3e-16)
     assert np.abs(P - np.conj(np.swapaxes(P, -1, -2))).max() == 0.0
+
+
+@pytest.mark.parametrize("T", [0.05, 1e-4])
+def test_find_mu_from_two_threads_on_one_stream(cuda, T):
+    """Two threads that find the mu of their own spectra on the same stream get what one thread gets."""
+    import threading
+
+    import jax_hf_b200 as G
+    from jax_hf_b200.utils import solve_mu
+    g = torch.Generator(device="cuda").manual_seed(2)
+    w = torch.full((128 * 200,), 1.0 / (128 * 200), dtype=torch.float64, device="cuda")
+    eps = [i + torch.randn(128 * 200, 8, dtype=torch.float64, device="cuda", generator=g) for i in range(2)]
+    call = (lambda e: float(G.find_chemical_potential(e, w, 2.7, T)), lambda e: float(solve_mu(e, w, 2.7, 0.3, T)))
+    for f in call:
+        want = [f(e) for e in eps]
+        got = [[], []]
+        threads = [threading.Thread(target=lambda i=i: got[i].extend(f(eps[i]) for _ in range(60))) for i in range(2)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        for i in range(2):
+            assert got[i] == [want[i]] * 60
