@@ -97,6 +97,11 @@ bool lu_solve(std::vector<double> A, std::vector<double> b, int n, std::vector<d
   return true;
 }
 
+// Flags of the loop's builds, for which its workspace is sized too.
+unsigned scf_flags(const hf_cg_problem* pb, bool fp32) {
+  return pb->fock_flags | HF_FOCK_NO_TWO_FACTOR | (fp32 ? HF_FOCK_FFT_FP32 : 0u);
+}
+
 struct Scf {
   cudaStream_t s;
   const hf_cg_problem* pb;
@@ -142,8 +147,7 @@ struct Scf {
       if (cf->fock_cb(cf->cb_user, s, P, Sg, H, F) != 0)
         return fail(HF_ERR_ABORTED, "hf_scf_solve: Fock callback failed");
     } else {
-      const unsigned flags = pb->fock_flags | HF_FOCK_NO_TWO_FACTOR | (fp32 ? HF_FOCK_FFT_FP32 : 0u);
-      if ((st = hf_fock_build(s, HF_C128, flags, pb->nk1, pb->nk2, nb, P, pb->h, pb->VR, pb->refP, pb->HH,
+      if ((st = hf_fock_build(s, HF_C128, scf_flags(pb, fp32), pb->nk1, pb->nk2, nb, P, pb->h, pb->VR, pb->refP, pb->HH,
                               pb->w2d, pb->n_contact, pb->contact_g, pb->contact_Oi, pb->contact_Oj, Sg, H, F,
                               at<void>(kFOCKWS), fock_ws)))
         return st;
@@ -231,7 +235,12 @@ static int scf_check(const hf_cg_problem* pb, const hf_scf_config* cf) {
 static int scf_sizes(const hf_cg_problem* pb, const hf_scf_config* cf, size_t* fock_ws, size_t* red_ws,
                      size_t* ops_ws) {
   int st;
-  if ((st = hf_fock_workspace_size(HF_C128, pb->fock_flags, pb->nk1, pb->nk2, pb->nb, fock_ws))) return st;
+  if ((st = hf_fock_workspace_size(HF_C128, scf_flags(pb, false), pb->nk1, pb->nk2, pb->nb, fock_ws))) return st;
+  if (cf->fp32_exchange) {
+    size_t f32 = 0;
+    if ((st = hf_fock_workspace_size(HF_C128, scf_flags(pb, true), pb->nk1, pb->nk2, pb->nb, &f32))) return st;
+    if (f32 > *fock_ws) *fock_ws = f32;
+  }
   if ((st = hf_reduce_workspace_size(pb->nk1, pb->nk2, pb->nb, red_ws))) return st;
   return hf_ops_workspace_size(ops_ws);
 }

@@ -57,3 +57,25 @@ def test_cotangents_are_materialised():
     assert y.is_neg()
     z = adjoint._dev_scalar(y, y.device)
     assert not z.is_neg() and float(z) == float(y)
+
+
+@pytest.mark.parametrize("engine", [0, _lib.FOCK_TILE_PLAN, _lib.FOCK_PIPE, _lib.FOCK_GENERIC_FFT])
+@pytest.mark.parametrize("n1,n2,nb", [(340, 24, 5), (340, 24, 9), (430, 24, 3), (120, 120, 8)])
+def test_scf_workspace_covers_the_builds_of_the_loop(engine, n1, n2, nb):
+    """The SCF driver builds without the two-factor passes, whose slot plan may be the smaller one: its
+    workspace is the one of a problem that asks for that itself."""
+    import ctypes as C
+
+    from jax_hf_b200.reference_scf import SCFConfig, _scf_config_struct, _ScfConfig
+    from jax_hf_b200.solver import _CgProblem
+    L = _lib.lib()
+    cf = _scf_config_struct(SCFConfig())
+    fn = L.hf_scf_workspace_size
+    fn.argtypes, fn.restype = [C.POINTER(_CgProblem), C.POINTER(_ScfConfig), C.POINTER(C.c_size_t)], C.c_int
+    sizes = []
+    for extra in (0, _lib.FOCK_NO_TWO_FACTOR):
+        pb = _CgProblem(n1, n2, nb, _lib.FOCK_EXCHANGE | _lib.FOCK_VR_REAL | engine | extra, 0.1, 1.0, 1.0)
+        need = C.c_size_t(0)
+        _lib.check(fn(C.byref(pb), C.byref(cf), C.byref(need)))
+        sizes.append(need.value)
+    assert sizes[0] == sizes[1]
