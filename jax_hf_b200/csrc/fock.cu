@@ -650,6 +650,12 @@ static int fork_join(ForkJoin** out) {
   return HF_OK;
 }
 
+// Register sides whose line shapes put 24 elements on a thread, which a tile plan of more than one band
+// leaves to the two-factor passes (launch_fock).
+static bool deep_tiles(int nk1, int nk2, int nb) {
+  return nb > 1 && fast_per_thread(nk1) >= 24 && fast_per_thread(nk2) >= 24;
+}
+
 // pc: the plan for the constant terms when it differs from the exchange plan (an
 // in-block mask: the Hartree and contact terms read every channel of the density).
 template <typename ST, typename FT>
@@ -683,8 +689,7 @@ static int launch_fock(FockParams& p, cudaStream_t stream, bool need_consts, con
     const bool two = !(p.flags & HF_FOCK_NO_TWO_FACTOR);
     // A single channel keeps them too (192 x 192 x 1 21.3 us against 22.3).  Packing a band-resolved V at
     // 96 x 96 x 8 in c64 is the one build seen to lose (19.6 -> 21.9; 52.8 -> 44.4 at 192).
-    const bool deep = two && p.nb > 1 && !p.rows_plan && !(p.flags & HF_FOCK_TILE_PLAN) && fast_per_thread(p.nk1) >= 24 &&
-                      fast_per_thread(p.nk2) >= 24;
+    const bool deep = two && !p.rows_plan && !(p.flags & HF_FOCK_TILE_PLAN) && deep_tiles(p.nk1, p.nk2, p.nb);
     if (!deep) {
       st = fast_fock<ST, FT>(p, stream, &handled);
       if (st != HF_OK || handled) return st;
@@ -727,10 +732,16 @@ using TuneKey = std::tuple<int, int, unsigned, int, int, int>;
 static std::mutex g_tune_mu;
 static std::map<TuneKey, unsigned> g_tune;
 
+// HF_FOCK_NO_TWO_FACTOR stays in the key where it changes which kernels run: a choice among the Stockham
+// stages says nothing about the two-factor passes, nor the other way round.
 static TuneKey tune_key(int dtype, unsigned flags, int nk1, int nk2, int nb) {
   int dev = 0;
   cudaGetDevice(&dev);
-  return TuneKey(dev, dtype, flags & ~(kEngineFlags | HF_FOCK_NO_TWO_FACTOR), nk1, nk2, nb);
+  const bool tiles = (flags & HF_FOCK_PACKING) || nb > 8;
+  const bool two = fast_length(nk1) && fast_length(nk2) ? tiles && deep_tiles(nk1, nk2, nb)
+                                                         : line_factors(nk1) && line_factors(nk2);
+  const unsigned drop = kEngineFlags | (two ? 0u : HF_FOCK_NO_TWO_FACTOR);
+  return TuneKey(dev, dtype, flags & ~drop, nk1, nk2, nb);
 }
 
 // flags with the stored engine choice applied (unless the caller set an engine flag)
@@ -1055,7 +1066,8 @@ extern "C" int hf_fock_autotune(void* stream, int dtype, unsigned flags, int nk1
   if (flags & kEngineFlags) return fail(HF_ERR_INVALID, "hf_fock_autotune chooses the engine flags itself");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const unsigned* cands = kTuneCand;
-  // the tile and pipeline candidates only differ from the default where the rows plan applies
+  // the pipeline only differs from the default where the rows plan applies, the tile plan there and where
+  // it brings the register passes back (deep_tiles)
   SlotPlan sp0;
   if ((st = get_plan(dtype, flags, nk1, nk2, nb, sp0))) return st;
   float times[kTuneCands] = {-1.f, -1.f, -1.f, -1.f};
@@ -1067,7 +1079,8 @@ extern "C" int hf_fock_autotune(void* stream, int dtype, unsigned flags, int nk1
   }
   int best = -1;
   for (int c = 0; c < kTuneCands && st == HF_OK; ++c) {
-    if ((c == 1 || c == 3) && !sp0.rows) continue;
+    if (c == 3 && !sp0.rows) continue;
+    if (c == 1 && !sp0.rows && (!deep_tiles(nk1, nk2, nb) || (flags & HF_FOCK_NO_TWO_FACTOR))) continue;
     const unsigned f = flags | cands[c];
     auto run = [&] {
       return fock_build_exact(stream, dtype, f, nk1, nk2, nb, P, h, VR, refP, HH, w2d, n_contact, contact_g,

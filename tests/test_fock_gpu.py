@@ -669,3 +669,48 @@ def test_find_mu_from_two_threads_on_one_stream(cuda, T):
             t.join()
         for i in range(2):
             assert got[i] == [want[i]] * 60
+
+
+def _tune_inputs(n, nb, V):
+    import jax_hf_b200 as G
+    prob, P, _ = _problem(n, n, nb, V, 3)
+    K = G.HartreeFockKernel(prob.weights, prob.hamiltonian, prob.coulomb_q, prob.T)
+    a = K.as_args()
+    return torch.as_tensor(P, device="cuda"), dict(
+        h=a["h"], VR=a["VR"], refP=a["refP"], HH=a["HH"], w2d=K.w2d, include_exchange=True, include_hartree=False,
+        exchange_hermitian_channel_packing=a["exchange_hermitian_channel_packing"])
+
+
+def test_autotuning_the_stockham_stages_leaves_other_builds_alone(cuda):
+    """Tuned with engine="stockham", a two-factor side compares two schedules of the Stockham stages; whichever
+    wins, the default build keeps the two-factor passes (the same bits as before), and a build tuned by
+    default leaves the Stockham one where it was."""
+    import jax_hf_b200 as G
+    from jax_hf_b200 import fock as Fk
+    P, kw = _tune_inputs(60, 3, "layer")
+    Fk.autotune_reset()
+    try:
+        before = G.build_fock(P, **kw)
+        for _ in range(20):  # two equal candidates: the noise of the timing picks one
+            G.build_fock(P, engine="stockham", autotune=True, autotune_reps=1, **kw)
+            if Fk.last_autotune["chosen"] == "generic":
+                break
+        after = G.build_fock(P, **kw)
+        assert all(torch.equal(x, y) for x, y in zip(before, after))
+    finally:
+        Fk.autotune_reset()
+
+
+def test_autotuner_times_the_register_passes_beside_the_two_factor_ones(cuda):
+    """96 x 96 packed runs the two-factor passes by default: the tile candidate is the register passes."""
+    import jax_hf_b200 as G
+    from jax_hf_b200 import fock as Fk
+    P, kw = _tune_inputs(96, 4, "scalar")
+    Fk.autotune_reset()
+    try:
+        G.build_fock(P, autotune=True, autotune_reps=1, **kw)
+        assert Fk.last_autotune["us"]["tile"] > 0 and "pipe" not in Fk.last_autotune["us"]
+        G.build_fock(P, engine="stockham", autotune=True, autotune_reps=1, **kw)
+        assert "tile" not in Fk.last_autotune["us"]
+    finally:
+        Fk.autotune_reset()
