@@ -261,10 +261,16 @@ __device__ __forceinline__ double cert_margin(int ka, int kb, double W) {
   return 1.25 * ((double)ka + (double)kb + 60.0) * 1.1102230246251565e-16 * W;
 }
 
+// What the margin is worth on the axis of x, and no less than the spacing of the numbers at m: probes any
+// closer are m itself.  Infinite where N is flat.
+__device__ __forceinline__ double probe_noise(double margin, double Z, double m) {
+  return Z > 0.0 ? fmax(margin / Z, 0x1p-52 * fabs(m)) : INFINITY;
+}
+
 // Offset of the two probes around a Newton iterate of N(x) = target that was moved by `step`.
 // |N''| <= N' / Td for every sum of Fermi functions, so a step of at most Td / 2 leaves the
 // iterate within step^2 / Td of the root; longer steps (and bracket midpoints) take twice the
-// step.  `noise` is the distance that the margin is worth.
+// step.  `noise`: probe_noise.
 __device__ __forceinline__ double probe_offset(double step, bool newton, double iTd, double noise) {
   return newton && step * iTd <= 0.5 ? fma(step * step, iTd, 1.5 * noise) : fmax(2.0 * step, 1.5 * noise);
 }
@@ -445,7 +451,7 @@ __global__ void __launch_bounds__(kPassThreads) k_mu_pass(const MuArgs a, MuStat
       r = m - (v[0] - a.target) / Z;
       const bool newton = Z > 0.0 && isfinite(r) && r > bl && r < bh;
       if (!newton) r = 0.5 * (bl + bh);
-      const double fw = Z > 0.0 ? margin / Z : INFINITY;
+      const double fw = probe_noise(margin, Z, m);
       st->done = A - B <= 4.0 * fw;  // as narrow as the margin allows
       d = probe_offset(fabs(r - m), newton, 1.0 / Td, fw);
     }
@@ -749,8 +755,10 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
     if (has_hint) {
       // Certified bracket from the hint.  N(x) = sum w / (1 + exp((e - x) / Td)) is
       // increasing in x; an evaluation N~(x) differs from it by at most E = (kpt + 24) u W
-      // (kpt terms summed per thread, a reduction tree of depth <= 14, about 6 u per term
-      // and u W for the rounding of the exponent's argument; W = sum w).  So once
+      // (kpt terms summed per thread, a reduction tree of depth <= 14, about 6 u per term, and u W for the
+      // rounding of the exponent's argument y, whose error u |y| moves a term by f (1 - f) u |y| < 0.23 u;
+      // as a product of two exponentials with |z| <= 2 in the second, by less than 1.3 u, and by 2 u for
+      // the second exponential and the product; W = sum w).  So once
       // N~(A) > target + margin with margin = cert_margin(...) >= 2E, every x >= A has
       // N~(x) > target: the bisection's decision at a midpoint m >= A is "above" without
       // an evaluation, and likewise "below" for m <= B once N~(B) < target - margin.
@@ -779,13 +787,17 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
         double r = m - (v[0] - a.target) / Z;
         const bool newton = Z > 0.0 && isfinite(r) && r > bl && r < bh;
         if (!newton) r = 0.5 * (bl + bh);
-        const double floor_w = Z > 0.0 ? margin / Z : INFINITY;
+        const double floor_w = probe_noise(margin, Z, m);
         if (A - B <= 4.0 * floor_w || ++t == kMuCertPasses) break;  // as narrow as the margin allows
         d = probe_offset(fabs(r - m), newton, iTd, floor_w);
         m = r;
-        // exp((e - m +- d) / Td) as a product where the factor is far from the range's ends
-        const bool fac = d * iTd < 30.0;
-        const double up = exp(d * iTd), dn = exp(-d * iTd);
+        // The probes are the rounded m - d and m + d, as they are recorded in A and B: what counts is the
+        // count at the recorded number (one half ulp of m beside it is more than the margin for a band that
+        // is narrow against its offset from zero).  exp((e - x) / Td) is the product of the exponential at m
+        // and the factor of the realised offset m - x where that is small.
+        const double pl = m - d, ph = m + d, zl = (m - pl) * iTd, zh = (m - ph) * iTd;
+        const bool fac = zl <= 2.0 && zh >= -2.0;
+        const double up = exp(zl), dn = exp(zh);
 #pragma unroll
         for (int j = 0; j < 5; ++j) v[j] = 0.0;
         visit([&](double ev, double w) {
@@ -793,8 +805,8 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
           const double f = cert_fermi(g);
           v[0] += w * f;
           v[1] += w * (f * (1.0 - f));
-          v[2] += w * cert_fermi(fac ? g * up : exp((ev - (m - d)) * iTd));
-          v[3] += w * cert_fermi(fac ? g * dn : exp((ev - (m + d)) * iTd));
+          v[2] += w * cert_fermi(fac ? g * up : exp((ev - pl) * iTd));
+          v[3] += w * cert_fermi(fac ? g * dn : exp((ev - ph) * iTd));
           v[4] += w;
         });
         cluster_sum_n<5, BT / 32>(cl, v, cslots, csm, parity);

@@ -714,3 +714,31 @@ def test_autotuner_times_the_register_passes_beside_the_two_factor_ones(cuda):
         assert "tile" not in Fk.last_autotune["us"]
     finally:
         Fk.autotune_reset()
+
+
+@pytest.mark.parametrize("center,width,T", [(10.0, 0.02, 1e-3), (10.0, 0.02, 1e-2), (1.0, 0.002, 1e-3),
+                                            (-300.0, 0.5, 1e-2), (1e4, 0.1, 0.05), (0.0, 1.0, 1e-3)])
+@pytest.mark.parametrize("nk", [576, 10368])
+def test_bisection_hint_keeps_the_result_of_narrow_bands(cuda, center, width, T, nk):
+    """Bands that are narrow against their offset from zero, where the spacing of the numbers at mu exceeds what
+    the certifying margin is worth: with a hint the result still has the bits of evaluating every level."""
+    from jax_hf_b200 import _lib
+    rng = np.random.default_rng(nk)
+    eps = torch.as_tensor(center + width * rng.standard_normal((nk, 4)), device="cuda")
+    w = torch.full((nk,), 1.0 / nk, device="cuda", dtype=torch.float64)
+    fills = rng.uniform(0.05, 3.95, 60)
+    L, st = _lib.lib(), _lib.stream_ptr(eps.device)
+    out = torch.zeros(4, len(fills), device="cuda", dtype=torch.float64)
+    hint = torch.zeros(3, len(fills), device="cuda", dtype=torch.float64)
+
+    def run(ne, h, o):
+        _lib.check(L.hf_find_mu(st, _lib.HF_C128, 0, nk, 1, 4, eps.data_ptr(), w.data_ptr(), ne, T, 0, h, o))
+
+    for i, ne in enumerate(fills):
+        run(ne, None, out[0, i:].data_ptr())
+    hint.copy_(out[0] + width * torch.tensor([[1e-8], [1e-4], [-0.3]], device="cuda"))
+    for j in range(3):
+        for i, ne in enumerate(fills):
+            run(ne, hint[j, i:].data_ptr(), out[j + 1, i:].data_ptr())
+    for j in range(1, 4):
+        assert torch.equal(out[j], out[0]), (out[j] != out[0]).sum()
