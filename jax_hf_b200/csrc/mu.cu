@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(kPassThreads) k_mu_pass(const MuArgs a, MuStat
   pdl_begin();
   if (a.active && !*a.active) return;
   if (STAGE != kStageRange && st->done) return;
-  constexpr int K = STAGE == kStageRange ? 3 : STAGE == kStageScan ? 8 : 5;
+  constexpr int K = STAGE == kStageRange ? 4 : STAGE == kStageScan ? 8 : 5;
   __shared__ double red[(kPassThreads / 32) * K];
   __shared__ bool last;
   const int gt = blockIdx.x * blockDim.x + threadIdx.x, gs = gridDim.x * blockDim.x;
@@ -349,13 +349,14 @@ __global__ void __launch_bounds__(kPassThreads) k_mu_pass(const MuArgs a, MuStat
 #pragma unroll
   for (int j = 0; j < K; ++j) v[j] = 0.0;
   auto fermi = [](double x) { return recip_seeded(1.0 + exp(x > 600.0 ? 600.0 : x)); };  // a NaN stays one
-  if constexpr (STAGE == kStageRange) {  // extremes and total weight
-    v[0] = INFINITY;
+  if constexpr (STAGE == kStageRange) {  // extremes, total and least weight
+    v[0] = v[3] = INFINITY;
     v[1] = -INFINITY;
     for_each_eps<RT, kMuCacheU>(a, gt, gs, [&](double e, double w) {
       v[0] = fmin(v[0], e);
       v[1] = fmax(v[1], e);
       v[2] += w;
+      v[3] = fmin(v[3], w);
     });
   } else if constexpr (STAGE == kStageScan) {  // N at 8 points inside [mn, mx]
     const double r = 1.0 / Td, m0 = st->mn, h = (st->mx - st->mn) * (1.0 / 9.0);
@@ -376,7 +377,8 @@ __global__ void __launch_bounds__(kPassThreads) k_mu_pass(const MuArgs a, MuStat
   }
   // block, then grid: fixed trees, so the sums do not depend on the order of arrival
   auto combine = [](int j, double x, double y) {
-    return STAGE == kStageRange && j == 0 ? fmin(x, y) : STAGE == kStageRange && j == 1 ? fmax(x, y) : x + y;
+    if (STAGE != kStageRange || j == 2) return x + y;
+    return j == 1 ? fmax(x, y) : fmin(x, y);
   };
   auto block_all = [&]() {  // v: the block's values in thread 0
 #pragma unroll
@@ -404,7 +406,7 @@ __global__ void __launch_bounds__(kPassThreads) k_mu_pass(const MuArgs a, MuStat
   if (!last) return;
   __threadfence();
 #pragma unroll
-  for (int j = 0; j < K; ++j) v[j] = STAGE == kStageRange && j < 2 ? (j ? -INFINITY : INFINITY) : 0.0;
+  for (int j = 0; j < K; ++j) v[j] = STAGE != kStageRange || j == 2 ? 0.0 : j == 1 ? -INFINITY : INFINITY;
   for (int b = threadIdx.x; b < (int)gridDim.x; b += kPassThreads)
 #pragma unroll
     for (int j = 0; j < K; ++j) v[j] = combine(j, v[j], __ldcg(part + b * K + j));
@@ -416,11 +418,17 @@ __global__ void __launch_bounds__(kPassThreads) k_mu_pass(const MuArgs a, MuStat
     st->mn = mn;
     st->mx = mx;
     st->W = v[2];
-    st->done = 0;
+    // a bracket decides levels only while N increases: with a negative weight every level is evaluated
+    st->done = v[3] < 0.0;
     st->A = INFINITY;
     st->B = -INFINITY;
     st->m = 0.5 * (mn + mx);
     st->d = 0.0;
+    const double span = mx - mn + 10.0 * fmax(a.T, 1e-6);
+    st->lo = mn - span;
+    st->hi = mx + span;
+    st->it = 0;
+    st->fixed = 0;
   } else {
     const int gk = (a.n + gs - 1) / gs;
     const double margin = cert_margin(gk, a.kpt, st->W);
@@ -1074,7 +1082,7 @@ int hf::find_mu_internal(void* stream, int dtype, int method, int nk1, int nk2, 
   // the grid-wide passes, given a workspace: for the bisection without a hint (with one, the
   // cluster kernel certifies its own bracket) and the warm-started Newton rule
   if (ws && ws_bytes >= kMuWsBytes && a.n >= (method == 2 ? kGridMinNewton : kGridMin) &&
-      (method == 2 ? mu0 != nullptr : method == 0 && !mu0)) {
+      (method == 2 ? mu0 != nullptr : method == 0 && !mu0 && T + 1e-12 > 0.0)) {
     MuState* st = static_cast<MuState*>(ws);
     double* part = reinterpret_cast<double*>(static_cast<char*>(ws) + 256);
     cudaStream_t s = static_cast<cudaStream_t>(stream);

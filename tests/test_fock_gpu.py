@@ -742,3 +742,29 @@ def test_bisection_hint_keeps_the_result_of_narrow_bands(cuda, center, width, T,
             run(ne, hint[j, i:].data_ptr(), out[j + 1, i:].data_ptr())
     for j in range(1, 4):
         assert torch.equal(out[j], out[0]), (out[j] != out[0]).sum()
+
+
+@pytest.mark.parametrize("T", [0.3, 0.02, -0.05])
+def test_grid_wide_bisection_where_the_count_is_not_monotonic(cuda, T):
+    """Weights of both signs (quadrature rules have them) and T < 0: no bracket can be certified there, so
+    hf_find_mu_ws evaluates the levels that hf_find_mu evaluates."""
+    from jax_hf_b200 import _lib
+    rng = np.random.default_rng(8)
+    nk, nb = 96 * 96, 4
+    bands, wn = rng.normal(size=(nk, nb)), np.ones(nk)
+    if T > 0:  # the count falls where the negative weights' eigenvalues lie
+        wn[::4] = -1.5
+        bands[::4] = 0.4 + 0.1 * bands[::4]
+    eps = torch.as_tensor(bands, device="cuda")
+    w = torch.as_tensor(wn / wn.sum(), device="cuda")
+    L, st = _lib.lib(), _lib.stream_ptr(eps.device)
+    n = _lib.C.c_size_t(0)
+    _lib.check(L.hf_mu_workspace_size(_lib.C.byref(n)))
+    ws = torch.full((n.value,), 255, dtype=torch.uint8, device="cuda")
+    fills = np.linspace(-0.2, nb + 0.2, 81)
+    out = torch.zeros(2, len(fills), dtype=torch.float64, device="cuda")
+    for i, ne in enumerate(fills):
+        args = (st, _lib.HF_C128, 0, nk, 1, nb, eps.data_ptr(), w.data_ptr(), ne, T, 0, None)
+        _lib.check(L.hf_find_mu(*args, out[0, i:].data_ptr()))
+        _lib.check(L.hf_find_mu_ws(*args, out[1, i:].data_ptr(), ws.data_ptr(), ws.numel()))
+    assert torch.equal(out[0], out[1])
