@@ -10,7 +10,7 @@
 // The retraction solves the Cayley transform directly,
 //   U(tau) = (I + tau d / 2)^{-1} (I - tau d / 2) = 2 (I + tau d / 2)^{-1} - I,
 // the form of _cayley_retract (solver.py:122-138), by in-place Gauss-Jordan
-// elimination; it equals the spectral form of the reference loop (solver.py:161-197,
+// elimination with row pivoting; it equals the spectral form of the reference loop (solver.py:161-197,
 // eigh(i d)) up to rounding and needs ~10x fewer FP64 operations per trial than a
 // Jacobi eigh.
 #pragma once
@@ -41,21 +41,31 @@ __device__ __forceinline__ double2 crecip(double2 z) {
   return make_double2(z.x * s, -z.y * s);
 }
 
+// What the pivot search compares: the larger part's magnitude to 2^-20, in the integer pipe
+// (the choice is free within a small factor, the FP64 pipe is not).
+__device__ __forceinline__ int pivot_key(double2 z) {
+  return max(__double2hiint(z.x) & 0x7fffffff, __double2hiint(z.y) & 0x7fffffff);
+}
+
 // Column c of U(tau) into u[] from column c of d (skew-Hermitian).  `on`: this lane
 // holds a real column of a live k-point.  SC: NB complex (the broadcast column).
 // Warp-uniform control flow.
 //
-// (I + tau d / 2)^{-1} by in-place Gauss-Jordan: step j turns column j into column j of the
-// inverse so far, so a lane updates one column of NB entries per step.  No pivoting: the
-// Hermitian part of I + tau d / 2 is I, and every Schur complement keeps a Hermitian part
-// >= I, so a pivot has modulus >= 1 and the elimination is stable (Golub & Van Loan,
-// Matrix Computations, sec. 4.3, on matrices with a positive definite Hermitian part).
-// Against the pivoted elimination of [M | I] it replaced (pivot search and run-time row
-// selects in every step, two columns per lane): the first line-search trial at 144 x 144,
-// nb = 8 takes 45 us (62 before; cold, launch list).
+// (I + tau d / 2)^{-1} by in-place Gauss-Jordan with row pivoting: step j turns column j into
+// column j of the inverse so far, so a lane updates one column of NB entries per step.  No pivot
+// vanishes without pivoting either (the Hermitian part of I + tau d / 2 is I), but the growth
+// is then bounded by |tau d|^2 (Golub & Van Loan, Matrix Computations, sec. 4.3), and the
+// mesh-norm limit on the step leaves single k-points steps of 10 to 100: at |tau d| = 80 with
+// occupied-empty blocks U was off unitary by 2e-14 (99% of random d, nb = 8), pivoted by 9e-16.
+// The rows are swapped in registers, by every lane of a warp in which some k-point's pivot is
+// not on the diagonal (none is for steps below 1 or so); the columns go back by a shuffle.
+// First line-search trial at 144 x 144, nb = 8 (cold, launch list): 49 us; 44 without the pivoting,
+// 62 for pivoted elimination of [M | I] with two columns per lane.
 template <int NB>
 __device__ __forceinline__ void cayley_cols(const double2 (&d)[NB], double tau, int c, bool on, double2* SC,
                                             double2 (&u)[NB]) {
+  constexpr unsigned kSame = 0x76543210u;
+  unsigned perm = kSame;  // nibble i: the row that is now in place i
   const double h = 0.5 * tau;
 #pragma unroll
   for (int r = 0; r < NB; ++r) u[r] = make_double2((r == c ? 1.0 : 0.0) + h * d[r].x, h * d[r].y);
@@ -66,6 +76,31 @@ __device__ __forceinline__ void cayley_cols(const double2 (&d)[NB], double tau, 
       for (int r = 0; r < NB; ++r) SC[r] = u[r];
     }
     __syncwarp();
+    int p = j, best = pivot_key(SC[j]);
+#pragma unroll
+    for (int r = j + 1; r < NB; ++r) {
+      const int key = pivot_key(SC[r]);
+      if (key > best) { best = key; p = r; }
+    }
+    if (__any_sync(0xffffffffu, p != j)) {
+      const unsigned x = ((perm >> 4 * j) ^ (perm >> 4 * p)) & 15u;
+      perm ^= x << 4 * j | x << 4 * p;
+      const double2 uj = u[j];
+#pragma unroll
+      for (int r = j + 1; r < NB; ++r) {
+        if (r == p) {
+          u[j] = u[r];
+          u[r] = uj;
+        }
+      }
+      __syncwarp();
+      if (on && c == j) {
+        const double2 t = SC[j];
+        SC[j] = SC[p];
+        SC[p] = t;
+      }
+      __syncwarp();
+    }
     if (on) {
       const double2 ip = crecip(SC[j]);
       const double2 pj = c == j ? ip : cmul(u[j], ip);  // row j of the updated column
@@ -78,6 +113,18 @@ __device__ __forceinline__ void cayley_cols(const double2 (&d)[NB], double tau, 
       u[j] = pj;
     }
     __syncwarp();
+  }
+  // column i of what is in the lanes is column perm[i] of the inverse
+  if (__any_sync(0xffffffffu, perm != kSame)) {
+    int src = 0;
+#pragma unroll
+    for (int i = 0; i < NB; ++i)
+      if (((perm >> 4 * i) & 15u) == (unsigned)c) src = i;
+#pragma unroll
+    for (int r = 0; r < NB; ++r) {
+      u[r].x = __shfl_sync(0xffffffffu, u[r].x, src, RowGroup<NB>::G);
+      u[r].y = __shfl_sync(0xffffffffu, u[r].y, src, RowGroup<NB>::G);
+    }
   }
   if (on) {
 #pragma unroll

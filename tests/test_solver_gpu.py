@@ -246,3 +246,40 @@ def test_cg_batch_rejects_hooks(cuda):
     with pytest.raises(ValueError, match="hooks"):
         solve_batch([K], [np.zeros((p.nk, p.nk, p.nb, p.nb), complex)], [p.n_electrons],
                     config=SolverConfig(block_sizes=(2, 2)))
+
+
+@pytest.mark.parametrize("nb", [2, 3, 4, 5, 6, 8])
+@pytest.mark.parametrize("bt_max", [0, 2])
+def test_cg_retraction_stays_unitary_for_long_steps(cuda, nb, bt_max):
+    """One CG step with Cayley steps |tau d| from 1 to 1e4 between occupied and empty states (max_step limits
+    the mesh norm only).  The Fock hook sees the density after the step: with occupations 0 and 1 it is
+    P = U p U^H, a projector as far as U is unitary.  Elimination with row pivoting keeps that to the
+    rounding of its n steps, a few ulp each and entry: 30 nb ulp."""
+    import jax_hf_b200 as G
+    from jax_hf_b200.solver import SolverConfig, solve
+    rng = np.random.default_rng(nb)
+    n, ne = 24, nb // 2
+    lev = np.linspace(-1, 1, nb)
+    lev = np.where(np.arange(nb) < ne, -1.0, 1.0) + 0.3 * lev
+    F0 = np.broadcast_to(np.diag(lev), (n, n, nb, nb)).astype(complex)
+    B = np.zeros_like(F0)
+    B[..., :ne, ne:] = rng.normal(size=(n, n, ne, nb - ne)) + 1j * rng.normal(size=(n, n, ne, nb - ne))
+    B *= 10.0 ** rng.uniform(0, 4, size=(n, n, 1, 1)) / np.linalg.norm(B, axis=(-2, -1), keepdims=True)
+    F1 = F0 + B + np.conj(np.swapaxes(B, -1, -2))
+    fock = [torch.as_tensor(F, device="cuda") for F in (F0, F1)]
+    seen = []
+
+    def build(P, **kw):
+        seen.append(P.clone())
+        zero = torch.zeros_like(P)
+        return zero, torch.zeros((1, 1, nb, nb), dtype=P.dtype, device=P.device), fock[min(len(seen) - 1, 1)]
+
+    K = G.HartreeFockKernel(np.full((n, n), 1.0 / n ** 2), F0.copy(), np.ones((n, n, 1, 1)), 1e-12)
+    solve(K, np.zeros((n, n, nb, nb), complex), float(ne), fock_build_fn=build,
+          config=SolverConfig(max_iter=2, max_step=1e9, denom_scale=1e-9, bt_max=bt_max, chunk=1))
+    P = seen[2].cpu().numpy()  # initial, first iteration, second iteration
+    assert np.abs(P - seen[1].cpu().numpy()).max() > 0.1
+    tr = np.einsum("xyii->xy", P).real
+    whole = np.abs(tr - np.round(tr)) < 1e-9  # all but a k-point whose state lies at mu (T = 1e-12)
+    assert whole.mean() > 0.95
+    assert np.abs(P @ P - P)[whole].max() <= 30 * nb * 1.2e-16
