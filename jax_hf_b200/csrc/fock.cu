@@ -321,11 +321,15 @@ __global__ void __launch_bounds__(kThreads) k_fock_col(const __grid_constant__ F
   }
 }
 
-// Reduces rho partials and forms the k-independent terms (fock.py:66-92).  One CTA: a warp
-// per slot sums the partials of the nk1 rows, then a thread per matrix entry forms the
-// terms, contact term by contact term as (O_i rho) O_j through shared memory.  Latency is
-// all that counts here; the serial form (a thread per slot down the rows, every thread
-// its own trace and triple product) took 26 us at 90 rows with two terms of nb = 6.
+// Reduces rho partials and forms the k-independent terms (fock.py:66-92).  One CTA; latency is all
+// that counts here.  The sums over the nk1 rows, the trace and the products keep the order of
+// additions of a thread per slot and a thread per matrix entry that walk them one by one (an
+// SCF loop amplifies a change of their rounding): the row sums read tiles of rows that all
+// threads have put into shared memory, four tiles in flight; the trace is a chain of additions
+// beside the first product; the triple product goes as (O_i rho) O_j through shared memory.
+// A build of the constant terms alone, 90 x 75 x 6 with two contact terms: 14.4 us, 26.5 with the
+// loads in the walks and the trace and both products in every thread; 49 x 49 x 16: 21.8 (23.2), with
+// two terms 27.9 (92).
 constexpr int kConstThreads = 1024;
 
 template <typename ST>
@@ -333,68 +337,92 @@ __global__ void __launch_bounds__(kConstThreads) k_fock_consts(const __grid_cons
   if (p.active && !*p.active) return;
   using SC = cpx_t<ST>;
   __shared__ double2 rho[kMaxNb * kMaxNb];
-  __shared__ double2 prod[kMaxNb * kMaxNb];
+  __shared__ double2 prod[kMaxNb * kMaxNb];  // tiles of row sums, the trace's terms, O_i rho
   __shared__ double2 tr;
-  const int nb = p.nb, nb2 = p.nb2, LS = p.LS, ns = p.ngroups * LS;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int nb = p.nb, nb2 = p.nb2, LS = p.LS, ns = p.ngroups * LS, tid = threadIdx.x;
   const bool packing = (p.flags & HF_FOCK_PACKING) != 0;
-  for (int c = threadIdx.x; c < nb2; c += blockDim.x) rho[c] = make_double2(0.0, 0.0);
+  for (int c = tid; c < nb2; c += blockDim.x) rho[c] = make_double2(0.0, 0.0);
   __syncthreads();
-  constexpr int U = 4, W = kConstThreads / 32;  // four slots per warp and turn: their loads overlap
-  for (int s0 = wid; s0 < ns; s0 += U * W) {
-    double2 t[U];
+  auto put = [&](int s, double2 t) {
+    const int c = p.chan[s];
+    if (c < 0) return;
+    rho[c] = t;
+    const int a = c / nb, b = c % nb;
+    if (packing && a != b) rho[b * nb + a] = conj(t);
+  };
+  if (ns <= kMaxNb * kMaxNb) {
+    constexpr int U = 4;
+    const int R = (kMaxNb * kMaxNb) / ns, n = p.nk1 * ns, step = R * ns;  // a tile is R rows
+    double2 t = make_double2(0.0, 0.0);
+    for (int base = 0; base < n; base += U * step) {
+      double2 v[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) t[u] = make_double2(0.0, 0.0);
-    for (int k1 = lane; k1 < p.nk1; k1 += 32)
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (s0 + u * W < ns) t[u] = cadd(t[u], p.rho_part[(size_t)k1 * ns + s0 + u * W]);
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int c = s0 + u * W < ns ? p.chan[s0 + u * W] : -1;
-      t[u].x = warp_sum(t[u].x);
-      t[u].y = warp_sum(t[u].y);
-      if (lane == 0 && c >= 0) {
-        rho[c] = t[u];
-        const int a = c / nb, b = c % nb;
-        if (packing && a != b) rho[b * nb + a] = conj(t[u]);
+      for (int u = 0; u < U; ++u) {
+        const int e = base + u * step + tid;
+        v[u] = tid < step && e < n ? p.rho_part[e] : make_double2(0.0, 0.0);
       }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int rows = min(R, (n - (base + u * step)) / ns);
+        if (rows <= 0) break;
+        if (tid < step) prod[tid] = v[u];
+        __syncthreads();
+        if (tid < ns)
+          for (int r = 0; r < rows; ++r) t = cadd(t, prod[r * ns + tid]);
+        __syncthreads();
+      }
+    }
+    if (tid < ns) put(tid, t);
+  } else {  // padded slots beyond one per thread
+    for (int s = tid; s < ns; s += blockDim.x) {
+      double2 t = make_double2(0.0, 0.0);
+      for (int k1 = 0; k1 < p.nk1; ++k1) t = cadd(t, p.rho_part[(size_t)k1 * ns + s]);
+      put(s, t);
     }
   }
   __syncthreads();
   // Hartree diagonal: HH @ n, n_a = Re rho_aa (fock.py:66-74)
   double hd = 0.0;
-  if (threadIdx.x < nb) {
+  if (tid < nb) {
     if (p.flags & HF_FOCK_HARTREE) {
-      const ST* HH = static_cast<const ST*>(p.HH) + threadIdx.x * nb;
+      const ST* HH = static_cast<const ST*>(p.HH) + tid * nb;
       for (int b = 0; b < nb; ++b) hd += (double)HH[b] * rho[b * nb + b].x;
     }
-    p.hdiag[threadIdx.x] = (double)(ST)hd;
+    p.hdiag[tid] = (double)(ST)hd;
   }
   // contact: sum_t g_t [Oi_t tr(Oj_t rho) - Oi_t rho Oj_t] (fock.py:77-92)
-  const int c = threadIdx.x, i = c / nb, l = c - i * nb;  // nb2 <= kConstThreads
+  const int c = tid, i = c / nb, l = c - i * nb;  // nb2 <= kConstThreads
   double2 acc = make_double2(0.0, 0.0);
   for (int t = 0; t < p.n_contact; ++t) {
     const SC* oi = static_cast<const SC*>(p.cOi) + (size_t)t * nb2;
     const SC* oj = static_cast<const SC*>(p.cOj) + (size_t)t * nb2;
-    if (wid == 0) {
-      double2 z = make_double2(0.0, 0.0);
-      for (int q = lane; q < nb2; q += 32) z = cfma(cvt<double2>(oj[q]), rho[(q % nb) * nb + q / nb], z);
-      z.x = warp_sum(z.x);
-      z.y = warp_sum(z.y);
-      if (lane == 0) tr = z;
-    }
+    // the roundings are spelled out where the compiler could choose which product of two it fuses
     if (c < nb2) {
-      double2 m = make_double2(0.0, 0.0);  // (O_i rho)_{il}
-      for (int k = 0; k < nb; ++k) m = cfma(cvt<double2>(oi[i * nb + k]), rho[k * nb + l], m);
-      prod[c] = m;
+      const double2 a = cvt<double2>(oj[c]), b = rho[l * nb + i];
+      prod[c] = make_double2(fma(a.x, b.x, -__dmul_rn(a.y, b.y)), fma(a.y, b.x, __dmul_rn(a.x, b.y)));
     }
+    __syncthreads();
+    if (tid >= kConstThreads - 32 && tid < kConstThreads - 30) {  // the trace's parts, a lane each
+      const double* q = reinterpret_cast<const double*>(prod) + (tid & 1);
+      double z = 0.0;
+#pragma unroll 8
+      for (int e = 0; e < nb2; ++e) z += q[2 * e];
+      reinterpret_cast<double*>(&tr)[tid & 1] = z;
+    }
+    double2 m = make_double2(0.0, 0.0);  // (O_i rho)_{il}
+    if (c < nb2)
+      for (int k = 0; k < nb; ++k) m = cadd(m, cmul(cvt<double2>(oi[i * nb + k]), rho[k * nb + l]));
+    __syncthreads();
+    if (c < nb2) prod[c] = m;
     __syncthreads();
     if (c < nb2) {
       const double g = (double)static_cast<const ST*>(p.cg)[t];
+      const double2 o = cvt<double2>(oi[c]);
+      const double2 ot = make_double2(fma(o.x, tr.x, -__dmul_rn(o.y, tr.y)), fma(o.x, tr.y, __dmul_rn(o.y, tr.x)));
+      const double2 hterm = cscale(ot, g);
       double2 f = make_double2(0.0, 0.0);
-      for (int k = 0; k < nb; ++k) f = cfma(prod[i * nb + k], cvt<double2>(oj[k * nb + l]), f);
-      acc = cadd(acc, cscale(csub(cmul(cvt<double2>(oi[c]), tr), f), g));
+      for (int k = 0; k < nb; ++k) f = cadd(f, cmul(prod[i * nb + k], cvt<double2>(oj[k * nb + l])));
+      acc = cadd(acc, csub(hterm, cscale(f, g)));
     }
     __syncthreads();
   }
@@ -402,7 +430,7 @@ __global__ void __launch_bounds__(kConstThreads) k_fock_consts(const __grid_cons
   if (p.Hout) {
     SC* Ho = static_cast<SC*>(p.Hout);
     if (c < nb2 && i != l) Ho[c] = mk<SC>(0.0, 0.0);
-    if (threadIdx.x < nb) Ho[threadIdx.x * nb + threadIdx.x] = mk<SC>((double)(ST)hd, 0.0);
+    if (tid < nb) Ho[tid * nb + tid] = mk<SC>((double)(ST)hd, 0.0);
   }
 }
 

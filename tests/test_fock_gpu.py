@@ -768,3 +768,57 @@ def test_grid_wide_bisection_where_the_count_is_not_monotonic(cuda, T):
         _lib.check(L.hf_find_mu(*args, out[0, i:].data_ptr()))
         _lib.check(L.hf_find_mu_ws(*args, out[1, i:].data_ptr(), ws.data_ptr(), ws.numel()))
     assert torch.equal(out[0], out[1])
+
+
+def _fma(x, y, z):
+    from fractions import Fraction
+    return float(Fraction(x) * Fraction(y) + Fraction(z))
+
+
+@pytest.mark.parametrize("n,nb", [(5, 3), (90, 6), (49, 16), (144, 2), (40, 8)])
+@pytest.mark.parametrize("packing", [False, True])
+def test_constant_terms_add_the_rows_one_by_one(cuda, n, nb, packing):
+    """The constant terms of a build keep the roundings of adding the mesh rows in order (an SCF loop's DIIS
+    amplifies any other order).  One k-point per row and weight 1 make a row's partial sum P itself, and the
+    identity as Hartree matrix makes H its running sum, so plain sequential sums are the oracle, bit for bit."""
+    import jax_hf_b200 as G
+    rng = np.random.default_rng(n + nb)
+    P = rng.normal(size=(n, 1, nb, nb)) + 1j * rng.normal(size=(n, 1, nb, nb))
+    P = 0.5 * (P + np.conj(np.swapaxes(P, -1, -2)))
+    t = lambda x: torch.as_tensor(x, device="cuda")
+    VR = t(np.ones((n, 1, 1, 1)))
+    _, H, _ = G.build_fock(t(P), h=t(np.zeros_like(P)), VR=VR, refP=None, HH=t(np.eye(nb)), w2d=t(np.ones((n, 1))),
+                           include_exchange=packing, include_hartree=True, exchange_hermitian_channel_packing=packing)
+    s = np.zeros(nb)
+    for k in range(n):
+        s = s + np.einsum("aa->a", P[k, 0]).real
+    assert np.array_equal(np.einsum("aa->a", H.cpu().numpy()[0, 0]).real, s)
+
+
+@pytest.mark.parametrize("nb", [1, 3, 8])
+def test_contact_term_keeps_its_roundings(cuda, nb):
+    """Sigma of one contact term at one k-point against the same sums in exact fused multiply-adds: products
+    a.x b.x - a.y b.y and a.x b.y + a.y b.x with one fused rounding each, added to the running sum."""
+    import jax_hf_b200 as G
+    rng = np.random.default_rng(nb)
+    P, Oi, Oj = (rng.normal(size=(nb, nb)) + 1j * rng.normal(size=(nb, nb)) for _ in range(3))
+    t = lambda x: torch.as_tensor(np.ascontiguousarray(x), device="cuda")
+    S, _, _ = G.build_fock(t(P[None, None]), h=t(np.zeros((1, 1, nb, nb), complex)), VR=None, refP=None,
+                           HH=t(np.zeros((nb, nb))), w2d=t(np.ones((1, 1))), include_exchange=False,
+                           include_hartree=True, exchange_hermitian_channel_packing=False,
+                           contact_g=t(np.array([1.0])), contact_Oi=t(Oi[None]), contact_Oj=t(Oj[None]))
+    prod = lambda a, b: complex(_fma(a.real, b.real, -(a.imag * b.imag)), _fma(a.imag, b.real, a.real * b.imag))
+
+    def dot(pairs):
+        z = 0j
+        for a, b in pairs:
+            z = z + prod(complex(a), complex(b))
+        return z
+
+    tr = dot([(Oj[a, b], P[b, a]) for a in range(nb) for b in range(nb)])
+    R = [[dot([(Oi[i, k], P[k, l]) for k in range(nb)]) for l in range(nb)] for i in range(nb)]
+    for i in range(nb):
+        for l in range(nb):
+            o = complex(Oi[i, l])
+            ht = complex(_fma(o.real, tr.real, -(o.imag * tr.imag)), _fma(o.real, tr.imag, o.imag * tr.real))
+            assert complex(S[0, 0, i, l].item()) == ht - dot([(R[i][k], Oj[k, l]) for k in range(nb)])
