@@ -52,7 +52,8 @@ __global__ void k_density(int batch, int nb, const cpx_t<RT>* __restrict__ Q, co
 // forming column c of X = Q diag(p) Q^H from a shared copy of Q read by broadcast; the copy
 // then takes X for the hermitisation.  The warp-per-matrix form above recomputes its
 // indices and reads both factors from shared memory per product: 65 us for 2401 matrices
-// of nb = 16 (cold, launch list), 10.5 us here.
+// of nb = 16 (cold, launch list), 12 us here.  The products and their order are that form's,
+// bit for bit: the SCF loops run either.
 template <typename RT, int NB>
 __global__ void __launch_bounds__(128) k_density_cols(int batch, const cpx_t<RT>* __restrict__ Q,
                                                       const RT* __restrict__ p, cpx_t<RT>* __restrict__ P) {
@@ -71,14 +72,14 @@ __global__ void __launch_bounds__(128) k_density_cols(int batch, const cpx_t<RT>
   __syncwarp();
   double2 x[NB];
   if (on) {
-    double2 cq[NB];
+    double2 qc[NB];
 #pragma unroll
-    for (int n = 0; n < NB; ++n) cq[n] = cscale(conj(SQ[c * LP + n]), sp[g][n]);
+    for (int n = 0; n < NB; ++n) qc[n] = SQ[c * LP + n];
 #pragma unroll
-    for (int r = 0; r < NB; ++r) {
+    for (int r = 0; r < NB; ++r) {  // warp_density's products and order: the same bits
       double2 acc = make_double2(0.0, 0.0);
 #pragma unroll
-      for (int n = 0; n < NB; ++n) acc = cfma(SQ[r * LP + n], cq[n], acc);
+      for (int n = 0; n < NB; ++n) acc = cadd(acc, cscale(cmulc(SQ[r * LP + n], qc[n]), sp[g][n]));
       x[r] = acc;
     }
   }

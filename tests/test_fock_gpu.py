@@ -822,3 +822,19 @@ def test_contact_term_keeps_its_roundings(cuda, nb):
             o = complex(Oi[i, l])
             ht = complex(_fma(o.real, tr.real, -(o.imag * tr.imag)), _fma(o.real, tr.imag, o.imag * tr.real))
             assert complex(S[0, 0, i, l].item()) == ht - dot([(R[i][k], Oj[k, l]) for k in range(nb)])
+
+
+@pytest.mark.parametrize("nb,dt", [(9, np.complex128), (12, np.complex128), (16, np.complex128), (3, np.complex64),
+                                   (8, np.complex64), (13, np.complex64)])
+@pytest.mark.parametrize("nk", [1, 45])
+def test_density_from_orbitals_has_the_bits_of_the_general_kernel(cuda, nb, dt, nk):
+    """The column kernel against the warp-per-matrix kernel, which takes the same orbitals padded with zeros
+    to 17 bands: the padding adds zeros to sums in the same order, so the bits are the same."""
+    from jax_hf_b200 import linalg as L
+    rng = np.random.default_rng(nb + nk)
+    Q = (rng.normal(size=(nk, nb, nb)) + 1j * rng.normal(size=(nk, nb, nb))).astype(dt)
+    p = rng.uniform(0, 1, size=(nk, nb)).astype(np.zeros(1, dt).real.dtype)
+    Qp, pp = np.zeros((nk, 17, 17), dt), np.zeros((nk, 17), p.dtype)
+    Qp[:, :nb, :nb], pp[:, :nb] = Q, p
+    t = lambda x: torch.as_tensor(x, device="cuda")
+    assert torch.equal(L.density_from_Qp(t(Q), t(p)), L.density_from_Qp(t(Qp), t(pp))[:, :nb, :nb])
