@@ -305,6 +305,9 @@ int hf_eigh(void* stream, int dtype, int batch, int nb, const void* A, void* w, 
  * previous SCF iteration's Fock matrix), the sweeps converge at once.  The result
  * is an exact decomposition either way (to the Jacobi tolerance). */
 int hf_eigh_warm(void* stream, int nk, int nb, const void* A, const void* Qin, void* Qout, void* w);
+/* hf_eigh by cyclic Jacobi at every size (a lane per column for complex128 and nb <= 8, a warp per
+ * matrix otherwise): the eigensolver of the SCF loops, whose trajectories rest on its roundings. */
+int hf_eigh_jacobi(void* stream, int dtype, int batch, int nb, const void* A, void* w, void* V);
 int hf_cayley_retract(void* stream, int dtype, int batch, int nb, const void* d, double tau,
                       void* U);
 int hf_cayley_spectral(void* stream, int dtype, int batch, int nb, const void* d, void* V,

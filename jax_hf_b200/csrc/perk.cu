@@ -349,12 +349,8 @@ extern "C" int hf_fock_orbital(void* stream, int dtype, int batch, int nb, const
   return HF_OK;
 }
 
-static int eigh_common(void* stream, int dtype, int batch, int nb, int mode, const void* A, void* w, void* V) {
-  int st = check_perk(dtype, batch, nb);
-  if (st) return st;
-  if (batch == 0) return HF_OK;
-  if (!A || !w || !V) return fail(HF_ERR_INVALID, "NULL argument");
-  if (nb >= 2 && nb <= 16) return hf::eigh_tri(stream, dtype, batch, nb, A, w, V, mode);
+// The warp-per-matrix Jacobi.
+static int eigh_warp(void* stream, int dtype, int batch, int nb, int mode, const void* A, void* w, void* V) {
   Launch L = warp_launch(batch, jacobi_smem_elems(nb));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (dtype == HF_C128) {
@@ -366,6 +362,24 @@ static int eigh_common(void* stream, int dtype, int batch, int nb, int mode, con
   }
   HF_LAUNCH_CHECK("k_eigh");
   return HF_OK;
+}
+
+static int eigh_common(void* stream, int dtype, int batch, int nb, int mode, const void* A, void* w, void* V) {
+  int st = check_perk(dtype, batch, nb);
+  if (st) return st;
+  if (batch == 0) return HF_OK;
+  if (!A || !w || !V) return fail(HF_ERR_INVALID, "NULL argument");
+  if (nb >= 2 && nb <= 16) return hf::eigh_tri(stream, dtype, batch, nb, A, w, V, mode);
+  return eigh_warp(stream, dtype, batch, nb, mode, A, w, V);
+}
+
+extern "C" int hf_eigh_jacobi(void* stream, int dtype, int batch, int nb, const void* A, void* w, void* V) {
+  int st = check_perk(dtype, batch, nb);
+  if (st) return st;
+  if (batch == 0) return HF_OK;
+  if (!A || !w || !V) return fail(HF_ERR_INVALID, "NULL argument");
+  if (dtype == HF_C128 && nb <= 8) return hf_eigh_warm(stream, batch, nb, A, nullptr, V, static_cast<double*>(w));
+  return eigh_warp(stream, dtype, batch, nb, 0, A, w, V);
 }
 
 extern "C" int hf_eigh(void* stream, int dtype, int batch, int nb, const void* A, void* w, void* V) {

@@ -122,11 +122,11 @@ struct Scf {
   bool fp32 = false;    // this build runs the exchange FFT in FP32
   bool mu_warm = false;  // a previous mu exists: the Newton-bracket start, or the bisection's hint
   bool eig_warm = false; // eigh started from the eigenvectors in kV (the previous decomposition)
-  // eigh by the lane-per-column Jacobi (nb <= 8), cold or warm.  The DIIS extrapolation
-  // solves a nearly singular system and amplifies the rounding of the eigensolver:
-  // with hf_eigh's tridiagonal solver the iteration counts of 14 of 27 random
-  // problems moved by 1 to 3 and the results by up to 1e-7 (within the tolerances), so the
-  // loop stays on the kernels whose trajectories are pinned by its stored results.
+  // eigh by the lane-per-column Jacobi (nb <= 8), cold or warm; above that the loop runs the
+  // warp-per-matrix Jacobi (hf_eigh_jacobi).  The DIIS extrapolation solves a nearly singular
+  // system and amplifies the rounding of the eigensolver: with hf_eigh's tridiagonal solver the
+  // iteration counts of 14 of 27 random problems moved by 1 to 3 or their results by up to
+  // 1e-7 (within the tolerances), so the loop stays on the kernels whose trajectories are stored.
   bool eig_cols = false;
   // herm(project(X)) in place (the caller's projector), or nothing without one
   int project(void* X) {
@@ -165,7 +165,7 @@ struct Scf {
     if (eig_cols) {  // from the previous eigenvectors when asked for and there are any
       if ((st = hf_eigh_warm(s, nk, nb, F, eig_warm ? at<void>(kV) : nullptr, at<void>(kV), at<double>(kEV))))
         return st;
-    } else if ((st = hf_eigh(s, HF_C128, nk, nb, F, at<double>(kEV), at<void>(kV)))) {
+    } else if ((st = hf_eigh_jacobi(s, HF_C128, nk, nb, F, at<double>(kEV), at<void>(kV)))) {
       return st;
     }
     // mu_method 2: Newton-bracket solver, from mu = 0 in the first call and from the previous

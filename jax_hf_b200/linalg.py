@@ -36,18 +36,16 @@ def eigh(A):
 
 
 def eigh_jacobi(A):
-    """The same decomposition by the cyclic Jacobi of the SCF loop (complex128, nb <= 8)."""
+    """The same decomposition by the cyclic Jacobi of the SCF loop (complex128)."""
     A = _as_dev(A)
     batch, nb = _batch(A)
-    # hf_eigh_warm takes no dtype: it reads and writes 16-byte elements
+    # the loop's buffers hold 16-byte elements
     if A.dtype != torch.complex128:
         raise TypeError(f"eigh_jacobi needs a complex128 array, got {A.dtype}")
-    if not 1 <= nb <= 8:
-        raise ValueError(f"eigh_jacobi needs 1 <= nb <= 8, got {nb}")
     w = torch.empty(A.shape[:-1], dtype=torch.float64, device=A.device)
     V = torch.empty_like(A)
-    _lib.check(_lib.lib().hf_eigh_warm(_lib.stream_ptr(A.device), batch, nb, A.data_ptr(), None, V.data_ptr(),
-                                       w.data_ptr()))
+    _lib.check(_lib.lib().hf_eigh_jacobi(_lib.stream_ptr(A.device), _lib.HF_C128, batch, nb, A.data_ptr(),
+                                         w.data_ptr(), V.data_ptr()))
     return w, V
 
 

@@ -27,7 +27,7 @@ import torch
 
 from . import _lib
 from .fock import build_fock, hf_energy
-from .linalg import density_from_Qp, eigh, eigh_jacobi
+from .linalg import density_from_Qp, eigh_jacobi
 from .utils import validate_electron_count
 
 
@@ -183,7 +183,7 @@ def _solve_scf_impl(kernel, P0, n_electrons, cfg, fock_build_fn):
 
     def density_from_fock(F):
         """reference_scf.py:87-96: eigh, bisection mu, level shift, occupations."""
-        ev, orb = eigh_jacobi(F) if F.shape[-1] <= 8 else eigh(F)
+        ev, orb = eigh_jacobi(F)
         mu_raw = ops.find_mu(ev, w2d, n_electrons, T, method=0)
         if cfg.level_shift != 0.0:
             shifted = ops.fermi(ev, mu_raw, T, 2, cfg.level_shift)

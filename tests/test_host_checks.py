@@ -22,14 +22,9 @@ def no_library(monkeypatch):
 
 @pytest.mark.parametrize("dtype", [torch.complex64, torch.float32, torch.float64])
 def test_eigh_jacobi_refuses_other_element_sizes(no_library, dtype):
-    """hf_eigh_warm has no dtype argument and takes 16-byte elements."""
+    """The SCF loop's eigensolver takes 16-byte elements."""
     with pytest.raises(TypeError, match="complex128"):
         linalg.eigh_jacobi(torch.zeros((3, 4, 4), dtype=dtype))
-
-
-def test_eigh_jacobi_refuses_more_bands_than_the_kernel(no_library):
-    with pytest.raises(ValueError, match="nb"):
-        linalg.eigh_jacobi(torch.zeros((3, 9, 9), dtype=torch.complex128))
 
 
 @pytest.mark.parametrize("dtype", [torch.complex64, torch.complex128, torch.float64])
