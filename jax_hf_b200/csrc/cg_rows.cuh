@@ -188,9 +188,9 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_cgr_density(CgArgs a, int fo
 // P = herm(Q diag(p) Q^H) from given occupations (hf_density_from_Qp for complex128,
 // nb <= 8): the density step of k_cgr_density without the Fermi function
 template <int NB>
-__global__ void __launch_bounds__(32 * kRowWarps) k_rows_density(int nk, const double2* __restrict__ Q,
-                                                                 const double* __restrict__ p,
-                                                                 double2* __restrict__ P) {
+__global__ void __launch_bounds__(32 * kRowWarps) k_rows_density(int nk, const double2* Q,
+                                                                 const double* p,
+                                                                 double2* P) {
   pdl_begin();
   using RG = RowGroup<NB>;
   constexpr int G = RG::G, KPW = RG::KPW, LP = RG::LP, MAT = RG::MAT;
@@ -748,7 +748,7 @@ __device__ __forceinline__ void jacobi_reg_cols(double2 (&a)[NB], double2 (&v)[N
 // Qout = Qin V.  Qin may equal Qout: a k-point's rows are read before they are written.
 constexpr int kEigWarps = 2;
 template <int NB>
-__device__ __forceinline__ void eig_cols(int nk, const double2* __restrict__ A, const double2* Qin, double2* Qout,
+__device__ __forceinline__ void eig_cols(int nk, const double2* A, const double2* Qin, double2* Qout,
                                          double* eps, double tol) {
   const bool rotate = Qin != nullptr;
   using RG = RowGroup<NB>;
@@ -869,7 +869,7 @@ __device__ __forceinline__ void eig_cols(int nk, const double2* __restrict__ A, 
 
 // Standalone eigensolve: eps, Qout <- eigh(A) (Qin == nullptr) or with the starting basis Qin.
 template <int NB>
-__global__ void __launch_bounds__(32 * kEigWarps, 8) k_eig_cols(int nk, const double2* __restrict__ A,
+__global__ void __launch_bounds__(32 * kEigWarps, 8) k_eig_cols(int nk, const double2* A,
                                                              const double2* Qin, double2* Qout, double* eps,
                                                              double tol) {
   pdl_begin();

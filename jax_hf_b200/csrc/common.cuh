@@ -226,7 +226,8 @@ __device__ __forceinline__ void block_reduce_all(KSum (&acc)[NS], Sink&& sink) {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
-// First statement of every kernel that launch_pdl launches, ahead of any early return: a
+// First statement of every kernel that launch_pdl launches, ahead of any early return (and no parameter of
+// such a kernel is __restrict__: its predecessor may still be at that memory): a
 // grid that ended without waiting would let its successor start before its predecessor ended.
 __device__ __forceinline__ void pdl_begin() {
   pdl_wait();

@@ -124,7 +124,7 @@ __device__ __forceinline__ bool qr_sweep(double (&d)[NB], double (&e)[NB], doubl
 // V diag(eps) V^H = herm(A) (mode 0) or herm(i A) (mode 1) for nk matrices, ascending.
 template <typename RT, int NB>
 __global__ void __launch_bounds__(TriShape<NB>::MAXM * TriShape<NB>::G, TriShape<NB>::CTAS)
-    k_eigh_tri(int nk, int mode, const cpx_t<RT>* __restrict__ A, RT* __restrict__ eps, cpx_t<RT>* V) {
+    k_eigh_tri(int nk, int mode, const cpx_t<RT>* A, RT* eps, cpx_t<RT>* V) {
   pdl_begin();
   using S = TriShape<NB>;
   constexpr int G = S::G, LP = S::LP;

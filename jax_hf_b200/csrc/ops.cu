@@ -30,8 +30,8 @@ __device__ __forceinline__ void write_partials(KSum (&acc)[NS], double* part, in
 // fixed-shape block reduction, so the result is deterministic for a launch shape.
 // (One warp walking every partial in one dependent chain took ~150 us at 592 blocks.)
 constexpr int kSumThreads = 128;
-__global__ void __launch_bounds__(kSumThreads) k_sum_partials(const double* __restrict__ part, int nblk, int ns,
-                                                              double* __restrict__ out) {
+__global__ void __launch_bounds__(kSumThreads) k_sum_partials(const double* part, int nblk, int ns,
+                                                              double* out) {
   pdl_begin();
   __shared__ double sm[2 * 32];
   const int q = blockIdx.x;
@@ -55,8 +55,8 @@ static int nblocks(size_t n) {
 // mode 0: fermidirac(eps - mu, T) = expit(-(eps - mu)/(T + 1e-12))  (utils.py:51-53)
 // mode 1: sigmoid((mu - eps)/max(T, 1e-12))                        (solver.py:394)
 // mode 2: eps + level_shift (1 - fermidirac(eps - mu, T))           (reference_scf.py:92)
-__global__ void k_fermi(size_t n, const double* __restrict__ eps, const double* __restrict__ mu, double T,
-                        int mode, double shift, double* __restrict__ out) {
+__global__ void k_fermi(size_t n, const double* eps, const double* mu, double T,
+                        int mode, double shift, double* out) {
   pdl_begin();
   const double m = mu[0];
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
@@ -70,10 +70,10 @@ __global__ void k_fermi(size_t n, const double* __restrict__ eps, const double* 
 // --------------------------------------------------------- SCF residuals --
 // delta = Pn - P, comm = F P - P F (stored), sums: w|delta|^2, w|comm|^2, w Re tr(F delta)
 // comm_slot (may be NULL): comm is the history slot *comm_slot of comm_stride elements each
-__global__ void k_scf_residuals(int nk, int nb, const double2* __restrict__ F, const double2* __restrict__ P,
-                                const double2* __restrict__ Pn, const double* __restrict__ w,
-                                double2* __restrict__ comm, double2* __restrict__ delta, double* part,
-                                const int* __restrict__ comm_slot, size_t comm_stride) {
+__global__ void k_scf_residuals(int nk, int nb, const double2* F, const double2* P,
+                                const double2* Pn, const double* w,
+                                double2* comm, double2* delta, double* part,
+                                const int* comm_slot, size_t comm_stride) {
   pdl_begin();
   if (comm && comm_slot) comm += (size_t)(*comm_slot) * comm_stride;
   extern __shared__ double2 smd[];
@@ -117,8 +117,8 @@ __global__ void k_scf_residuals(int nk, int nb, const double2* __restrict__ F, c
 // N (history slots) is a template parameter so that every loop has a compile-time
 // trip count and the N (N + 1) / 2 accumulators stay in registers.
 template <int N>
-__global__ void k_gram(size_t stride, size_t len, int nb2, const double2* __restrict__ R,
-                       const double* __restrict__ w, double* part) {
+__global__ void k_gram(size_t stride, size_t len, int nb2, const double2* R,
+                       const double* w, double* part) {
   pdl_begin();
   constexpr int np = N * (N + 1) / 2;
   // a thread sums its few elements in plain FP64; the thread, block and grid partials
@@ -148,8 +148,8 @@ __global__ void k_gram(size_t stride, size_t len, int nb2, const double2* __rest
 // the SCF driver keeps the rest of B and refreshes the row with one launch.  Every
 // entry is formed exactly as in k_gram (fma(x_i, x_j, y_i y_j) is symmetric in i, j).
 template <int N>
-__global__ void k_gram_row(size_t stride, size_t len, int nb2, const double2* __restrict__ R, int inew,
-                           const double* __restrict__ w, double* part, const int* __restrict__ inew_dev = nullptr) {
+__global__ void k_gram_row(size_t stride, size_t len, int nb2, const double2* R, int inew,
+                           const double* w, double* part, const int* inew_dev = nullptr) {
   pdl_begin();
   if (inew_dev) inew = *inew_dev;
   double acc[N];
@@ -171,8 +171,8 @@ __global__ void k_gram_row(size_t stride, size_t len, int nb2, const double2* __
 }
 
 // out = sum_i c_i X_i (+ optional herm)
-__global__ void k_lincomb(int n, size_t stride, size_t len, int nb, const double2* __restrict__ X,
-                          const double* __restrict__ c, double2* __restrict__ out) {
+__global__ void k_lincomb(int n, size_t stride, size_t len, int nb, const double2* X,
+                          const double* c, double2* out) {
   pdl_begin();
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < len; e += (size_t)gridDim.x * blockDim.x) {
     double2 acc = make_double2(0.0, 0.0);
@@ -182,8 +182,8 @@ __global__ void k_lincomb(int n, size_t stride, size_t len, int nb, const double
 }
 
 // out = a x + b y, hermitised when herm != 0 (complex arrays, nb x nb per k)
-__global__ void k_axpby(size_t nk, int nb, double a, const double2* __restrict__ x, double b,
-                        const double2* __restrict__ y, int herm, double2* __restrict__ out) {
+__global__ void k_axpby(size_t nk, int nb, double a, const double2* x, double b,
+                        const double2* y, int herm, double2* out) {
   pdl_begin();
   const int nb2 = nb * nb;
   const size_t n = nk * nb2;
@@ -198,17 +198,17 @@ __global__ void k_axpby(size_t nk, int nb, double a, const double2* __restrict__
   }
 }
 
-__global__ void k_axpby_real(size_t n, double a, const double* __restrict__ x, double b,
-                             const double* __restrict__ y, double* __restrict__ out) {
+__global__ void k_axpby_real(size_t n, double a, const double* x, double b,
+                             const double* y, double* out) {
   pdl_begin();
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x)
     out[e] = a * x[e] + (y ? b * y[e] : 0.0);
 }
 
 // joint inner product sum_k wX_k sum Re(conj(aX) bX) + sum_k wp_k sum ap bp  (solver.py:205-233, 783-787)
-__global__ void k_jdot(size_t nk, int nb, const double2* __restrict__ aX, const double2* __restrict__ bX,
-                       const double* __restrict__ wX, const double* __restrict__ ap, const double* __restrict__ bp,
-                       const double* __restrict__ wp, double* part) {
+__global__ void k_jdot(size_t nk, int nb, const double2* aX, const double2* bX,
+                       const double* wX, const double* ap, const double* bp,
+                       const double* wp, double* part) {
   pdl_begin();
   KSum acc[1];
   const int nb2 = nb * nb;
@@ -269,8 +269,8 @@ __global__ void k_jdot_multi(size_t nk, int nb, const __grid_constant__ JdotMult
 
 // ---------------------------------------------------------------- Newton --
 // G = skew((p_j - p_i) Ft) offdiag, eps = Re diag(Ft)                 (solver.py:898-900)
-__global__ void k_orbital_grad(size_t nk, int nb, const double2* __restrict__ Ft, const double* __restrict__ p,
-                               double2* __restrict__ G, double* __restrict__ eps) {
+__global__ void k_orbital_grad(size_t nk, int nb, const double2* Ft, const double* p,
+                               double2* G, double* eps) {
   pdl_begin();
   const int nb2 = nb * nb;
   const size_t n = nk * nb2;
@@ -290,10 +290,10 @@ __global__ void k_orbital_grad(size_t nk, int nb, const double2* __restrict__ Ft
 }
 
 // z = (rX / sqrt(gap^2 + lam^2), rp p(1-p)/T) with p clipped to [occ_clip, 1-occ_clip]; sum w2d zp
-__global__ void k_newton_prec(size_t nk, int nb, const double2* __restrict__ rX, const double* __restrict__ rp,
-                              const double* __restrict__ eps, const double* __restrict__ p, double lam, double T,
-                              double clipv, const double* __restrict__ w2d, double2* __restrict__ zX,
-                              double* __restrict__ zp, double* part) {
+__global__ void k_newton_prec(size_t nk, int nb, const double2* rX, const double* rp,
+                              const double* eps, const double* p, double lam, double T,
+                              double clipv, const double* w2d, double2* zX,
+                              double* zp, double* part) {
   pdl_begin();
   KSum acc[1];
   const int nb2 = nb * nb;
@@ -315,15 +315,15 @@ __global__ void k_newton_prec(size_t nk, int nb, const double2* __restrict__ rX,
   write_partials<1>(acc, part);
 }
 
-__global__ void k_sub_scalar(size_t n, double* __restrict__ x, const double* __restrict__ c, double scale) {
+__global__ void k_sub_scalar(size_t n, double* x, const double* c, double scale) {
   pdl_begin();
   const double v = c[0] * scale;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) x[e] -= v;
 }
 
 // dP = herm(Q M Q^H), M = X o (p_j - p_i) + diag(dp)                 (solver.py:916-919)
-__global__ void k_newton_dP(int nk, int nb, const double2* __restrict__ Q, const double2* __restrict__ X,
-                            const double* __restrict__ dp, const double* __restrict__ p, double2* __restrict__ dP) {
+__global__ void k_newton_dP(int nk, int nb, const double2* Q, const double2* X,
+                            const double* dp, const double* p, double2* dP) {
   pdl_begin();
   extern __shared__ double2 smd[];
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5, wpb = blockDim.x >> 5;
@@ -368,12 +368,12 @@ __global__ void k_newton_dP(int nk, int nb, const double2* __restrict__ Q, const
 
 // St = Q^H (Fr - h) Q; A = Ft X - X Ft + St; C = dpij Ft + pij A;
 // HX = skew(C) offdiag; Hp = Re diag(A) + T/(pc(1-pc)) dp            (solver.py:920-929)
-__global__ void k_newton_hvp(int nk, int nb, const double2* __restrict__ Q, const double2* __restrict__ Ft,
-                             const double2* __restrict__ X, const double* __restrict__ dp,
-                             const double* __restrict__ p, const double2* __restrict__ Fr,
-                             const double2* __restrict__ h, double T, double clipv, double pen,
-                             const double2* __restrict__ dPpen, double2* __restrict__ HX, double* __restrict__ Hp,
-                             const double* __restrict__ w2d, double* part) {
+__global__ void k_newton_hvp(int nk, int nb, const double2* Q, const double2* Ft,
+                             const double2* X, const double* dp,
+                             const double* p, const double2* Fr,
+                             const double2* h, double T, double clipv, double pen,
+                             const double2* dPpen, double2* HX, double* Hp,
+                             const double* w2d, double* part) {
   pdl_begin();
   extern __shared__ double2 smd[];
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5, wpb = blockDim.x >> 5;
@@ -430,8 +430,8 @@ __global__ void k_newton_hvp(int nk, int nb, const double2* __restrict__ Q, cons
 }
 
 // C = A B per k
-__global__ void k_matmul(int nk, int nb, const double2* __restrict__ A, const double2* __restrict__ B,
-                         double2* __restrict__ Cm) {
+__global__ void k_matmul(int nk, int nb, const double2* A, const double2* B,
+                         double2* Cm) {
   pdl_begin();
   extern __shared__ double2 smd[];
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5, wpb = blockDim.x >> 5;
@@ -452,7 +452,7 @@ __global__ void k_matmul(int nk, int nb, const double2* __restrict__ A, const do
   }
 }
 
-__global__ void k_real_diag(size_t nk, int nb, const double2* __restrict__ A, double* __restrict__ d) {
+__global__ void k_real_diag(size_t nk, int nb, const double2* A, double* d) {
   pdl_begin();
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < nk * nb; e += (size_t)gridDim.x * blockDim.x) {
     const size_t k = e / nb;
@@ -520,8 +520,8 @@ int hf::scf_residuals_slot(void* stream, int nk, int nb, const void* F, const vo
   return finish(HF_S, (double*)ws, g, 3, sums3);
 }
 
-__global__ void k_copy_to_slot(size_t n, const double2* __restrict__ x, double2* __restrict__ hist,
-                               const int* __restrict__ slot) {
+__global__ void k_copy_to_slot(size_t n, const double2* x, double2* hist,
+                               const int* slot) {
   pdl_begin();
   double2* dst = hist + (size_t)(*slot) * n;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x)

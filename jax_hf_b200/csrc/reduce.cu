@@ -17,8 +17,8 @@ static int red_blocks(size_t n) {
   return (int)b;
 }
 
-__global__ void k_red_final(const double* __restrict__ part, int nparts, int mode, double T,
-                            const double* __restrict__ E, double* __restrict__ out, const int* active) {
+__global__ void k_red_final(const double* part, int nparts, int mode, double T,
+                            const double* E, double* out, const int* active) {
   pdl_begin();
   if (active && !*active) return;
   __shared__ double sm[64];
@@ -38,9 +38,9 @@ __global__ void k_red_final(const double* __restrict__ part, int nparts, int mod
 
 template <typename RT>
 __global__ void __launch_bounds__(kRedThreads)
-k_energy_part(int nk, int nb, const cpx_t<RT>* __restrict__ P, const cpx_t<RT>* __restrict__ h,
-              const cpx_t<RT>* __restrict__ S, const cpx_t<RT>* __restrict__ H, int H_mode,
-              const RT* __restrict__ w, double* __restrict__ part, const int* active) {
+k_energy_part(int nk, int nb, const cpx_t<RT>* P, const cpx_t<RT>* h,
+              const cpx_t<RT>* S, const cpx_t<RT>* H, int H_mode,
+              const RT* w, double* part, const int* active) {
   pdl_begin();
   if (active && !*active) return;
   __shared__ double sm[64];
@@ -68,8 +68,8 @@ k_energy_part(int nk, int nb, const cpx_t<RT>* __restrict__ P, const cpx_t<RT>* 
 // sum_k w_k sum_i [p log p + (1-p) log1p(-p)], p clipped to [1e-14, 1-1e-14]
 template <typename RT>
 __global__ void __launch_bounds__(kRedThreads)
-k_entropy_part(int nk, int nb, const RT* __restrict__ p, const RT* __restrict__ w,
-               double* __restrict__ part) {
+k_entropy_part(int nk, int nb, const RT* p, const RT* w,
+               double* part) {
   pdl_begin();
   __shared__ double sm[64];
   const size_t n = (size_t)nk * nb;

@@ -74,3 +74,36 @@ def test_scf_workspace_covers_the_builds_of_the_loop(engine, n1, n2, nb):
         _lib.check(fn(C.byref(pb), C.byref(cf), C.byref(need)))
         sizes.append(need.value)
     assert sizes[0] == sizes[1]
+
+
+def _kernels():
+    """(file, name, parameters, body) of every __global__ function in the sources."""
+    import re
+    from pathlib import Path
+    csrc = Path(__file__).resolve().parents[1] / "jax_hf_b200" / "csrc"
+    for f in sorted([*csrc.glob("*.cu"), *csrc.glob("*.cuh")]):
+        s = f.read_text()
+        for m in re.finditer(r"__global__", s):
+            head = s[m.start():s.index("{", m.start())]
+            if ";" in head:
+                continue
+            bounds = re.match(r"__global__\s+void\s*(__launch_bounds__\s*\((?:[^()]|\((?:[^()]|\([^()]*\))*\))*\))?", head)
+            rest = head[bounds.end():]
+            depth, i = 1, m.start() + len(head) + 1
+            while depth:
+                depth += {"{": 1, "}": -1}.get(s[i], 0)
+                i += 1
+            yield f.name, rest[:rest.index("(")].strip(), rest[rest.index("("):], s[m.start() + len(head):i]
+
+
+def test_dependently_launched_kernels_read_through_plain_pointers():
+    """A kernel launched with programmatic serialization starts while its predecessor still writes what it will
+    read and reads what it will write.  __restrict__ would let the compiler read through the non-coherent
+    path, and move accesses across the wait: both take memory that no one else touches while the kernel runs."""
+    seen, bad = 0, []
+    for f, name, params, body in _kernels():
+        if "pdl_begin()" in body or "pdl_wait()" in body:
+            seen += 1
+            if "__restrict__" in params:
+                bad.append(f"{f}: {name}")
+    assert seen > 30 and not bad, bad
