@@ -271,10 +271,10 @@ int hf_free_energy(void* stream, int dtype, int nk1, int nk2, int nb, const doub
 int hf_find_mu(void* stream, int dtype, int method, int nk1, int nk2, int nb, const void* eps,
                const void* weights, double n_electrons, double T, int maxiter, const double* mu0,
                double* mu_out);
-/* The same with a workspace (hf_mu_workspace_size bytes, 256-byte aligned): from some ten
- * thousand eigenvalues on, the bisection without a hint and the warm-started Newton rule run
- * their evaluations over the whole device instead of one cluster.  The bisection's result is
- * bit-identical to hf_find_mu's. */
+/* The same with a workspace (hf_mu_workspace_size bytes, 256-byte aligned), with the same bits: from
+ * 16384 eigenvalues on the bisection without a hint leaves out the evaluations that a certified
+ * bracket decides, and from 131072 (the bisection) or 163840 (the warm-started Newton rule) on the
+ * evaluations run over the whole device instead of one cluster. */
 int hf_mu_workspace_size(size_t* bytes);
 int hf_find_mu_ws(void* stream, int dtype, int method, int nk1, int nk2, int nb, const void* eps,
                   const void* weights, double n_electrons, double T, int maxiter, const double* mu0,

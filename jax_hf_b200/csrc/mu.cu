@@ -40,6 +40,7 @@ constexpr int kMuThreads = 1024;
 constexpr int kMuMaxCluster = 16;  // non-portable size, used when the device schedules it
 constexpr int kBisLevels = 2;  // bisection levels per pass of the 256-thread variant
 constexpr int kMuCertPasses = 6;  // Newton passes of a hinted bisection (certified bracket)
+constexpr int kMuCertPassesCold = 12;  // from the middle of the spectrum
 
 struct MuArgs {
   const void* eps;
@@ -50,6 +51,7 @@ struct MuArgs {
   double* out;
   const int* active;  // optional device flag: return at once when *active == 0
   int cache;          // elements per thread kept in shared memory as (eps, w); 0: read from L2
+  int certify;        // bisection: certify a bracket from the middle of the spectrum (without a hint)
   int kpt;                    // eigenvalues per thread of the cluster kernel
   const struct MuState* pre;  // what the grid-wide passes found, or nullptr
 };
@@ -267,12 +269,18 @@ __device__ __forceinline__ double probe_noise(double margin, double Z, double m)
   return Z > 0.0 ? fmax(margin / Z, 0x1p-52 * fabs(m)) : INFINITY;
 }
 
+// Whether a bracket of this width is as narrow as evaluations with this margin make it: a few times the noise
+// at an iterate m whose count n is next to the target (where N is flat at the target, at once: every
+// level inside has to be evaluated).  Away from the target the noise at m says nothing.
+__device__ __forceinline__ bool bracket_done(double width, double n, double target, double margin, double noise) {
+  return fabs(n - target) <= 16.0 * margin && width <= 4.0 * noise;
+}
+
 // Offset of the two probes around a Newton iterate of N(x) = target that was moved by `step`.
 // |N''| <= N' / Td for every sum of Fermi functions, so a step of at most Td / 2 leaves the
-// iterate within step^2 / Td of the root; longer steps (and bracket midpoints) take twice the
-// step.  `noise`: probe_noise.
-__device__ __forceinline__ double probe_offset(double step, bool newton, double iTd, double noise) {
-  return newton && step * iTd <= 0.5 ? fma(step * step, iTd, 1.5 * noise) : fmax(2.0 * step, 1.5 * noise);
+// iterate within step^2 / Td of the root; longer steps take twice the step.  `noise`: probe_noise.
+__device__ __forceinline__ double probe_offset(double step, double iTd, double noise) {
+  return step * iTd <= 0.5 ? fma(step * step, iTd, 1.5 * noise) : fmax(2.0 * step, 1.5 * noise);
 }
 
 // Bisection levels that need no evaluation: every midpoint >= A is decided "above", every one
@@ -315,17 +323,22 @@ __device__ __forceinline__ bool newton_step(double g, double Z, double& lo, doub
 // (atomic ticket, no spin) takes the step, and the cluster kernel finishes from MuState.
 // Every pass returns at once when the state says done.  The bisection's passes certify a
 // bracket (see the hinted bisection below), the levels inside it are evaluated two per pass,
-// and the cluster kernel finishes what is left.
-// 144 x 144, nb = 8 (166k eigenvalues): the bisection of the cluster kernel alone takes 353 us.
+// and the cluster kernel finishes what is left (with its shared-memory cache: inside a gap that is
+// some forty levels).
 constexpr int kPassThreads = 256;
 constexpr int kPassBlocks = 296;   // two CTAs per SM
 constexpr int kPassSums = 8;
-// Eigenvalues from which the passes are used.  Bisection: 116 us by the cluster kernel against
-// 58 on 16384, 344 against 78 on 165888.  The warm-started Newton rule has only 4 to 8 evaluations,
-// each a launch here and a cluster barrier there: 20 us (cluster) against 27 on 41472, 25
-// against 29 to 45 against 39 on 131072 (T = 0.2, 0.01), 40 against 36 on 165888, 65 against
-// 45 on 294912.
-constexpr int kGridMin = 16384, kGridMinNewton = 131072;
+// Eigenvalues from which a call with a workspace certifies a bracket for the bisection, in the cluster kernel
+// (kCertMin) or by the passes (kGridMin).  What that gives depends on the spectrum, in us against every level
+// in the cluster kernel: for a metal (T = 0.1) 44 against 118 on 16384, 60 against 164 on 38416, 78 against 235
+// on 98304, 77 against 281 on 131072.  With the target inside a gap (gap 2, T = 0.01) the count is flat to its
+// rounding and every level there is evaluated: 121 against 118, 168 against 164, 238 against 235, 284 against 281
+// (one pass to see it).  Passes from 65536 on would take 70 for the metal of 98304, but 202 against 188 in the gap
+// on 65536, where the idle ones show.  kGridMinNewton: the warm-started Newton rule has only 4 to 8
+// evaluations, each a launch here and a cluster barrier there: 39 us in the cluster kernel against 39, 70 against
+// 50 and 95 against 61 by the passes on 165888 (T = 0.1, 0.01, 0.001), 21.1 against 22.9 where a gap ends it
+// after one; on 131072 39 against 40, 55 against 44, 17.2 against 21.0.
+constexpr int kCertMin = 16384, kGridMin = 131072, kGridMinNewton = 163840;
 constexpr int kNewtonPasses = 5;   // method 2: Newton steps queued ahead of the cluster kernel
 constexpr int kLevelPasses = 5;    // bisection: passes of two levels each behind them
 constexpr int kCertPasses = 7;     // bisection: certifying passes, the first one a scan of 8 points
@@ -460,8 +473,8 @@ __global__ void __launch_bounds__(kPassThreads) k_mu_pass(const MuArgs a, MuStat
       const bool newton = Z > 0.0 && isfinite(r) && r > bl && r < bh;
       if (!newton) r = 0.5 * (bl + bh);
       const double fw = probe_noise(margin, Z, m);
-      st->done = A - B <= 4.0 * fw;  // as narrow as the margin allows
-      d = probe_offset(fabs(r - m), newton, 1.0 / Td, fw);
+      st->done = bracket_done(bh - bl, v[0], a.target, margin, fw);
+      d = newton ? probe_offset(fabs(r - m), 1.0 / Td, fw) : 0.0;  // no probes around a middle
     }
     st->A = A;
     st->B = B;
@@ -709,7 +722,7 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
       mn = fmin(mn, v);
       mx = fmax(mx, v);
       const double p = expit(div_by(mu0v - v, Tf, rTf));
-      N0 += w * p;
+      N0 = fma(w, p, N0);  // as k_mu_newton adds
       Z0 += div_by(w * (p * (1.0 - p)), Tf, rTf);
     });
   } else if (has_hint) {  // the first Newton evaluation of the hinted bisection with the extremes
@@ -722,7 +735,7 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
       const double f = cert_fermi(exp((v - hint) * r));
       hv[2] += w * f;
       hv[3] += w * (f * (1.0 - f));
-      hv[4] += w;
+      hv[4] += w < 0.0 ? NAN : w;  // N does not increase then: no bracket
     });
   } else if (!a.pre) {
     visit([&](double v, double) {
@@ -760,9 +773,9 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
     int it = 0;
     bool fixed = false;
     double A = INFINITY, B = -INFINITY;
-    if (has_hint) {
-      // Certified bracket from the hint.  N(x) = sum w / (1 + exp((e - x) / Td)) is
-      // increasing in x; an evaluation N~(x) differs from it by at most E = (kpt + 24) u W
+    if (has_hint || a.certify) {
+      // Certified bracket from the hint, or from the middle of the spectrum.  For weights >= 0
+      // N(x) = sum w / (1 + exp((e - x) / Td)) is increasing in x; an evaluation N~(x) differs from it by at most E = (kpt + 24) u W
       // (kpt terms summed per thread, a reduction tree of depth <= 14, about 6 u per term, and u W for the
       // rounding of the exponent's argument y, whose error u |y| moves a term by f (1 - f) u |y| < 0.23 u;
       // as a product of two exponentials with |z| <= 2 in the second, by less than 1.3 u, and by 2 u for
@@ -775,50 +788,59 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
       // levels whose midpoints lie outside (B, A) are replayed without evaluations and
       // only the last few levels are evaluated.  The decisions, and so the result, are
       // those of evaluating every level.
-      // The first evaluation came with the extremes, at the hint itself.  With that and the
-      // probes at step^2 / Td a call on 2304 eigenvalues (T = 0.1) takes 17.8 us for 19.4 with
-      // a hint 1e-7 off the root and 19.9 for 23.8 with one 1e-2 off, on 165888 83 for 106 and 93 for 121 (then
-      // 16.0, 17.8, 82 and 92 with the interleaved trees of cluster_sum_n).
-      const int kpt = (a.n + gs - 1) / gs;
-      double m = hint, d = 0.0;
+      // With a hint the first evaluation came with the extremes, at the hint itself: a call on 2304
+      // eigenvalues (T = 0.1) takes 16.0 us with a hint 1e-7 off the root and 17.8 with one 1e-2 off,
+      // 49 without a hint.
+      const int kpt = (a.n + gs - 1) / gs, passes = has_hint ? kMuCertPasses : kMuCertPassesCold;
+      double m = has_hint ? hint : 0.5 * (mn + mx), d = 0.0, width = INFINITY;
+      double nA = 0.0, nB = 0.0;  // the counts at A and B
       double v[5] = {hv[2], hv[3], hv[2], hv[2], hv[4]};  // N(m), N'(m) Td, N(m - d), N(m + d), W
       for (int t = 0;;) {
+        if (t > 0 || !has_hint) {
+          // The probes are the rounded m - d and m + d, as they are recorded in A and B: what counts is the
+          // count at the recorded number (one half ulp of m beside it is more than the margin for a band
+          // that is narrow against its offset from zero).  exp((e - x) / Td) is the product of the
+          // exponential at m and the factor of the realised offset m - x where that is small.
+          const double pl = m - d, ph = m + d, zl = (m - pl) * iTd, zh = (m - ph) * iTd;
+          const bool fac = zl <= 2.0 && zh >= -2.0;
+          const double up = exp(zl), dn = exp(zh);
+#pragma unroll
+          for (int j = 0; j < 5; ++j) v[j] = 0.0;
+          visit([&](double ev, double w) {
+            const double g = exp((ev - m) * iTd);
+            const double f = cert_fermi(g);
+            v[0] += w * f;
+            v[1] += w * (f * (1.0 - f));
+            v[2] += w * cert_fermi(fac ? g * up : exp((ev - pl) * iTd));
+            v[3] += w * cert_fermi(fac ? g * dn : exp((ev - ph) * iTd));
+            v[4] += w < 0.0 ? NAN : w;  // N does not increase then: no bracket
+          });
+          cluster_sum_n<5, BT / 32>(cl, v, cslots, csm, parity);
+          parity ^= 1;
+        }
         const double margin = cert_margin(kpt, kpt, v[4]);
+        if (isnan(margin)) break;
         const double xs[3] = {m, m - d, m + d}, ns[3] = {v[0], v[2], v[3]};
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
-          if (ns[q] > a.target + margin) A = fmin(A, xs[q]);
-          if (ns[q] < a.target - margin) B = fmax(B, xs[q]);
+          if (ns[q] > a.target + margin && xs[q] < A) { A = xs[q]; nA = ns[q]; }
+          if (ns[q] < a.target - margin && xs[q] > B) { B = xs[q]; nB = ns[q]; }
         }
+        if (isinf(A)) nA = v[4];
         const double Z = v[1] * iTd;
         const double bl = fmax(B, lo), bh = fmin(A, hi);
         double r = m - (v[0] - a.target) / Z;
-        const bool newton = Z > 0.0 && isfinite(r) && r > bl && r < bh;
+        // a step that left more than half of the bracket is followed by its middle
+        const bool slow = bh - bl > 0.5 * width;
+        width = bh - bl;
+        const bool newton = Z > 0.0 && isfinite(r) && r > bl && r < bh && !slow;
         if (!newton) r = 0.5 * (bl + bh);
         const double floor_w = probe_noise(margin, Z, m);
-        if (A - B <= 4.0 * floor_w || ++t == kMuCertPasses) break;  // as narrow as the margin allows
-        d = probe_offset(fabs(r - m), newton, iTd, floor_w);
+        if (bracket_done(width, v[0], a.target, margin, floor_w) || ++t == passes) break;
+        // fewer than one level in 30 Td over the bracket: N is a staircase, which Newton's rule does not climb
+        if (!has_hint && (nA - nB) * Td * a.n < 0.03 * v[4] * width) break;
+        d = newton ? probe_offset(fabs(r - m), iTd, floor_w) : 0.0;  // no probes around a middle
         m = r;
-        // The probes are the rounded m - d and m + d, as they are recorded in A and B: what counts is the
-        // count at the recorded number (one half ulp of m beside it is more than the margin for a band that
-        // is narrow against its offset from zero).  exp((e - x) / Td) is the product of the exponential at m
-        // and the factor of the realised offset m - x where that is small.
-        const double pl = m - d, ph = m + d, zl = (m - pl) * iTd, zh = (m - ph) * iTd;
-        const bool fac = zl <= 2.0 && zh >= -2.0;
-        const double up = exp(zl), dn = exp(zh);
-#pragma unroll
-        for (int j = 0; j < 5; ++j) v[j] = 0.0;
-        visit([&](double ev, double w) {
-          const double g = exp((ev - m) * iTd);
-          const double f = cert_fermi(g);
-          v[0] += w * f;
-          v[1] += w * (f * (1.0 - f));
-          v[2] += w * cert_fermi(fac ? g * up : exp((ev - pl) * iTd));
-          v[3] += w * cert_fermi(fac ? g * dn : exp((ev - ph) * iTd));
-          v[4] += w;
-        });
-        cluster_sum_n<5, BT / 32>(cl, v, cslots, csm, parity);
-        parity ^= 1;
       }
     } else if (a.pre) {  // what the grid-wide passes left
       A = a.pre->A;
@@ -929,7 +951,7 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
       } else {
         visit([&](double ev, double w) {
           const double p = expit(div_by(mu - ev, Tj, rTj));
-          N += w * p;
+          N = fma(w, p, N);
           Z += div_by(w * (p * (1.0 - p)), Tj, rTj);
         });
         cluster_sum2(cl, N, Z, slots, wsm, parity);
@@ -1079,10 +1101,12 @@ int hf::find_mu_internal(void* stream, int dtype, int method, int nk1, int nk2, 
     a.cache = per <= kMuCacheMax ? (int)per : 0;
     a.kpt = (int)per;
   }
-  // the grid-wide passes, given a workspace: for the bisection without a hint (with one, the
-  // cluster kernel certifies its own bracket) and the warm-started Newton rule
-  if (ws && ws_bytes >= kMuWsBytes && a.n >= (method == 2 ? kGridMinNewton : kGridMin) &&
-      (method == 2 ? mu0 != nullptr : method == 0 && !mu0 && T + 1e-12 > 0.0)) {
+  // the grid-wide passes, given a workspace: for the bisection without a hint (with one, or below
+  // kGridMin, the cluster kernel certifies its own bracket) and the warm-started Newton rule
+  const bool bisect = method == 0 && !mu0 && T + 1e-12 > 0.0 && a.n >= kCertMin;
+  const bool grid = ws && ws_bytes >= kMuWsBytes;
+  if (grid && bisect && a.n < kGridMin) a.certify = 1;
+  if (grid && (method == 2 ? mu0 != nullptr && a.n >= kGridMinNewton : bisect && a.n >= kGridMin)) {
     MuState* st = static_cast<MuState*>(ws);
     double* part = reinterpret_cast<double*>(static_cast<char*>(ws) + 256);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -1090,7 +1114,6 @@ int hf::find_mu_internal(void* stream, int dtype, int method, int nk1, int nk2, 
                          : launch_passes<double>(s, a, csize, st, part, ws_ready);
     if (e) return e;
     a.pre = st;
-    a.cache = 0;  // mostly nothing is left to do: no shared-memory cache to set up (the same order without it)
   }
   const size_t cache_bytes = (size_t)a.cache * threads * sizeof(double2);
   cudaLaunchConfig_t cfg = {};

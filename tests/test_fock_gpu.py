@@ -838,3 +838,60 @@ def test_density_from_orbitals_has_the_bits_of_the_general_kernel(cuda, nb, dt, 
     Qp[:, :nb, :nb], pp[:, :nb] = Q, p
     t = lambda x: torch.as_tensor(x, device="cuda")
     assert torch.equal(L.density_from_Qp(t(Q), t(p)), L.density_from_Qp(t(Qp), t(pp))[:, :nb, :nb])
+
+
+def _mu_pair(eps, w, ne, T, method, mu0, maxiter=0):
+    """hf_find_mu and hf_find_mu_ws (a dirty workspace) on the same eigenvalues."""
+    from jax_hf_b200 import _lib
+    L, s = _lib.lib(), _lib.stream_ptr(eps.device)
+    n = _lib.C.c_size_t(0)
+    _lib.check(L.hf_mu_workspace_size(_lib.C.byref(n)))
+    ws = torch.full((n.value,), 255, dtype=torch.uint8, device="cuda")
+    out = torch.zeros(2, dtype=torch.float64, device="cuda")
+    m0 = None if mu0 is None else torch.tensor(mu0, dtype=torch.float64, device="cuda")
+    nk, nb = eps.numel() // eps.shape[-1], eps.shape[-1]
+    args = (s, _lib.HF_C128 if eps.dtype == torch.float64 else _lib.HF_C64, method, nk, 1, nb, eps.data_ptr(),
+            w.data_ptr(), ne, T, maxiter, _lib.ptr(m0))
+    _lib.check(L.hf_find_mu(*args, out.data_ptr()))
+    _lib.check(L.hf_find_mu_ws(*args, out[1:].data_ptr(), ws.data_ptr(), ws.numel()))
+    return out.tolist()
+
+
+@pytest.mark.parametrize("nk,nb", [(24577, 8), (160 * 161, 8), (97 * 97, 24), (163841, 1), (40001, 5)])
+@pytest.mark.parametrize("T", [0.2, 0.01, 1e-4])
+def test_grid_wide_newton_has_the_bits_of_the_cluster_kernel(cuda, nk, nb, T):
+    """Method 2 from the threshold of the passes on: the same sums in the same order, so the same bits,
+    for starts inside and outside the bracket and for iteration limits that stop in and behind the passes."""
+    rng = np.random.default_rng(nk)
+    eps = torch.as_tensor(rng.normal(size=(nk, nb)), device="cuda")
+    w = rng.uniform(0.5, 1.5, size=nk)
+    w = torch.as_tensor(w / w.sum(), device="cuda")
+    for ne, mu0, maxiter in ((0.4 * nb, 0.0, 25), (0.4 * nb, -0.2, 25), (0.7 * nb, 40.0, 25), (0.02 * nb, -900.0, 25),
+                             (0.4 * nb, 0.3, 1), (0.4 * nb, 0.3, 3), (0.4 * nb, 0.3, 6), (0.4 * nb, 0.3, 8)):
+        a, b = _mu_pair(eps, w, ne, T, 2, mu0, maxiter)
+        assert a == b, (ne, mu0, maxiter)
+
+
+@pytest.mark.parametrize("n", [16384, 40000, 131071, 131072, 196612])
+@pytest.mark.parametrize("kind,T", [("metal", 0.05), ("gap", 0.01), ("gap", 1e-5), ("staircase", 1e-5), ("flat band", 1e-3),
+                                    ("two bands", 0.01), ("narrow", 1e-3), ("single", 0.02)])
+def test_certified_bisection_has_the_bits_of_every_level(cuda, n, kind, T):
+    """Without a hint, on both sides of the thresholds: in and beside gaps, at temperatures below the spacing of the
+    levels, for flat and narrow bands, in single precision, with a short iteration limit."""
+    rng = np.random.default_rng(n)
+    e = rng.normal(size=(n // 4, 4))
+    if kind == "gap":
+        e = np.abs(e) + 1.0
+        e[:, :2] *= -1.0
+    elif kind == "flat band":
+        e[:, :2] *= 1e-3
+    elif kind == "two bands":
+        e = rng.uniform(-1, 1, size=e.shape) - np.where(np.arange(4) < 1, 30.0, 0.0)
+    elif kind == "narrow":
+        e = 50.0 + 0.01 * e
+    dt = torch.float32 if kind == "single" else torch.float64
+    eps = torch.as_tensor(e, device="cuda", dtype=dt)
+    w = torch.full((n // 4,), 4.0 / n, device="cuda", dtype=dt)
+    for ne, maxiter in ((2.0, 0), (0.7, 0), (1.0, 0), (3.37, 0), (0.001, 0), (2.5, 7)):
+        a, b = _mu_pair(eps, w, ne, T, 0, None, maxiter)
+        assert a == b, (ne, maxiter)
