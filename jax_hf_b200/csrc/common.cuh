@@ -28,7 +28,7 @@ int jdot_multi(void* stream, size_t nk, int nb, int n, const void* const* aX, co
                double* out, void* ws);
 int gram_row_slot(void* stream, int n, const int* slot, size_t stride, int nk, int nb, const void* R,
                   const double* w, double* b_out, void* ws);
-// eigh of herm(A) (mode 0) or herm(i A) (mode 1), 2 <= nb <= 16, ascending, by
+// eigh of herm(A) (mode 0) or herm(i A) (mode 1), nb <= 16, ascending, by
 // tridiagonalisation and QR (eigh.cu); eps and V in A's precision
 int eigh_tri(void* stream, int dtype, int nk, int nb, const void* A, void* eps, void* V, int mode);
 // P = herm(Q diag(p) Q^H), complex128, nb <= 8, lane-per-column kernel (solver_cg.cu)

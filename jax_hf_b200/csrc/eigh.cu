@@ -1,4 +1,4 @@
-// Batched eigh of small Hermitian matrices, 2 <= nb <= 16: tridiagonalisation and
+// Batched eigh of small Hermitian matrices, nb <= 16: for nb >= 2 tridiagonalisation and
 // implicit-shift QR (Golub & Van Loan, Matrix Computations, secs. 8.3.1-8.3.5).
 //
 // What bounds it: a matrix is one k-point (1 KiB at nb = 8), the bytes are nothing, and
@@ -364,6 +364,26 @@ __global__ void __launch_bounds__(TriShape<NB>::MAXM * TriShape<NB>::G, TriShape
   }
 }
 
+// nb = 1: the eigenvalue is the entry's real part (mode 1: of i A), the eigenvector 1.
+template <typename RT>
+__global__ void k_eigh_one(int nk, int mode, const cpx_t<RT>* A, RT* eps, cpx_t<RT>* V) {
+  pdl_begin();
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nk; k += gridDim.x * blockDim.x) {
+    const cpx_t<RT> a = A[k];
+    eps[k] = mode == 1 ? -a.y : a.x;
+    V[k] = mk<cpx_t<RT>>(1.0, 0.0);
+  }
+}
+
+template <typename RT>
+int launch_one(cudaStream_t s, int nk, int mode, const void* A, void* eps, void* V) {
+  const int blocks = (nk + 255) / 256;
+  launch_pdl(k_eigh_one<RT>, blocks < 148 * 8 ? blocks : 148 * 8, 256, 0, s, nk, mode,
+             static_cast<const cpx_t<RT>*>(A), static_cast<RT*>(eps), static_cast<cpx_t<RT>*>(V));
+  HF_LAUNCH_CHECK("k_eigh_one");
+  return HF_OK;
+}
+
 template <typename RT, int NB>
 int launch_tri(cudaStream_t s, int nk, int mode, const void* A, void* eps, void* V) {
   using S = TriShape<NB>;
@@ -382,9 +402,10 @@ int launch_tri(cudaStream_t s, int nk, int mode, const void* A, void* eps, void*
 }  // namespace
 
 // nb <= 16: beyond that a column no longer fits a lane's registers (perk.cu's warp-per-matrix
-// Jacobi takes nb = 17 .. 32, and nb = 1).
+// Jacobi takes nb = 17 .. 32).
 int eigh_tri(void* stream, int dtype, int nk, int nb, const void* A, void* eps, void* V, int mode) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (nb == 1) return dtype == HF_C128 ? launch_one<double>(s, nk, mode, A, eps, V) : launch_one<float>(s, nk, mode, A, eps, V);
   switch (nb) {
 #define HF_NB_CASE(N)                                                                \
   case N:                                                                            \
@@ -395,7 +416,7 @@ int eigh_tri(void* stream, int dtype, int nk, int nb, const void* A, void* eps, 
 #undef HF_NB_CASE
     default: break;
   }
-  return fail(HF_ERR_UNSUPPORTED, "eigh_tri: needs 2 <= nb <= 16");
+  return fail(HF_ERR_UNSUPPORTED, "eigh_tri: needs nb <= 16");
 }
 
 }  // namespace hf

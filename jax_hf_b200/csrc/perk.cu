@@ -1,8 +1,8 @@
 // Per-k small nb x nb kernels: one warp per matrix, matrices staged in shared
 // memory (double precision internally, storage precision at the boundary).
 //
-// Eigendecomposition for 2 <= nb <= 16: eigh.cu.  Otherwise cyclic Jacobi with complex Hermitian rotations in the
-// round-robin parallel ordering (Jacobi 1846; Golub & Van Loan, Matrix
+// Eigendecomposition for nb <= 16: eigh.cu.  Above, and for the SCF loops (hf_eigh_jacobi), cyclic
+// Jacobi with complex Hermitian rotations in the round-robin parallel ordering (Jacobi 1846; Golub & Van Loan, Matrix
 // Computations, sec. 8.5): each round applies nb/2 disjoint rotations at once
 // (lanes over rows/columns), sweeps repeat until no off-diagonal entry exceeds
 // 1e-17 ||A||_F (1e-8 in single precision) or 60 sweeps.  Eigenvalues are
@@ -369,7 +369,7 @@ static int eigh_common(void* stream, int dtype, int batch, int nb, int mode, con
   if (st) return st;
   if (batch == 0) return HF_OK;
   if (!A || !w || !V) return fail(HF_ERR_INVALID, "NULL argument");
-  if (nb >= 2 && nb <= 16) return hf::eigh_tri(stream, dtype, batch, nb, A, w, V, mode);
+  if (nb <= 16) return hf::eigh_tri(stream, dtype, batch, nb, A, w, V, mode);
   return eigh_warp(stream, dtype, batch, nb, mode, A, w, V);
 }
 

@@ -895,3 +895,17 @@ def test_certified_bisection_has_the_bits_of_every_level(cuda, n, kind, T):
     for ne, maxiter in ((2.0, 0), (0.7, 0), (1.0, 0), (3.37, 0), (0.001, 0), (2.5, 7)):
         a, b = _mu_pair(eps, w, ne, T, 0, None, maxiter)
         assert a == b, (ne, maxiter)
+
+
+@pytest.mark.parametrize("dt", [np.complex128, np.complex64])
+@pytest.mark.parametrize("nk", [1, 257, 400000])
+def test_eigh_of_one_band(cuda, dt, nk):
+    """nb = 1: the real part (of i A for the Cayley spectral form) and the eigenvector 1, exactly."""
+    from jax_hf_b200 import linalg as L
+    rng = np.random.default_rng(nk)
+    A = (rng.normal(size=(nk, 1, 1)) + 1j * rng.normal(size=(nk, 1, 1))).astype(dt)
+    t = torch.as_tensor(A, device="cuda")
+    w, V = L.eigh(t)
+    assert np.array_equal(w.cpu().numpy()[:, 0], A[:, 0, 0].real) and bool((V == 1).all())
+    V1, lam = L.cayley_spectral_setup(t)
+    assert np.array_equal(lam.cpu().numpy()[:, 0], -A[:, 0, 0].imag) and bool((V1 == 1).all())
