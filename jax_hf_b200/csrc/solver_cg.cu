@@ -107,69 +107,9 @@ __global__ void k_cg_init(CgArgs a, const double2* __restrict__ P0, const double
   }
 }
 
-// Rotation threshold of the init / finalize eigensolves, relative to |A|_F: at the
+// Rotation threshold of the lane-per-column eigensolve, relative to |A|_F: at the
 // double-precision rounding level, so converged rotations are not re-made from noise.
 constexpr double kEigTol = 1e-15;
-
-// eps, Q <- eigh(A) per k (A = F0 at init, or Ft = Q^H F Q at finalize with Q <- Q V)
-__global__ void k_cg_eig(CgArgs a, const double2* __restrict__ A, int rotate) {
-  extern __shared__ double2 sm[];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-  const int nb = a.nb, nb2 = nb * nb;
-  double2* m = sm + (size_t)w * (jacobi_smem_elems(nb) + 2 * nb2);
-  double2* v = m + nb2;
-  double2* scr = v + nb2;
-  double2* q = scr + nb + 40;
-  double2* t = q + nb2;
-  double* wv = reinterpret_cast<double*>(scr);
-  for (int k = blockIdx.x * wpb + w; k < a.nk; k += gridDim.x * wpb) {
-    const size_t base = (size_t)k * nb2;
-    if (rotate) {
-      for (int e = lane; e < nb2; e += 32) { q[e] = a.Q[base + e]; m[e] = A[base + e]; }
-      __syncwarp();
-      warp_qhaq(q, m, t, nb, lane);  // m <- Q^H F Q
-      __syncwarp();
-    } else {
-      for (int e = lane; e < nb2; e += 32) m[e] = A[base + e];
-      __syncwarp();
-    }
-    // hermitise (jnp.linalg.eigh symmetrises its input)
-    for (int e = lane; e < nb2; e += 32) {
-      const int i = e / nb, j = e - i * nb;
-      if (i < j) {
-        const double2 x = m[e], y = m[j * nb + i];
-        const double2 hxy = make_double2(0.5 * (x.x + y.x), 0.5 * (x.y - y.y));
-        m[e] = hxy;
-        m[j * nb + i] = conj(hxy);
-      } else if (i == j) {
-        m[e].y = 0.0;
-      }
-    }
-    __syncwarp();
-    warp_jacobi_eigh(m, v, scr + nb, nb, lane, kEigTol);
-    for (int e = lane; e < nb; e += 32) wv[e] = m[e * nb + e].x;
-    __syncwarp();
-    for (int i = lane; i < nb; i += 32) {
-      const double wi = wv[i];
-      int r = 0;
-      for (int j = 0; j < nb; ++j) r += (wv[j] < wi) || (wv[j] == wi && j < i);
-      a.eps[(size_t)k * nb + r] = wi;
-      for (int row = 0; row < nb; ++row) t[row * nb + r] = v[row * nb + i];
-    }
-    __syncwarp();
-    if (rotate) {  // Q <- Q V
-      for (int e = lane; e < nb2; e += 32) {
-        const int i = e / nb, j = e - i * nb;
-        double2 acc = make_double2(0.0, 0.0);
-        for (int n = 0; n < nb; ++n) acc = cadd(acc, cmul(q[i * nb + n], t[n * nb + j]));
-        a.Q[base + e] = acc;
-      }
-    } else {
-      for (int e = lane; e < nb2; e += 32) a.Q[base + e] = t[e];
-    }
-    __syncwarp();
-  }
-}
 
 // ---------------------------------------------- density: p and P = herm(Q p Q^H)
 __global__ void k_cg_density(CgArgs a, int force) {
@@ -746,7 +686,7 @@ struct CgRun {
   int nblk;
 };
 
-static size_t smem_eig(int nb) { return (jacobi_smem_elems(nb) + 2 * (size_t)nb * nb) * sizeof(double2) * kSolverWarps; }
+static size_t smem_dir(int nb) { return (jacobi_smem_elems(nb) + 2 * (size_t)nb * nb) * sizeof(double2) * kSolverWarps; }
 
 static int set_smem(const void* fn, size_t) { return allow_max_dynamic_smem(fn); }
 
@@ -845,14 +785,10 @@ static int cg_density(CgRun& r, cudaStream_t s, int force) {
 
 // eps, Q <- eigh(A): of F0 at init, of the final F at finalize.  The reference decomposes
 // Q^H F Q there and rotates Q (solver.py:622-626), the same eigenvectors up to a phase each;
-// for nb <= 16 decomposing F itself is cheaper than forming Q^H F Q and Q V (144 x 144,
-// nb = 8: 75 us against 195 us for a warm-started Jacobi).
-static int cg_eig(CgRun& r, cudaStream_t s, const double2* A, int rotate) {
-  const int nb = r.a.nb;
-  if (nb <= 16) return hf_eigh(s, HF_C128, r.a.nk, nb, A, r.a.eps, r.a.Q);
-  k_cg_eig<<<r.nblk, 32 * kSolverWarps, smem_eig(nb), s>>>(r.a, A, rotate);
-  HF_LAUNCH_CHECK("k_cg_eig");
-  return HF_OK;
+// decomposing F itself is cheaper than forming Q^H F Q and Q V (144 x 144, nb = 8: 75 us
+// against 195 us for a warm-started Jacobi).
+static int cg_eig(CgRun& r, cudaStream_t s, const double2* A) {
+  return hf_eigh(s, HF_C128, r.a.nk, r.a.nb, A, r.a.eps, r.a.Q);
 }
 
 template <int NB>
@@ -917,7 +853,7 @@ static int cg_iteration_warp(CgRun& r, cudaStream_t s, const hf_cg_config& cf, b
   HF_LAUNCH_CHECK("k_cg_grad1");
   k_cg_grad2<<<r.nblk, 256, 0, s>>>(r.a);
   HF_LAUNCH_CHECK("k_cg_grad2");
-  k_cg_dir<<<r.nblk, blk, smem_eig(nb), s>>>(r.a);
+  k_cg_dir<<<r.nblk, blk, smem_dir(nb), s>>>(r.a);
   HF_LAUNCH_CHECK("k_cg_dir");
   const size_t sm_tr = (2 * (size_t)nb2 + nb) * 16 * kSolverWarps;
   const int bt = cf.bt_max;
@@ -1068,8 +1004,7 @@ int CgSolver::setup(const hf_cg_problem* pb_, const hf_cg_config* cf_, void* Q, 
   chunk = cf->chunk > 0 ? cf->chunk : 4;
   graphs = cf->fock_cb == nullptr && cf->project_cb == nullptr && s != nullptr;
   const int nb = pb->nb, nb2 = nb * nb;
-  if ((st = set_smem((const void*)k_cg_eig, smem_eig(nb)))) return st;
-  if ((st = set_smem((const void*)k_cg_dir, smem_eig(nb)))) return st;
+  if ((st = set_smem((const void*)k_cg_dir, smem_dir(nb)))) return st;
   if ((st = set_smem((const void*)k_cg_update, (4 * (size_t)nb2 + nb) * 16 * kSolverWarps))) return st;
   if ((st = set_smem((const void*)k_cg_grad1, 3 * (size_t)nb2 * 16 * kSolverWarps))) return st;
   return HF_OK;
@@ -1094,7 +1029,7 @@ int CgSolver::init_ops(const void* P0) {
                                    pb->weight_sum);
   HF_LAUNCH_CHECK("k_cg_init");
   if ((st = cg_fock(r, s, false, nullptr))) return st;
-  if ((st = cg_eig(r, s, a.F, 0))) return st;
+  if ((st = cg_eig(r, s, a.F))) return st;
   return cg_mu(r, s, cf->mu_maxiter, nullptr);
 }
 
@@ -1174,7 +1109,7 @@ int CgSolver::finalize_ops(bool device_switch) {
   if ((st = cg_density(r, s, 1))) return st;
   if ((st = cg_project(r, s))) return st;
   if ((st = cg_fock(r, s, false, nullptr))) return st;
-  if ((st = cg_eig(r, s, a.F, 1))) return st;  // reads the current Q, writes the caller's buffer
+  if ((st = cg_eig(r, s, a.F))) return st;  // into the caller's buffer
   k_cg_qsel_reset<<<1, 1, 0, s>>>(a);
   HF_LAUNCH_CHECK("k_cg_qsel_reset");
   if ((st = cg_mu(r, s, cf->mu_maxiter, nullptr))) return st;

@@ -909,3 +909,14 @@ def test_eigh_of_one_band(cuda, dt, nk):
     assert np.array_equal(w.cpu().numpy()[:, 0], A[:, 0, 0].real) and bool((V == 1).all())
     V1, lam = L.cayley_spectral_setup(t)
     assert np.array_equal(lam.cpu().numpy()[:, 0], -A[:, 0, 0].imag) and bool((V1 == 1).all())
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), -float("inf")])
+def test_certified_bisection_with_a_non_finite_eigenvalue(cuda, bad):
+    """A non-finite eigenvalue below the threshold of the grid-wide passes: no bracket, the bits of every level."""
+    rng = np.random.default_rng(6)
+    e = rng.normal(size=(9000, 3))
+    e[77, 1] = bad
+    w = torch.full((9000,), 1.0 / 9000, dtype=torch.float64, device="cuda")
+    a, b = _mu_pair(torch.as_tensor(e, device="cuda"), w, 1.1, 0.05, 0, None)
+    assert a == b or (a != a and b != b)
