@@ -178,10 +178,11 @@ __device__ __forceinline__ KSum block_reduce(KSum v, double* sm) {
   return r;
 }
 
-// Block-wide compensated sums of NS quantities (block_reduce on each, the same trees), side by side: a compensated merge is a chain of ten dependent additions, so one
-// quantity after the other left the block waiting 2 NS times.  The warps' results go
-// through shared memory once, and warp w finishes quantities w, w + nw, ...  Returns the sums of
-// quantity q in lane 0 of warp q % nw; call with every thread.
+// Block-wide compensated sums of NS quantities (block_reduce on each, the same trees), side by
+// side: a compensated merge is a chain of ten dependent additions, so one quantity after the
+// other left the block waiting 2 NS times.  The warps' results go through shared memory once,
+// and warp w finishes quantities w, w + nw, ...  sink(q, sums of quantity q) runs in lane 0 of
+// warp q % nw; call with every thread of a block of at most 256.
 template <int NS, class Sink>
 __device__ __forceinline__ void block_reduce_all(KSum (&acc)[NS], Sink&& sink) {
   constexpr int MW = 8;  // warps per block at most (256 threads)
@@ -226,9 +227,9 @@ __device__ __forceinline__ void block_reduce_all(KSum (&acc)[NS], Sink&& sink) {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
-// First statement of every kernel that launch_pdl launches, ahead of any early return (and no parameter of
-// such a kernel is __restrict__: its predecessor may still be at that memory): a
-// grid that ended without waiting would let its successor start before its predecessor ended.
+// First statement of every kernel that launch_pdl launches, ahead of any early return: a grid that
+// ended without waiting would let its successor start before its predecessor ended.  No parameter
+// of such a kernel is __restrict__, since its predecessor may still be at that memory.
 __device__ __forceinline__ void pdl_begin() {
   pdl_wait();
   pdl_launch_dependents();

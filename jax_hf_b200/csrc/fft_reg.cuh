@@ -5,7 +5,8 @@
 // unrolling).  Composite N = A*B is split Cooley-Tukey style: A-point DFTs over
 // x[n2 + B n1], the twiddle W_N^{n2 k1}, B-point DFTs, output X[k1 + A k2].
 // Radices 2/3/4/5/8 are the butterflies of fft_engine.cuh; other primes use a
-// direct DFT with the products of conjugate terms shared.  Inner twiddles are compile-time constants (CtTwiddle).
+// direct DFT with the products of conjugate terms shared.  Inner twiddles are compile-time
+// constants (CtTwiddle).
 //
 // Line FFT of length N = N1*N2 over TPL threads per line (TPL | N1, TPL | N2):
 //   pattern A: thread t holds x[n2 + N2 n1] for n2 = t + TPL i (i < N2/TPL), all n1

@@ -715,8 +715,9 @@ static int launch_fock(FockParams& p, cudaStream_t stream, bool need_consts, con
     // thread keep the register passes, whose DFTs have no run-time switch: 72 and 144 sides lose 3 to 25 %, 16 to
     // 36 up to 40 %; and so does the row plan (96 x 96 x 4 14.4 us against 16.8).
     const bool two = !(p.flags & HF_FOCK_NO_TWO_FACTOR);
-    // A single channel keeps them too (192 x 192 x 1 21.3 us against 22.3).  Packing a band-resolved V at
-    // 96 x 96 x 8 in c64 is the one build seen to lose (19.6 -> 21.9; 52.8 -> 44.4 at 192).
+    // A single channel keeps them too (192 x 192 x 1 21.3 us against 22.3).  c64 at 96 x 192 is the one shape
+    // seen to lose (packed nb 6 22.5 -> 24.3, nb 8 25.3 -> 26.2; at 192 x 192 x 8 53.9 -> 43.9), which the
+    // autotuner settles.
     const bool deep = two && !p.rows_plan && !(p.flags & HF_FOCK_TILE_PLAN) && deep_tiles(p.nk1, p.nk2, p.nb);
     if (!deep) {
       st = fast_fock<ST, FT>(p, stream, &handled);

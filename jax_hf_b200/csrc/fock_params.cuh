@@ -112,7 +112,7 @@ inline int line_factors(int n) {
 // Launches the fast passes when both mesh lengths have a fast shape.
 template <typename ST, typename FT>
 int fast_fock(FockParams& p, cudaStream_t stream, bool* handled);
-// Launches the two-factor passes where both sides have two factors of at most 16.
+// Launches the two-factor and dense passes where both sides have line_factors.
 template <typename ST, typename FT>
 int two_fock(FockParams& p, cudaStream_t stream, bool* handled);
 // Launches the bulk-copy pipelined passes (fock_pipe.cuh) where they apply.

@@ -9,7 +9,10 @@
 // so three kernels serve all sides.  16 slot lanes x T line parts, T = max(N1, N2):
 // thread t takes column n2 = t of the first step and row k1 = t of the second; where the
 // factors differ the surplus threads sit one step out.  No thread holds data across a
-// phase, so a CTA of up to 256 threads stays within 128 registers and two CTAs fill an SM.
+// phase, so that two CTAs of up to 256 threads fill an SM at 128 registers.  FP32 transforms and the
+// forward pass fit them; of the FP64 ones the inverse row pass spills (2.0 KB of stores and
+// 2.5 KB of loads over its sixteen cases: the epilogue holds h across the IDFT) and the column pass
+// 92 and 372 B.
 //
 // What bounds it: the passes move the same bytes as the register engine's (each pass reads
 // and writes the spectrum once) and their DFTs are a few hundred FP64 operations per

@@ -2,8 +2,8 @@
 // memory (double precision internally, storage precision at the boundary).
 //
 // Eigendecomposition for nb <= 16: eigh.cu.  Above, and for the SCF loops (hf_eigh_jacobi), cyclic
-// Jacobi with complex Hermitian rotations in the round-robin parallel ordering (Jacobi 1846; Golub & Van Loan, Matrix
-// Computations, sec. 8.5): each round applies nb/2 disjoint rotations at once
+// Jacobi with complex Hermitian rotations in the round-robin parallel ordering (Jacobi 1846;
+// Golub & Van Loan, Matrix Computations, sec. 8.5): each round applies nb/2 disjoint rotations at once
 // (lanes over rows/columns), sweeps repeat until no off-diagonal entry exceeds
 // 1e-17 ||A||_F (1e-8 in single precision) or 60 sweeps.  Eigenvalues are
 // returned ascending, eigenvectors as columns (A = V diag(w) V^H), like LAPACK

@@ -1,4 +1,4 @@
-"""Per-k small-matrix operations on the GPU (one warp per k-point).
+"""Per-k small-matrix operations on the GPU.
 
 Wrappers of the C ABI for the nb x nb kernels used by the solvers
 (solver.py:42-49, 108-197; linalg.eigh).  Leading axes are flattened into a
