@@ -73,7 +73,9 @@ def _consts(rho, kernel):
 
 def _cotangent(g):
     """A complex cotangent as its numbers in memory: autograd may hand over a lazily conjugated view."""
-    return None if g is None else g.to(torch.complex128).resolve_conj().resolve_neg().contiguous()
+    if g is None or (g.dtype is torch.complex128 and g.is_contiguous() and not (g.is_conj() or g.is_neg())):
+        return g
+    return g.to(torch.complex128).resolve_conj().resolve_neg().contiguous()
 
 
 def _fock_vjp(kernel, P, gS, gF, gH, want_h):
@@ -148,6 +150,8 @@ def _energy_vjp_H(gE, P, w2d):
 
 def _dev_scalar(g, dev):
     """A cotangent as a contiguous float64 device scalar (no host read)."""
+    if g.dtype is torch.float64 and g.device == dev and not g.is_neg():
+        return g
     return g.to(dev, torch.float64).resolve_neg().contiguous()
 
 
@@ -268,7 +272,8 @@ def objective(P, p, kernel, h=None):
     if kernel.dtype != torch.complex128:
         raise ValueError("the hand-written adjoint runs in complex128; build the kernel in complex128")
     # the adjoints read 16-byte elements; autograd carries the conversion back to the caller's type
-    P, h = (t.to(torch.complex128).contiguous() for t in (P, h))
+    P, h = (t if t.dtype is torch.complex128 and t.is_contiguous() else t.to(torch.complex128).contiguous()
+            for t in (P, h))
     return _ObjectiveFn.apply(P, p.to(torch.float64).contiguous(), h, kernel)
 
 
