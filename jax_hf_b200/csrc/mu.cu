@@ -773,7 +773,8 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
     int it = 0;
     bool fixed = false;
     double A = INFINITY, B = -INFINITY;
-    if (has_hint || a.certify) {
+    constexpr bool COLD = BT > 256;  // a.certify is for large spectra only
+    if (has_hint || (COLD && a.certify)) {
       // Certified bracket from the hint, or from the middle of the spectrum.  For weights >= 0
       // N(x) = sum w / (1 + exp((e - x) / Td)) is increasing in x; an evaluation N~(x) differs from it by at most E = (kpt + 24) u W
       // (kpt terms summed per thread, a reduction tree of depth <= 14, about 6 u per term, and u W for the
@@ -791,12 +792,12 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
       // With a hint the first evaluation came with the extremes, at the hint itself: a call on 2304
       // eigenvalues (T = 0.1) takes 16.0 us with a hint 1e-7 off the root and 17.8 with one 1e-2 off,
       // 49 without a hint.
-      const int kpt = (a.n + gs - 1) / gs, passes = has_hint ? kMuCertPasses : kMuCertPassesCold;
-      double m = has_hint ? hint : 0.5 * (mn + mx), d = 0.0, width = INFINITY;
-      double nA = 0.0, nB = 0.0;  // the counts at A and B
+      const int kpt = (a.n + gs - 1) / gs, passes = !COLD || has_hint ? kMuCertPasses : kMuCertPassesCold;
+      double m = !COLD || has_hint ? hint : 0.5 * (mn + mx), d = 0.0, width = INFINITY;
+      double nA = INFINITY, nB = 0.0;  // the counts at A and B (without a hint)
       double v[5] = {hv[2], hv[3], hv[2], hv[2], hv[4]};  // N(m), N'(m) Td, N(m - d), N(m + d), W
       for (int t = 0;;) {
-        if (t > 0 || !has_hint) {
+        if (t > 0 || (COLD && !has_hint)) {
           // The probes are the rounded m - d and m + d, as they are recorded in A and B: what counts is the
           // count at the recorded number (one half ulp of m beside it is more than the margin for a band
           // that is narrow against its offset from zero).  exp((e - x) / Td) is the product of the
@@ -823,10 +824,9 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
         const double xs[3] = {m, m - d, m + d}, ns[3] = {v[0], v[2], v[3]};
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
-          if (ns[q] > a.target + margin && xs[q] < A) { A = xs[q]; nA = ns[q]; }
-          if (ns[q] < a.target - margin && xs[q] > B) { B = xs[q]; nB = ns[q]; }
+          if (ns[q] > a.target + margin) A = fmin(A, xs[q]);
+          if (ns[q] < a.target - margin) B = fmax(B, xs[q]);
         }
-        if (isinf(A)) nA = v[4];
         const double Z = v[1] * iTd;
         const double bl = fmax(B, lo), bh = fmin(A, hi);
         double r = m - (v[0] - a.target) / Z;
@@ -838,7 +838,11 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
         const double floor_w = probe_noise(margin, Z, m);
         if (bracket_done(width, v[0], a.target, margin, floor_w) || ++t == passes) break;
         // fewer than one level in 30 Td over the bracket: N is a staircase, which Newton's rule does not climb
-        if (!has_hint && (nA - nB) * Td * a.n < 0.03 * v[4] * width) break;
+        if (COLD && !has_hint) {
+          if (v[0] > a.target) nA = fmin(nA, v[0]);
+          else nB = fmax(nB, v[0]);
+          if ((fmin(nA, v[4]) - nB) * Td * a.n < 0.03 * v[4] * width) break;
+        }
         d = newton ? probe_offset(fabs(r - m), iTd, floor_w) : 0.0;  // no probes around a middle
         m = r;
       }
