@@ -796,28 +796,32 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
       double m = !COLD || has_hint ? hint : 0.5 * (mn + mx), d = 0.0, width = INFINITY;
       double nA = INFINITY, nB = 0.0;  // the counts at A and B (without a hint)
       double v[5] = {hv[2], hv[3], hv[2], hv[2], hv[4]};  // N(m), N'(m) Td, N(m - d), N(m + d), W
-      for (int t = 0;;) {
-        if (t > 0 || (COLD && !has_hint)) {
-          // The probes are the rounded m - d and m + d, as they are recorded in A and B: what counts is the
-          // count at the recorded number (one half ulp of m beside it is more than the margin for a band
-          // that is narrow against its offset from zero).  exp((e - x) / Td) is the product of the
-          // exponential at m and the factor of the realised offset m - x where that is small.
-          const double pl = m - d, ph = m + d, zl = (m - pl) * iTd, zh = (m - ph) * iTd;
-          const bool fac = zl <= 2.0 && zh >= -2.0;
-          const double up = exp(zl), dn = exp(zh);
+      auto evaluate = [&] {
+        // The probes are the rounded m - d and m + d, as they are recorded in A and B: what counts is the
+        // count at the recorded number (one half ulp of m beside it is more than the margin for a band
+        // that is narrow against its offset from zero).  exp((e - x) / Td) is the product of the
+        // exponential at m and the factor of the realised offset m - x where that is small.
+        const double pl = m - d, ph = m + d, zl = (m - pl) * iTd, zh = (m - ph) * iTd;
+        const bool fac = zl <= 2.0 && zh >= -2.0;
+        const double up = exp(zl), dn = exp(zh);
 #pragma unroll
-          for (int j = 0; j < 5; ++j) v[j] = 0.0;
-          visit([&](double ev, double w) {
-            const double g = exp((ev - m) * iTd);
-            const double f = cert_fermi(g);
-            v[0] += w * f;
-            v[1] += w * (f * (1.0 - f));
-            v[2] += w * cert_fermi(fac ? g * up : exp((ev - pl) * iTd));
-            v[3] += w * cert_fermi(fac ? g * dn : exp((ev - ph) * iTd));
-            v[4] += w < 0.0 ? NAN : w;  // N does not increase then: no bracket
-          });
-          cluster_sum_n<5, BT / 32>(cl, v, cslots, csm, parity);
-          parity ^= 1;
+        for (int j = 0; j < 5; ++j) v[j] = 0.0;
+        visit([&](double ev, double w) {
+          const double g = exp((ev - m) * iTd);
+          const double f = cert_fermi(g);
+          v[0] += w * f;
+          v[1] += w * (f * (1.0 - f));
+          v[2] += w * cert_fermi(fac ? g * up : exp((ev - pl) * iTd));
+          v[3] += w * cert_fermi(fac ? g * dn : exp((ev - ph) * iTd));
+          v[4] += w < 0.0 ? NAN : w;  // N does not increase then: no bracket
+        });
+        cluster_sum_n<5, BT / 32>(cl, v, cslots, csm, parity);
+        parity ^= 1;
+      };
+      for (int t = 0;;) {
+        // one copy of the evaluation in each kernel: a loop's calls find the instruction cache cold
+        if constexpr (COLD) {
+          if (t > 0 || !has_hint) evaluate();
         }
         const double margin = cert_margin(kpt, kpt, v[4]);
         if (isnan(margin)) break;
@@ -845,6 +849,7 @@ __global__ void __launch_bounds__(BT) k_find_mu(const MuArgs a) {
         }
         d = newton ? probe_offset(fabs(r - m), iTd, floor_w) : 0.0;  // no probes around a middle
         m = r;
+        if constexpr (!COLD) evaluate();
       }
     } else if (a.pre) {  // what the grid-wide passes left
       A = a.pre->A;
